@@ -1537,14 +1537,16 @@ __global__ void k_tier(u32 n, u32 K, const u64 *__restrict__ work, const u64 *__
 }
 
 // ------------------------------------------------------------------ ranking
-// Mover flags, and every node's rank reset (k_set_rank then ranks the movers) and cascaded gain
-// zeroed.
-__global__ void k_move_flags(u32 n, const u32 *__restrict__ target, u32 *__restrict__ flag, u32 *__restrict__ rank,
-                             unsigned long long *__restrict__ g2) {
+// A node's state in the cascade: {rank, partition}, rank NONE unless it moves. One 8-byte gather
+// tells a hyperedge's pin apart from an earlier mover.
+// Mover flags, and every node's state without a rank (k_set_rank then ranks the movers) and
+// cascaded gain zeroed.
+__global__ void k_move_flags(u32 n, const u32 *__restrict__ target, const u32 *__restrict__ part,
+                             u32 *__restrict__ flag, uint2 *__restrict__ state, unsigned long long *__restrict__ g2) {
     u32 v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v < n) {
         flag[v] = target[v] != NONE ? 1u : 0u;
-        rank[v] = NONE;
+        state[v] = make_uint2(NONE, part[v]);
         g2[v] = 0;
     }
 }
@@ -1556,12 +1558,12 @@ __global__ void k_move_keys(const u32 *__restrict__ mv, const u32 *__restrict__ 
     hi[i] = (u32)(k >> 32);
     lo[i] = (u32)k;
 }
-// rank[mv[i]] = i; also the size-event count 2M into *twice.
-__global__ void k_set_rank(const u32 *__restrict__ mv, const u32 *__restrict__ dM, u32 *__restrict__ rank,
+// The rank of mover mv[i] is i; also the size-event count 2M into *twice.
+__global__ void k_set_rank(const u32 *__restrict__ mv, const u32 *__restrict__ dM, uint2 *__restrict__ state,
                            u32 *__restrict__ twice) {
     u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *twice = 2 * *dM;
-    if (i < *dM) rank[mv[i]] = i;
+    if (i < *dM) state[mv[i]].x = i;
 }
 
 // k-way pair ranking (include/axc.h AXC_PAIR_RANK_MAX_K): the moves, in (gain desc, id asc)
@@ -1624,7 +1626,8 @@ struct CascadeArgs {
     u32 e;
     int encourage;
     const u64 *off;
-    const u32 *pins, *nsrc, *wfx, *lam, *cpart, *ccnt, *cdcnt, *rank, *part, *target;
+    const u32 *pins, *nsrc, *wfx, *lam, *cpart, *ccnt, *cdcnt, *part, *target;
+    const uint2 *state;  // [n] {rank, partition}
     unsigned long long *g2;
     // inbound-set transitions (INCC): a (partition, hyperedge) destination count going 0 -> 1 or
     // 1 -> 0 at a move's rank; appended as (partition, rank, +-1)
@@ -1672,6 +1675,19 @@ __device__ __forceinline__ void emit_at(const CascadeArgs &A, u32 s, u32 p, u32 
 }
 __device__ __forceinline__ void emit_transition(const CascadeArgs &A, u32 p, u32 r, int32_t d) {
     emit_at(A, atomicAdd(A.dT, 1u), p, r, d);
+}
+// The transitions of one mover (leave: p loses its last destination pin, join: q gains its first),
+// with one reservation for the lanes that call it together.
+__device__ __forceinline__ void emit_pair(const CascadeArgs &A, bool leave, u32 p, bool join, u32 q, u32 r) {
+    const u32 am = __activemask(), lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const u32 bp = __ballot_sync(am, leave), bq = __ballot_sync(am, join);
+    const u32 tot = __popc(bp) + __popc(bq), lead = __ffs(am) - 1;
+    if (!tot) return;
+    u32 s0 = 0;
+    if (!A.tdense && lane == lead) s0 = atomicAdd(A.dT, tot);
+    s0 = __shfl_sync(am, s0, lead);
+    if (leave) emit_at(A, s0 + __popc(bp & lt), p, r, -1);
+    if (join) emit_at(A, s0 + __popc(bp) + __popc(bq & lt), q, r, +1);
 }
 
 // Table slots of every mover's source and target partition, sl[i] = slot(p) | slot(q) << 16,
@@ -1830,15 +1846,227 @@ __device__ void cascade_sweep_warp(const CascadeArgs &A, u32 h, const u64 *mv, c
     }
 }
 
-// The hyperedges that hold a mover: every incidence of every mover flags its hyperedge (flag[]
-// zeroed before), then the flags are compacted into the cascade's list. One warp per mover.
+// The cascade over hyperedges of at most CM_LEN pins needs no table and no sort of a hyperedge's
+// movers: a pin whose rank is below a mover's counts in its target partition, every other pin in its
+// own, which gives the counts the mover finds when all better-ranked moves are applied. Two
+// kernels, of which one acts, by the round's mover count (cascade_dense):
+//  - few movers, k_cascade_movers: G lanes take one mover, a lane one incidence at a time, and
+//    re-read the hyperedge's pins. Its cost follows the movers alone, and a mover's gain is one
+//    sum over its lanes.
+//  - many movers, k_cascade_dense: a warp stages the pins of consecutive hyperedges in shared
+//    memory, each read once, and every mover among them runs over its hyperedge there.
+constexpr u32 CM_LEN = 128;
+constexpr u32 CM_THREADS = 256;
+constexpr u32 CD_STAGE = 512;        // pins a warp of the dense kernel stages at a time
+constexpr u32 CD_MAX_K = 32768;      // partitions its packed states hold
+static_assert(CM_LEN <= CD_STAGE, "every short hyperedge fits the stage");
+
+struct MoverArgs {
+    const u32 *mv, *dM;
+    const u64 *toff;
+    const u32 *touch, *nin;
+    int longs;  // the level holds longer hyperedges, whose kernels add to g2 as well
+    int dense;  // k_cascade_dense is launched too
+    u32 n, copies;     // nodes; counters in dM (one per copy with slots)
+    u64 len16;         // 16 times the mean length of the short hyperedge at a short incidence
+    u32 per_warp;      // hyperedges a warp of the dense kernel looks at
+};
+
+// Whether the dense kernel acts: the movers' incidences hold at least as many pins as the level.
+__device__ __forceinline__ bool cascade_dense(const MoverArgs &V) {
+    if (!V.dense) return false;
+    u64 M = 0;
+    for (u32 t = 0; t < V.copies; ++t) M += V.dM[t];
+    return M * V.len16 >= 16ull * V.n;
+}
+
+// One incidence of the mover of rank r (node u, moving p -> q) in hyperedge h: its part of the
+// cascaded gain, and its inbound transitions when u is one of h's destinations.
+template <bool TRACK>
+__device__ __forceinline__ i64 cascade_incidence(const CascadeArgs &A, u32 h, u32 u, u32 r, u32 p, u32 q, bool dst) {
+    const u64 a = A.off[h], len64 = A.off[h + 1] - a;
+    if (len64 > CM_LEN) return 0;
+    const u32 len = (u32)len64, w = A.wfx[h], ns = TRACK ? A.nsrc[h] : 0u;
+    u32 cp = 0, cq = 0, dp = 0, dq = 0;
+    constexpr u32 U = 4;  // pins whose loads are in flight together
+    for (u32 i0 = 0; i0 < len; i0 += U) {
+        u32 v[U];
+        uint2 st[U];
+#pragma unroll
+        for (u32 x = 0; x < U; ++x) v[x] = i0 + x < len ? A.pins[a + i0 + x] : u;
+#pragma unroll
+        for (u32 x = 0; x < U; ++x) st[x] = A.state[v[x]];
+#pragma unroll
+        for (u32 x = 0; x < U; ++x)
+            if (i0 + x < len) {
+                const u32 s = st[x].x < r ? A.target[v[x]] : st[x].y;
+                cp += s == p;
+                cq += s == q;
+                if (TRACK && i0 + x >= ns) {
+                    dp += s == p;
+                    dq += s == q;
+                }
+            }
+    }
+    if (TRACK) emit_pair(A, dst && dp == 1, p, dst && dq == 0, q, r);
+    return leave_gain(A.encourage, w, cp) - (cq == 0 ? (i64)w : 0);
+}
+
+// Movers of at most CM_HEAVY * G incidences (a lane's share stays bounded); the others take a block
+// each (k_cascade_movers_heavy).
+constexpr u32 CM_HEAVY = 128;
+template <u32 G, bool TRACK>
+__global__ void __launch_bounds__(CM_THREADS) k_cascade_movers(CascadeArgs A, MoverArgs V) {
+    const u32 lane = threadIdx.x & 31u, gl = lane & (G - 1);
+    const u32 gmask = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
+    if (cascade_dense(V)) return;
+    const u32 M = *V.dM, ng = gridDim.x * (CM_THREADS / G);
+    for (u32 r = blockIdx.x * (CM_THREADS / G) + threadIdx.x / G; r < M; r += ng) {
+        const u32 u = V.mv[r];
+        const u64 t0 = V.toff[u], deg = V.toff[u + 1] - t0;
+        if (deg > CM_HEAVY * G) continue;
+        const u32 p = A.part[u], q = A.target[u], nin_u = TRACK ? V.nin[u] : 0u;
+        i64 sum = 0;
+        for (u32 j = gl; j < (u32)deg; j += G)
+            sum += cascade_incidence<TRACK>(A, V.touch[t0 + j], u, r, p, q, TRACK && j < nin_u);
+        __syncwarp(gmask);
+#pragma unroll
+        for (u32 o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(gmask, sum, o);
+        if (gl == 0) {
+            if (V.longs) atomicAdd(&A.g2[u], (unsigned long long)sum);
+            else A.g2[u] = (unsigned long long)sum;
+        }
+    }
+}
+template <bool TRACK>
+__global__ void __launch_bounds__(CM_THREADS) k_cascade_movers_heavy(CascadeArgs A, MoverArgs V, u32 min_deg) {
+    if (cascade_dense(V)) return;
+    const u32 M = *V.dM;
+    for (u32 r = blockIdx.x; r < M; r += gridDim.x) {
+        const u32 u = V.mv[r];
+        const u64 t0 = V.toff[u], deg = V.toff[u + 1] - t0;
+        if (deg <= min_deg) continue;
+        const u32 p = A.part[u], q = A.target[u], nin_u = TRACK ? V.nin[u] : 0u;
+        i64 sum = 0;
+        for (u64 j = threadIdx.x; j < deg; j += CM_THREADS)
+            sum += cascade_incidence<TRACK>(A, V.touch[t0 + j], u, r, p, q, TRACK && j < nin_u);
+        sum = warp_sum(sum);
+        if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(&A.g2[u], (unsigned long long)sum);  // g2 starts at zero
+    }
+}
+
+// A staged pin: its rank, and partition | target << 15 | destination << 31 (target 0 without a
+// rank); its node beside it.
+template <bool TRACK>
+__global__ void __launch_bounds__(CM_THREADS) k_cascade_dense(CascadeArgs A, MoverArgs V) {
+    constexpr u32 NW = CM_THREADS / 32;
+    __shared__ uint2 ss[NW][CD_STAGE];
+    __shared__ u32 sn[NW][CD_STAGE];
+    if (!cascade_dense(V)) return;
+    const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    uint2 *st = ss[w];
+    u32 *nd = sn[w];
+    const u32 step = gridDim.x * NW * V.per_warp;
+    for (u32 h0 = (blockIdx.x * NW + w) * V.per_warp; h0 < A.e; h0 += step) {
+        const u32 h = h0 + lane;
+        const bool mine = lane < V.per_warp && h < A.e;
+        const u64 a = mine ? A.off[h] : 0, len64 = mine ? A.off[h + 1] - a : 0;
+        const u32 len = len64 <= CM_LEN ? (u32)len64 : 0u;  // longer ones are not taken here
+        const u32 wh = mine ? A.wfx[h] : 0u, ns = TRACK && mine ? A.nsrc[h] : 0u;
+        u32 x = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if ((int)lane >= o) x += y;
+        }
+        const u32 excl = x - len;
+        // as many of the hyperedges as the stage holds at a time
+        for (u32 lo = 0; lo < 32;) {
+            const u32 b0 = __shfl_sync(0xFFFFFFFFu, excl, lo);
+            const u32 hi = lo + __popc(__ballot_sync(0xFFFFFFFFu, lane >= lo && x - b0 <= CD_STAGE));
+            const u32 T = __shfl_sync(0xFFFFFFFFu, x, hi - 1) - b0;
+            bool movers = false;
+            for (u32 f0 = 0; f0 < T; f0 += 32) {
+                const u32 f = f0 + lane;
+                u32 ol = lo, oh = hi - 1;  // owner: the last hyperedge starting at or before f
+                for (int it = 0; it < 5; ++it) {
+                    const u32 mid = (ol + oh + 1) >> 1;
+                    const u32 em = __shfl_sync(0xFFFFFFFFu, excl, mid & 31);
+                    if (ol < oh) { if (em - b0 <= f) ol = mid; else oh = mid - 1; }
+                }
+                const u32 eo = __shfl_sync(0xFFFFFFFFu, excl, ol) - b0;
+                const u64 ao = __shfl_sync(0xFFFFFFFFu, a, ol);
+                const u32 no = TRACK ? __shfl_sync(0xFFFFFFFFu, ns, ol) : 0u;
+                if (f >= T) continue;
+                const u32 v = A.pins[ao + (f - eo)];
+                const uint2 s = A.state[v];
+                u32 y = s.y;
+                if (s.x != NONE) {
+                    movers = true;
+                    y |= A.target[v] << 15;
+                }
+                if (TRACK && f - eo >= no) y |= 1u << 31;
+                st[f] = make_uint2(s.x, y);
+                nd[f] = v;
+            }
+            __syncwarp();
+            if (__any_sync(0xFFFFFFFFu, movers)) {
+                for (u32 f0 = 0; f0 < T; f0 += 32) {
+                    const u32 f = f0 + lane;
+                    const uint2 me = f < T ? st[f] : make_uint2(NONE, 0);
+                    const bool act = me.x != NONE;
+                    if (!__any_sync(0xFFFFFFFFu, act)) continue;
+                    u32 ol = lo, oh = hi - 1;
+                    for (int it = 0; it < 5; ++it) {
+                        const u32 mid = (ol + oh + 1) >> 1;
+                        const u32 em = __shfl_sync(0xFFFFFFFFu, excl, mid & 31);
+                        if (ol < oh) { if (em - b0 <= f) ol = mid; else oh = mid - 1; }
+                    }
+                    const u32 eo = __shfl_sync(0xFFFFFFFFu, excl, ol) - b0, lno = __shfl_sync(0xFFFFFFFFu, len, ol);
+                    const u32 wo = __shfl_sync(0xFFFFFFFFu, wh, ol);
+                    const u32 p = me.y & 0x7FFFu, q = (me.y >> 15) & 0x7FFFu;
+                    u32 cp = 0, cq = 0, dp = 0, dq = 0;
+                    if (act) {
+#pragma unroll 4
+                        for (u32 j = eo; j < eo + lno; ++j) {
+                            const uint2 o = st[j];
+                            const u32 s = (o.x < me.x ? o.y >> 15 : o.y) & 0x7FFFu;
+                            cp += s == p;
+                            cq += s == q;
+                            if (TRACK) {
+                                dp += s == p && (o.y >> 31);
+                                dq += s == q && (o.y >> 31);
+                            }
+                        }
+                        const i64 d = leave_gain(A.encourage, wo, cp) - (cq == 0 ? (i64)wo : 0);
+                        if (d) atomicAdd(&A.g2[nd[f]], (unsigned long long)d);
+                    }
+                    if (TRACK) {
+                        __syncwarp();
+                        const bool dst = act && (me.y >> 31);
+                        emit_pair(A, dst && dp == 1, p, dst && dq == 0, q, me.x);
+                    }
+                }
+            }
+            __syncwarp();  // the stage is no longer read
+            lo = hi;
+        }
+    }
+}
+
+// The hyperedges of more than CM_LEN pins that hold a mover: every such incidence of every mover
+// flags its hyperedge (flag[] zeroed before), then the flags are compacted into the cascade's
+// list. One warp per mover.
 __global__ void k_mover_hedges(const u32 *__restrict__ mv, const u32 *__restrict__ dM, const u64 *__restrict__ toff,
-                               const u32 *__restrict__ touch, u32 *__restrict__ flag) {
+                               const u32 *__restrict__ touch, const u64 *__restrict__ off, u32 *__restrict__ flag) {
     const u32 lane = threadIdx.x & 31u, nw = (gridDim.x * blockDim.x) >> 5;
     const u32 M = *dM;
     for (u32 r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < M; r += nw) {
         const u32 u = mv[r];
-        for (u64 j = toff[u] + lane; j < toff[u + 1]; j += 32) flag[touch[j]] = 1u;
+        for (u64 j = toff[u] + lane; j < toff[u + 1]; j += 32) {
+            const u32 h = touch[j];
+            if (off[h + 1] - off[h] > CM_LEN) flag[h] = 1u;
+        }
     }
 }
 
@@ -1858,7 +2086,7 @@ __global__ void k_cascade_warp(CascadeArgs A, const u32 *__restrict__ list, cons
         u32 m = 0;
         for (u64 base = a; base < b; base += 32) {
             u64 k = base + lane;
-            u32 v = k < b ? A.pins[k] : 0, r = k < b ? A.rank[v] : NONE;
+            u32 v = k < b ? A.pins[k] : 0, r = k < b ? A.state[v].x : NONE;
             bool mvr = r != NONE;
             u32 bal = __ballot_sync(0xFFFFFFFFu, mvr);
             if (mvr) {
@@ -1953,7 +2181,7 @@ __device__ __forceinline__ u32 cascade_gather(const CascadeArgs &A, u32 h, u64 *
     u32 mymax = 0;
     for (u64 base = a; base < b; base += blockDim.x) {  // same trip count in every thread
         const u64 k = base + threadIdx.x;
-        const u32 v = k < b ? A.pins[k] : 0, r = k < b ? A.rank[v] : NONE;
+        const u32 v = k < b ? A.pins[k] : 0, r = k < b ? A.state[v].x : NONE;
         const bool mvr = r != NONE;
         const u32 bal = __ballot_sync(0xFFFFFFFFu, mvr);
         u32 wbase = 0;
@@ -2326,7 +2554,8 @@ __device__ __forceinline__ Best warp_best_prefix(Best b) {
 // writes the mover count and the size-event count, as k_move_flags ... k_set_rank do.
 __global__ void __launch_bounds__(RSS_WARPS * 32) k_rank_small(u32 n, const u32 *__restrict__ target,
                                                               const i64 *__restrict__ gain, u64 gbound, u32 kb,
-                                                              u32 *__restrict__ mv, u32 *__restrict__ rank,
+                                                              const u32 *__restrict__ part, u32 *__restrict__ mv,
+                                                              uint2 *__restrict__ state,
                                                               unsigned long long *__restrict__ g2, u32 *__restrict__ dM,
                                                               u32 *__restrict__ twice) {
     extern __shared__ u32 sm[];
@@ -2335,7 +2564,7 @@ __global__ void __launch_bounds__(RSS_WARPS * 32) k_rank_small(u32 n, const u32 
     for (u32 b = 0; b < n; b += blockDim.x) {
         const u32 v = b + threadIdx.x;
         const bool f = v < n && target[v] != NONE;
-        if (v < n) { rank[v] = NONE; g2[v] = 0; }
+        if (v < n) { state[v] = make_uint2(NONE, part[v]); g2[v] = 0; }
         i64 tot;
         const i64 incl = block_incl_scan_i64(f ? 1 : 0, sh, tot);
         if (f) {
@@ -2366,7 +2595,7 @@ __global__ void __launch_bounds__(RSS_WARPS * 32) k_rank_small(u32 n, const u32 
     for (u32 i = threadIdx.x; i < M; i += blockDim.x) {
         const u32 v = vo[i];
         mv[i] = v;
-        rank[v] = i;
+        state[v].x = i;
     }
     if (threadIdx.x == 0) {
         *dM = M;
@@ -2571,6 +2800,8 @@ struct LevelPrep {
     u64 block_work_max = 0;  // largest gain-work bound of the block tier (sizes its shared table)
     u64 gain_bound = 0;     // no gain exceeds this (sum of incident weights)
     u64 max_len = 0;         // largest hyperedge
+    u64 max_deg = 0;         // largest degree
+    u64 short_pins = 0, short_sq = 0;  // pins of hyperedges of at most CM_LEN pins; sum of their squared lengths
     u64 dst_pins = 0;        // destination pins (bounds the inbound events: 2 per pin)
     u64 tier_deg[3] = {0, 0, 0};  // incidence entries of each gain tier (kernel timer only)
     u32 census_K = 0;        // nonzero: partition-indexed census over this many partitions, and
@@ -2619,21 +2850,25 @@ void setup_refine_kernels(Ctx &c) {
 __global__ void k_level_bounds(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ nsrc,
                                unsigned long long *__restrict__ out);
 
-// Largest gain-work bound over all nodes (out[0]) and over the block tier (out[1]).
+// Largest gain-work bound over all nodes (out[0]) and over the block tier (out[1]); the largest
+// degree (out[2]).
 __global__ void k_tier_max(u32 n, u32 K, const u64 *__restrict__ work, const u64 *__restrict__ toff,
                            unsigned long long *__restrict__ out) {
     u32 u = blockIdx.x * blockDim.x + threadIdx.x;
-    u64 all = 0, blk = 0;
+    u64 all = 0, blk = 0, deg = 0;
     if (u < n) {
-        const u64 wk = work[u], deg = toff[u + 1] - toff[u];
+        const u64 wk = work[u];
+        deg = toff[u + 1] - toff[u];
         all = wk;
         if (gain_tier(n, K, wk, deg) == 1u) blk = wk;
     }
     all = warp_max_u64(all);
     blk = warp_max_u64(blk);
+    deg = warp_max_u64(deg);
     if ((threadIdx.x & 31) == 0) {
         if (all) atomicMax(&out[0], (unsigned long long)all);
         if (blk) atomicMax(&out[1], (unsigned long long)blk);
+        if (deg) atomicMax(&out[2], (unsigned long long)deg);
     }
 }
 
@@ -2643,9 +2878,10 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K) {
     LevelPrep lp;
     const u32 e = L.e, n = L.n;
     // [0] census block list, [1] census huge list, [2..4] node tiers, [5] gain bound,
-    // [6] largest work, [7] largest block-tier work, [8] largest hyperedge, [9] destination pins
-    u64 *dc = c.arena.alloc<u64>(10);
-    AXC_CUDA(cudaMemsetAsync(dc, 0, 80, c.stream));
+    // [6] largest work, [7] largest block-tier work, [8] largest degree, [9] largest hyperedge,
+    // [10] destination pins, [11] pins of short hyperedges, [12] the sum of their squared lengths
+    u64 *dc = c.arena.alloc<u64>(13);
+    AXC_CUDA(cudaMemsetAsync(dc, 0, 104, c.stream));
     lp.census_K = K <= CD_K ? K : 0;
     if (e) {
         u32 *flag = c.arena.alloc<u32>(e);
@@ -2660,7 +2896,7 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K) {
             LAUNCH(c, k_flag_len, cdiv(e, 256), 256, 0, e, L.off, (u64)CS_BLOCK_CAP, ~0ull, flag);
             compact_indices_dn(c, flag, lp.hhuge, e, (u32 *)(dc + 1));
         }
-        LAUNCH(c, k_level_bounds, cdiv(e, 256), 256, 0, e, L.off, L.nsrc, (unsigned long long *)(dc + 8));
+        LAUNCH(c, k_level_bounds, cdiv(e, 256), 256, 0, e, L.off, L.nsrc, (unsigned long long *)(dc + 9));
     }
     if (n) {
         u64 *work = c.arena.alloc<u64>(n);
@@ -2675,16 +2911,19 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K) {
         }
         LAUNCH(c, k_tier_max, cdiv(n, 256), 256, 0, n, K, work, L.toff, (unsigned long long *)(dc + 6));
     }
-    u64 h[10];
-    fetch(c, h, dc, 80);
+    u64 h[13];
+    fetch(c, h, dc, 104);
     lp.n_hblock = (u32)h[0];
     lp.n_hhuge = (u32)h[1];
     for (int t = 0; t < 3; ++t) lp.ncount[t] = (u32)h[2 + t];
     lp.gain_bound = h[5];
     lp.heavy_work_max = lp.ncount[2] ? h[6] : 0;
     lp.block_work_max = h[7];
-    lp.max_len = h[8];
-    lp.dst_pins = h[9];
+    lp.max_deg = h[8];
+    lp.max_len = h[9];
+    lp.dst_pins = h[10];
+    lp.short_pins = h[11];
+    lp.short_sq = h[12];
     if (lp.n_hhuge) {
         lp.huge_tab = c.arena.alloc<u64>(lp.n_hhuge + 1);
         LAUNCH(c, k_tab_sizes, cdiv(lp.n_hhuge + 1, 256), 256, 0, lp.hhuge, lp.n_hhuge, L.off, lp.huge_tab);
@@ -2991,6 +3230,27 @@ static void inc_census_round(Ctx &c, const DLevel &L, const LevelPrep &lp, const
     AXC_CUDA(cudaMemsetAsync(ic.dirty, 0, (size_t)L.e * 4, c.stream));
 }
 
+// The lanes per mover follow the level's mean degree.
+template <u32 G, bool TRACK>
+static void run_cascade_movers_g(Ctx &c, const CascadeArgs &C, const MoverArgs &V, u32 n, u64 max_deg) {
+    LAUNCH_AS(c, "k_cascade_movers", (k_cascade_movers<G, TRACK>),
+              std::min<u32>(cdiv((u64)n * G, CM_THREADS), (u32)c.sms * 8), CM_THREADS, 0, C, V);
+    if (max_deg > CM_HEAVY * G)
+        LAUNCH_AS(c, "k_cascade_movers_heavy", (k_cascade_movers_heavy<TRACK>), (u32)c.sms * 4, CM_THREADS, 0, C, V,
+                  CM_HEAVY * G);
+}
+template <bool TRACK>
+static void run_cascade_movers(Ctx &c, const CascadeArgs &C, const MoverArgs &V, u32 n, u64 P, u64 max_deg) {
+    if (V.dense)
+        LAUNCH_AS(c, "k_cascade_dense", k_cascade_dense<TRACK>,
+                  std::min<u32>(cdiv(C.e, (CM_THREADS / 32) * V.per_warp), (u32)c.sms * 4), CM_THREADS, 0, C, V);
+    const u64 deg = P / n;
+    if (deg < 6) run_cascade_movers_g<4, TRACK>(c, C, V, n, max_deg);
+    else if (deg < 12) run_cascade_movers_g<8, TRACK>(c, C, V, n, max_deg);
+    else if (deg < 24) run_cascade_movers_g<16, TRACK>(c, C, V, n, max_deg);
+    else run_cascade_movers_g<32, TRACK>(c, C, V, n, max_deg);
+}
+
 // The launches of one round, with no host synchronization: safe to capture in a CUDA graph.
 // dyn (device, optional) holds the round's discount and round number for graph replays. Returns
 // the device word that says whether the moves were applied; its arena slot lies below `keep`,
@@ -3029,14 +3289,16 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     // small levels: ranking, validity and the best prefix in one block each (SMALL_*)
     const bool small = rp.K <= VS_MAX_K && n <= (u32)RSS_CAP && rp.copies == 1;
     // movers in id order, then ranked by (gain desc, id asc)
-    u32 *flag = c.arena.alloc<u32>(n), *mv = c.arena.alloc<u32>(n), *rank = c.arena.alloc<u32>(n);
+    u32 *flag = c.arena.alloc<u32>(n), *mv = c.arena.alloc<u32>(n);
+    uint2 *state = (uint2 *)c.arena.alloc<u64>(n);
     unsigned long long *g2 = c.arena.alloc<unsigned long long>(n);  // cascaded gains, zeroed here
     const u32 kb = bits_for(lp.gain_bound);
-    u32 *khi = c.arena.alloc<u32>(n), *klo = c.arena.alloc<u32>(n);
+    u32 *khi = flag, *klo = c.arena.alloc<u32>(n);  // the flags are spent when the keys are made
     if (small) {
-        LAUNCH(c, k_rank_small, 1, RSS_WARPS * 32, RSS_SMEM, n, target, gain, lp.gain_bound, kb, mv, rank, g2, dM, dSE);
+        LAUNCH(c, k_rank_small, 1, RSS_WARPS * 32, RSS_SMEM, n, target, gain, lp.gain_bound, kb, part, mv, state,
+               g2, dM, dSE);
     } else {
-    LAUNCH(c, k_move_flags, cdiv(n, 256), 256, 0, n, target, flag, rank, g2);
+    LAUNCH(c, k_move_flags, cdiv(n, 256), 256, 0, n, target, part, flag, state, g2);
     compact_indices_dn(c, flag, mv, n, dM);
     LAUNCH(c, k_move_keys, cdiv(n, 256), 256, 0, mv, dM, gain, lp.gain_bound, khi, klo);
     if (kb > 32) {
@@ -3075,7 +3337,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         LAUNCH(c, k_copy_keys, cdiv(n, 256), 256, 0, mv, dM, rp.copy_n, ck);
         radix_sort_pairs_dn(c, ck, mv, dM, n, bits_for(rp.copies - 1));
     }
-    if (!small || pairs || rp.copies > 1) LAUNCH(c, k_set_rank, cdiv(n, 256), 256, 0, mv, dM, rank, dSE);
+    if (!small || pairs || rp.copies > 1) LAUNCH(c, k_set_rank, cdiv(n, 256), 256, 0, mv, dM, state, dSE);
     // cascade
 
     // inbound-set transitions (INCC): each destination pin of a mover gives at most two
@@ -3097,22 +3359,32 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     {
         CascadeArgs C;
         C.e = L.e; C.encourage = rp.encourage ? 1 : 0; C.off = L.off; C.pins = L.pins; C.nsrc = L.nsrc;
-        C.wfx = wfx; C.lam = cs.lam; C.cpart = cs.part; C.ccnt = cs.cnt; C.cdcnt = cs.dcnt; C.rank = rank;
+        C.wfx = wfx; C.lam = cs.lam; C.cpart = cs.part; C.ccnt = cs.cnt; C.cdcnt = cs.dcnt; C.state = state;
         C.part = part; C.target = target; C.g2 = g2;
         C.track = track ? 1 : 0; C.tp = tp; C.tr = tr; C.tdv = tdv; C.dT = dT; C.tcap = tcap;
         C.tdense = tdense; C.dense_stride = n;
         C.status = c.d_status;
         C.K = rp.K;
         C.pbytes = c.profiling("k_cascade_warp") ? c.d_prof_bytes() : nullptr;
-        const bool direct = rp.K <= CC_DIRECT_K;
+        const bool direct = C.K <= CC_DIRECT_K;
         size_t m1 = c.arena.mark();
-        u32 *big = c.arena.alloc<u32>(L.e ? L.e : 1), *huge = c.arena.alloc<u32>(L.e ? L.e : 1);
-        u32 *big2 = c.arena.alloc<u32>(L.e ? L.e : 1);
-        if (L.e) {
-            // only the hyperedges that hold a mover: flagged from the movers' incidences
+        const bool longs = lp.max_len > CM_LEN;
+        // a warp of the dense kernel looks at 32 hyperedges, or fewer where that leaves the GPU idle
+        u32 per_warp = 32;
+        while (per_warp > 4 && L.e / per_warp < (u32)c.sms * 16) per_warp >>= 1;
+        // few nodes of many short incidences: a lane of the mover kernel would walk through several
+        // of them one after the other while the dense kernel reads the whole level in a few microseconds
+        const bool always = L.P / n > 128 && lp.short_pins <= (2u << 20);
+        const MoverArgs V{mv, dM, L.toff, L.touch, L.nin, longs ? 1 : 0, rp.K <= CD_MAX_K ? 1 : 0, n, 1u,
+                          always ? 1ull << 40 : lp.short_pins ? 16 * lp.short_sq / lp.short_pins : 0, per_warp};
+        if (lp.short_pins && track) run_cascade_movers<true>(c, C, V, n, L.P, lp.max_deg);
+        else if (lp.short_pins) run_cascade_movers<false>(c, C, V, n, L.P, lp.max_deg);
+        if (longs) {
+            u32 *big = c.arena.alloc<u32>(L.e), *huge = c.arena.alloc<u32>(L.e), *big2 = c.arena.alloc<u32>(L.e);
+            // only the long hyperedges that hold a mover: flagged from the movers' incidences
             u32 *hflag = c.arena.alloc<u32>(L.e), *hlist = c.arena.alloc<u32>(L.e);
             AXC_CUDA(cudaMemsetAsync(hflag, 0, (size_t)L.e * 4, c.stream));
-            LAUNCH(c, k_mover_hedges, (u32)c.sms * 8, 256, 0, mv, dM, L.toff, L.touch, hflag);
+            LAUNCH(c, k_mover_hedges, (u32)c.sms * 8, 256, 0, mv, dM, L.toff, L.touch, L.off, hflag);
             compact_indices_dn(c, hflag, hlist, L.e, dHl);
             int per_w = 1;
             AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_w, k_cascade_warp, CC_WARPS * 32, 0));
@@ -3122,7 +3394,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
             u32 smov = 128;
             while (smov < lp.max_len && smov < cascade_block_movers(c)) smov <<= 1;
             // hashed tables: sized for the level's largest hyperedge within the block's limit
-            const u32 stab = direct ? std::max(2 * rp.K, 32u)  // tk: the sweep's 2K lane masks
+            const u32 stab = direct ? std::max(2 * C.K, 32u)  // tk: the sweep's 2K lane masks
                                     : (u32)std::min<u64>(cascade_cap(std::min<u64>(lp.max_len, rp.K),
                                                                      std::min<u64>(lp.max_len, smov)),
                                                          CB_TAB_HASH);
@@ -3314,16 +3586,21 @@ __global__ void k_round_next(cudaGraphConditionalHandle h, u32 *__restrict__ rs,
 __global__ void k_level_bounds(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ nsrc,
                                unsigned long long *__restrict__ out) {
     u32 h = blockIdx.x * blockDim.x + threadIdx.x;
-    u64 len = 0, dst = 0;
+    u64 len = 0, dst = 0, sp = 0, sq = 0;
     if (h < e) {
         len = off[h + 1] - off[h];
         dst = len - nsrc[h];
+        if (len <= CM_LEN) { sp = len; sq = len * len; }
     }
+    sp = warp_sum(sp);
+    sq = warp_sum(sq);
     len = warp_max_u64(len);
     dst = warp_sum(dst);
     if ((threadIdx.x & 31) == 0) {
         atomicMax(&out[0], (unsigned long long)len);
         atomicAdd(&out[1], (unsigned long long)dst);
+        if (sp) atomicAdd(&out[2], (unsigned long long)sp);
+        if (sq) atomicAdd(&out[3], (unsigned long long)sq);
     }
 }
 
