@@ -109,13 +109,6 @@ __global__ void k_try_keys(u32 n, u32 salt, u32 *__restrict__ key, u32 *__restri
     const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v < n) { key[v] = mix32(v ^ salt); ord[v] = v; }
 }
-__global__ void k_copy_conn(u64 eS, u32 e2, const u32 *__restrict__ lam, const u32 *__restrict__ wfxS,
-                            unsigned long long *__restrict__ conn) {
-    const u64 h = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= eS) return;
-    const u32 l = lam[h];
-    if (l > 1) atomicAdd(&conn[h / e2], (unsigned long long)wfxS[h] * (l - 1));
-}
 __global__ void k_pick_copy(u32 n, const u32 *__restrict__ partS, u32 best, u32 k, u32 *__restrict__ part) {
     const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v < n) part[v] = partS[(u64)best * n + v] - best * k;
@@ -224,11 +217,9 @@ bool kway_multistart(Ctx &c, const DLevel &L, const u32 *wfx, u32 k, u32 omega, 
     RefineParams rp{nc * k, omega, 0x7FFFFFFFu, false, AXC_KWAY_TRY_ROUNDS, seed};
     rp.copies = nc;
     rp.copy_n = n;
-    refine_level(c, S, wfxS, rp, partS);
-    Census cs = build_census(c, S, partS);
     unsigned long long *conn = c.arena.alloc<unsigned long long>(nc);
     AXC_CUDA(cudaMemsetAsync(conn, 0, (size_t)nc * 8, c.stream));
-    LAUNCH(c, k_copy_conn, cdiv((u64)S.e, 256), 256, 0, (u64)S.e, e2, cs.lam, wfxS, conn);
+    refine_level(c, S, wfxS, rp, partS, conn);
     std::vector<u64> h(nc);
     fetch(c, h.data(), (const u64 *)conn, (size_t)nc * 8);
     u32 best = 0;

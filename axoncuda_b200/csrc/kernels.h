@@ -54,8 +54,10 @@ struct RefineParams {
     u32 copies = 1, copy_n = 0;
 };
 void setup_refine_kernels(Ctx &c);
-// all refinement rounds of one level; part[n] is updated in place; returns rounds applied
-u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp, u32 *part);
+// all refinement rounds of one level; part[n] is updated in place; returns rounds applied. With
+// copy_conn (device, [copies], zeroed) every copy's connectivity is added there.
+u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp, u32 *part,
+                 unsigned long long *copy_conn = nullptr);
 // one round's proposals only (parity stage)
 void refine_gains_only(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp, const u32 *part,
                        u32 discount, u32 round, u32 *target, i64 *gain);

@@ -21,6 +21,7 @@
 // are built once per level. Inside a round every count stays in device memory; the host reads a
 // single word per round (whether moves were applied), which drives the round schedule.
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -653,6 +654,7 @@ constexpr u32 GN_BLOCK = 256;
 constexpr u32 GN_BLOCK_W = 4096;
 constexpr u32 GN_WARP_DEG = 256;      // incidences one warp takes; more go to a block
 constexpr u32 GN_SMALL_LEVEL = 1024;  // levels with at most this many nodes use blocks only
+constexpr u32 KW_WARP_DEG = 1024;     // incidences one group of lanes takes in the k-way gains
 constexpr u32 GM_WARP_DEG = 4096;     // incidences one warp takes in the mask gains; more go to a block
 
 // ------------------------------------------------------------------ partition-indexed gains
@@ -1523,17 +1525,18 @@ __global__ void k_list_max(const u32 *__restrict__ list, u32 nl, const u64 *__re
 // table in shared memory, 2 = one block with the table in global scratch. Levels of at most
 // GN_SMALL_LEVEL nodes use no warp tier: their few nodes carry long census chains, which a block
 // splits over its warps while the rest of the GPU would idle anyway.
-__device__ __forceinline__ u32 gain_tier(u32 n, u32 K, u64 wk, u64 deg) {
+__device__ __forceinline__ u32 gain_tier(u32 n, u32 K, u64 wk, u64 deg, u32 kway) {
+    if (kway) return (n > GN_SMALL_LEVEL && deg <= KW_WARP_DEG) ? 0u : 1u;
     if (K <= GN_DIRECT_K)  // partition-indexed gains: a warp or a block, by incidences
         return (n > GN_SMALL_LEVEL && deg <= GM_WARP_DEG) ? 0u : 1u;
     if (wk > GN_BLOCK_W) return 2u;
     return (n > GN_SMALL_LEVEL && wk <= GN_WARP_W && deg <= GN_WARP_DEG) ? 0u : 1u;
 }
-__global__ void k_tier(u32 n, u32 K, const u64 *__restrict__ work, const u64 *__restrict__ toff, u32 tier,
+__global__ void k_tier(u32 n, u32 K, const u64 *__restrict__ work, const u64 *__restrict__ toff, u32 tier, u32 kway,
                        u32 *__restrict__ flag) {
     u32 u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= n) return;
-    flag[u] = gain_tier(n, K, work[u], toff[u + 1] - toff[u]) == tier ? 1u : 0u;
+    flag[u] = gain_tier(n, K, work[u], toff[u + 1] - toff[u], kway) == tier ? 1u : 0u;
 }
 
 // ------------------------------------------------------------------ ranking
@@ -1642,6 +1645,12 @@ struct CascadeArgs {
     u32 dense_stride;
     u32 *status;
     u32 K;  // partitions: with K <= CC_DIRECT_K the per-hyperedge tables are indexed by partition id
+    // without a census (k-way levels of few partitions per copy): K partitions and ce hyperedges
+    // of one copy; the tables hold copy-local partitions, counted from the pins (lam, cpart null)
+    u32 ce;
+    // movers in slots (k-way copies ranked by one block each): copy t's from slot t * cn, dM[t] of
+    // them; 0: ranks [0, *dM)
+    u32 cn;
     // when set (kernel timer on k_cascade_warp): each hyperedge's algorithmic bytes are added here
     unsigned long long *pbytes;
 };
@@ -1650,11 +1659,17 @@ constexpr u32 MV_DST = 0x80000000u;  // mover flag in the node field: the pin is
 constexpr u32 CC_DIRECT_K = 256;
 
 __device__ __forceinline__ bool cascade_direct(const CascadeArgs &A) { return A.K <= CC_DIRECT_K; }
+__device__ __forceinline__ u32 cascade_base(const CascadeArgs &A, u32 h) { return A.ce ? (h / A.ce) * A.K : 0u; }
 
 // The hyperedge's census into the table: partition -> (pins, destination pins). Block- or
 // warp-wide over threads [t0, t0 + nt); direct tables hold K slots, hashed ones `cap`.
-__device__ __forceinline__ void cascade_fill(const CascadeArgs &A, u64 a, u32 lm, u32 *tk, u32 *tc, u32 *td, u32 cap,
-                                             u32 t0, u32 nt) {
+__device__ __forceinline__ void cascade_fill(const CascadeArgs &A, u32 h, u64 a, u64 b, u32 lm, u32 *tk, u32 *tc,
+                                             u32 *td, u32 cap, u32 t0, u32 nt) {
+    if (!A.lam) {
+        const u32 base = cascade_base(A, h);
+        for (u64 k = a + t0; k < b; k += nt) atomicAdd(&tc[A.state[A.pins[k]].y - base], 1u);
+        return;
+    }
     const bool direct = cascade_direct(A);
     for (u32 i = t0; i < lm; i += nt) {
         const u32 q = A.cpart[a + i];
@@ -1693,12 +1708,13 @@ __device__ __forceinline__ void emit_pair(const CascadeArgs &A, bool leave, u32 
 // Table slots of every mover's source and target partition, sl[i] = slot(p) | slot(q) << 16,
 // gathered in parallel so the sequential sweep reads no global memory. Hashed tables insert the
 // partitions missing from the census (their counts stay zero); they need cap <= 65536.
-__device__ __forceinline__ void cascade_slots(const CascadeArgs &A, const u64 *mv, u32 *sl, u32 m, u32 *tk, u32 cap,
-                                              u32 t0, u32 nt) {
+__device__ __forceinline__ void cascade_slots(const CascadeArgs &A, u32 h, const u64 *mv, u32 *sl, u32 m, u32 *tk,
+                                              u32 cap, u32 t0, u32 nt) {
     const bool direct = cascade_direct(A);
+    const u32 base = cascade_base(A, h);
     for (u32 i = t0; i < m; i += nt) {
         const u32 v = (u32)mv[i] & ~MV_DST;
-        const u32 p = A.part[v], q = A.target[v];
+        const u32 p = A.part[v] - base, q = A.target[v] - base;
         u32 sp = p, sq = q;  // direct tables: the slot is the partition id
         if (!direct) {
             sp = hash_find_or_insert(tk, cap - 1, p);
@@ -1920,9 +1936,11 @@ __global__ void __launch_bounds__(CM_THREADS) k_cascade_movers(CascadeArgs A, Mo
     const u32 lane = threadIdx.x & 31u, gl = lane & (G - 1);
     const u32 gmask = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
     if (cascade_dense(V)) return;
-    const u32 M = *V.dM, ng = gridDim.x * (CM_THREADS / G);
-    for (u32 r = blockIdx.x * (CM_THREADS / G) + threadIdx.x / G; r < M; r += ng) {
-        const u32 u = V.mv[r];
+    const u32 ng = gridDim.x * (CM_THREADS / G), end = A.cn ? V.n : *V.dM;
+    for (u32 x = blockIdx.x * (CM_THREADS / G) + threadIdx.x / G; x < end; x += ng) {
+        const u32 r = A.cn ? x % A.cn : x;
+        if (A.cn && r >= V.dM[x / A.cn]) continue;
+        const u32 u = V.mv[x];
         const u64 t0 = V.toff[u], deg = V.toff[u + 1] - t0;
         if (deg > CM_HEAVY * G) continue;
         const u32 p = A.part[u], q = A.target[u], nin_u = TRACK ? V.nin[u] : 0u;
@@ -1941,9 +1959,11 @@ __global__ void __launch_bounds__(CM_THREADS) k_cascade_movers(CascadeArgs A, Mo
 template <bool TRACK>
 __global__ void __launch_bounds__(CM_THREADS) k_cascade_movers_heavy(CascadeArgs A, MoverArgs V, u32 min_deg) {
     if (cascade_dense(V)) return;
-    const u32 M = *V.dM;
-    for (u32 r = blockIdx.x; r < M; r += gridDim.x) {
-        const u32 u = V.mv[r];
+    const u32 end = A.cn ? V.n : *V.dM;
+    for (u32 x = blockIdx.x; x < end; x += gridDim.x) {
+        const u32 r = A.cn ? x % A.cn : x;
+        if (A.cn && r >= V.dM[x / A.cn]) continue;
+        const u32 u = V.mv[x];
         const u64 t0 = V.toff[u], deg = V.toff[u + 1] - t0;
         if (deg <= min_deg) continue;
         const u32 p = A.part[u], q = A.target[u], nin_u = TRACK ? V.nin[u] : 0u;
@@ -2058,10 +2078,12 @@ __global__ void __launch_bounds__(CM_THREADS) k_cascade_dense(CascadeArgs A, Mov
 // flags its hyperedge (flag[] zeroed before), then the flags are compacted into the cascade's
 // list. One warp per mover.
 __global__ void k_mover_hedges(const u32 *__restrict__ mv, const u32 *__restrict__ dM, const u64 *__restrict__ toff,
-                               const u32 *__restrict__ touch, const u64 *__restrict__ off, u32 *__restrict__ flag) {
+                               const u32 *__restrict__ touch, const u64 *__restrict__ off, u32 cn, u32 slots,
+                               u32 *__restrict__ flag) {
     const u32 lane = threadIdx.x & 31u, nw = (gridDim.x * blockDim.x) >> 5;
-    const u32 M = *dM;
-    for (u32 r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < M; r += nw) {
+    const u32 end = cn ? slots : *dM;
+    for (u32 r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < end; r += nw) {
+        if (cn && r % cn >= dM[r / cn]) continue;
         const u32 u = mv[r];
         for (u64 j = toff[u] + lane; j < toff[u + 1]; j += 32) {
             const u32 h = touch[j];
@@ -2103,7 +2125,7 @@ __global__ void k_cascade_warp(CascadeArgs A, const u32 *__restrict__ list, cons
             bytes += bytes_read;
             continue;
         }
-        const u32 lm = A.lam[h];
+        const u32 lm = A.lam ? A.lam[h] : 0;
         const bool direct = cascade_direct(A);
         const u32 cap = direct ? A.K : cascade_cap32(lm, m);
         if (m > CC_MOV || cap > CC_TAB) {
@@ -2131,9 +2153,9 @@ __global__ void k_cascade_warp(CascadeArgs A, const u32 *__restrict__ list, cons
         const u32 ntk = direct ? 2 * A.K : cap;
         for (u32 i = lane; i < ntk; i += 32) tk[w][i] = direct ? 0u : NONE;
         __syncwarp();
-        cascade_fill(A, a, lm, tk[w], tc[w], td[w], cap, lane, 32);
+        cascade_fill(A, h, a, b, lm, tk[w], tc[w], td[w], cap, lane, 32);
         __syncwarp();
-        cascade_slots(A, mvs[w], sl[w], m, tk[w], cap, lane, 32);
+        cascade_slots(A, h, mvs[w], sl[w], m, tk[w], cap, lane, 32);
         __syncwarp();
         cascade_sweep_warp(A, h, mvs[w], sl[w], m, tk[w], tc[w], td[w], direct ? tk[w] : nullptr);
     }
@@ -2278,10 +2300,10 @@ __device__ __forceinline__ void cascade_block_one(const CascadeArgs &A, u32 h, u
     __syncthreads();
     if (radix) block_radix_sort_hi(mvs, m, 32 - __clz(rmax), wsum);
     else block_bitonic_u64(mvs, P);
-    cascade_fill(A, A.off[h], A.lam[h], tk, tc, td, cap, threadIdx.x, blockDim.x);
+    cascade_fill(A, h, A.off[h], A.off[h + 1], A.lam ? A.lam[h] : 0, tk, tc, td, cap, threadIdx.x, blockDim.x);
     __syncthreads();
     if (sl) {
-        cascade_slots(A, mvs, sl, m, tk, cap, threadIdx.x, blockDim.x);
+        cascade_slots(A, h, mvs, sl, m, tk, cap, threadIdx.x, blockDim.x);
         __syncthreads();
     }
     if (sl) {
@@ -2771,6 +2793,558 @@ __global__ void k_apply_seg(const u32 *__restrict__ mv, const u32 *__restrict__ 
     part[v] = target[v];
 }
 
+// ------------------------------------------------------------------ k-way levels of few partitions
+// K-way rounds without an inbound limit need no census entries when a copy holds at most KW_K
+// partitions. A hyperedge's record is two K-bit masks of MW words: the partitions present, and
+// those holding exactly one of its pins. With w its weight, a node in partition p gains w for
+// every incidence where p is single (what leaving saves) and pays w for every incidence where
+// the target is absent: both are bits, so a node's gains are sums over its incidences' records
+// and no per-pin sums are kept. A level keeps its records across its rounds; after each apply
+// the hyperedges of the moved nodes are flagged, and the next round rewrites only those. The
+// copies of a multi-start use partition ids local to their copy, so a record is as wide as one
+// copy's partitions whatever the number of copies.
+constexpr u32 KW_K = 256;
+constexpr u32 KW_SHORT = 8;      // pins one lane reads; longer hyperedges take the warp
+constexpr u32 KW_THREADS = 256;
+
+struct KwArgs {
+    const u64 *off;
+    const u32 *pins, *part;
+    u32 e, ce, k;    // hyperedges; hyperedges and partitions of one copy
+    u32 *rec;        // [e * 2 * MW]: present words, then single words
+    uint8_t *dirty;  // [e]
+    u32 per_warp;    // hyperedges one warp looks at (at most 32)
+};
+
+template <u32 MW>
+__device__ __forceinline__ void kw_add(u32 (&any)[MW], u32 (&mul)[MW], u32 q) {
+    const u32 bit = 1u << (q & 31u);
+#pragma unroll
+    for (u32 x = 0; x < MW; ++x) {  // no branch: the words stay in registers
+        const u32 m = MW == 1 || x == (q >> 5) ? bit : 0u;
+        mul[x] |= any[x] & m;
+        any[x] |= m;
+    }
+}
+template <u32 MW>
+__device__ __forceinline__ void kw_store(u32 *rec, const u32 (&any)[MW], const u32 (&mul)[MW]) {
+    u32 out[2 * MW];
+#pragma unroll
+    for (u32 x = 0; x < MW; ++x) {
+        out[x] = any[x];
+        out[MW + x] = any[x] & ~mul[x];
+    }
+    store_words<2 * MW>(rec, out);
+}
+
+// The records of the flagged hyperedges, which are unflagged. A warp looks at per_warp hyperedges:
+// a lane does its own when it has at most KW_SHORT pins, the warp the others one by one.
+template <u32 MW>
+__global__ void __launch_bounds__(KW_THREADS) k_kway_records(KwArgs A) {
+    const u32 lane = threadIdx.x & 31u;
+    const u32 h0 = (blockIdx.x * (KW_THREADS / 32) + (threadIdx.x >> 5)) * A.per_warp;
+    const u32 h = h0 + lane;
+    bool mine = lane < A.per_warp && h < A.e && A.dirty[h];
+    const u64 a = mine ? A.off[h] : 0, len64 = mine ? A.off[h + 1] - a : 0;
+    mine = mine && len64 <= CD_WARP_LEN;  // longer ones are k_kway_records_block's
+    const u32 len = mine ? (u32)len64 : 0;
+    const u32 base = mine ? (h / A.ce) * A.k : 0;
+    if (mine) A.dirty[h] = 0;
+    u32 any[MW], mul[MW];
+#pragma unroll
+    for (u32 x = 0; x < MW; ++x) any[x] = mul[x] = 0;
+    if (mine && len <= KW_SHORT) {
+        u32 q[KW_SHORT];
+#pragma unroll
+        for (u32 i = 0; i < KW_SHORT; ++i) q[i] = i < len ? A.part[A.pins[a + i]] - base : NONE;
+#pragma unroll
+        for (u32 i = 0; i < KW_SHORT; ++i)
+            if (i < len) kw_add<MW>(any, mul, q[i]);
+        kw_store<MW>(A.rec + (u64)h * (2 * MW), any, mul);
+    }
+    u32 rest = __ballot_sync(0xFFFFFFFFu, mine && len > KW_SHORT);
+    while (rest) {
+        const u32 t = __ffs(rest) - 1;
+        rest &= rest - 1;
+        const u64 at = __shfl_sync(0xFFFFFFFFu, a, t);
+        const u32 lt = __shfl_sync(0xFFFFFFFFu, len, t), bt = __shfl_sync(0xFFFFFFFFu, base, t);
+#pragma unroll
+        for (u32 x = 0; x < MW; ++x) any[x] = mul[x] = 0;
+#pragma unroll 4
+        for (u32 i = lane; i < lt; i += 32) kw_add<MW>(any, mul, A.part[A.pins[at + i]] - bt);
+#pragma unroll
+        for (u32 o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (u32 x = 0; x < MW; ++x) {
+                const u32 a2 = __shfl_xor_sync(0xFFFFFFFFu, any[x], o), m2 = __shfl_xor_sync(0xFFFFFFFFu, mul[x], o);
+                mul[x] |= m2 | (any[x] & a2);
+                any[x] |= a2;
+            }
+        if (lane == 0) kw_store<MW>(A.rec + (u64)(h0 + t) * (2 * MW), any, mul);
+    }
+}
+
+// Hyperedges above CD_WARP_LEN pins (the level's block list), one block each, when flagged.
+template <u32 MW>
+__global__ void __launch_bounds__(KW_THREADS) k_kway_records_block(KwArgs A, const u32 *__restrict__ list, u32 nlist) {
+    __shared__ u32 cnt[MW * 32];
+    for (u32 idx = blockIdx.x; idx < nlist; idx += gridDim.x) {
+        const u32 h = list[idx];
+        if (!A.dirty[h]) continue;  // uniform over the block
+        const u64 a = A.off[h], b = A.off[h + 1];
+        const u32 base = (h / A.ce) * A.k;
+        for (u32 i = threadIdx.x; i < MW * 32; i += KW_THREADS) cnt[i] = 0;
+        __syncthreads();
+        for (u64 i = a + threadIdx.x; i < b; i += KW_THREADS) atomicAdd(&cnt[A.part[A.pins[i]] - base], 1u);
+        __syncthreads();
+        for (u32 x = threadIdx.x >> 5; x < MW; x += KW_THREADS / 32) {
+            const u32 c = cnt[x * 32 + (threadIdx.x & 31u)];
+            const u32 any = __ballot_sync(0xFFFFFFFFu, c > 0), one = __ballot_sync(0xFFFFFFFFu, c == 1);
+            if ((threadIdx.x & 31u) == 0) {
+                A.rec[(u64)h * (2 * MW) + x] = any;
+                A.rec[(u64)h * (2 * MW) + MW + x] = one;
+            }
+        }
+        if (threadIdx.x == 0) A.dirty[h] = 0;
+        __syncthreads();
+    }
+}
+
+// Connectivity of every copy from the records: conn[t] += w * (partitions present - 1).
+template <u32 MW>
+__global__ void __launch_bounds__(KW_THREADS) k_kway_conn(KwArgs A, const u32 *__restrict__ wfx,
+                                                          unsigned long long *__restrict__ conn) {
+    const u32 t = blockIdx.y;
+    u64 s = 0;
+    for (u32 j = blockIdx.x * KW_THREADS + threadIdx.x; j < A.ce; j += gridDim.x * KW_THREADS) {
+        const u64 h = (u64)t * A.ce + j;
+        u32 any[MW], l = 0;
+        load_words<MW>(A.rec + h * (2 * MW), any);
+#pragma unroll
+        for (u32 x = 0; x < MW; ++x) l += __popc(any[x]);
+        if (l > 1) s += (u64)wfx[h] * (l - 1);
+    }
+    s = warp_sum(s);
+    if ((threadIdx.x & 31u) == 0 && s) atomicAdd(&conn[t], (unsigned long long)s);
+}
+
+struct KwGain {
+    const u32 *rec;
+    u32 k, cn;  // partitions and nodes of one copy
+    const u32 *list;
+    u32 nl;
+};
+
+// Best target of node u from the lanes' connectivities: lane `own` of a group of G holds those of
+// its partitions own, own + G, ... (conn[x]); the group's lane 0 writes the move. A partition
+// without connectivity gains at most saving - wtot <= 0, so presence needs no test.
+template <u32 G, u32 C, class T>
+__device__ __forceinline__ void kw_move(const GainArgs &A, u32 u, u32 base, u32 pl, u32 k, u32 own, u32 gmask,
+                                        const T (&conn)[C], T saving, T wtot) {
+    Cand best{INT64_MIN, 0};
+    const u64 s = A.nsize[u], need = s - s / A.discount;
+#pragma unroll
+    for (u32 x = 0; x < C; ++x) {
+        const u32 q = own + G * x;
+        if (q >= k || q == pl || conn[x] == 0) continue;
+        if (A.psize[base + q] + need > A.omega) continue;
+        const Cand c{(i64)saving - ((i64)wtot - (i64)conn[x]),
+                     ((u64)mix32(base + q + A.round + A.seed) << 32) | (u64)(~(base + q))};
+        if (cand_better(c, best)) best = c;
+    }
+#pragma unroll
+    for (u32 o = G / 2; o > 0; o >>= 1) {
+        Cand d;
+        d.g = __shfl_xor_sync(gmask, best.g, o);
+        d.tie = __shfl_xor_sync(gmask, best.tie, o);
+        if (cand_better(d, best)) best = d;
+    }
+    if (own == 0) write_move(A, u, best);
+}
+
+// One group of G lanes per node (G a power of two, at least k for one word): lane l owns
+// partitions l, l + G, ... (C of them) and reads every incidence's record, the same addresses across the group. T: u32 when
+// no node's incident weights pass 2^32, else u64.
+template <u32 MW, u32 G, class T>
+__global__ void __launch_bounds__(KW_THREADS) k_kway_gain(GainArgs A0, KwGain V) {
+    static_assert(MW == 1 || G == 32, "one word: a lane per partition; more: a lane per bit of each");
+    constexpr u32 C = MW;
+    const GainArgs A = gain_args_now(A0);
+    const u32 lane = threadIdx.x & 31u, own = lane & (G - 1);
+    const u32 gmask = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
+    const u32 idx = blockIdx.x * (KW_THREADS / G) + threadIdx.x / G;
+    if (idx >= V.nl) return;
+    const u32 u = V.list[idx], base = (u / V.cn) * V.k, pl = A.part[u] - base;
+    const u64 t0 = A.toff[u];
+    const u32 deg = (u32)(A.toff[u + 1] - t0);
+    T conn[C], saving = 0, wtot = 0;
+#pragma unroll
+    for (u32 x = 0; x < C; ++x) conn[x] = 0;
+#pragma unroll 4
+    for (u32 j = 0; j < deg; ++j) {
+        const u32 h = A.touch[t0 + j], w = A.wfx[h];
+        const u32 *r = V.rec + (u64)h * (2 * MW);
+        u32 any[MW];
+        u32 sg;
+        if constexpr (MW == 1) {
+            const uint2 v = *(const uint2 *)r;
+            any[0] = v.x;
+            sg = v.y;
+        } else {
+            load_words<MW>(r, any);
+            sg = r[MW + (pl >> 5)];
+        }
+        wtot += w;
+        if ((sg >> (pl & 31u)) & 1u) saving += w;
+#pragma unroll
+        for (u32 x = 0; x < C; ++x)
+            if ((any[x] >> own) & 1u) conn[x] += w;
+    }
+    kw_move<G, C, T>(A, u, base, pl, V.k, own, gmask, conn, saving, wtot);
+}
+
+// At most 4 partitions: a group of G lanes per node takes the incidences side by side, each lane
+// with a sum per partition, summed over the group at the end.
+template <u32 G, class T>
+__global__ void __launch_bounds__(KW_THREADS) k_kway_gain_few(GainArgs A0, KwGain V) {
+    const GainArgs A = gain_args_now(A0);
+    const u32 lane = threadIdx.x & 31u, own = lane & (G - 1);
+    const u32 gmask = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
+    const u32 idx = blockIdx.x * (KW_THREADS / G) + threadIdx.x / G;
+    if (idx >= V.nl) return;
+    const u32 u = V.list[idx], base = (u / V.cn) * V.k, pl = A.part[u] - base;
+    const u64 t0 = A.toff[u];
+    const u32 deg = (u32)(A.toff[u + 1] - t0);
+    T conn[4] = {0, 0, 0, 0}, saving = 0, wtot = 0;
+#pragma unroll 2
+    for (u32 j = own; j < deg; j += G) {
+        const u32 h = A.touch[t0 + j], w = A.wfx[h];
+        const uint2 r = *(const uint2 *)(V.rec + (u64)h * 2);
+        wtot += w;
+        if ((r.y >> pl) & 1u) saving += w;
+#pragma unroll
+        for (u32 x = 0; x < 4; ++x)
+            if ((r.x >> x) & 1u) conn[x] += w;
+    }
+    __syncwarp(gmask);
+#pragma unroll
+    for (u32 o = G / 2; o > 0; o >>= 1) {
+        wtot += __shfl_xor_sync(gmask, wtot, o);
+        saving += __shfl_xor_sync(gmask, saving, o);
+#pragma unroll
+        for (u32 x = 0; x < 4; ++x) conn[x] += __shfl_xor_sync(gmask, conn[x], o);
+    }
+    T mine[1] = {own == 0 ? conn[0] : own == 1 ? conn[1] : own == 2 ? conn[2] : own == 3 ? conn[3] : (T)0};
+    kw_move<G, 1, T>(A, u, base, pl, V.k, own, gmask, mine, saving, wtot);
+}
+
+// One block per node (heavy nodes and small levels): each warp takes every eighth incidence with a
+// lane per 32 partitions as above, and the warps' sums meet in shared memory.
+template <u32 MW, class T>
+__global__ void __launch_bounds__(KW_THREADS) k_kway_gain_block(GainArgs A0, KwGain V) {
+    constexpr u32 NW = KW_THREADS / 32;
+    const GainArgs A = gain_args_now(A0);
+    __shared__ T sc[NW][MW * 32], ss[NW], sw[NW];
+    const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    for (u32 idx = blockIdx.x; idx < V.nl; idx += gridDim.x) {
+        const u32 u = V.list[idx], base = (u / V.cn) * V.k, pl = A.part[u] - base;
+        const u64 t0 = A.toff[u], deg = A.toff[u + 1] - t0;
+        T conn[MW], saving = 0, wtot = 0;
+#pragma unroll
+        for (u32 x = 0; x < MW; ++x) conn[x] = 0;
+#pragma unroll 4
+        for (u64 j = w; j < deg; j += NW) {
+            const u32 h = A.touch[t0 + j], wh = A.wfx[h];
+            const u32 *r = V.rec + (u64)h * (2 * MW);
+            u32 any[MW];
+            load_words<MW>(r, any);
+            const u32 sg = r[MW + (pl >> 5)];
+            wtot += wh;
+            if ((sg >> (pl & 31u)) & 1u) saving += wh;
+#pragma unroll
+            for (u32 x = 0; x < MW; ++x)
+                if ((any[x] >> lane) & 1u) conn[x] += wh;
+        }
+#pragma unroll
+        for (u32 x = 0; x < MW; ++x) sc[w][x * 32 + lane] = conn[x];
+        if (lane == 0) { ss[w] = saving; sw[w] = wtot; }
+        __syncthreads();
+        if (w == 0) {
+            saving = wtot = 0;
+            for (u32 i = 0; i < NW; ++i) { saving += ss[i]; wtot += sw[i]; }
+#pragma unroll
+            for (u32 x = 0; x < MW; ++x) {
+                conn[x] = 0;
+                for (u32 i = 0; i < NW; ++i) conn[x] += sc[i][x * 32 + lane];
+            }
+            kw_move<32, MW, T>(A, u, base, pl, V.k, lane, 0xFFFFFFFFu, conn, saving, wtot);
+        }
+        __syncthreads();  // warp 0 has read the sums
+    }
+}
+
+// After the apply: the hyperedges of the moved nodes are flagged for the next round's records. The
+// movers of copy t are mv[t * cn, ...) in rank order and its first applied[t] moved (one copy:
+// the movers up to the best prefix's rank).
+__global__ void k_kway_mark(const u32 *__restrict__ mv, u32 cn, u32 copies, const u32 *__restrict__ applied,
+                            const u64 *__restrict__ toff, const u32 *__restrict__ touch, uint8_t *__restrict__ dirty) {
+    const u32 lane = threadIdx.x & 31u, nw = (gridDim.x * blockDim.x) >> 5;
+    const u32 w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    for (u32 t = 0; t < copies; ++t) {
+        const u32 M = applied[t];
+        for (u32 i = w0; i < M; i += nw) {
+            const u32 v = mv[(u64)t * cn + i];
+            for (u64 j = toff[v] + lane; j < toff[v + 1]; j += 32) dirty[touch[j]] = 1;
+        }
+    }
+}
+
+// The same after the ranking of larger levels: the movers mv[0, *dM) in rank order, their copies in
+// ck (null: one copy), those up to their copy's best rank moved where its apply flag is set.
+__global__ void k_kway_mark_ranked(const u32 *__restrict__ mv, const u32 *__restrict__ dM, const u32 *__restrict__ ck,
+                                   const Best *__restrict__ best, const u32 *__restrict__ apply,
+                                   const u64 *__restrict__ toff, const u32 *__restrict__ touch,
+                                   uint8_t *__restrict__ dirty) {
+    const u32 lane = threadIdx.x & 31u, nw = (gridDim.x * blockDim.x) >> 5, M = *dM;
+    for (u32 i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < M; i += nw) {
+        const u32 t = ck ? ck[i] : 0;
+        if (!apply[t] || i > best[t].r) continue;
+        const u32 v = mv[i];
+        for (u64 j = toff[v] + lane; j < toff[v + 1]; j += 32) dirty[touch[j]] = 1;
+    }
+}
+
+// ---- ranking, validity and the best prefix of k-way copies of at most RSS_CAP nodes -----------
+// A copy's moves depend on no other copy, so one block ranks each copy's moves in shared memory
+// (a level of one copy is the case copies = 1), and ranks, prefixes and the best prefix are per
+// copy. The order is that of the launches for larger levels: moves by (gain desc, id asc), the
+// i-th of a -> b beside the i-th of b -> a, pairs by (pair gain desc, position, direction).
+struct CopyArgs {
+    u32 cn, k;                  // nodes and partitions of one copy
+    u32 n;                      // nodes of all copies
+    const u32 *target, *nsize;
+    const i64 *gain;
+    u32 *part;
+    u64 gbound, pbound;         // bounds of the gains and of the pair gains
+    u32 kb, pb, gb;             // their bits; bits of a direction group
+    u32 *mv;                    // [n] movers of copy t in rank order from t * cn
+    u32 *dM;                    // [copies] movers
+    uint2 *state;               // [n]
+    unsigned long long *g2;     // [n] cascaded gains (zeroed here)
+    i64 *psn;                   // [n] pair gain of a mover
+    i64 *vs;                    // [n] size violations by rank (zeroed here)
+    u64 *psize;                 // [copies * k]
+    u32 *applied;               // [copies]
+    u32 *apply;                 // any copy moved
+    u64 omega;
+};
+
+// Stable sort of the block's (key, node) pairs by a 64-bit key of `bits` bits: the low words are in
+// sm (as block_radix_sort takes them), the high words come from hi(node).
+template <class F>
+__device__ __forceinline__ void copy_sort64(u32 *sm, u32 M, u32 bits, const u32 *&ko, const u32 *&vo, F &&hi) {
+    block_radix_sort(sm, M, bits < 32 ? bits : 32, ko, vo);
+    if (bits <= 32) return;
+    u32 hv[RSS_ITEMS], nv[RSS_ITEMS];
+#pragma unroll
+    for (int x = 0; x < RSS_ITEMS; ++x) {
+        const u32 i = threadIdx.x + (u32)x * blockDim.x;
+        nv[x] = i < M ? vo[i] : 0u;
+        hv[x] = i < M ? hi(nv[x]) : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < RSS_ITEMS; ++x) {
+        const u32 i = threadIdx.x + (u32)x * blockDim.x;
+        if (i < M) { sm[i] = hv[x]; sm[RSS_CAP + i] = nv[x]; }
+    }
+    block_radix_sort(sm, M, bits - 32, ko, vo);
+}
+
+__global__ void __launch_bounds__(RSS_WARPS * 32) k_copy_rank(CopyArgs A) {
+    extern __shared__ u32 sm[];
+    __shared__ i64 sh[32];
+    const u32 t = blockIdx.x, v0 = t * A.cn, base = t * A.k, T = blockDim.x;
+    u32 M = 0;
+    for (u32 b = 0; b < A.cn; b += T) {
+        const u32 i = b + threadIdx.x, v = v0 + i;
+        const bool f = i < A.cn && A.target[v] != NONE;
+        if (i < A.cn) {
+            A.state[v] = make_uint2(NONE, A.part[v]);
+            A.g2[v] = 0;
+            A.vs[v] = 0;
+        }
+        i64 tot;
+        const i64 incl = block_incl_scan_i64(f ? 1 : 0, sh, tot);
+        if (f) {
+            const u32 pos = M + (u32)incl - 1;
+            sm[pos] = (u32)(A.gbound - (u64)A.gain[v]);
+            sm[RSS_CAP + pos] = v;
+        }
+        M += (u32)tot;
+    }
+    const u32 *ko, *vo;
+    copy_sort64(sm, M, A.kb, ko, vo, [&](u32 v) { return (u32)((A.gbound - (u64)A.gain[v]) >> 32); });
+    // by direction group, each in gain order
+    u32 key[RSS_ITEMS], nd[RSS_ITEMS];
+#pragma unroll
+    for (int x = 0; x < RSS_ITEMS; ++x) {
+        const u32 i = threadIdx.x + (u32)x * T;
+        if (i >= M) continue;
+        const u32 u = vo[i], p = A.part[u] - base, q = A.target[u] - base;
+        nd[x] = u;
+        key[x] = (((p < q ? p : q) * A.k + (p < q ? q : p)) << 1) | (p < q ? 0u : 1u);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < RSS_ITEMS; ++x) {
+        const u32 i = threadIdx.x + (u32)x * T;
+        if (i < M) { sm[i] = key[x]; sm[RSS_CAP + i] = nd[x]; }
+    }
+    block_radix_sort(sm, M, A.gb, ko, vo);
+    // partners: the i-th move of a group and the i-th of the opposite one. fl[j] counts the moves
+    // that follow the group order at position j: both of a pair at its first direction's position.
+    u32 pk[RSS_ITEMS];  // a paired second direction's partner position, else NONE
+    i64 ps[RSS_ITEMS];
+    u32 *fl = const_cast<u32 *>(ko == sm ? sm + 2 * RSS_CAP : sm);  // the buffers not holding (ko, vo)
+#pragma unroll
+    for (int x = 0; x < RSS_ITEMS; ++x) {
+        const u32 j = threadIdx.x + (u32)x * T;
+        if (j >= M) continue;
+        const u32 g = ko[j], d = g & 1u, u = vo[j];
+        const u32 i = j - lower_bound_u32(ko, M, g);
+        const u32 s2 = lower_bound_u32(ko, M, g ^ 1u), e2 = lower_bound_u32(ko, M, (g ^ 1u) + 1u);
+        nd[x] = u;
+        ps[x] = A.gain[u];
+        pk[x] = NONE;
+        u32 f = 1;
+        if (i < e2 - s2) {
+            ps[x] += A.gain[vo[s2 + i]];
+            if (d) pk[x] = s2 + i;
+            f = d ? 0u : 2u;
+        }
+        fl[j] = f;
+    }
+    __syncthreads();
+    // exclusive prefix of fl in place: a move's place by (pair position, direction)
+    {
+        u32 run = 0;
+        for (u32 b = 0; b < M; b += T) {
+            const u32 j = b + threadIdx.x;
+            const u32 f = j < M ? fl[j] : 0u;
+            i64 tot;
+            const i64 incl = block_incl_scan_i64((i64)f, sh, tot);
+            if (j < M) fl[j] = run + (u32)incl - f;
+            run += (u32)tot;
+        }
+    }
+    __syncthreads();
+    u32 at[RSS_ITEMS];
+#pragma unroll
+    for (int x = 0; x < RSS_ITEMS; ++x) {
+        const u32 j = threadIdx.x + (u32)x * T;
+        if (j < M) at[x] = pk[x] != NONE ? fl[pk[x]] + 1 : fl[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < RSS_ITEMS; ++x) {
+        const u32 j = threadIdx.x + (u32)x * T;
+        if (j >= M) continue;
+        sm[at[x]] = (u32)(A.pbound - (u64)ps[x]);
+        sm[RSS_CAP + at[x]] = nd[x];
+        if (A.pb > 32) A.psn[nd[x]] = ps[x];
+    }
+    __syncthreads();
+    copy_sort64(sm, M, A.pb, ko, vo, [&](u32 v) { return (u32)((A.pbound - (u64)A.psn[v]) >> 32); });
+    for (u32 i = threadIdx.x; i < M; i += T) {
+        const u32 v = vo[i];
+        A.mv[v0 + i] = v;
+        A.state[v].x = i;
+    }
+    if (threadIdx.x == 0) {
+        A.dM[t] = M;
+        if (t == 0) *A.apply = 0;
+    }
+}
+
+// Size violations of every prefix: one block per partition of every copy runs its size along the
+// copy's movers; vs[r] += excess(after rank r) - excess(before).
+constexpr u32 CV_SIZE_THREADS = 512;
+__global__ void __launch_bounds__(CV_SIZE_THREADS) k_copy_sizes(CopyArgs A) {
+    __shared__ i64 sh[32];
+    const u32 p = blockIdx.x, t = p / A.k, v0 = t * A.cn, M = A.dM[t];
+    i64 run = (i64)A.psize[p];
+    const i64 om = (i64)A.omega;
+    for (u32 b = 0; b < M; b += CV_SIZE_THREADS) {
+        const u32 r = b + threadIdx.x;
+        i64 d = 0;
+        if (r < M) {
+            const u32 v = A.mv[v0 + r];
+            if (A.part[v] == p) d = -(i64)A.nsize[v];
+            else if (A.target[v] == p) d = (i64)A.nsize[v];
+        }
+        if (!__syncthreads_or(d != 0)) continue;
+        i64 tot;
+        const i64 incl = block_incl_scan_i64(d, sh, tot);
+        if (d != 0) {
+            const i64 after = run + incl, before = after - d;
+            const i64 dx = (after > om ? after - om : 0) - (before > om ? before - om : 0);
+            if (dx) atomicAdd((unsigned long long *)&A.vs[v0 + r], (unsigned long long)dx);
+        }
+        run += tot;
+    }
+}
+
+// The best prefix of every copy and its application, one block each; the partition sizes follow.
+__global__ void __launch_bounds__(1024) k_copy_tail(CopyArgs A) {
+    __shared__ i64 sh[32];
+    __shared__ Best bsh[32];
+    __shared__ Best s_best;
+    __shared__ int dlo[KW_K], dhi[KW_K];  // size changes in units of 1 and 2^16: at most RSS_CAP terms each
+    const u32 t = blockIdx.x, v0 = t * A.cn, base = t * A.k, M = A.dM[t];
+    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_best = Best{0, 0, 0, 0xFFFFFFFFu};
+    for (u32 i = threadIdx.x; i < A.k; i += blockDim.x) dlo[i] = dhi[i] = 0;
+    i64 rg = 0, rs = 0;
+    for (u32 b0 = 0; b0 < M; b0 += blockDim.x) {
+        const u32 r = b0 + threadIdx.x;
+        const bool in = r < M;
+        i64 tg, ts;
+        const i64 pg = rg + block_incl_scan_i64(in ? (i64)A.g2[A.mv[v0 + r]] : 0, sh, tg);
+        const i64 ps = rs + block_incl_scan_i64(in ? A.vs[v0 + r] : 0, sh, ts);
+        const Best b = warp_best_prefix(Best{1u, ps, pg, in ? r : 0xFFFFFFFFu});
+        if (lane == 0) bsh[w] = b;
+        __syncthreads();
+        if (w == 0) {
+            const Best x = warp_best_prefix(bsh[lane]);
+            if (lane == 0) s_best = best_pick(s_best, x);
+        }
+        rg += tg;
+        rs += ts;
+    }
+    __syncthreads();
+    const Best x = s_best;
+    const bool ok = x.r != 0xFFFFFFFFu && x.vs <= 0 && x.g >= 0;
+    if (threadIdx.x == 0) {
+        A.applied[t] = ok ? x.r + 1 : 0u;
+        if (ok) *A.apply = 1u;
+    }
+    if (!ok) return;
+    for (u32 i = threadIdx.x; i <= x.r; i += blockDim.x) {
+        const u32 v = A.mv[v0 + i], p = A.part[v] - base, q = A.target[v] - base, s = A.nsize[v];
+        A.part[v] = base + q;
+        atomicAdd(&dlo[p], -(int)(s & 0xFFFFu));
+        atomicAdd(&dlo[q], (int)(s & 0xFFFFu));
+        if (s >> 16) {
+            atomicAdd(&dhi[p], -(int)(s >> 16));
+            atomicAdd(&dhi[q], (int)(s >> 16));
+        }
+    }
+    __syncthreads();
+    for (u32 i = threadIdx.x; i < A.k; i += blockDim.x)
+        A.psize[base + i] = (u64)((i64)A.psize[base + i] + (i64)dlo[i] + ((i64)dhi[i] << 16));
+}
+
 GainArgs make_gain_args(const DLevel &L, const u32 *wfx, const RefineParams &rp, const Census &cs, const u32 *part,
                         const u64 *psize, const u64 *pinb, u32 discount, u32 round, u32 *target, i64 *gain,
                         u32 *status) {
@@ -2845,6 +3419,7 @@ void setup_refine_kernels(Ctx &c) {
                                   (int)cudaSharedmemCarveoutMaxShared));
     AXC_CUDA(cudaFuncSetAttribute(k_cands_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CV_BLOCK_SMEM));
     AXC_CUDA(cudaFuncSetAttribute(k_rank_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
+    AXC_CUDA(cudaFuncSetAttribute(k_copy_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
 }
 
 __global__ void k_level_bounds(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ nsrc,
@@ -2852,7 +3427,7 @@ __global__ void k_level_bounds(u32 e, const u64 *__restrict__ off, const u32 *__
 
 // Largest gain-work bound over all nodes (out[0]) and over the block tier (out[1]); the largest
 // degree (out[2]).
-__global__ void k_tier_max(u32 n, u32 K, const u64 *__restrict__ work, const u64 *__restrict__ toff,
+__global__ void k_tier_max(u32 n, u32 K, const u64 *__restrict__ work, const u64 *__restrict__ toff, u32 kway,
                            unsigned long long *__restrict__ out) {
     u32 u = blockIdx.x * blockDim.x + threadIdx.x;
     u64 all = 0, blk = 0, deg = 0;
@@ -2860,7 +3435,7 @@ __global__ void k_tier_max(u32 n, u32 K, const u64 *__restrict__ work, const u64
         const u64 wk = work[u];
         deg = toff[u + 1] - toff[u];
         all = wk;
-        if (gain_tier(n, K, wk, deg) == 1u) blk = wk;
+        if (gain_tier(n, K, wk, deg, kway) == 1u) blk = wk;
     }
     all = warp_max_u64(all);
     blk = warp_max_u64(blk);
@@ -2874,7 +3449,8 @@ __global__ void k_tier_max(u32 n, u32 K, const u64 *__restrict__ work, const u64
 
 // Everything the level's rounds need sized on the host comes back in one round trip (a second
 // one only when some hyperedge is longer than CS_BLOCK_CAP).
-static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K) {
+// kway: the level's rounds take the k-way records (no census lists; two gain tiers, by degree).
+static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, bool kway = false) {
     LevelPrep lp;
     const u32 e = L.e, n = L.n;
     // [0] census block list, [1] census huge list, [2..4] node tiers, [5] gain bound,
@@ -2882,7 +3458,7 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K) {
     // [10] destination pins, [11] pins of short hyperedges, [12] the sum of their squared lengths
     u64 *dc = c.arena.alloc<u64>(13);
     AXC_CUDA(cudaMemsetAsync(dc, 0, 104, c.stream));
-    lp.census_K = K <= CD_K ? K : 0;
+    lp.census_K = K <= CD_K || kway ? K : 0;
     if (e) {
         u32 *flag = c.arena.alloc<u32>(e);
         lp.hblock = c.arena.alloc<u32>(e);
@@ -2904,12 +3480,13 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K) {
         LAUNCH(c, k_gain_bounds, cdiv((u64)n * 32, 256), 256, 0, n, K, L.toff, L.touch, L.off, wfx, work,
                (unsigned long long *)(dc + 5));
         u32 *flag = c.arena.alloc<u32>(n);
-        for (u32 t = 0; t < 3; ++t) {
+        for (u32 t = 0; t < (kway ? 2u : 3u); ++t) {
             lp.ntier[t] = c.arena.alloc<u32>(n);
-            LAUNCH(c, k_tier, cdiv(n, 256), 256, 0, n, K, work, L.toff, t, flag);
+            LAUNCH(c, k_tier, cdiv(n, 256), 256, 0, n, K, work, L.toff, t, kway ? 1u : 0u, flag);
             compact_indices_dn(c, flag, lp.ntier[t], n, (u32 *)(dc + 2 + t));
         }
-        LAUNCH(c, k_tier_max, cdiv(n, 256), 256, 0, n, K, work, L.toff, (unsigned long long *)(dc + 6));
+        LAUNCH(c, k_tier_max, cdiv(n, 256), 256, 0, n, K, work, L.toff, kway ? 1u : 0u,
+               (unsigned long long *)(dc + 6));
     }
     u64 h[13];
     fetch(c, h, dc, 104);
@@ -3082,6 +3659,14 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
     }
 }
 
+__global__ void k_copy_conn(u64 eS, u32 e2, const u32 *__restrict__ lam, const u32 *__restrict__ wfxS,
+                            unsigned long long *__restrict__ conn) {
+    const u64 h = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (h >= eS) return;
+    const u32 l = lam[h];
+    if (l > 1) atomicAdd(&conn[h / e2], (unsigned long long)wfxS[h] * (l - 1));
+}
+
 Census build_census(Ctx &c, const DLevel &L, const u32 *part) {
     Census cs = alloc_census(c, L);
     size_t m = c.arena.mark();
@@ -3251,25 +3836,124 @@ static void run_cascade_movers(Ctx &c, const CascadeArgs &C, const MoverArgs &V,
     else run_cascade_movers_g<32, TRACK>(c, C, V, n, max_deg);
 }
 
+// The records of a level's k-way rounds (k_kway_*), kept across them.
+struct KwayLevel {
+    u32 k = 0, mw = 0, cn = 0, ce = 0;  // partitions, mask words, nodes and hyperedges of one copy
+    u32 *rec = nullptr;                 // [e * 2 * mw]
+    uint8_t *dirty = nullptr;           // [e]
+    bool slots = false;                 // copies ranked by one block each (k_copy_*)
+    u64 *psize = nullptr;               // [K] with slots: kept by k_copy_tail
+};
+
+// K-way rounds without an inbound limit whose copies hold at most KW_K partitions.
+static bool kway_eligible(const DLevel &L, const RefineParams &rp) {
+    return !rp.encourage && !inbound_binds(L, rp) && L.e && rp.K / rp.copies <= KW_K;
+}
+
+static void kway_init(Ctx &c, const DLevel &L, const RefineParams &rp, const u32 *part, KwayLevel &kw) {
+    kw.k = rp.K / rp.copies;
+    kw.mw = mask_words(kw.k);
+    kw.cn = L.n / rp.copies;
+    kw.ce = L.e / rp.copies;
+    kw.slots = kw.cn <= (u32)RSS_CAP;
+    kw.rec = c.arena.alloc<u32>((u64)L.e * 2 * kw.mw);
+    kw.dirty = c.arena.alloc<uint8_t>(L.e);
+    AXC_CUDA(cudaMemsetAsync(kw.dirty, 1, L.e, c.stream));
+    if (kw.slots) {
+        kw.psize = c.arena.alloc<u64>(rp.K);
+        part_sizes(c, L.n, part, L.nsize, kw.psize, rp.K);
+    }
+}
+
+static KwArgs kway_args(const DLevel &L, const u32 *part, const KwayLevel &kw) {
+    // a lane per hyperedge where most have few pins; fewer per warp where the warp reads each
+    const u64 len = L.P / L.e;
+    return KwArgs{L.off, L.pins, part, L.e, kw.ce, kw.k, kw.rec, kw.dirty, len <= 2 * KW_SHORT ? 32u : len <= 64 ? 8u : 2u};
+}
+
+// Runs f(MW) for the level's mask words.
+template <class F>
+static void kway_words(u32 mw, F &&f) {
+    switch (mw) {
+        case 1: f(std::integral_constant<u32, 1>()); break;
+        case 2: f(std::integral_constant<u32, 2>()); break;
+        case 4: f(std::integral_constant<u32, 4>()); break;
+        default: f(std::integral_constant<u32, 8>()); break;
+    }
+}
+
+static void kway_records(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *part, const KwayLevel &kw) {
+    const KwArgs A = kway_args(L, part, kw);
+    kway_words(kw.mw, [&](auto mw) {
+        constexpr u32 MW = decltype(mw)::value;
+        LAUNCH_AS(c, "k_kway_records", k_kway_records<MW>, cdiv(L.e, (KW_THREADS / 32) * A.per_warp), KW_THREADS, 0, A);
+        if (lp.n_hblock)
+            LAUNCH_AS(c, "k_kway_records_block", k_kway_records_block<MW>, lp.n_hblock, KW_THREADS, 0, A, lp.hblock,
+                      lp.n_hblock);
+    });
+}
+
+// Gains from the records. Light nodes: a group of lanes per node, at least one lane per partition
+// up to 32 (at most 4 partitions: lanes side by side over the incidences, as many as the mean
+// degree fills); heavy nodes and small levels: a block per node.
+template <class T>
+static void kway_gains_t(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainArgs &A, const KwayLevel &kw) {
+    KwGain V{kw.rec, kw.k, kw.cn, lp.ntier[0], lp.ncount[0]};
+    const auto grid = [&](u32 G) { return cdiv((u64)lp.ncount[0] * G, KW_THREADS); };
+    if (lp.ncount[0] && kw.k <= 4) {
+        const u64 deg = L.P / L.n;
+        if (deg < 8) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain_few<4, T>), grid(4), KW_THREADS, 0, A, V);
+        else if (deg < 24) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain_few<8, T>), grid(8), KW_THREADS, 0, A, V);
+        else if (deg < 64) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain_few<16, T>), grid(16), KW_THREADS, 0, A, V);
+        else LAUNCH_AS(c, "k_kway_gain", (k_kway_gain_few<32, T>), grid(32), KW_THREADS, 0, A, V);
+    } else if (lp.ncount[0]) {
+        if (kw.k <= 8) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain<1, 8, T>), grid(8), KW_THREADS, 0, A, V);
+        else if (kw.k <= 16) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain<1, 16, T>), grid(16), KW_THREADS, 0, A, V);
+        else if (kw.k <= 32) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain<1, 32, T>), grid(32), KW_THREADS, 0, A, V);
+        else if (kw.k <= 64) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain<2, 32, T>), grid(32), KW_THREADS, 0, A, V);
+        else if (kw.k <= 128) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain<4, 32, T>), grid(32), KW_THREADS, 0, A, V);
+        else LAUNCH_AS(c, "k_kway_gain", (k_kway_gain<8, 32, T>), grid(32), KW_THREADS, 0, A, V);
+    }
+    if (lp.ncount[1]) {
+        V.list = lp.ntier[1];
+        V.nl = lp.ncount[1];
+        kway_words(kw.mw, [&](auto mw) {
+            LAUNCH_AS(c, "k_kway_gain_block", (k_kway_gain_block<decltype(mw)::value, T>), lp.ncount[1], KW_THREADS, 0, A,
+                      V);
+        });
+    }
+}
+static void kway_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainArgs &A, const KwayLevel &kw) {
+    if (c.profiling("k_kway_gain")) c.prof_bytes += gain_bytes(lp, 0);
+    if (c.profiling("k_kway_gain_block")) c.prof_bytes += gain_bytes(lp, 1);
+    if (lp.gain_bound < (1ull << 32)) kway_gains_t<u32>(c, L, lp, A, kw);
+    else kway_gains_t<unsigned long long>(c, L, lp, A, kw);
+}
+
 // The launches of one round, with no host synchronization: safe to capture in a CUDA graph.
 // dyn (device, optional) holds the round's discount and round number for graph replays. Returns
 // the device word that says whether the moves were applied; its arena slot lies below `keep`,
 // the mark the caller releases to after reading it.
 static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *wfx, const RefineParams &rp,
-                       u32 *part, u32 discount, u32 round, const u32 *dyn, size_t &keep, IncCensus *ic) {
+                       u32 *part, u32 discount, u32 round, const u32 *dyn, size_t &keep, IncCensus *ic,
+                       const KwayLevel *kw) {
     const u32 n = L.n;
+    const bool slots = kw && kw->slots;
     u32 *apply = c.arena.alloc<u32>(1);
     keep = c.arena.mark();
     Census cs;
-    if (ic) {
+    if (kw) {
+        kway_records(c, L, lp, part, *kw);
+    } else if (ic) {
         inc_census_round(c, L, lp, part, *ic);
         cs = ic->cs;
     } else {
         cs = census_for_gains(c, L, lp, wfx, rp, part);
     }
-    u64 *psize = c.arena.alloc<u64>(rp.K), *pinb = c.arena.alloc<u64>(rp.K);
-    part_sizes(c, n, part, L.nsize, psize, rp.K);
-    if (inbound_binds(L, rp)) {
+    u64 *psize = slots ? kw->psize : c.arena.alloc<u64>(rp.K), *pinb = kw ? nullptr : c.arena.alloc<u64>(rp.K);
+    if (!slots) part_sizes(c, n, part, L.nsize, psize, rp.K);
+    if (kw) {  // no inbound limit, and gains that read no inbound counts
+    } else if (inbound_binds(L, rp)) {
         part_inbound(c, L, cs, pinb, rp.K);
     } else {
         AXC_CUDA(cudaMemsetAsync(pinb, 0, (size_t)rp.K * 8, c.stream));
@@ -3278,7 +3962,8 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     i64 *gain = c.arena.alloc<i64>(n);
     GainArgs A = make_gain_args(L, wfx, rp, cs, part, psize, pinb, discount, round, target, gain, c.d_status);
     A.dyn = dyn;
-    run_gains(c, L, lp, A, cs);
+    if (kw) kway_gains(c, L, lp, A, *kw);
+    else run_gains(c, L, lp, A, cs);
     // counters on the device: [0] M movers, [1] 2M size events, [2] inbound transitions,
     // [3] cascade hyperedges for the block kernel, [4] for the scratch kernel, [5] for the block
     // kernel's full-size launch after its middle tier, [6] hyperedges holding a mover
@@ -3287,14 +3972,23 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     u32 *dM = cnt, *dSE = cnt + 1, *dT = cnt + 2, *dBig = cnt + 3, *dHuge = cnt + 4, *dBig2 = cnt + 5;
     u32 *dHl = cnt + 6;  // hyperedges holding a mover
     // small levels: ranking, validity and the best prefix in one block each (SMALL_*)
-    const bool small = rp.K <= VS_MAX_K && n <= (u32)RSS_CAP && rp.copies == 1;
+    const bool small = !slots && rp.K <= VS_MAX_K && n <= (u32)RSS_CAP && rp.copies == 1;
+    CopyArgs ca{};
     // movers in id order, then ranked by (gain desc, id asc)
     u32 *flag = c.arena.alloc<u32>(n), *mv = c.arena.alloc<u32>(n);
     uint2 *state = (uint2 *)c.arena.alloc<u64>(n);
     unsigned long long *g2 = c.arena.alloc<unsigned long long>(n);  // cascaded gains, zeroed here
     const u32 kb = bits_for(lp.gain_bound);
     u32 *khi = flag, *klo = c.arena.alloc<u32>(n);  // the flags are spent when the keys are made
-    if (small) {
+    if (slots) {
+        const u64 pbound = 2 * lp.gain_bound;
+        u32 *dMc = c.arena.alloc<u32>(2 * (u64)rp.copies);
+        ca = CopyArgs{kw->cn, kw->k, n, target, L.nsize, gain, part, lp.gain_bound, pbound, kb, bits_for(pbound),
+                      bits_for(2 * (u64)kw->k * kw->k), mv, dMc, state, g2, c.arena.alloc<i64>(n),
+                      c.arena.alloc<i64>(n), psize, dMc + rp.copies, apply, rp.omega};
+        dM = dMc;
+        LAUNCH(c, k_copy_rank, rp.copies, RSS_WARPS * 32, RSS_SMEM, ca);
+    } else if (small) {
         LAUNCH(c, k_rank_small, 1, RSS_WARPS * 32, RSS_SMEM, n, target, gain, lp.gain_bound, kb, part, mv, state,
                g2, dM, dSE);
     } else {
@@ -3312,7 +4006,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         radix_sort_pairs_dn(c, klo, mv, dM, n, kb);
     }
     }
-    const bool pairs = !rp.encourage && rp.K <= PAIR_RANK_MAX_K;
+    const bool pairs = !slots && !rp.encourage && rp.K <= PAIR_RANK_MAX_K;
     if (pairs) {  // k-way: moves in p <-> q pairs
         u32 *gk = khi, *pos = klo;  // the gain keys are spent
         LAUNCH(c, k_pair_group, cdiv(n, 256), 256, 0, mv, dM, part, target, rp.K, gk, pos);
@@ -3332,12 +4026,12 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         AXC_CUDA(cudaMemcpyAsync(mv, node, (size_t)n * 4, cudaMemcpyDeviceToDevice, c.stream));
     }
     u32 *ck = nullptr;  // copies: the copy of every rank, ascending
-    if (rp.copies > 1) {
+    if (rp.copies > 1 && !slots) {
         ck = c.arena.alloc<u32>(n);
         LAUNCH(c, k_copy_keys, cdiv(n, 256), 256, 0, mv, dM, rp.copy_n, ck);
         radix_sort_pairs_dn(c, ck, mv, dM, n, bits_for(rp.copies - 1));
     }
-    if (!small || pairs || rp.copies > 1) LAUNCH(c, k_set_rank, cdiv(n, 256), 256, 0, mv, dM, state, dSE);
+    if (!slots && (!small || pairs || rp.copies > 1)) LAUNCH(c, k_set_rank, cdiv(n, 256), 256, 0, mv, dM, state, dSE);
     // cascade
 
     // inbound-set transitions (INCC): each destination pin of a mover gives at most two
@@ -3364,7 +4058,9 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         C.track = track ? 1 : 0; C.tp = tp; C.tr = tr; C.tdv = tdv; C.dT = dT; C.tcap = tcap;
         C.tdense = tdense; C.dense_stride = n;
         C.status = c.d_status;
-        C.K = rp.K;
+        C.K = kw ? kw->k : rp.K;
+        C.ce = kw ? kw->ce : 0;
+        C.cn = slots ? kw->cn : 0;
         C.pbytes = c.profiling("k_cascade_warp") ? c.d_prof_bytes() : nullptr;
         const bool direct = C.K <= CC_DIRECT_K;
         size_t m1 = c.arena.mark();
@@ -3375,7 +4071,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         // few nodes of many short incidences: a lane of the mover kernel would walk through several
         // of them one after the other while the dense kernel reads the whole level in a few microseconds
         const bool always = L.P / n > 128 && lp.short_pins <= (2u << 20);
-        const MoverArgs V{mv, dM, L.toff, L.touch, L.nin, longs ? 1 : 0, rp.K <= CD_MAX_K ? 1 : 0, n, 1u,
+        const MoverArgs V{mv, dM, L.toff, L.touch, L.nin, longs ? 1 : 0, rp.K <= CD_MAX_K ? 1 : 0, n, C.cn ? rp.copies : 1u,
                           always ? 1ull << 40 : lp.short_pins ? 16 * lp.short_sq / lp.short_pins : 0, per_warp};
         if (lp.short_pins && track) run_cascade_movers<true>(c, C, V, n, L.P, lp.max_deg);
         else if (lp.short_pins) run_cascade_movers<false>(c, C, V, n, L.P, lp.max_deg);
@@ -3384,7 +4080,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
             // only the long hyperedges that hold a mover: flagged from the movers' incidences
             u32 *hflag = c.arena.alloc<u32>(L.e), *hlist = c.arena.alloc<u32>(L.e);
             AXC_CUDA(cudaMemsetAsync(hflag, 0, (size_t)L.e * 4, c.stream));
-            LAUNCH(c, k_mover_hedges, (u32)c.sms * 8, 256, 0, mv, dM, L.toff, L.touch, L.off, hflag);
+            LAUNCH(c, k_mover_hedges, (u32)c.sms * 8, 256, 0, mv, dM, L.toff, L.touch, L.off, C.cn, n, hflag);
             compact_indices_dn(c, hflag, hlist, L.e, dHl);
             int per_w = 1;
             AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_w, k_cascade_warp, CC_WARPS * 32, 0));
@@ -3429,6 +4125,13 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
             }
         }
         c.arena.release(m1);
+    }
+    if (slots) {  // every copy's prefixes, application and partition sizes
+        LAUNCH(c, k_copy_sizes, rp.K, CV_SIZE_THREADS, 0, ca);
+        LAUNCH(c, k_copy_tail, rp.copies, 1024, 0, ca);
+        LAUNCH(c, k_kway_mark, (u32)c.sms * 8, 256, 0, mv, kw->cn, rp.copies, ca.applied, L.toff, L.touch, kw->dirty);
+        c.arena.release(keep);
+        return apply;
     }
     // prefix gains in rank order
     // per-rank deltas of the cascaded gain, the size violations and the inbound violations, in
@@ -3492,6 +4195,8 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         LAUNCH(c, k_best_seg, rp.copies, 256, 0, pre, n, track ? 1 : 0, dM, ck, bs, capply, apply);
         LAUNCH(c, k_apply_seg, cdiv(n, 256), 256, 0, mv, dM, ck, target, bs, capply, part, ic ? ic->prev : nullptr,
                ic ? ic->stamp : nullptr, ic ? (const u32 *)ic->ctr : nullptr);
+        if (kw)
+            LAUNCH(c, k_kway_mark_ranked, (u32)c.sms * 8, 256, 0, mv, dM, ck, bs, capply, L.toff, L.touch, kw->dirty);
     } else {
         const u32 nbk = cdiv(n, 256) < 64u ? cdiv(n, 256) : 64u;
         Best *bb = (Best *)c.arena.alloc<u64>(4 * (nbk + 1));
@@ -3499,6 +4204,9 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         LAUNCH(c, k_best_final, 1, 1, 0, bb + 1, nbk, pre, n, track ? 1 : 0, bb, apply);
         LAUNCH(c, k_apply, cdiv(n, 256), 256, 0, mv, target, bb, apply, part, ic ? ic->prev : nullptr,
                ic ? ic->stamp : nullptr, ic ? (const u32 *)ic->ctr : nullptr);
+        if (kw)
+            LAUNCH(c, k_kway_mark_ranked, (u32)c.sms * 8, 256, 0, mv, dM, (const u32 *)nullptr, bb, apply, L.toff,
+                   L.touch, kw->dirty);
     }
     if (ic) {  // flag the moved nodes' hyperedges for the next census, then count the round
         LAUNCH(c, k_mark_moved, (u32)c.sms * 8, 256, 0, mv, dM, ic->stamp, ic->ctr, L.toff, L.touch, ic->dirty);
@@ -3524,10 +4232,10 @@ static bool round_result(Ctx &c, const u32 *apply) {
 
 // One round, launched eagerly; returns true when moves were applied.
 static bool refine_round(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *wfx, const RefineParams &rp,
-                         u32 *part, u32 discount, u32 round, IncCensus *ic) {
+                         u32 *part, u32 discount, u32 round, IncCensus *ic, const KwayLevel *kw) {
     const size_t m0 = c.arena.mark();
     size_t keep;
-    const u32 *apply = round_body(c, L, lp, wfx, rp, part, discount, round, nullptr, keep, ic);
+    const u32 *apply = round_body(c, L, lp, wfx, rp, part, discount, round, nullptr, keep, ic, kw);
     const bool r = round_result(c, apply);
     c.arena.release(m0);
     return r;
@@ -3608,7 +4316,7 @@ __global__ void k_level_bounds(u32 e, const u64 *__restrict__ off, const u32 *__
 // (round_body) followed by k_round_next, which applies the round schedule on the device. Returns
 // the rounds run.
 static u32 refine_level_loop(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *wfx, const RefineParams &rp,
-                             u32 *part, IncCensus *ic) {
+                             u32 *part, IncCensus *ic, const KwayLevel *kw) {
     const u32 R = rp.rounds;
     u32 *dyn = c.arena.alloc<u32>(2), *rs = c.arena.alloc<u32>(4);
     {
@@ -3641,7 +4349,7 @@ static u32 refine_level_loop(Ctx &c, const DLevel &L, const LevelPrep &lp, const
     AXC_CUDA(cudaStreamBeginCaptureToGraph(c.stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     c.capturing = true;
     try {
-        apply = round_body(c, L, lp, wfx, rp, part, 1, 0, dyn, keep, ic);
+        apply = round_body(c, L, lp, wfx, rp, part, 1, 0, dyn, keep, ic, kw);
         LAUNCH(c, k_round_next, 1, 1, 0, h, rs, dyn, apply, c.d_status);
     } catch (...) {
         c.capturing = false;
@@ -3670,17 +4378,9 @@ static u32 refine_level_loop(Ctx &c, const DLevel &L, const LevelPrep &lp, const
     return done;
 }
 
-u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp, u32 *part) {
+static u32 refine_rounds(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *wfx, const RefineParams &rp, u32 *part,
+                         IncCensus *ic, const KwayLevel *kw) {
     const u32 R = rp.rounds;
-    if (R == 0 || L.n == 0) return 0;
-    size_t m = c.arena.mark();
-    LevelPrep lp = prepare_level(c, L, wfx, rp.K);
-    // one census kept across the rounds where the level allows it (k_census_inc_*)
-    IncCensus icv, *ic = nullptr;
-    if (inc_census_eligible(L, lp, rp) && inc_census_enabled()) {
-        inc_census_init(c, L, wfx, rp, icv);
-        ic = &icv;
-    }
     // Graph replays need the round's scalars in device memory. Kernel-timer pairs captured in the
     // graph are read back after every replay; the bytes of the captured launches count per replay.
     const bool graph = R > 1;
@@ -3690,9 +4390,7 @@ u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp
     // variable AXC_ROUND_LOOP=0 also selects the replays (the same kernels and results; profilers
     // that do not follow kernels into conditional graph nodes see them then).
     if (graph && !c.prof_on && round_loop_enabled()) {
-        const u32 done = refine_level_loop(c, L, lp, wfx, rp, part, ic);
-        c.arena.release(m);
-        return done;
+        return refine_level_loop(c, L, lp, wfx, rp, part, ic, kw);
     }
     size_t ev0 = 0, ev1 = 0;
     u64 bytes_per_round = 0;
@@ -3708,7 +4406,7 @@ u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp
         AXC_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
         c.capturing = true;
         try {
-            apply = round_body(c, L, lp, wfx, rp, part, 1, 0, dyn, keep, ic);
+            apply = round_body(c, L, lp, wfx, rp, part, 1, 0, dyn, keep, ic, kw);
         } catch (...) {
             c.capturing = false;
             cudaGraph_t junk = nullptr;
@@ -3743,7 +4441,7 @@ u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp
             c.prof_collect(ev0, ev1);
             c.prof_bytes += bytes_per_round;
         } else {
-            applied = refine_round(c, L, lp, wfx, rp, part, discount, r, ic);
+            applied = refine_round(c, L, lp, wfx, rp, part, discount, r, ic, kw);
         }
         if (!applied) {
             if (r < R / 3) r = R / 2;
@@ -3752,6 +4450,35 @@ u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp
         }
     }
     if (graph) c.prof_used = ev0;  // the captured pairs go back to the pool with the graph
+    return done;
+}
+
+u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp, u32 *part,
+                 unsigned long long *copy_conn) {
+    if (rp.rounds == 0 || L.n == 0) return 0;
+    const size_t m = c.arena.mark();
+    const bool kway = kway_eligible(L, rp);
+    const LevelPrep lp = prepare_level(c, L, wfx, rp.K, kway);
+    // state kept across the rounds: the k-way records, or one census where the level allows it
+    KwayLevel kw;
+    IncCensus ic;
+    const bool inc = !kway && inc_census_eligible(L, lp, rp) && inc_census_enabled();
+    if (kway) kway_init(c, L, rp, part, kw);
+    if (inc) inc_census_init(c, L, wfx, rp, ic);
+    const u32 done = refine_rounds(c, L, lp, wfx, rp, part, inc ? &ic : nullptr, kway ? &kw : nullptr);
+    if (copy_conn && kway) {  // from the records, brought up to date with the last round's moves
+        kway_records(c, L, lp, part, kw);
+        const KwArgs A = kway_args(L, part, kw);
+        const dim3 grid(std::min<u32>(cdiv(kw.ce, KW_THREADS), std::max(1u, (u32)c.sms * 8 / rp.copies)), rp.copies);
+        kway_words(kw.mw, [&](auto mw) {
+            k_kway_conn<decltype(mw)::value><<<grid, KW_THREADS, 0, c.stream>>>(A, wfx, copy_conn);
+            c.launches++;
+            AXC_CUDA(cudaGetLastError());
+        });
+    } else if (copy_conn) {
+        const Census cs = build_census(c, L, part);
+        LAUNCH(c, k_copy_conn, cdiv((u64)L.e, 256), 256, 0, (u64)L.e, L.e / rp.copies, cs.lam, wfx, copy_conn);
+    }
     c.arena.release(m);
     return done;
 }
