@@ -474,21 +474,14 @@ struct GainArgs {
     u32 *status;
     const u32 *dyn;  // when set: discount and round read from device memory (graph replays)
     const i64 *save; // partition-indexed gains: each node's saving from leaving its partition
-    u32 K;           // partitions: with K <= GN_DIRECT_K the tables are indexed by partition id
+    u32 K;           // partitions
 };
 
 constexpr u32 GN_DIRECT_K = 256;
 
-// Slots of a node's table: K (rounded up) when indexed by partition id, else from its work bound.
-// Rounds with K <= GN_DIRECT_K take the mask kernels (k_gain_mask_*); the partition-indexed
-// branches of the table kernels below are kept so that those kernels stay correct for any K.
-__device__ __forceinline__ bool gain_direct(const GainArgs &A) { return A.K <= GN_DIRECT_K; }
-__device__ __forceinline__ u32 gain_cap(const GainArgs &A, u64 work, u32 cap_max) {
+// Slots of a node's hash table from its work bound.
+__device__ __forceinline__ u32 gain_cap(u64 work, u32 cap_max) {
     u32 cap = 32;
-    if (gain_direct(A)) {
-        while (cap < A.K) cap <<= 1;
-        return cap;
-    }
     while (cap < 2 * work && cap < cap_max) cap <<= 1;
     return cap;
 }
@@ -536,25 +529,12 @@ __host__ __device__ __forceinline__ u32 table_cap(u64 work, u32 cap_max) {
 // `stride` entries. A batch's hyperedge metadata loads in parallel; its census entries are then
 // flattened across the lanes (each lane finds its entry's hyperedge by a 5-step search over the
 // prefix of the batch's lambdas). saving and wtot are per-lane partial sums.
-//
-// With `trk` the block counts the distinct partitions it inserts. In a first try (limit below the
-// table size) passing the limit, or a full table, sets *ovf and the warps stop at their next batch;
-// the caller retries the node with a larger table. With trk->used the inserted slots are listed,
-// so the caller can scan and clear only those.
-struct GainTrack {
-    u32 *ndist;
-    u32 limit;
-    volatile u32 *ovf;
-    u32 *used;
-};
 __device__ __forceinline__ void gain_flat(const GainArgs &A, u32 u, u32 p, u32 *keys, unsigned long long *conn,
-                                          u32 *dconn, u32 mask, u32 first, u32 stride, i64 &saving, i64 &wtot,
-                                          const GainTrack *trk = nullptr) {
+                                          u32 *dconn, u32 mask, u32 first, u32 stride, i64 &saving, i64 &wtot) {
     const u32 lane = threadIdx.x & 31u;
     const u64 t0 = A.toff[u];
     const u32 deg = (u32)(A.toff[u + 1] - t0), nin_u = A.nin[u];
     for (u32 jb = first; jb < deg; jb += stride) {
-        if (trk && __any_sync(0xFFFFFFFFu, *trk->ovf != 0)) return;
         const u32 j = jb + lane;
         const bool has = j < deg;
         const u32 h = has ? A.touch[t0 + j] : 0;
@@ -590,27 +570,8 @@ __device__ __forceinline__ void gain_flat(const GainArgs &A, u32 u, u32 p, u32 *
                 saving += leave_gain(A.encourage, wo, A.ccnt[k]);
                 continue;
             }
-            u32 slot;
-            if (gain_direct(A)) {  // the slot is the partition id: no probing
-                slot = q;
-                keys[q] = q;
-            } else if (trk) {
-                bool fresh;
-                slot = hash_insert_fresh(keys, mask, q, fresh);
-                if (slot == NONE) {  // full: a first try overflows, a sized table is an error
-                    if (trk->limit <= mask) *trk->ovf = 1u;
-                    else atomicExch(A.status, DEV_HASH_FULL);
-                    continue;
-                }
-                if (fresh) {
-                    const u32 idx = atomicAdd(trk->ndist, 1u);
-                    if (trk->used) trk->used[idx] = slot;
-                    if (idx >= trk->limit) *trk->ovf = 1u;
-                }
-            } else {
-                slot = hash_find_or_insert(keys, mask, q);
-                if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); continue; }
-            }
+            const u32 slot = hash_find_or_insert(keys, mask, q);
+            if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); continue; }
             atomicAdd(&conn[slot], (unsigned long long)wo);
             if (io && A.cdcnt[k] > 0) atomicAdd(&dconn[slot], 1u);
         }
@@ -883,7 +844,7 @@ __global__ void __launch_bounds__(GN_WARPS * 32) k_gain_warp(GainArgs A0, const 
     const u32 u = list[idx], p = A.part[u];
     u32 *keys = tk[w], *dconn = td[w];
     unsigned long long *conn = tcw[w];
-    const u32 cap = gain_cap(A, work[u], 2 * GN_WARP_W);
+    const u32 cap = gain_cap(work[u], 2 * GN_WARP_W);
     for (u32 i = lane; i < cap; i += 32) { keys[i] = NONE; dconn[i] = 0; conn[i] = 0; }
     __syncwarp();
     i64 saving = 0, wtot = 0;
@@ -909,83 +870,35 @@ __global__ void __launch_bounds__(GN_WARPS * 32) k_gain_warp(GainArgs A0, const 
     }
 }
 
-// One block per node. Three table modes:
-// - shared, sized (gtab null, try_limit 0): the node's table bound fits in shared memory;
-// - shared, first try (try_limit > 0): a cap_max-slot shared table for nodes whose bound does not
-//   fit; a node with more than try_limit distinct partitions is appended to retry / *nretry;
-// - global (gtab set): this block's slice of gtab, sized by the bound. Inserted slots are listed
-//   in this block's slice of gused, so candidates are read from and cleared in those slots only;
-//   the slice is cleared once at the start.
-// With dnl set, the node count is read from device memory.
-__global__ void __launch_bounds__(GN_BLOCK) k_gain_block(GainArgs A0, const u32 *__restrict__ list, u32 nl,
-                                                        const u32 *__restrict__ dnl, u32 cap_max, u32 *gtab,
-                                                        u32 *gused, const u64 *__restrict__ work, u32 try_limit,
-                                                        u32 *__restrict__ retry, u32 *__restrict__ nretry) {
+// One block per node, for nodes of the block tier when K > GS_K: a shared table sized by the node's
+// bound.
+__global__ void __launch_bounds__(GN_BLOCK) k_gain_block(GainArgs A0, const u32 *__restrict__ list, u32 nl, u32 cap_max,
+                                                        const u64 *__restrict__ work) {
     const GainArgs A = gain_args_now(A0);
     extern __shared__ unsigned long long dyn64[];
     __shared__ i64 red[2][32];
     __shared__ Cand cred[32];
-    __shared__ u32 ndist, ovf;
-    if (dnl) nl = *dnl;
-    // this block's global slice: conn u64 [cap_max], keys and dconn u32 [cap_max]; a node uses
-    // the first `cap` slots of each, and leaves every slot empty again when it is done
-    u32 *gbase = gtab ? gtab + (u64)blockIdx.x * 4 * cap_max : nullptr;
-    u32 *used = gtab ? gused + (u64)blockIdx.x * cap_max : nullptr;
-    if (gtab && blockIdx.x < nl) {
-        for (u32 i = threadIdx.x; i < 2 * cap_max; i += blockDim.x) gbase[i] = 0;
-        for (u32 i = threadIdx.x; i < cap_max; i += blockDim.x) { gbase[2 * cap_max + i] = NONE; gbase[3 * cap_max + i] = 0; }
-    }
     for (u32 idx = blockIdx.x; idx < nl; idx += gridDim.x) {
         const u32 u = list[idx], p = A.part[u];
-        unsigned long long *conn;
-        u32 *keys, *dconn;
-        const u32 cap = try_limit ? cap_max : gain_cap(A, work[u], cap_max);
-        if (gtab) {
-            conn = (unsigned long long *)gbase;
-            keys = gbase + 2 * cap_max;
-            dconn = keys + cap_max;
-        } else {
-            conn = dyn64;
-            keys = (u32 *)(dyn64 + cap);
-            dconn = keys + cap;
-            for (u32 i = threadIdx.x; i < cap; i += blockDim.x) { keys[i] = NONE; dconn[i] = 0; conn[i] = 0; }
-        }
-        if (threadIdx.x == 0) { ndist = 0; ovf = 0; }
+        const u32 cap = gain_cap(work[u], cap_max);
+        unsigned long long *conn = dyn64;
+        u32 *keys = (u32 *)(dyn64 + cap), *dconn = keys + cap;
+        for (u32 i = threadIdx.x; i < cap; i += blockDim.x) { keys[i] = NONE; dconn[i] = 0; conn[i] = 0; }
         __syncthreads();
-        const bool track = (try_limit || gtab) && !gain_direct(A);
-        const GainTrack trk{&ndist, try_limit ? try_limit : cap, &ovf, used};
         i64 saving = 0, wtot = 0;
-        gain_flat(A, u, p, keys, conn, dconn, cap - 1, 32 * (threadIdx.x >> 5), blockDim.x, saving, wtot,
-                  track ? &trk : nullptr);
+        gain_flat(A, u, p, keys, conn, dconn, cap - 1, 32 * (threadIdx.x >> 5), blockDim.x, saving, wtot);
         saving = warp_sum(saving);
         wtot = warp_sum(wtot);
         if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = saving; red[1][threadIdx.x >> 5] = wtot; }
         __syncthreads();
-        if (ovf) {  // first try overflowed: the global tier takes the node
-            if (threadIdx.x == 0) retry[atomicAdd(nretry, 1u)] = u;
-            __syncthreads();
-            continue;
-        }
         saving = 0;
         wtot = 0;
         for (u32 i = 0; i < blockDim.x / 32; ++i) { saving += red[0][i]; wtot += red[1][i]; }
         Cand best{INT64_MIN, 0};
-        const bool listed = track && used;
-        const u32 nscan = listed ? ndist : cap;
-        for (u32 t = threadIdx.x; t < nscan; t += blockDim.x) {
-            const u32 i = listed ? used[t] : t;
+        for (u32 i = threadIdx.x; i < cap; i += blockDim.x) {
             if (keys[i] == NONE) continue;
-            Cand c = gain_candidate(A, u, keys[i], conn[i], dconn[i], saving, wtot);
+            const Cand c = gain_candidate(A, u, keys[i], conn[i], dconn[i], saving, wtot);
             if (cand_better(c, best)) best = c;
-        }
-        if (gtab) {
-            __syncthreads();  // every candidate is read before the slots are emptied
-            for (u32 t = threadIdx.x; t < nscan; t += blockDim.x) {
-                const u32 i = listed ? used[t] : t;
-                keys[i] = NONE;
-                conn[i] = 0;
-                dconn[i] = 0;
-            }
         }
         best = warp_best(best);
         if ((threadIdx.x & 31) == 0) cred[threadIdx.x >> 5] = best;
@@ -994,13 +907,7 @@ __global__ void __launch_bounds__(GN_BLOCK) k_gain_block(GainArgs A0, const u32 
             Cand b = cred[0];
             for (u32 i = 1; i < blockDim.x / 32; ++i)
                 if (cand_better(cred[i], b)) b = cred[i];
-            if (b.g != INT64_MIN && b.g > 0) {
-                A.target[u] = ~(u32)b.tie;
-                A.gain[u] = b.g;
-            } else {
-                A.target[u] = NONE;
-                A.gain[u] = 0;
-            }
+            write_move(A, u, b);
         }
         __syncthreads();
     }
@@ -1108,6 +1015,211 @@ __device__ __forceinline__ void census_flat(const GainArgs &A, u32 u, u32 first,
             const u32 io = __shfl_sync(0xFFFFFFFFu, ib, lo);
             if (fi < total) f(ao + (fi - eo), A.cpart[ao + (fi - eo)], wo, io);
         }
+    }
+}
+
+// ------------------------------------------------------------------ gains for GN_DIRECT_K < K <= GS_K
+// Nodes beyond a warp's hash table take a block and sums indexed by partition. What bounds them is
+// the census entries of a node's hyperedges (tens of thousands at a spiking network's
+// partitions), so there are two forms, chosen per level by run_gains:
+//  - k_gain_table: one shared add per census entry into K-entry tables. The connectivity is one
+//    u32 where no node's incident weights pass 2^32, else a low and a high word: 64-bit shared
+//    adds would be compare-and-swap loops.
+//  - k_gain_planes: for equal weights and hyperedges of at least as many pins as mask words. A
+//    candidate's connectivity is then a count of incidences whose K-bit mask holds it. A lane owns
+//    one mask word and adds whole words into bit-plane counters (carry-save adders, eight
+//    incidences at a time): 32 partitions per instruction, whatever the number of entries.
+template <bool WIDE>
+__global__ void __launch_bounds__(GN_BLOCK) k_gain_table(GainArgs A0, const u32 *__restrict__ list, u32 nl) {
+    const GainArgs A = gain_args_now(A0);
+    extern __shared__ u32 gt_dyn[];
+    u32 *lo = gt_dyn, *dconn = lo + A.K, *hi = dconn + A.K;  // hi only when WIDE
+    __shared__ i64 red[2][GN_BLOCK / 32];
+    __shared__ Cand cred[GN_BLOCK / 32];
+    const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (u32 idx = blockIdx.x; idx < nl; idx += gridDim.x) {
+        const u32 u = list[idx], p = A.part[u];
+        const u32 deg = (u32)(A.toff[u + 1] - A.toff[u]);
+        for (u32 i = threadIdx.x; i < (WIDE ? 3 : 2) * A.K; i += GN_BLOCK) gt_dyn[i] = 0;
+        __syncthreads();
+        i64 saving = 0, wtot = 0;
+        census_flat(A, u, 32 * warp, GN_BLOCK, deg, wtot, [&](u64 k, u32 q, u32 w, u32 io) {
+            if (q == p) { saving += leave_gain(A.encourage, w, A.ccnt[k]); return; }
+            if (io && A.cdcnt[k] > 0) atomicAdd(&dconn[q], 1u);
+            if (WIDE) {
+                const u32 old = atomicAdd(&lo[q], w);
+                if (old + w < old) atomicAdd(&hi[q], 1u);
+            } else {
+                atomicAdd(&lo[q], w);
+            }
+        });
+        saving = warp_sum(saving);
+        wtot = warp_sum(wtot);
+        if (lane == 0) { red[0][warp] = saving; red[1][warp] = wtot; }
+        __syncthreads();
+        saving = wtot = 0;
+        for (u32 i = 0; i < GN_BLOCK / 32; ++i) { saving += red[0][i]; wtot += red[1][i]; }
+        Cand best{INT64_MIN, 0};
+        for (u32 q = threadIdx.x; q < A.K; q += GN_BLOCK) {
+            const u64 conn = WIDE ? ((u64)hi[q] << 32) | lo[q] : (u64)lo[q];
+            if (conn == 0) continue;  // absent, or never a positive gain
+            const Cand c = gain_candidate(A, u, q, conn, dconn[q], saving, wtot);
+            if (cand_better(c, best)) best = c;
+        }
+        best = warp_best(best);
+        if (lane == 0) cred[warp] = best;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            Cand b = cred[0];
+            for (u32 i = 1; i < GN_BLOCK / 32; ++i)
+                if (cand_better(cred[i], b)) b = cred[i];
+            write_move(A, u, b);
+        }
+        __syncthreads();
+    }
+}
+
+constexpr u32 GP_PLANES = 14;   // bits of a lane's counters
+constexpr u32 GP_MAX_MW = 128;  // mask words (K <= GS_K)
+static_assert(GS_K <= 32 * GP_MAX_MW, "every K of the plane gains has a mask");
+
+// Per-hyperedge masks of MW <= GP_MAX_MW words from the census entries; one warp per hyperedge.
+__global__ void __launch_bounds__(128) k_census_masks_wide(u32 e, const u64 *__restrict__ off,
+                                                           const u32 *__restrict__ lam, const u32 *__restrict__ cpart,
+                                                           const u32 *__restrict__ cdcnt, u32 MW,
+                                                           u32 *__restrict__ mask, u32 *__restrict__ dmask) {
+    __shared__ u32 sm[4][GP_MAX_MW], sd[4][GP_MAX_MW];
+    const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.x * 4 + w;
+    if (h >= e) return;
+    for (u32 i = lane; i < MW; i += 32) sm[w][i] = sd[w][i] = 0;
+    __syncwarp();
+    const u64 a = off[h];
+    const u32 lm = lam[h];
+    for (u32 j = lane; j < lm; j += 32) {
+        const u32 q = cpart[a + j], bit = 1u << (q & 31u);
+        atomicOr(&sm[w][q >> 5], bit);
+        if (cdcnt[a + j] > 0) atomicOr(&sd[w][q >> 5], bit);
+    }
+    __syncwarp();
+    for (u32 i = lane; i < MW; i += 32) {
+        mask[(u64)h * MW + i] = sm[w][i];
+        dmask[(u64)h * MW + i] = sd[w][i];
+    }
+}
+
+// a + b + c of one bit position: sum into l, carry into h.
+__device__ __forceinline__ void csa(u32 &h, u32 &l, u32 a, u32 b, u32 c) {
+    const u32 x = a ^ b;
+    h = (a & b) | (x & c);
+    l = x ^ c;
+}
+// Bit-plane counters of mask word `wl` over the incidences slot, slot + S, ... below jend of the
+// node's list t: plane b of bit i counts 2^b incidences whose word has bit i.
+__device__ __forceinline__ void plane_count(const u32 *__restrict__ t, u32 jend, const u32 *__restrict__ mask, u32 MW,
+                                            u32 wl, u32 slot, u32 S, u32 (&pl)[GP_PLANES]) {
+#pragma unroll
+    for (u32 b = 0; b < GP_PLANES; ++b) pl[b] = 0;
+    for (u32 j = slot; j < jend; j += 8 * S) {
+        u32 x[8];
+#pragma unroll
+        for (u32 r = 0; r < 8; ++r) x[r] = j + r * S < jend ? t[j + r * S] : NONE;
+#pragma unroll
+        for (u32 r = 0; r < 8; ++r) x[r] = x[r] != NONE && wl < MW ? mask[(u64)x[r] * MW + wl] : 0u;
+        u32 t0, t1, f0, f1, e0;
+        csa(t0, pl[0], pl[0], x[0], x[1]);
+        csa(t1, pl[0], pl[0], x[2], x[3]);
+        csa(f0, pl[1], pl[1], t0, t1);
+        csa(t0, pl[0], pl[0], x[4], x[5]);
+        csa(t1, pl[0], pl[0], x[6], x[7]);
+        csa(f1, pl[1], pl[1], t0, t1);
+        csa(e0, pl[2], pl[2], f0, f1);
+#pragma unroll
+        for (u32 b = 3; b < GP_PLANES; ++b) {
+            const u32 c = pl[b] & e0;
+            pl[b] ^= e0;
+            e0 = c;
+        }
+    }
+}
+// The counters of lanes l and l ^ o added (both get the sum).
+__device__ __forceinline__ void plane_merge(u32 (&pl)[GP_PLANES], u32 o) {
+    u32 c = 0;
+#pragma unroll
+    for (u32 b = 0; b < GP_PLANES; ++b) {
+        const u32 y = __shfl_xor_sync(0xFFFFFFFFu, pl[b], o);
+        u32 h;
+        csa(h, pl[b], pl[b], y, c);
+        c = h;
+    }
+}
+
+// One block per node; MWP, the power of two from MW up, lanes per incidence. w: the level's weight.
+template <u32 MWP>
+__global__ void __launch_bounds__(GN_BLOCK) k_gain_planes(GainArgs A0, const u32 *__restrict__ list, u32 nl,
+                                                         const u32 *__restrict__ mask, const u32 *__restrict__ dmask,
+                                                         u32 MW, u32 w) {
+    constexpr u32 S = GN_BLOCK / MWP;                // incidences side by side
+    constexpr u32 ROWS = MWP < 32 ? GN_BLOCK / 32 : S;  // counters per word once a warp's are merged
+    const GainArgs A = gain_args_now(A0);
+    __shared__ u32 pc[GP_PLANES][ROWS * MWP], pd[GP_PLANES][ROWS * MWP];
+    __shared__ Cand cred[GN_BLOCK / 32];
+    const u32 wl = threadIdx.x & (MWP - 1), slot = threadIdx.x / MWP;
+    const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (u32 idx = blockIdx.x; idx < nl; idx += gridDim.x) {
+        const u32 u = list[idx], p = A.part[u];
+        const u64 t0 = A.toff[u];
+        const u32 deg = (u32)(A.toff[u + 1] - t0), nin = A.nin[u];
+        // planes that can be set: the bits of the most incidences one counter sees
+        u32 nb = 32 - __clz((deg + S - 1) / S * (MWP < 32 ? 32 / MWP : 1));
+        nb = nb < GP_PLANES ? nb : GP_PLANES;
+#pragma unroll 1
+        for (u32 pass = 0; pass < 2; ++pass) {
+            u32 pl[GP_PLANES];
+            plane_count(A.touch + t0, pass ? nin : deg, pass ? dmask : mask, MW, wl, slot, S, pl);
+            if (MWP < 32)
+#pragma unroll
+                for (u32 o = 16; o >= MWP; o >>= 1) plane_merge(pl, o);
+            const u32 row = MWP < 32 ? warp * MWP + wl : threadIdx.x;
+            if (MWP >= 32 || lane < MWP)
+#pragma unroll
+                for (u32 b = 0; b < GP_PLANES; ++b)
+                    if (b < nb) (pass ? pd : pc)[b][row] = pl[b];
+        }
+        __syncthreads();
+        const i64 saving = A.save[u], wtot = (i64)((u64)deg * w);
+        Cand best{INT64_MIN, 0};
+        for (u32 q = threadIdx.x; q < A.K; q += GN_BLOCK) {
+            const u32 wd = q >> 5, sh = q & 31u;
+            u32 cnt = 0;
+            for (u32 b = 0; b < nb; ++b) {
+                u32 c = 0;
+#pragma unroll
+                for (u32 r = 0; r < ROWS; ++r) c += (pc[b][r * MWP + wd] >> sh) & 1u;
+                cnt += c << b;
+            }
+            if (cnt == 0 || q == p) continue;
+            u32 dc = 0;
+            for (u32 b = 0; b < nb; ++b) {
+                u32 c = 0;
+#pragma unroll
+                for (u32 r = 0; r < ROWS; ++r) c += (pd[b][r * MWP + wd] >> sh) & 1u;
+                dc += c << b;
+            }
+            const Cand c = gain_candidate(A, u, q, (u64)cnt * w, dc, saving, wtot);
+            if (cand_better(c, best)) best = c;
+        }
+        best = warp_best(best);
+        if (lane == 0) cred[warp] = best;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            Cand b = cred[0];
+            for (u32 i = 1; i < GN_BLOCK / 32; ++i)
+                if (cand_better(cred[i], b)) b = cred[i];
+            write_move(A, u, b);
+        }
+        // the next node's counters are written after every thread has passed this barrier and
+        // read the previous ones before it
+        __syncthreads();
     }
 }
 
@@ -1513,13 +1625,6 @@ __global__ void k_list_degree(const u32 *__restrict__ list, u32 nl, const u64 *_
     u64 d = i < nl ? toff[list[i] + 1] - toff[list[i]] : 0;
     d = warp_sum(d);
     if ((threadIdx.x & 31) == 0 && d) atomicAdd(out, (unsigned long long)d);
-}
-__global__ void k_list_max(const u32 *__restrict__ list, u32 nl, const u64 *__restrict__ v,
-                           unsigned long long *__restrict__ out) {
-    u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    u64 m = i < nl ? v[list[i]] : 0;
-    m = warp_max_u64(m);
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(out, (unsigned long long)m);
 }
 // Gain tiers: 0 = one warp (small table, at most GN_WARP_DEG incidences), 1 = one block with the
 // table in shared memory, 2 = one block with the table in global scratch. Levels of at most
@@ -3370,12 +3475,13 @@ struct LevelPrep {
     u32 *ntier[3] = {nullptr, nullptr, nullptr};
     u32 ncount[3] = {0, 0, 0};
     u64 *work = nullptr;     // per-node table bound of the gains
-    u64 heavy_work_max = 0;  // largest gain-work bound of the heavy tier
     u64 block_work_max = 0;  // largest gain-work bound of the block tier (sizes its shared table)
     u64 gain_bound = 0;     // no gain exceeds this (sum of incident weights)
     u64 max_len = 0;         // largest hyperedge
     u64 max_deg = 0;         // largest degree
     u64 short_pins = 0, short_sq = 0;  // pins of hyperedges of at most CM_LEN pins; sum of their squared lengths
+    bool uniform = false;    // every hyperedge has the weight `weight`
+    u32 weight = 0;
     u64 dst_pins = 0;        // destination pins (bounds the inbound events: 2 per pin)
     u64 tier_deg[3] = {0, 0, 0};  // incidence entries of each gain tier (kernel timer only)
     u32 census_K = 0;        // nonzero: partition-indexed census over this many partitions, and
@@ -3412,6 +3518,7 @@ static bool round_loop_enabled() {
 
 void setup_refine_kernels(Ctx &c) {
     AXC_CUDA(cudaFuncSetAttribute(k_census_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 2 * CS_BLOCK_CAP * 4));
+    AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * GN_BLOCK_W * 16));
     AXC_CUDA(cudaFuncSetAttribute(k_cascade_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CB_DYN_MAX));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_SMEM));
@@ -3423,7 +3530,7 @@ void setup_refine_kernels(Ctx &c) {
 }
 
 __global__ void k_level_bounds(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ nsrc,
-                               unsigned long long *__restrict__ out);
+                               const u32 *__restrict__ wfx, unsigned long long *__restrict__ out);
 
 // Largest gain-work bound over all nodes (out[0]) and over the block tier (out[1]); the largest
 // degree (out[2]).
@@ -3455,9 +3562,10 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
     const u32 e = L.e, n = L.n;
     // [0] census block list, [1] census huge list, [2..4] node tiers, [5] gain bound,
     // [6] largest work, [7] largest block-tier work, [8] largest degree, [9] largest hyperedge,
-    // [10] destination pins, [11] pins of short hyperedges, [12] the sum of their squared lengths
-    u64 *dc = c.arena.alloc<u64>(13);
-    AXC_CUDA(cudaMemsetAsync(dc, 0, 104, c.stream));
+    // [10] destination pins, [11] largest weight, [12] complement of the smallest, [13] pins of short
+    // hyperedges, [14] the sum of their squared lengths
+    u64 *dc = c.arena.alloc<u64>(15);
+    AXC_CUDA(cudaMemsetAsync(dc, 0, 120, c.stream));
     lp.census_K = K <= CD_K || kway ? K : 0;
     if (e) {
         u32 *flag = c.arena.alloc<u32>(e);
@@ -3472,7 +3580,7 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
             LAUNCH(c, k_flag_len, cdiv(e, 256), 256, 0, e, L.off, (u64)CS_BLOCK_CAP, ~0ull, flag);
             compact_indices_dn(c, flag, lp.hhuge, e, (u32 *)(dc + 1));
         }
-        LAUNCH(c, k_level_bounds, cdiv(e, 256), 256, 0, e, L.off, L.nsrc, (unsigned long long *)(dc + 9));
+        LAUNCH(c, k_level_bounds, cdiv(e, 256), 256, 0, e, L.off, L.nsrc, wfx, (unsigned long long *)(dc + 9));
     }
     if (n) {
         u64 *work = c.arena.alloc<u64>(n);
@@ -3488,19 +3596,22 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
         LAUNCH(c, k_tier_max, cdiv(n, 256), 256, 0, n, K, work, L.toff, kway ? 1u : 0u,
                (unsigned long long *)(dc + 6));
     }
-    u64 h[13];
-    fetch(c, h, dc, 104);
+    u64 h[15];
+    fetch(c, h, dc, 120);
     lp.n_hblock = (u32)h[0];
     lp.n_hhuge = (u32)h[1];
     for (int t = 0; t < 3; ++t) lp.ncount[t] = (u32)h[2 + t];
     lp.gain_bound = h[5];
-    lp.heavy_work_max = lp.ncount[2] ? h[6] : 0;
     lp.block_work_max = h[7];
     lp.max_deg = h[8];
     lp.max_len = h[9];
     lp.dst_pins = h[10];
-    lp.short_pins = h[11];
-    lp.short_sq = h[12];
+    lp.short_pins = h[13];
+    lp.short_sq = h[14];
+    if (e && (u32)h[11] == ~(u32)h[12]) {
+        lp.uniform = true;
+        lp.weight = (u32)h[11];
+    }
     if (lp.n_hhuge) {
         lp.huge_tab = c.arena.alloc<u64>(lp.n_hhuge + 1);
         LAUNCH(c, k_tab_sizes, cdiv(lp.n_hhuge + 1, 256), 256, 0, lp.hhuge, lp.n_hhuge, L.off, lp.huge_tab);
@@ -3566,17 +3677,6 @@ static Census alloc_census(Ctx &c, const DLevel &L) {
 // move, gain and rank).
 static u64 gain_bytes(const LevelPrep &lp, int t) { return 8 * lp.tier_deg[t] + 16 * (u64)lp.ncount[t]; }
 
-// Distinct partitions a node may reach in the first try of the heavy gain tier: 3/4 of the
-// table, or fewer when the environment variable AXC_GAIN_TRY_LIMIT asks for it (at least 1),
-// which sends more nodes to the global retry; the tests use it to reach that path on small inputs.
-static u32 gain_try_limit(u32 cap) {
-    const u32 lim = cap / 4 * 3;
-    const char *s = std::getenv("AXC_GAIN_TRY_LIMIT");
-    if (!s || !*s) return lim;
-    const unsigned long v = std::strtoul(s, nullptr, 10);
-    return v < 1 ? 1u : (v < lim ? (u32)v : lim);
-}
-
 template <u32 MW>
 static void run_gains_masked(Ctx &c, const LevelPrep &lp, const GainArgs &A, const Census &cs) {
     if (lp.ncount[0])
@@ -3584,6 +3684,21 @@ static void run_gains_masked(Ctx &c, const LevelPrep &lp, const GainArgs &A, con
                cs.mask, cs.dmask);
     if (lp.ncount[1])
         LAUNCH(c, k_gain_mask_block<MW>, lp.ncount[1], GN_BLOCK, 0, A, lp.ntier[1], lp.ncount[1], cs.mask, cs.dmask);
+}
+
+// Lanes per incidence of k_gain_planes at K partitions: the power of two from its mask words up.
+static u32 plane_lanes(u32 K) {
+    u32 l = 16;
+    while (32 * l < K) l <<= 1;
+    return l;
+}
+// Plane gains: equal weights, a block tier at GN_DIRECT_K < K <= GS_K, counters that hold the
+// largest degree, and hyperedges of at least as many pins as mask words on average. A node's work is
+// then its incidences times K / 32 words against (at most) times their census entries.
+static bool plane_gains(const DLevel &L, const LevelPrep &lp, u32 K) {
+    if (!lp.uniform || !lp.ncount[1] || K <= GN_DIRECT_K || K > GS_K || !L.e) return false;
+    const u32 lanes = plane_lanes(K), S = GN_BLOCK / lanes, rows = lanes < 32 ? 32 / lanes : 1;
+    return (lp.max_deg / S + 1) * rows < (1u << GP_PLANES) && L.P / L.e >= (K + 31) / 32;
 }
 
 static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainArgs &A, const Census &cs) {
@@ -3602,13 +3717,33 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
     if (c.profiling("k_gain_warp") && lp.ncount[0]) c.prof_bytes += gain_bytes(lp, 0);
     if (c.profiling("k_gain_block")) c.prof_bytes += gain_bytes(lp, 1) + gain_bytes(lp, 2);
     LAUNCH(c, k_gain_warp, cdiv(lp.ncount[0], GN_WARPS), GN_WARPS * 32, 0, A, lp.ntier[0], lp.ncount[0], lp.work);
-    if (lp.ncount[1]) {
+    if (lp.ncount[1] && plane_gains(L, lp, A.K)) {
+        const size_t m = c.arena.mark();
+        const u32 MW = (A.K + 31) / 32;
+        u32 *mask = c.arena.alloc<u32>((u64)L.e * MW), *dmask = c.arena.alloc<u32>((u64)L.e * MW);
+        LAUNCH(c, k_census_masks_wide, cdiv(L.e, 4), 128, 0, L.e, L.off, cs.lam, cs.part, cs.dcnt, MW, mask, dmask);
+        const auto launch = [&](auto lanes) {
+            LAUNCH_AS(c, "k_gain_planes", k_gain_planes<decltype(lanes)::value>, lp.ncount[1], GN_BLOCK, 0, A,
+                      lp.ntier[1], lp.ncount[1], mask, dmask, MW, lp.weight);
+        };
+        switch (plane_lanes(A.K)) {
+            case 16: launch(std::integral_constant<u32, 16>()); break;
+            case 32: launch(std::integral_constant<u32, 32>()); break;
+            case 64: launch(std::integral_constant<u32, 64>()); break;
+            default: launch(std::integral_constant<u32, 128>()); break;
+        }
+        c.arena.release(m);
+    } else if (lp.ncount[1] && A.K <= GS_K) {
+        if (lp.gain_bound < (1ull << 32))
+            LAUNCH_AS(c, "k_gain_table", k_gain_table<false>, lp.ncount[1], GN_BLOCK, (size_t)A.K * 8, A, lp.ntier[1],
+                      lp.ncount[1]);
+        else
+            LAUNCH_AS(c, "k_gain_table", k_gain_table<true>, lp.ncount[1], GN_BLOCK, (size_t)A.K * 12, A, lp.ntier[1],
+                      lp.ncount[1]);
+    } else if (lp.ncount[1]) {
         // shared table sized by the tier's largest bound (16 B per slot)
-        u32 cap1 = table_cap(lp.block_work_max, 2 * GN_BLOCK_W);
-        if (A.K <= GN_DIRECT_K)  // indexed by partition id: K slots (rounded up) per node
-            while (cap1 < A.K) cap1 <<= 1;
-        LAUNCH(c, k_gain_block, lp.ncount[1], GN_BLOCK, cap1 * 16, A, lp.ntier[1], lp.ncount[1], (const u32 *)nullptr,
-               cap1, (u32 *)nullptr, (u32 *)nullptr, lp.work, 0u, (u32 *)nullptr, (u32 *)nullptr);
+        const u32 cap1 = table_cap(lp.block_work_max, 2 * GN_BLOCK_W);
+        LAUNCH(c, k_gain_block, lp.ncount[1], GN_BLOCK, cap1 * 16, A, lp.ntier[1], lp.ncount[1], cap1, lp.work);
     }
     if (lp.ncount[2] && A.K > GS_K) {  // the sampled rule (include/axc.h AXC_SPARSE_GAIN_*)
         size_t m = c.arena.mark();
@@ -3632,29 +3767,6 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
             LAUNCH(c, k_cands_block, lp.n_hhuge, CV_BLOCK, 0, A, C, lp.hhuge, lp.n_hhuge, gtab, (const u64 *)lp.huge_tab);
         }
         LAUNCH(c, k_cands_best, cdiv(rows, 256), 256, 0, A, C, lp.ntier[2], rows);
-        c.arena.release(m);
-    } else if (lp.ncount[2]) {
-        size_t m = c.arena.mark();
-        const u32 *heavy = lp.ntier[2];
-        const u32 *dn = nullptr;
-        if (A.K > GN_DIRECT_K) {
-            // Bounds overestimate: partitions recur across a node's hyperedges. First try with the
-            // largest shared table; a node with more than 3/4 of its slots distinct is retried.
-            const u32 cap_try = 2 * GN_BLOCK_W;
-            u32 *retry = c.arena.alloc<u32>(lp.ncount[2]), *nretry = c.arena.alloc<u32>(1);
-            AXC_CUDA(cudaMemsetAsync(nretry, 0, 4, c.stream));
-            LAUNCH(c, k_gain_block, lp.ncount[2], GN_BLOCK, cap_try * 16, A, lp.ntier[2], lp.ncount[2],
-                   (const u32 *)nullptr, cap_try, (u32 *)nullptr, (u32 *)nullptr, lp.work, gain_try_limit(cap_try), retry,
-                   nretry);
-            heavy = retry;
-            dn = nretry;
-        }
-        u32 cap = 64;
-        while (cap < 2 * lp.heavy_work_max && cap < (1u << 28)) cap <<= 1;
-        u32 grid = lp.ncount[2] < (u32)c.sms * 2 ? lp.ncount[2] : (u32)c.sms * 2;
-        u32 *gtab = c.arena.alloc<u32>((u64)grid * 4 * cap), *gused = c.arena.alloc<u32>((u64)grid * cap);
-        LAUNCH(c, k_gain_block, grid, GN_BLOCK, 0, A, heavy, lp.ncount[2], dn, cap, gtab, gused, lp.work, 0u,
-               (u32 *)nullptr, (u32 *)nullptr);
         c.arena.release(m);
     }
 }
@@ -3730,7 +3842,7 @@ static Census census_for_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, con
                                const u32 *part) {
     Census cs = alloc_census(c, L);
     const bool direct = rp.K <= GN_DIRECT_K;
-    if (direct) {
+    if (direct || plane_gains(L, lp, rp.K)) {
         cs.save = c.arena.alloc<i64>(L.n ? L.n : 1);
         AXC_CUDA(cudaMemsetAsync(cs.save, 0, (size_t)L.n * 8, c.stream));
         cs.wfx = wfx;
@@ -4290,25 +4402,33 @@ __global__ void k_round_next(cudaGraphConditionalHandle h, u32 *__restrict__ rs,
     cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
-// level bounds that need the offsets: the largest hyperedge and the destination pin count
+// level bounds over the hyperedges: the longest, the destination pin count, the largest weight and
+// the largest complement of a weight (the smallest weight)
 __global__ void k_level_bounds(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ nsrc,
-                               unsigned long long *__restrict__ out) {
+                               const u32 *__restrict__ wfx, unsigned long long *__restrict__ out) {
     u32 h = blockIdx.x * blockDim.x + threadIdx.x;
     u64 len = 0, dst = 0, sp = 0, sq = 0;
+    u32 w = 0, nw = 0;
     if (h < e) {
         len = off[h + 1] - off[h];
         dst = len - nsrc[h];
+        w = wfx[h];
+        nw = ~w;
         if (len <= CM_LEN) { sp = len; sq = len * len; }
     }
     sp = warp_sum(sp);
     sq = warp_sum(sq);
     len = warp_max_u64(len);
     dst = warp_sum(dst);
+    w = __reduce_max_sync(0xFFFFFFFFu, w);
+    nw = __reduce_max_sync(0xFFFFFFFFu, nw);
     if ((threadIdx.x & 31) == 0) {
         atomicMax(&out[0], (unsigned long long)len);
         atomicAdd(&out[1], (unsigned long long)dst);
-        if (sp) atomicAdd(&out[2], (unsigned long long)sp);
-        if (sq) atomicAdd(&out[3], (unsigned long long)sq);
+        atomicMax(&out[2], (unsigned long long)w);
+        atomicMax(&out[3], (unsigned long long)nw);
+        if (sp) atomicAdd(&out[4], (unsigned long long)sp);
+        if (sq) atomicAdd(&out[5], (unsigned long long)sq);
     }
 }
 
