@@ -1,7 +1,9 @@
 // Device primitives owned by the library (no Thrust/CUB): single-pass scans and compaction
 // (decoupled look-back over 2048-element tiles, Merrill & Garland 2016), a stable LSD radix sort
-// with warp-level match_any ranking, fills and reductions. Every launch goes through the
+// with one launch per pass, fills and reductions. Every launch goes through the
 // context's stream.
+#include <algorithm>
+
 #include "common.cuh"
 #include "blocksort.cuh"
 
@@ -186,17 +188,13 @@ __device__ TO lookback_prefix(const ScanState &S, u32 epoch, u32 t, TO tile_tota
 }
 
 // Scan: out[i] = sum of in[0..i) (exclusive) or in[0..i] (inclusive), in one pass.
-// With skip_n set, a launch whose *skip_n is at most skip_le does nothing: every block returns
-// before it takes a tile ticket, so the tile state is left as the previous launch left it.
 template <class TI, class TO, bool INCL>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_lb(const TI *__restrict__ in, TO *__restrict__ out, u64 n,
-                                                        ScanState S, u32 *status, const u32 *__restrict__ skip_n,
-                                                        u32 skip_le) {
+                                                        ScanState S, u32 *status) {
     __shared__ TO wt[33];
     __shared__ TO stage[SCAN_TILE + SCAN_TILE / 32];
     __shared__ u32 s_tile, s_epoch;
     __shared__ TO s_prefix;
-    if (skip_n && *skip_n <= skip_le) return;
     u32 epoch;
     const u32 t = lb_enter(S, s_tile, s_epoch, epoch);
     const u64 base = (u64)t * SCAN_TILE;
@@ -263,11 +261,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_compact_lb(const u32 *__restri
 }
 
 template <class TI, class TO, bool INCL = false>
-void scan_impl(Ctx &c, const TI *in, TO *out, u64 n, const u32 *skip_n = nullptr, u32 skip_le = 0) {
+void scan_impl(Ctx &c, const TI *in, TO *out, u64 n) {
     if (n == 0) return;
     const u32 tiles = cdiv(n, SCAN_TILE);
     if (tiles <= c.scan.cap_tiles) {
-        LAUNCH(c, (k_scan_lb<TI, TO, INCL>), tiles, SCAN_THREADS, 0, in, out, n, c.scan, c.d_status, skip_n, skip_le);
+        LAUNCH(c, (k_scan_lb<TI, TO, INCL>), tiles, SCAN_THREADS, 0, in, out, n, c.scan, c.d_status);
         return;
     }
     if (INCL) throw Error(AXC_EOVERFLOW, "inclusive scan longer than the look-back tile state");
@@ -297,72 +295,228 @@ __global__ void k_offsets_tail(const u32 *counts, u64 *out, u64 n) {
 }
 
 // ------------------------------------------------------------------ radix sort
+// Stable LSD sort of (key, value) pairs in 8-bit passes, one launch per pass (the single-pass
+// scheme of Adinets and Merrill, "Onesweep", 2022, over this file's bounded look-back): one first
+// launch counts the digits of every pass; in a pass, tiles take tickets, rank their items by
+// digit, look back digit by digit over their predecessors' counts and write each item once, from
+// shared memory in digit order. A pass whose digit is the same in every key moves nothing and is
+// left out (fixed-point gains of unweighted nets share their low 18 bits), so the buffers swap
+// once per pass that ran, and a last launch brings an odd number of them home.
 constexpr int RS_WARPS = 8;
-constexpr int RS_ITEMS = 8;  // rounds of 32 per warp
-constexpr int RS_TILE = RS_WARPS * 32 * RS_ITEMS;
+// Rounds of 32 per warp: 16 (tiles of 4096) for large arrays, 4 (tiles of 1024) up to RS_SMALL_N
+// elements, where larger tiles would leave most of the GPU without one.
+constexpr int RS_ITEMS_LARGE = 16, RS_ITEMS_SMALL = 4;
+constexpr u64 RS_SMALL_N = 1u << 19;
+constexpr int RS_PASSES = 4;
+constexpr u32 RS_DIG = 256;
 
-// k_rs_hist / k_rs_scatter: with d_n set, a count of at most skip_le means the one-block sort
-// has already sorted the data, and the launch does nothing.
-__global__ void k_rs_hist(const u32 *__restrict__ keys, u64 n, u32 shift, u32 *__restrict__ hist,
-                          u32 tiles, const u32 *__restrict__ d_n, u32 skip_le) {
-    if (d_n && *d_n <= skip_le) return;
-    __shared__ u32 cnt[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) cnt[i] = 0;
+// Tile states hold a digit's count in the low bits and 1 (aggregate) or 2 (inclusive prefix) in the
+// top two: u32 words while every count fits 30 bits, else u64.
+struct SortState {
+    u32 *keys, *vals, *k2, *v2;
+    u64 n;             // capacity
+    const u32 *d_n;    // count in device memory (at most n), or null
+    u32 skip_le;       // with d_n: a count of at most this was sorted by one block of the first launch
+    u32 passes;
+    u32 *hist;         // [RS_PASSES][256] digit counts, then their exclusive prefixes
+    u32 *ctrl;         // [0, RS_PASSES) tile tickets, [4] first-launch blocks done, [5] passes left out
+    void *st0, *st1;   // [tiles * 256] tile states, used in turn by the passes that run
+};
+__device__ __forceinline__ u64 rs_count(const SortState &S) { return S.d_n ? (u64)*S.d_n : S.n; }
+
+// First launch: a count that one block holds is sorted there and then; else every pass's digit counts.
+__global__ void __launch_bounds__(RSS_WARPS * 32) k_rs_first(SortState S, u32 bits) {
+    extern __shared__ u32 sm[];
+    __shared__ u32 last;
+    const u64 n = rs_count(S);
+    if (S.d_n && n <= S.skip_le) {
+        if (blockIdx.x) return;
+        const u32 m = (u32)n;
+        for (u32 i = threadIdx.x; i < m; i += blockDim.x) { sm[i] = S.keys[i]; sm[RSS_CAP + i] = S.vals[i]; }
+        const u32 *ko, *vo;
+        block_radix_sort(sm, m, bits, ko, vo);
+        for (u32 i = threadIdx.x; i < m; i += blockDim.x) { S.keys[i] = ko[i]; S.vals[i] = vo[i]; }
+        return;
+    }
+    u32 *cnt = sm;  // [passes][256]
+    for (u32 i = threadIdx.x; i < S.passes * RS_DIG; i += blockDim.x) cnt[i] = 0;
     __syncthreads();
-    if (d_n) n = *d_n;  // element count resident on the device (tiles past it count nothing)
-    const u64 base = (u64)blockIdx.x * RS_TILE;
-    for (int j = threadIdx.x; j < RS_TILE; j += blockDim.x) {
-        u64 i = base + j;
-        if (i < n) atomicAdd(&cnt[(keys[i] >> shift) & 255u], 1u);
+    const u64 step = (u64)gridDim.x * blockDim.x, n32 = (n + 31) & ~31ull;
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n32; i += step) {  // whole warps
+        const bool in = i < n;
+        const u32 k = in ? S.keys[i] : 0u;
+        for (u32 p = 0; p < S.passes; ++p) {
+            const u32 d = in ? (k >> (8 * p)) & 255u : 256u;
+            int same;
+            __match_all_sync(0xFFFFFFFFu, d, &same);
+            if (same) {  // one digit over the warp: one add instead of 32 to one word
+                if ((threadIdx.x & 31u) == 0 && in) atomicAdd(&cnt[p * RS_DIG + d], 32u);
+            } else if (in) {
+                atomicAdd(&cnt[p * RS_DIG + d], 1u);
+            }
+        }
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += blockDim.x) hist[(u64)d * tiles + blockIdx.x] = cnt[d];
+    for (u32 i = threadIdx.x; i < S.passes * RS_DIG; i += blockDim.x)
+        if (cnt[i]) atomicAdd(&S.hist[i], cnt[i]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&S.ctrl[4], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    // the last block: digit bases of every pass (one warp each), and the passes left out
+    const u32 p = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    if (p >= S.passes) return;
+    u32 v[8], s = 0;
+    bool all = false;
+    for (u32 k = 0; k < 8; ++k) {
+        v[k] = *(volatile u32 *)&S.hist[p * RS_DIG + lane * 8 + k];
+        all |= (u64)v[k] == n;
+        s += v[k];
+    }
+    u32 x = s;
+    for (u32 o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    u32 pre = x - s;
+    for (u32 k = 0; k < 8; ++k) { S.hist[p * RS_DIG + lane * 8 + k] = pre; pre += v[k]; }
+    if (__any_sync(0xFFFFFFFFu, all) && lane == 0) atomicOr(&S.ctrl[5], 1u << p);
 }
 
-__global__ void k_rs_scatter(const u32 *__restrict__ kin, const u32 *__restrict__ vin, u32 *__restrict__ kout,
-                             u32 *__restrict__ vout, u64 n, u32 shift, const u32 *__restrict__ offs,
-                             u32 tiles, const u32 *__restrict__ d_n, u32 skip_le) {
-    if (d_n && *d_n <= skip_le) return;
-    __shared__ u32 wcnt[RS_WARPS][256];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (d_n) n = *d_n;
-    for (int i = threadIdx.x; i < RS_WARPS * 256; i += blockDim.x) (&wcnt[0][0])[i] = 0;
+// Passes that ran before pass p: their parity says which buffers hold the data.
+__device__ __forceinline__ u32 rs_parity(const SortState &S, u32 p) {
+    return __popc(~S.ctrl[5] & ((1u << p) - 1u)) & 1u;
+}
+
+template <class ST, int RS_ITEMS>
+__global__ void __launch_bounds__(RS_WARPS * 32, RS_ITEMS > 8 ? 3 : 6) k_rs_pass(SortState S, u32 p, u32 *status) {
+    constexpr u32 RS_TILE = RS_WARPS * 32 * RS_ITEMS;
+    constexpr int FS = (int)sizeof(ST) * 8 - 2;  // shift of the flag
+    extern __shared__ u32 sm[];                  // sorted keys, then values
+    __shared__ u32 wcnt[RS_WARPS][RS_DIG], lbase[RS_DIG], gbase[RS_DIG], wsum[RS_WARPS];
+    __shared__ u32 s_tile;
+    const u64 n = rs_count(S);
+    if (S.d_n && n <= S.skip_le) return;
+    if ((S.ctrl[5] >> p) & 1u) return;
+    const u32 par = rs_parity(S, p), shift = 8 * p;
+    const u32 *kin = par ? S.k2 : S.keys, *vin = par ? S.v2 : S.vals;
+    u32 *kout = par ? S.keys : S.k2, *vout = par ? S.vals : S.v2;
+    ST *st = (ST *)(par ? S.st1 : S.st0), *st_next = (ST *)(par ? S.st0 : S.st1);
+    const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  for (;;) {  // tiles by ticket: the grid follows the GPU, not the capacity
+    if (threadIdx.x == 0) s_tile = atomicAdd(&S.ctrl[p], 1u);
+    for (u32 i = threadIdx.x; i < RS_WARPS * RS_DIG; i += blockDim.x) (&wcnt[0][0])[i] = 0;
     __syncthreads();
-    const u64 base = (u64)blockIdx.x * RS_TILE + (u64)w * 32 * RS_ITEMS;
-    u32 dig[RS_ITEMS], loc[RS_ITEMS], key[RS_ITEMS], val[RS_ITEMS];
-    const u32 lt = (1u << lane) - 1u;
+    const u32 tile = s_tile;
+    const u64 t0 = (u64)tile * RS_TILE;
+    if (t0 >= n) return;
+    const u32 cnt = (u32)(n - t0 < RS_TILE ? n - t0 : RS_TILE);
+    st_next[(u64)tile * RS_DIG + threadIdx.x] = 0;  // the next pass's state (its last reader has finished)
+    const u64 base = t0 + (u64)w * 32 * RS_ITEMS;
+    u32 key[RS_ITEMS], loc[RS_ITEMS];
 #pragma unroll
     for (int r = 0; r < RS_ITEMS; ++r) {
-        u64 i = base + (u64)r * 32 + lane;
-        bool ok = i < n;
-        key[r] = ok ? kin[i] : 0u;
-        val[r] = ok ? vin[i] : 0u;
-        u32 d = ok ? ((key[r] >> shift) & 255u) : 256u;
-        dig[r] = d;
-        u32 peers = __match_any_sync(0xFFFFFFFFu, d);
-        u32 before = ok ? wcnt[w][d] : 0u;
+        const u64 i = base + (u64)r * 32 + lane;
+        key[r] = i < n ? kin[i] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < RS_ITEMS; ++r) {
+        const bool ok = base + (u64)r * 32 + lane < n;
+        const u32 d = ok ? ((key[r] >> shift) & 255u) : 256u;
+        const u32 peers = __match_any_sync(0xFFFFFFFFu, d);
+        const u32 before = ok ? wcnt[w][d] : 0u;
         loc[r] = before + __popc(peers & lt);
         __syncwarp();
         if (ok && (peers & lt) == 0) wcnt[w][d] = before + __popc(peers);
         __syncwarp();
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += blockDim.x) {
-        u32 run = offs[(u64)d * tiles + blockIdx.x];
-        for (int ww = 0; ww < RS_WARPS; ++ww) {
-            u32 t = wcnt[ww][d];
-            wcnt[ww][d] = run;
-            run += t;
+    u32 val[RS_ITEMS];  // in flight during the look-back
+#pragma unroll
+    for (int r = 0; r < RS_ITEMS; ++r) {
+        const u64 i = base + (u64)r * 32 + lane;
+        val[r] = i < n ? vin[i] : 0u;
+    }
+    // thread d: the tile's count of digit d and its warps' offsets within it
+    const u32 d = threadIdx.x;
+    u32 tot = 0;
+#pragma unroll
+    for (int ww = 0; ww < RS_WARPS; ++ww) {
+        const u32 t = wcnt[ww][d];
+        wcnt[ww][d] = tot;
+        tot += t;
+    }
+    volatile ST *mine = st + (u64)tile * RS_DIG + d;
+    *mine = ((ST)(tile ? 1 : 2) << FS) | (ST)tot;
+    // exclusive prefix of the tile's counts over the digits
+    u32 x = tot;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= (u32)o) x += y;
+    }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    u32 lb = x - tot;
+    for (u32 ww = 0; ww < w; ++ww) lb += wsum[ww];
+    lbase[d] = lb;
+    // look back over the predecessors' counts of digit d: a word carries count and flag together
+    ST excl = 0;
+    if (tile) {
+        bool gave_up = false, done = false;
+        constexpr int WIN = 8;  // predecessors read at once
+        for (long long j = (long long)tile - 1; j >= 0 && !done && !gave_up; j -= WIN) {
+            ST v[WIN];
+#pragma unroll
+            for (int x = 0; x < WIN; ++x) v[x] = j - x >= 0 ? *(volatile const ST *)(st + (j - x) * RS_DIG + d) : ((ST)2 << FS);
+#pragma unroll
+            for (int x = 0; x < WIN; ++x) {
+                if (done || gave_up) continue;
+                for (u32 it = 0; !(v[x] >> FS); ++it) {
+                    if (it >= LB_SPIN_LIMIT) { gave_up = true; break; }
+                    if (it > 64) __nanosleep(32);
+                    v[x] = *(volatile const ST *)(st + (j - x) * RS_DIG + d);
+                }
+                excl += v[x] & (((ST)1 << FS) - 1);
+                done = (v[x] >> FS) == 2;
+            }
+        }
+        if (gave_up) atomicExch(status, (u32)DEV_SPIN_LIMIT);
+        *mine = ((ST)2 << FS) | (excl + (ST)tot);
+    }
+    gbase[d] = S.hist[p * RS_DIG + d] + (u32)excl - lb;  // position of the tile's digit-d run, less its place in it
+    __syncthreads();
+    u32 *sk = sm, *sv = sm + RS_TILE;
+#pragma unroll
+    for (int r = 0; r < RS_ITEMS; ++r) {
+        if (base + (u64)r * 32 + lane < n) {
+            const u32 dg = (key[r] >> shift) & 255u;
+            const u32 pos = lbase[dg] + wcnt[w][dg] + loc[r];
+            sk[pos] = key[r];
+            sv[pos] = val[r];
         }
     }
     __syncthreads();
-#pragma unroll
-    for (int r = 0; r < RS_ITEMS; ++r) {
-        if (dig[r] < 256u) {
-            u32 pos = wcnt[w][dig[r]] + loc[r];
-            kout[pos] = key[r];
-            vout[pos] = val[r];
+    for (u32 i = threadIdx.x; i < cnt; i += RS_WARPS * 32) {
+        const u32 k = sk[i];
+        const u32 pos = gbase[(k >> shift) & 255u] + i;
+        if (pos < n) {  // holds unless a wait gave up
+            kout[pos] = k;
+            vout[pos] = sv[i];
         }
+    }
+    __syncthreads();  // the tile's shared state is no longer read
+  }
+}
+
+// An odd number of passes left the data in k2, v2.
+__global__ void k_rs_home(SortState S) {
+    const u64 n = rs_count(S);
+    if ((S.d_n && n <= S.skip_le) || !rs_parity(S, S.passes)) return;
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
+        S.keys[i] = S.k2[i];
+        S.vals[i] = S.v2[i];
     }
 }
 
@@ -420,7 +574,6 @@ __global__ void k_compact_write(const u32 *flags, const u32 *pos, u32 *out, u64 
 __global__ void __launch_bounds__(RSS_WARPS * 32) k_rs_small(u32 *__restrict__ keys, u32 *__restrict__ vals, u32 n_cap,
                                                              const u32 *__restrict__ d_n, u32 bits) {
     extern __shared__ u32 sm[];
-    if (d_n && *d_n > n_cap) return;  // more than one block holds: the multi-pass sort takes it
     const u32 n = d_n ? *d_n : n_cap;
     for (u32 i = threadIdx.x; i < n; i += blockDim.x) { sm[i] = keys[i]; sm[RSS_CAP + i] = vals[i]; }
     const u32 *ko, *vo;
@@ -460,6 +613,7 @@ void lookback_selftest(Ctx &c, u32 spin_limit) {
 
 void setup_prim_kernels() {
     AXC_CUDA(cudaFuncSetAttribute(k_rs_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
+    AXC_CUDA(cudaFuncSetAttribute(k_rs_first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
 }
 
 void scan_state_create(Ctx &c, u32 cap_tiles) {
@@ -568,37 +722,35 @@ void radix_sort_pairs(Ctx &c, u32 *keys, u32 *vals, u64 n, u32 bits) {
 // Same, with the element count read from device memory (d_n, at most n); no host round trip.
 void radix_sort_pairs_dn(Ctx &c, u32 *keys, u32 *vals, const u32 *d_n, u64 n, u32 bits) {
     if ((!d_n && n <= 1) || n == 0 || bits == 0) return;
+    bits = std::min(bits, 32u);
     if (n <= (u64)RSS_CAP) {  // one block, every pass in shared memory
         LAUNCH(c, k_rs_small, 1, RSS_WARPS * 32, RSS_SMEM, keys, vals, (u32)n, d_n, bits);
         return;
     }
-    // Capacity above one block. With the count on the device both forms are launched: the
-    // one-block sort acts when the count fits it, the passes below when it does not (each kernel
-    // reads the count and returns at once otherwise), and an even number of passes leaves the
-    // data in place either way.
-    u32 skip_le = 0;
-    u32 passes = (bits + 7) / 8;
-    if (d_n) {
-        LAUNCH(c, k_rs_small, 1, RSS_WARPS * 32, RSS_SMEM, keys, vals, (u32)RSS_CAP, d_n, bits);
-        skip_le = RSS_CAP;
-        passes += passes & 1u;
+    const size_t m = c.arena.mark();
+    const u32 tile = RS_WARPS * 32 * (n <= RS_SMALL_N ? RS_ITEMS_SMALL : RS_ITEMS_LARGE);
+    const u64 tiles = (n + tile - 1) / tile;
+    SortState S{keys, vals, c.arena.alloc<u32>(n), c.arena.alloc<u32>(n), n, d_n, (u32)RSS_CAP, (bits + 7) / 8};
+    const bool wide = n >= (1ull << 30);
+    const size_t st_bytes = tiles * RS_DIG * (wide ? 8 : 4);
+    constexpr size_t head = RS_PASSES * RS_DIG + 64;  // hist and ctrl, in words before the first states
+    char *mem = c.arena.alloc<char>(head * 4 + st_bytes);
+    S.hist = (u32 *)mem;
+    S.ctrl = S.hist + RS_PASSES * RS_DIG;
+    S.st0 = mem + head * 4;
+    S.st1 = c.arena.alloc<char>(st_bytes);
+    AXC_CUDA(cudaMemsetAsync(mem, 0, head * 4 + st_bytes, c.stream));
+    LAUNCH(c, k_rs_first, std::min<u32>((u32)c.sms, cdiv(n, RSS_CAP)), RSS_WARPS * 32, RSS_SMEM, S, bits);
+    const u32 grid = (u32)std::min<u64>(tiles, (u64)c.sms * 6);
+    for (u32 p = 0; p < S.passes; ++p) {
+        const auto pass = [&](auto kernel) {
+            LAUNCH_AS(c, "k_rs_pass", kernel, grid, RS_WARPS * 32, (size_t)tile * 8, S, p, c.d_status);
+        };
+        if (wide) pass(k_rs_pass<unsigned long long, RS_ITEMS_LARGE>);
+        else if (n <= RS_SMALL_N) pass(k_rs_pass<u32, RS_ITEMS_SMALL>);
+        else pass(k_rs_pass<u32, RS_ITEMS_LARGE>);
     }
-    size_t m = c.arena.mark();
-    const u32 tiles = cdiv(n, RS_TILE);
-    u32 *k2 = c.arena.alloc<u32>(n), *v2 = c.arena.alloc<u32>(n);
-    u32 *hist = c.arena.alloc<u32>((u64)tiles * 256);
-    u32 *ka = keys, *va = vals, *kb = k2, *vb = v2;
-    for (u32 pass = 0, shift = 0; pass < passes; ++pass, shift += 8) {
-        LAUNCH(c, k_rs_hist, tiles, 256, 0, ka, n, shift, hist, tiles, d_n, skip_le);
-        scan_impl<u32, u32>(c, hist, hist, (u64)tiles * 256, d_n, skip_le);
-        LAUNCH(c, k_rs_scatter, tiles, RS_WARPS * 32, 0, ka, va, kb, vb, n, shift, hist, tiles, d_n, skip_le);
-        std::swap(ka, kb);
-        std::swap(va, vb);
-    }
-    if (ka != keys) {
-        AXC_CUDA(cudaMemcpyAsync(keys, ka, n * 4, cudaMemcpyDeviceToDevice, c.stream));
-        AXC_CUDA(cudaMemcpyAsync(vals, va, n * 4, cudaMemcpyDeviceToDevice, c.stream));
-    }
+    LAUNCH(c, k_rs_home, std::min<u32>(cdiv(n, 256), (u32)c.sms * 8), 256, 0, S);
     c.arena.release(m);
 }
 

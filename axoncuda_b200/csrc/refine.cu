@@ -1695,34 +1695,46 @@ __device__ __forceinline__ u32 lower_bound_u32(const u32 *a, u32 n, u32 x) {
 }
 // After the stable sort by group key: the move at position j is the i-th of its group; the i-th of
 // the opposite direction is its partner. Pair gain into psn[node] (indexed by node, so later
-// passes can rebuild the key after any permutation), (pair position << 1 | d) into k1.
-__global__ void k_pair_keys(const u32 *__restrict__ gk, const u32 *__restrict__ pos, const u32 *__restrict__ dM,
+// passes can rebuild the key after any permutation). The order by (pair position, direction), a
+// pair's first direction at its own position and the second one after it, needs no sort: follow[j]
+// counts the moves placed at position j (both of a pair at its first direction's, none at its
+// second's), and its prefix sums are the places; pk[j] is a paired second direction's pair
+// position, else NONE.
+__global__ void k_pair_keys(const u32 *__restrict__ gk, const u32 *__restrict__ pos, const u32 *__restrict__ dM, u32 n,
                             const u32 *__restrict__ mv, const i64 *__restrict__ gain, i64 *__restrict__ psn,
-                            u32 *__restrict__ k1, u32 *__restrict__ node) {
+                            u32 *__restrict__ pk, u32 *__restrict__ node, u32 *__restrict__ follow) {
     const u32 M = *dM, j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= M) return;
+    if (j >= M) {
+        if (j < n) follow[j] = 0;
+        return;
+    }
     const u32 g = gk[j], d = g & 1u;
     const u32 i = j - lower_bound_u32(gk, M, g);
     const u32 s2 = lower_bound_u32(gk, M, g ^ 1u), e2 = lower_bound_u32(gk, M, (g ^ 1u) + 1u);
     const u32 u = mv[pos[j]];
     i64 ps = gain[u];
-    u32 pk = j;
-    if (i < e2 - s2) {
-        ps += gain[mv[pos[s2 + i]]];
-        if (d) pk = s2 + i;
-    }
+    const bool paired = i < e2 - s2;
+    if (paired) ps += gain[mv[pos[s2 + i]]];
     psn[u] = ps;
-    k1[j] = (pk << 1) | d;
+    pk[j] = paired && d ? s2 + i : NONE;
+    follow[j] = paired ? (d ? 0u : 2u) : 1u;
     node[j] = u;
 }
-// Descending pair-gain keys of the permuted movers (hi and lo words of pbound - ps).
-__global__ void k_pair_gain_keys(const u32 *__restrict__ node, const u32 *__restrict__ dM, const i64 *__restrict__ psn,
-                                 u64 pbound, u32 *__restrict__ hi, u32 *__restrict__ lo) {
+// Each move at its place, with the low word of its descending pair-gain key (pbound - ps).
+__global__ void k_pair_place(const u32 *__restrict__ node, const u32 *__restrict__ dM, const u32 *__restrict__ pk,
+                             const u32 *__restrict__ place, const i64 *__restrict__ psn, u64 pbound,
+                             u32 *__restrict__ mv, u32 *__restrict__ lo) {
     const u32 j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= *dM) return;
-    const u64 k = pbound - (u64)psn[node[j]];
-    hi[j] = (u32)(k >> 32);
-    lo[j] = (u32)k;
+    const u32 u = node[j], at = pk[j] != NONE ? place[pk[j]] + 1 : place[j];
+    mv[at] = u;
+    lo[at] = (u32)(pbound - (u64)psn[u]);
+}
+// High words of the permuted movers' descending pair-gain keys.
+__global__ void k_pair_gain_high(const u32 *__restrict__ mv, const u32 *__restrict__ dM, const i64 *__restrict__ psn,
+                                 u64 pbound, u32 *__restrict__ hi) {
+    const u32 j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < *dM) hi[j] = (u32)((pbound - (u64)psn[mv[j]]) >> 32);
 }
 
 // ------------------------------------------------------------------ cascade
@@ -4124,18 +4136,17 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         LAUNCH(c, k_pair_group, cdiv(n, 256), 256, 0, mv, dM, part, target, rp.K, gk, pos);
         radix_sort_pairs_dn(c, gk, pos, dM, n, bits_for(2 * (u64)rp.K * rp.K));
         i64 *psn = c.arena.alloc<i64>(n);
-        u32 *k1 = c.arena.alloc<u32>(n), *node = c.arena.alloc<u32>(n);
-        LAUNCH(c, k_pair_keys, cdiv(n, 256), 256, 0, gk, pos, dM, mv, gain, psn, k1, node);
-        radix_sort_pairs_dn(c, k1, node, dM, n, bits_for(2 * (u64)n));
+        u32 *pk = c.arena.alloc<u32>(n), *node = c.arena.alloc<u32>(n), *follow = c.arena.alloc<u32>(n);
+        LAUNCH(c, k_pair_keys, cdiv(n, 256), 256, 0, gk, pos, dM, n, mv, gain, psn, pk, node, follow);
+        scan_excl_u32(c, follow, follow, n);
         const u64 pbound = 2 * lp.gain_bound;
         const u32 pb = bits_for(pbound);
-        LAUNCH(c, k_pair_gain_keys, cdiv(n, 256), 256, 0, node, dM, psn, pbound, khi, klo);
-        radix_sort_pairs_dn(c, klo, node, dM, n, pb < 32 ? pb : 32);
+        LAUNCH(c, k_pair_place, cdiv(n, 256), 256, 0, node, dM, pk, follow, psn, pbound, mv, klo);
+        radix_sort_pairs_dn(c, klo, mv, dM, n, pb < 32 ? pb : 32);
         if (pb > 32) {
-            LAUNCH(c, k_pair_gain_keys, cdiv(n, 256), 256, 0, node, dM, psn, pbound, khi, klo);
-            radix_sort_pairs_dn(c, khi, node, dM, n, pb - 32);
+            LAUNCH(c, k_pair_gain_high, cdiv(n, 256), 256, 0, mv, dM, psn, pbound, khi);
+            radix_sort_pairs_dn(c, khi, mv, dM, n, pb - 32);
         }
-        AXC_CUDA(cudaMemcpyAsync(mv, node, (size_t)n * 4, cudaMemcpyDeviceToDevice, c.stream));
     }
     u32 *ck = nullptr;  // copies: the copy of every rank, ascending
     if (rp.copies > 1 && !slots) {
