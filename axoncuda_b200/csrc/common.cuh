@@ -302,6 +302,9 @@ void scan_excl_u32(Ctx &c, const u32 *in, u32 *out, u64 n);
 void scan_excl_u64(Ctx &c, const u64 *in, u64 *out, u64 n);
 void scan_excl_i64(Ctx &c, const i64 *in, i64 *out, u64 n);
 void scan_incl_i64(Ctx &c, const i64 *in, i64 *out, u64 n);
+// The exclusive scan of *d_n (at most n) elements, for capacities n that scan_fits.
+bool scan_fits(const Ctx &c, u64 n);
+void scan_excl_i64_dn(Ctx &c, const i64 *in, i64 *out, const u32 *d_n, u64 n);
 // one look-back wait on a tile flag that nothing publishes, polled spin_limit times (the
 // failure path of the scans' bounded waits); throws AXC_EINTERNAL when it gave up
 void lookback_selftest(Ctx &c, u32 spin_limit);

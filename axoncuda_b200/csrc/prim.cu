@@ -187,45 +187,52 @@ __device__ TO lookback_prefix(const ScanState &S, u32 epoch, u32 t, TO tile_tota
     return t > 0 ? *s_prefix : TO(0);
 }
 
-// Scan: out[i] = sum of in[0..i) (exclusive) or in[0..i] (inclusive), in one pass.
+// Scan: out[i] = sum of in[0..i) (exclusive) or in[0..i] (inclusive), in one pass. Blocks take tiles
+// by ticket until none is left; with d_n the element count is *d_n (at most n), so a launch over a
+// large capacity that holds few elements costs its few tiles.
 template <class TI, class TO, bool INCL>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_lb(const TI *__restrict__ in, TO *__restrict__ out, u64 n,
-                                                        ScanState S, u32 *status) {
+                                                        ScanState S, u32 *status, const u32 *__restrict__ d_n) {
     __shared__ TO wt[33];
     __shared__ TO stage[SCAN_TILE + SCAN_TILE / 32];
     __shared__ u32 s_tile, s_epoch;
     __shared__ TO s_prefix;
+    if (d_n) n = *d_n < n ? *d_n : n;
     u32 epoch;
-    const u32 t = lb_enter(S, s_tile, s_epoch, epoch);
-    const u64 base = (u64)t * SCAN_TILE;
-    for (int j = 0; j < SCAN_ITEMS; ++j) {
-        int li = j * SCAN_THREADS + threadIdx.x;
-        u64 i = base + li;
-        stage[li + li / 32] = i < n ? (TO)in[i] : TO(0);
-    }
-    __syncthreads();
-    TO loc[SCAN_ITEMS];
-    TO s = 0;
+    for (;;) {
+        const u32 t = lb_enter(S, s_tile, s_epoch, epoch);
+        const u64 base = (u64)t * SCAN_TILE;
+        if (base >= n) break;
+        for (int j = 0; j < SCAN_ITEMS; ++j) {
+            int li = j * SCAN_THREADS + threadIdx.x;
+            u64 i = base + li;
+            stage[li + li / 32] = i < n ? (TO)in[i] : TO(0);
+        }
+        __syncthreads();
+        TO loc[SCAN_ITEMS];
+        TO s = 0;
 #pragma unroll
-    for (int j = 0; j < SCAN_ITEMS; ++j) {
-        int li = threadIdx.x * SCAN_ITEMS + j;
-        loc[j] = stage[li + li / 32];
-        s += loc[j];
-    }
-    TO tot;
-    TO pre = block_excl_scan<TO>(s, wt, tot);
-    pre += lookback_prefix<TO>(S, epoch, t, tot, status, &s_prefix);
+        for (int j = 0; j < SCAN_ITEMS; ++j) {
+            int li = threadIdx.x * SCAN_ITEMS + j;
+            loc[j] = stage[li + li / 32];
+            s += loc[j];
+        }
+        TO tot;
+        TO pre = block_excl_scan<TO>(s, wt, tot);
+        pre += lookback_prefix<TO>(S, epoch, t, tot, status, &s_prefix);
 #pragma unroll
-    for (int j = 0; j < SCAN_ITEMS; ++j) {
-        int li = threadIdx.x * SCAN_ITEMS + j;
-        stage[li + li / 32] = INCL ? pre + loc[j] : pre;
-        pre += loc[j];
-    }
-    __syncthreads();
-    for (int j = 0; j < SCAN_ITEMS; ++j) {
-        int li = j * SCAN_THREADS + threadIdx.x;
-        u64 i = base + li;
-        if (i < n) out[i] = stage[li + li / 32];
+        for (int j = 0; j < SCAN_ITEMS; ++j) {
+            int li = threadIdx.x * SCAN_ITEMS + j;
+            stage[li + li / 32] = INCL ? pre + loc[j] : pre;
+            pre += loc[j];
+        }
+        __syncthreads();
+        for (int j = 0; j < SCAN_ITEMS; ++j) {
+            int li = j * SCAN_THREADS + threadIdx.x;
+            u64 i = base + li;
+            if (i < n) out[i] = stage[li + li / 32];
+        }
+        __syncthreads();  // the tile's shared state is no longer read
     }
     lb_leave(S, epoch);
 }
@@ -261,13 +268,15 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_compact_lb(const u32 *__restri
 }
 
 template <class TI, class TO, bool INCL = false>
-void scan_impl(Ctx &c, const TI *in, TO *out, u64 n) {
+void scan_impl(Ctx &c, const TI *in, TO *out, u64 n, const u32 *d_n = nullptr) {
     if (n == 0) return;
     const u32 tiles = cdiv(n, SCAN_TILE);
     if (tiles <= c.scan.cap_tiles) {
-        LAUNCH(c, (k_scan_lb<TI, TO, INCL>), tiles, SCAN_THREADS, 0, in, out, n, c.scan, c.d_status);
+        LAUNCH_AS(c, "k_scan_lb", (k_scan_lb<TI, TO, INCL>), std::min<u32>(tiles, (u32)c.sms * 8), SCAN_THREADS, 0, in,
+                  out, n, c.scan, c.d_status, d_n);
         return;
     }
+    if (d_n) throw Error(AXC_EINTERNAL, "scan of a device count longer than the look-back tile state");
     if (INCL) throw Error(AXC_EOVERFLOW, "inclusive scan longer than the look-back tile state");
     if (tiles == 1) {
         LAUNCH(c, (k_tile_scan<TI, TO>), 1, SCAN_THREADS, 0, in, out, (const TO *)nullptr, n);
@@ -593,6 +602,8 @@ void scan_excl_u32(Ctx &c, const u32 *in, u32 *out, u64 n) { scan_impl<u32, u32>
 void scan_excl_u64(Ctx &c, const u64 *in, u64 *out, u64 n) { scan_impl<u64, u64>(c, in, out, n); }
 void scan_excl_i64(Ctx &c, const i64 *in, i64 *out, u64 n) { scan_impl<i64, i64>(c, in, out, n); }
 void scan_incl_i64(Ctx &c, const i64 *in, i64 *out, u64 n) { scan_impl<i64, i64, true>(c, in, out, n); }
+bool scan_fits(const Ctx &c, u64 n) { return cdiv(n, SCAN_TILE) <= c.scan.cap_tiles; }
+void scan_excl_i64_dn(Ctx &c, const i64 *in, i64 *out, const u32 *d_n, u64 n) { scan_impl<i64, i64>(c, in, out, n, d_n); }
 
 void lookback_selftest(Ctx &c, u32 spin_limit) {
     const size_t m = c.arena.mark();

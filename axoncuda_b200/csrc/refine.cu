@@ -2490,43 +2490,48 @@ __global__ void k_gather_g2(const u32 *__restrict__ mv, const u32 *__restrict__ 
     }
 }
 
+// The event kernels loop over the device's counts: their capacities (two events per node, two
+// transitions per destination pin) are mostly empty.
+__device__ __forceinline__ u64 grid_first() { return (u64)blockIdx.x * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ u64 grid_step() { return (u64)gridDim.x * blockDim.x; }
 // size events: 2r = leave p, 2r+1 = join q
 __global__ void k_size_events(const u32 *__restrict__ mv, const u32 *__restrict__ dM, const u32 *__restrict__ part,
                               const u32 *__restrict__ target, u32 *__restrict__ key, u32 *__restrict__ val) {
-    u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 2 * *dM) return;
-    u32 v = mv[i >> 1];
-    key[i] = (i & 1) ? target[v] : part[v];
-    val[i] = i;
+    const u64 ne = 2 * (u64)*dM;
+    for (u64 i = grid_first(); i < ne; i += grid_step()) {
+        const u32 v = mv[i >> 1];
+        key[i] = (i & 1) ? target[v] : part[v];
+        val[i] = (u32)i;
+    }
 }
 __global__ void k_size_delta(const u32 *__restrict__ mv, const u32 *__restrict__ val, const u32 *__restrict__ dne,
-                             u32 nmax, const u32 *__restrict__ nsize, i64 *__restrict__ d) {
-    u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nmax) return;
-    if (i >= *dne) { d[i] = 0; return; }
-    u32 ev = val[i];
-    i64 s = nsize[mv[ev >> 1]];
-    d[i] = (ev & 1) ? s : -s;
+                             const u32 *__restrict__ nsize, i64 *__restrict__ d) {
+    const u32 ne = *dne;
+    for (u64 i = grid_first(); i < ne; i += grid_step()) {
+        const u32 ev = val[i];
+        const i64 s = nsize[mv[ev >> 1]];
+        d[i] = (ev & 1) ? s : -s;
+    }
 }
 __global__ void k_size_flags(const u32 *__restrict__ key, const u32 *__restrict__ val, const i64 *__restrict__ d,
                              const i64 *__restrict__ E, const u32 *__restrict__ dne, const u64 *__restrict__ psize,
                              u64 omega, unsigned long long *__restrict__ Vs) {
-    u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 ne = *dne;
-    if (i >= ne) return;
-    u32 p = key[i];
-    u32 st = lower_bound_u32(key, ne, p);
-    i64 before = (i64)psize[p] + (E[i] - E[st]);
-    i64 after = before + d[i];
-    i64 exb = before > (i64)omega ? before - (i64)omega : 0;
-    i64 exa = after > (i64)omega ? after - (i64)omega : 0;
-    if (exa != exb) atomicAdd(&Vs[val[i] >> 1], (unsigned long long)(exa - exb));
+    for (u64 i = grid_first(); i < ne; i += grid_step()) {
+        const u32 p = key[i];
+        const u32 st = lower_bound_u32(key, ne, p);
+        const i64 before = (i64)psize[p] + (E[i] - E[st]);
+        const i64 after = before + d[i];
+        const i64 exb = before > (i64)omega ? before - (i64)omega : 0;
+        const i64 exa = after > (i64)omega ? after - (i64)omega : 0;
+        if (exa != exb) atomicAdd(&Vs[val[i] >> 1], (unsigned long long)(exa - exb));
+    }
 }
 
 __global__ void k_gather_by_dn(const u32 *__restrict__ src, const u32 *__restrict__ idx, u32 *__restrict__ dst,
                                const u32 *__restrict__ dn) {
-    u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < *dn) dst[i] = src[idx[i]];
+    const u32 n = *dn;
+    for (u64 i = grid_first(); i < n; i += grid_step()) dst[i] = src[idx[i]];
 }
 // transition keys: (partition, rank) in one word when both fit, else the rank alone (the
 // partition is then a second stable pass). The count is clamped to the capacity nmax first (an
@@ -2534,24 +2539,25 @@ __global__ void k_gather_by_dn(const u32 *__restrict__ src, const u32 *__restric
 __global__ void k_trans_keys(u32 *__restrict__ dT, u64 nmax, const u32 *__restrict__ tp,
                              const u32 *__restrict__ tr, u32 rbits, int combined, u32 *__restrict__ key,
                              u32 *__restrict__ perm) {
-    u64 j = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    const u64 cnt = *dT < nmax ? *dT : nmax;
-    if (j == 0 && cnt < *dT) atomicMin(dT, (u32)cnt);
-    if (j >= cnt) return;
-    key[j] = combined ? ((tp[j] << rbits) | tr[j]) : tr[j];
-    perm[j] = (u32)j;
+    const u64 j0 = grid_first(), cnt = *dT < nmax ? *dT : nmax;
+    if (j0 == 0 && cnt < *dT) atomicMin(dT, (u32)cnt);
+    for (u64 j = j0; j < cnt; j += grid_step()) {
+        key[j] = combined ? ((tp[j] << rbits) | tr[j]) : tr[j];
+        perm[j] = (u32)j;
+    }
 }
-// after ordering by (p, r): partition, rank and delta of position i
-__global__ void k_trans_perm(const u32 *__restrict__ perm, const u32 *__restrict__ dT, u64 nmax,
+// after ordering by (p, r): partition, rank and delta of position i; the deltas of [*dT, nz) are zero
+__global__ void k_trans_perm(const u32 *__restrict__ perm, const u32 *__restrict__ dT, u64 nz,
                              const u32 *__restrict__ tp, const u32 *__restrict__ tr, const int32_t *__restrict__ td,
                              u32 *__restrict__ sp, u32 *__restrict__ sr, i64 *__restrict__ sd) {
-    u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nmax) return;
-    if (i >= *dT) { sd[i] = 0; return; }
-    const u32 j = perm[i];
-    sp[i] = tp[j];
-    sr[i] = tr[j];
-    sd[i] = td[j];
+    const u64 nt = *dT, end = nt > nz ? nt : nz;
+    for (u64 i = grid_first(); i < end; i += grid_step()) {
+        if (i >= nt) { sd[i] = 0; continue; }
+        const u32 j = perm[i];
+        sp[i] = tp[j];
+        sr[i] = tr[j];
+        sd[i] = td[j];
+    }
 }
 // per partition, the running inbound-set size along the move sequence; an event that makes the
 // partition exceed delta adds +1 at its rank, one that brings it back adds -1. The first event of a
@@ -2559,16 +2565,16 @@ __global__ void k_trans_perm(const u32 *__restrict__ perm, const u32 *__restrict
 __global__ void k_trans_flags(const u32 *__restrict__ sp, const u32 *__restrict__ sr, const i64 *__restrict__ sd,
                               const i64 *__restrict__ E, const u32 *__restrict__ dT, const u64 *__restrict__ pinb,
                               u64 delta, unsigned long long *__restrict__ Vi) {
-    u32 j = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 nt = *dT;
-    if (j >= nt) return;
-    const u32 p = sp[j];
-    const u32 st = lower_bound_u32(sp, nt, p);  // the partition's first transition (sp is sorted)
-    const i64 before = (i64)pinb[p] + (E[j] - E[st]);
-    const i64 after = before + sd[j];
-    const bool was_bad = (j != st) && before > (i64)delta;
-    const bool is_bad = after > (i64)delta;
-    if (was_bad != is_bad) atomicAdd(&Vi[sr[j]], (unsigned long long)(i64)(is_bad ? 1 : -1));
+    for (u64 j = grid_first(); j < nt; j += grid_step()) {
+        const u32 p = sp[j];
+        const u32 st = lower_bound_u32(sp, nt, p);  // the partition's first transition (sp is sorted)
+        const i64 before = (i64)pinb[p] + (E[j] - E[st]);
+        const i64 after = before + sd[j];
+        const bool was_bad = (j != st) && before > (i64)delta;
+        const bool is_bad = after > (i64)delta;
+        if (was_bad != is_bad) atomicAdd(&Vi[sr[j]], (unsigned long long)(i64)(is_bad ? 1 : -1));
+    }
 }
 
 // ---- size and inbound validity of every prefix on small levels: one block per partition ----------
@@ -4276,12 +4282,13 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         size_t m1 = c.arena.mark();
         const u32 nemax = 2 * n;
         u32 *key = c.arena.alloc<u32>(nemax), *val = c.arena.alloc<u32>(nemax);
-        LAUNCH(c, k_size_events, cdiv(nemax, 256), 256, 0, mv, dM, part, target, key, val);
+        const u32 ge = std::min<u32>(cdiv(nemax, 256), (u32)c.sms * 8);
+        LAUNCH(c, k_size_events, ge, 256, 0, mv, dM, part, target, key, val);
         radix_sort_pairs_dn(c, key, val, dSE, nemax, bits_for(rp.K ? rp.K - 1 : 0));
         i64 *d = c.arena.alloc<i64>(nemax), *E = c.arena.alloc<i64>(nemax);
-        LAUNCH(c, k_size_delta, cdiv(nemax, 256), 256, 0, mv, val, dSE, nemax, L.nsize, d);
-        scan_excl_i64(c, d, E, nemax);
-        LAUNCH(c, k_size_flags, cdiv(nemax, 256), 256, 0, key, val, d, E, dSE, psize, (u64)rp.omega,
+        LAUNCH(c, k_size_delta, ge, 256, 0, mv, val, dSE, L.nsize, d);
+        scan_excl_i64_dn(c, d, E, dSE, nemax);
+        LAUNCH(c, k_size_flags, ge, 256, 0, key, val, d, E, dSE, psize, (u64)rp.omega,
                (unsigned long long *)Vs);
         c.arena.release(m1);
     }
@@ -4293,19 +4300,22 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         const u32 rb = bits_for(n ? n - 1 : 0), pb = bits_for(rp.K ? rp.K - 1 : 0);
         const bool combined = rb + pb <= 32;
         u32 *key = c.arena.alloc<u32>(nt), *perm = c.arena.alloc<u32>(nt);
-        LAUNCH(c, k_trans_keys, cdiv(nt, 256), 256, 0, dT, nt, tp, tr, rb, combined ? 1 : 0, key, perm);
+        const u32 gt = std::min<u32>(cdiv(nt, 256), (u32)c.sms * 8);
+        LAUNCH(c, k_trans_keys, gt, 256, 0, dT, nt, tp, tr, rb, combined ? 1 : 0, key, perm);
         if (combined) {
             radix_sort_pairs_dn(c, key, perm, dT, nt, rb + pb);
         } else {
             radix_sort_pairs_dn(c, key, perm, dT, nt, rb);
-            LAUNCH(c, k_gather_by_dn, cdiv(nt, 256), 256, 0, tp, perm, key, dT);
+            LAUNCH(c, k_gather_by_dn, gt, 256, 0, tp, perm, key, dT);
             radix_sort_pairs_dn(c, key, perm, dT, nt, pb);
         }
         u32 *sp = c.arena.alloc<u32>(nt), *sr = key;
         i64 *sd = c.arena.alloc<i64>(nt), *E2 = c.arena.alloc<i64>(nt);
-        LAUNCH(c, k_trans_perm, cdiv(nt, 256), 256, 0, perm, dT, nt, tp, tr, tdv, sp, sr, sd);
-        scan_excl_i64(c, sd, E2, nt);
-        LAUNCH(c, k_trans_flags, cdiv(nt, 256), 256, 0, sp, sr, sd, E2, dT, pinb, (u64)rp.delta,
+        const bool fits = scan_fits(c, nt);  // else the whole capacity is scanned, past the count as zeros
+        LAUNCH(c, k_trans_perm, fits ? gt : cdiv(nt, 256), 256, 0, perm, dT, fits ? 0 : nt, tp, tr, tdv, sp, sr, sd);
+        if (fits) scan_excl_i64_dn(c, sd, E2, dT, nt);
+        else scan_excl_i64(c, sd, E2, nt);
+        LAUNCH(c, k_trans_flags, gt, 256, 0, sp, sr, sd, E2, dT, pinb, (u64)rp.delta,
                (unsigned long long *)Vi);
         c.arena.release(m1);
     }
