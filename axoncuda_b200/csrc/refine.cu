@@ -927,17 +927,19 @@ __global__ void __launch_bounds__(GN_BLOCK) k_gain_block(GainArgs A0, const u32 
 constexpr u32 GS_K = AXC_SPARSE_GAIN_K;
 constexpr u32 GS_SAMPLE = AXC_SPARSE_GAIN_SAMPLE;
 constexpr u32 GS_C = AXC_SPARSE_GAIN_CANDIDATES;
-constexpr u32 GS_TAB = 2 * GS_SAMPLE;                // sample table slots: at most half full
+constexpr u32 GS_TAB = 2 * GS_SAMPLE;  // hashed sample table: at most half full
 constexpr u32 GS_BLOCK = 256;
-constexpr u32 GS_PER_SM = 2;                         // resident sample blocks per SM
-constexpr u32 GS_DC_BITS = 13;                       // a slot's inbound count (<= GS_SAMPLE) in its low bits
-constexpr u64 GS_DC_MASK = (1ull << GS_DC_BITS) - 1;
-constexpr u64 GS_RULED_OUT = 1ull << 63;             // slot mark: the size or inbound bound rules it out
-static_assert(GS_SAMPLE <= GS_DC_MASK && GS_DC_BITS + 32 + 13 <= 64 && GS_SAMPLE <= 8192,
-              "packed slot: inbound count below the connectivity (<= GS_SAMPLE u32 weights)");
-static_assert(GS_TAB <= 65536, "used-slot list holds 16-bit slots");
-constexpr size_t GS_SMEM = (size_t)GS_TAB * 12 + (size_t)GS_SAMPLE * 2;  // packed u64 and key u32 per
-                                                     // slot; the used-slot list (u16)
+constexpr u32 GS_LIST = 256;           // keys the final selection of the candidates looks at
+// A slot of the sample table holds a partition's sampled connectivity and inbound count in 32-bit
+// words (64-bit shared adds would be compare-and-swap loops). Equal weights: one word, incidences
+// holding the partition above, inbound ones with a destination pin in it below. Else the low word
+// of the connectivity, and a word with its carries above, the inbound count below and GS_ZERO set
+// by a zero weight, so that a present slot is never all zero.
+constexpr u32 GS_HI = 16, GS_LOW = 0xFFFFu, GS_ZERO = 0x80000000u;
+static_assert(GS_SAMPLE < GS_LOW / 2, "counts and carries fit their half words");
+// The table is indexed by partition where that takes no more room than the hashed one (UNI: one
+// word per slot against a key and one), which also makes its scans read psize and pinb in order.
+constexpr u32 GS_DIRECT_UNI = 2 * GS_TAB, GS_DIRECT_GEN = GS_TAB + GS_TAB / 2;
 // Nodes outside the sampled kernels (gain tiers 0 and 1) have at most GN_BLOCK_W census entries,
 // so their sample would be the whole node and the exact kernels give the rule's result.
 static_assert(GN_BLOCK_W <= GS_SAMPLE, "tier-1 nodes must fit the sample");
@@ -1252,101 +1254,123 @@ struct CandAcc {
     unsigned long long *sacc, *wacc;  // [rows]
 };
 
-// Inserts k into the descending list top[0, GS_C) (keys not above the last entry drop out).
-__device__ __forceinline__ void skey_insert(SKey (&top)[GS_C], SKey k) {
-#pragma unroll
-    for (u32 i = 0; i < GS_C; ++i)
-        if (skey_better(k, top[i])) {
-            const SKey t = top[i];
-            top[i] = k;
-            k = t;
-        }
-}
-// The warp's best of its lanes' lists, GS_C times: out[r] = the r-th best over the warp (empty
-// keys are {0, 0}, below every real key, whose low word holds ~q with q < 2^32 - 2).
-__device__ __forceinline__ void skey_warp_top(SKey (&top)[GS_C], SKey *out) {
-    const u32 lane = threadIdx.x & 31u;
-    for (u32 r = 0; r < GS_C; ++r) {
-        SKey b = top[0];
-        u32 bl = lane;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const SKey c{__shfl_xor_sync(0xFFFFFFFFu, b.hi, o), __shfl_xor_sync(0xFFFFFFFFu, b.lo, o)};
-            const u32 cl = __shfl_xor_sync(0xFFFFFFFFu, bl, o);
-            if (skey_better(c, b) || (!skey_better(b, c) && cl < bl)) { b = c; bl = cl; }
-        }
-        if (lane == 0) out[r] = b;
-        if (lane == bl) {  // the winner drops its head
-#pragma unroll
-            for (u32 i = 0; i + 1 < GS_C; ++i) top[i] = top[i + 1];
-            top[GS_C - 1] = SKey{0, 0};
-        }
-    }
-}
-
-__global__ void __launch_bounds__(GS_BLOCK, GS_PER_SM) k_gain_sample(GainArgs A0, const u32 *__restrict__ list, u32 nl,
-                                                             CandAcc C) {
+// UNI: every hyperedge has the weight w. DIRECT: slots are partitions (T = K), else a hash table of
+// T = GS_TAB slots. One block per node at a time; the table is empty between nodes: the last scan
+// of a node clears it.
+template <bool UNI, bool DIRECT>
+__global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const u32 *__restrict__ list, u32 nl, CandAcc C,
+                                                         u32 T, u32 weight) {
     const GainArgs A = gain_args_now(A0);
-    extern __shared__ unsigned long long gs_dyn[];
-    unsigned long long *sacc = gs_dyn;       // [GS_TAB]: sampled connectivity << GS_DC_BITS | inbound count
-    u32 *keys = (u32 *)(gs_dyn + GS_TAB);    // [GS_TAB]
-    unsigned short *used = (unsigned short *)(keys + GS_TAB);  // [GS_SAMPLE]: the slots the node filled
-    __shared__ unsigned long long wsh[GS_BLOCK / 32];
+    extern __shared__ u32 gs_tab[];
+    u32 *v0 = gs_tab, *v1 = UNI ? nullptr : gs_tab + T, *keys = DIRECT ? nullptr : gs_tab + (UNI ? 1 : 2) * T;
+    constexpr u32 NW = GS_BLOCK / 32;
+    __shared__ unsigned long long wsh[NW];
     __shared__ unsigned long long s_acc;
-    __shared__ Cand cred[GS_BLOCK / 32];
-    __shared__ SKey kred[(GS_BLOCK / 32) * GS_C];
-    __shared__ u32 ndist;
-    // the first GS_BLOCK incidences: exclusive census prefix (entry GS_BLOCK or m = the sample's
-    // total), census offset and weight
+    __shared__ Cand cred[NW];
+    __shared__ SKey kred[NW], kout[GS_C], klist[GS_LIST];
+    __shared__ u32 nkeys;
+    // the first GS_BLOCK incidences: exclusive census prefix (entry m = the sample's total when m is
+    // at most GS_BLOCK), census offset and weight
     __shared__ u32 s_ex[GS_BLOCK + 1], s_w[GS_BLOCK];
     __shared__ u64 s_off[GS_BLOCK];
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (u32 i = threadIdx.x; i < GS_TAB; i += GS_BLOCK) { keys[i] = NONE; sacc[i] = 0; }
+    for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
+        v0[i] = 0;
+        if (!UNI) v1[i] = 0;
+        if (!DIRECT) keys[i] = NONE;
+    }
+    // slot contents
+    const auto present = [&](u32 i) { return UNI ? v0[i] != 0 : (v0[i] | v1[i]) != 0; };
+    const auto conn_of = [&](u32 i) {
+        return UNI ? (u64)(v0[i] >> GS_HI) * weight : ((u64)((v1[i] & ~GS_ZERO) >> GS_HI) << 32) | v0[i];
+    };
+    const auto dcon_of = [&](u32 i) { return UNI ? v0[i] & GS_LOW : v1[i] & GS_LOW; };
+    const auto part_of = [&](u32 i) { return DIRECT ? i : keys[i]; };
+    const auto clear = [&](u32 i) {
+        v0[i] = 0;
+        if (!UNI) v1[i] = 0;
+        if (!DIRECT) keys[i] = NONE;
+    };
+    const auto key_of = [&](u32 i) {
+        const u32 q = part_of(i);
+        return SKey{conn_of(i), ((u64)mix32(q + A.round + A.seed) << 32) | (u64)(~q)};
+    };
     for (u32 idx = blockIdx.x; idx < nl; idx += gridDim.x) {
         const u32 u = list[idx], p = A.part[u];
         const u64 t0 = A.toff[u];
         const u32 deg = (u32)(A.toff[u + 1] - t0), nin_u = A.nin[u];
-        if (threadIdx.x == 0) ndist = 0;
-        // 1. the sample: the longest incidence prefix with at most GS_SAMPLE census entries
+        // 1. the sample: the longest incidence prefix with at most GS_SAMPLE census entries. Nodes at
+        // this many partitions mostly pass it within 32 incidences, which every warp looks at.
         u32 m = 0;
         u64 acc = 0;
-        for (u32 base = 0; base < deg; base += GS_BLOCK) {
-            const u32 j = base + threadIdx.x;
-            const u32 h = j < deg ? A.touch[t0 + j] : 0;
-            const u32 lm = j < deg ? A.lam[h] : 0;
-            if (base == 0 && j < deg) {
-                s_off[j] = A.off[h];
-                s_w[j] = A.wfx[h];
-            }
+        {
+            const u32 h = lane < deg ? A.touch[t0 + lane] : 0;
+            const u32 lm = lane < deg ? A.lam[h] : 0;
             u64 x = lm;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const u64 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
                 if ((int)lane >= o) x += y;
             }
-            if (lane == 31) wsh[warp] = x;
-            __syncthreads();
-            for (u32 i = 0; i < warp; ++i) x += wsh[i];
-            if (base == 0) s_ex[threadIdx.x] = (u32)(x - lm < GS_SAMPLE ? x - lm : GS_SAMPLE);  // exact for j < m
-            const bool take = j < deg && acc + x <= GS_SAMPLE;
-            const u32 cnt = (u32)__syncthreads_count(take);
-            if (cnt > 0 && threadIdx.x == cnt - 1) s_acc = acc + x;
-            __syncthreads();
-            m += cnt;
-            if (cnt > 0) acc = s_acc;
-            if (cnt < GS_BLOCK) break;
+            m = __popc(__ballot_sync(0xFFFFFFFFu, lane < deg && x <= GS_SAMPLE));
+            if (m) acc = __shfl_sync(0xFFFFFFFFu, x, m - 1);
+            if (warp == 0 && lane < m) {
+                s_off[lane] = A.off[h];
+                s_w[lane] = UNI ? weight : A.wfx[h];
+                s_ex[lane] = (u32)(x - lm);
+                if (lane == m - 1) s_ex[m] = (u32)x;
+            }
         }
-        if (threadIdx.x == 0 && m <= GS_BLOCK) s_ex[m] = (u32)acc;
+        if (m == 32 && deg > 32) {  // uniform over the block: the general prefix
+            __syncthreads();
+            m = 0;
+            acc = 0;
+            for (u32 base = 0; base < deg; base += GS_BLOCK) {
+                const u32 j = base + threadIdx.x;
+                const u32 h = j < deg ? A.touch[t0 + j] : 0;
+                const u32 lm = j < deg ? A.lam[h] : 0;
+                if (base == 0 && j < deg) {
+                    s_off[j] = A.off[h];
+                    s_w[j] = A.wfx[h];
+                }
+                u64 x = lm;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const u64 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                    if ((int)lane >= o) x += y;
+                }
+                if (lane == 31) wsh[warp] = x;
+                __syncthreads();
+                for (u32 i = 0; i < warp; ++i) x += wsh[i];
+                if (base == 0) s_ex[threadIdx.x] = (u32)(x - lm < GS_SAMPLE ? x - lm : GS_SAMPLE);  // exact for j < m
+                const bool take = j < deg && acc + x <= GS_SAMPLE;
+                const u32 cnt = (u32)__syncthreads_count(take);
+                if (cnt > 0 && threadIdx.x == cnt - 1) s_acc = acc + x;
+                __syncthreads();
+                m += cnt;
+                if (cnt > 0) acc = s_acc;
+                if (cnt < GS_BLOCK) break;
+            }
+            if (threadIdx.x == 0 && m <= GS_BLOCK) s_ex[m] = (u32)acc;
+        }
         __syncthreads();
         // 2. sampled connectivity; saving and wtot are exact when the sample is the whole node
         i64 saving = 0, wtot = 0;
         const auto put = [&](u64 k, u32 q, u32 w, bool dst) {
             if (q == p) { saving += leave_gain(A.encourage, w, A.ccnt[k]); return; }
-            bool fresh = false;
-            const u32 slot = hash_insert_fresh(keys, GS_TAB - 1, q, fresh);
-            if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); return; }
-            if (fresh) used[atomicAdd(&ndist, 1u)] = (unsigned short)slot;  // at most GS_SAMPLE distinct keys
-            atomicAdd(&sacc[slot], ((unsigned long long)w << GS_DC_BITS) | (dst ? 1ull : 0ull));
+            u32 slot = q;
+            if (!DIRECT) {
+                slot = hash_find_or_insert(keys, T - 1, q);
+                if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); return; }
+            }
+            if (UNI) {
+                atomicAdd(&v0[slot], (1u << GS_HI) | (dst ? 1u : 0u));
+            } else {
+                const u32 old = atomicAdd(&v0[slot], w);
+                const u32 up = (old + w < old ? 1u << GS_HI : 0u) | (dst ? 1u : 0u);
+                if (up) atomicAdd(&v1[slot], up);
+                if (w == 0) atomicOr(&v1[slot], GS_ZERO);
+            }
         };
         if (m <= GS_BLOCK) {
             // the sample's acc entries split evenly over the block: thread t takes entries t,
@@ -1377,110 +1401,112 @@ __global__ void __launch_bounds__(GS_BLOCK, GS_PER_SM) k_gain_sample(GainArgs A0
             census_flat(A, u, 32 * warp, GS_BLOCK, m, wtot,
                         [&](u64 k, u32 q, u32 w, u32 io) { put(k, q, w, io && q != p && A.cdcnt[k] > 0); });
         }
+        if (threadIdx.x == 0) nkeys = 0;
         __syncthreads();
-        const u32 nd = ndist;
         const u64 s = A.nsize[u];
         if (m == deg) {  // 3a. the whole node: exact, as the table kernels
             saving = (i64)block_sum_u64((u64)saving, wsh);
             wtot = (i64)block_sum_u64((u64)wtot, wsh);
             Cand best{INT64_MIN, 0};
-            for (u32 t = threadIdx.x; t < nd; t += GS_BLOCK) {
-                const u32 i = used[t];
-                const Cand c = gain_candidate(A, u, keys[i], sacc[i] >> GS_DC_BITS, (u32)(sacc[i] & GS_DC_MASK), saving,
-                                              wtot);
+            for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
+                if (!present(i)) continue;
+                const Cand c = gain_candidate(A, u, part_of(i), conn_of(i), dcon_of(i), saving, wtot);
                 if (cand_better(c, best)) best = c;
+                clear(i);
             }
             best = warp_best(best);
             if (lane == 0) cred[warp] = best;
             __syncthreads();
             if (threadIdx.x == 0) {
                 Cand b = cred[0];
-                for (u32 i = 1; i < GS_BLOCK / 32; ++i)
+                for (u32 i = 1; i < NW; ++i)
                     if (cand_better(cred[i], b)) b = cred[i];
                 write_move(A, u, b);  // spos[u] stays NONE
             }
-        } else {
-            // 3b. the GS_C best by (sampled connectivity, tie hash, -id) among the keys the size
-            // limit and the inbound bound do not rule out. Pass 1 marks the ruled-out slots and
-            // takes each warp's best key; the least of those GS_BLOCK / 32 >= GS_C keys is no
-            // better than the GS_C-th best, so pass 2 lists only the keys at or above it
-            // (per-thread lists, then per warp, then warp 0 over the warps' lists).
-            const u64 in_sample = m < nin_u ? m : nin_u;
-            SKey best1{0, 0};
-            constexpr u32 U = 4;  // keys per thread whose partition loads are in flight together
-            for (u32 t0 = threadIdx.x; t0 < nd; t0 += U * GS_BLOCK) {
-                u32 qs[U], is[U];
-                u64 ps[U], pb[U];
-#pragma unroll
-                for (u32 r = 0; r < U; ++r) {
-                    const u32 t = t0 + r * GS_BLOCK;
-                    is[r] = t < nd ? used[t] : 0;
-                    qs[r] = t < nd ? keys[is[r]] : NONE;
-                    ps[r] = qs[r] != NONE ? A.psize[qs[r]] : 0;
-                    pb[r] = qs[r] != NONE ? A.pinb[qs[r]] : 0;
-                }
-#pragma unroll
-                for (u32 r = 0; r < U; ++r) {
-                    const u32 q = qs[r], i = is[r];
-                    if (q == NONE) continue;
-                    const u64 v = sacc[i];
-                    if (ps[r] + s - s / A.discount > A.omega || pb[r] + in_sample - (v & GS_DC_MASK) > A.delta) {
-                        sacc[i] = v | GS_RULED_OUT;
-                        continue;
-                    }
-                    const SKey k{v >> GS_DC_BITS, ((u64)mix32(q + A.round + A.seed) << 32) | (u64)(~q)};
-                    if (skey_better(k, best1)) best1 = k;
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const SKey c{__shfl_xor_sync(0xFFFFFFFFu, best1.hi, o), __shfl_xor_sync(0xFFFFFFFFu, best1.lo, o)};
-                if (skey_better(c, best1)) best1 = c;
-            }
-            if (lane == 0) kred[warp] = best1;
             __syncthreads();
-            SKey thr = kred[0];
-            for (u32 w2 = 1; w2 < GS_BLOCK / 32; ++w2)
-                if (skey_better(thr, kred[w2])) thr = kred[w2];
-            __syncthreads();  // kred is reused below
-            SKey top[GS_C];
-#pragma unroll
-            for (u32 r = 0; r < GS_C; ++r) top[r] = SKey{0, 0};
-            for (u32 t = threadIdx.x; t < nd; t += GS_BLOCK) {
-                const u32 i = used[t];
-                const u64 v = sacc[i];
-                if (v & GS_RULED_OUT) continue;
-                const u32 q = keys[i];
-                const SKey k{v >> GS_DC_BITS, ((u64)mix32(q + A.round + A.seed) << 32) | (u64)(~q)};
-                if (!skey_better(thr, k)) skey_insert(top, k);
+            continue;
+        }
+        // 3b. the GS_C best by (sampled connectivity, tie hash, -id) among the keys the size limit and
+        // the inbound bound do not rule out. Pass 1 empties the ruled-out slots and takes each warp's
+        // best key; the least of those NW >= GS_C keys is no better than the GS_C-th best, so pass 2
+        // lists the keys at or above it (a few dozen), whose ranks are counted pairwise.
+        const u64 in_sample = m < nin_u ? m : nin_u, need = s - s / A.discount;
+        SKey best1{0, 0};
+#pragma unroll 4
+        for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
+            if (!present(i)) continue;
+            const u32 q = part_of(i);
+            if (A.psize[q] + need > A.omega || A.pinb[q] + in_sample - dcon_of(i) > A.delta) {
+                clear(i);  // (its key goes as well: nothing is inserted any more)
+                continue;
             }
-            skey_warp_top(top, kred + warp * GS_C);
-            __syncthreads();
-            if (warp == 0) {
+            const SKey k = key_of(i);
+            if (skey_better(k, best1)) best1 = k;
+        }
 #pragma unroll
-                for (u32 r = 0; r < GS_C; ++r) top[r] = SKey{0, 0};
-                for (u32 t = lane; t < (GS_BLOCK / 32) * GS_C; t += 32) skey_insert(top, kred[t]);
-                __syncwarp();  // every lane has read kred before lane 0 overwrites its head
-                skey_warp_top(top, kred);
-                __syncwarp();
-                if (lane < GS_C) {  // the candidates and a zeroed accumulator row (row = list index)
-                    const SKey b = kred[lane];
-                    C.cand[(u64)u * GS_C + lane] = (b.hi | b.lo) ? ~(u32)b.lo : NONE;
-                    C.conn[(u64)idx * GS_C + lane] = 0;
-                    C.dcon[(u64)idx * GS_C + lane] = 0;
+        for (int o = 16; o > 0; o >>= 1) {
+            const SKey c{__shfl_xor_sync(0xFFFFFFFFu, best1.hi, o), __shfl_xor_sync(0xFFFFFFFFu, best1.lo, o)};
+            if (skey_better(c, best1)) best1 = c;
+        }
+        if (lane == 0) kred[warp] = best1;
+        if (threadIdx.x < GS_C) kout[threadIdx.x] = SKey{0, 0};
+        __syncthreads();
+        SKey thr = kred[0];
+        for (u32 w2 = 1; w2 < NW; ++w2)
+            if (skey_better(thr, kred[w2])) thr = kred[w2];
+        for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
+            if (!present(i) || conn_of(i) < thr.hi) continue;
+            const SKey k = key_of(i);
+            if (skey_better(thr, k)) continue;
+            const u32 at = atomicAdd(&nkeys, 1u);
+            if (at < GS_LIST) klist[at] = k;
+        }
+        __syncthreads();
+        const u32 nk = nkeys;
+        if (nk <= GS_LIST) {
+            if (threadIdx.x < nk) {
+                const SKey k = klist[threadIdx.x];
+                u32 rank = 0;
+                for (u32 j = 0; j < nk && rank < GS_C; ++j) rank += skey_better(klist[j], k);
+                if (rank < GS_C) kout[rank] = k;
+            }
+        } else {  // a warp without keys leaves a threshold that lists too many: GS_C block-wide maxima
+            SKey prev{~0ull, ~0ull};
+            for (u32 r = 0; r < GS_C; ++r) {
+                SKey b{0, 0};
+                for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
+                    if (!present(i)) continue;
+                    const SKey k = key_of(i);
+                    if (skey_better(prev, k) && skey_better(k, b)) b = k;
                 }
-                if (lane == 0) {
-                    C.sacc[idx] = 0;
-                    C.wacc[idx] = 0;
-                    C.spos[u] = idx;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const SKey c{__shfl_xor_sync(0xFFFFFFFFu, b.hi, o), __shfl_xor_sync(0xFFFFFFFFu, b.lo, o)};
+                    if (skey_better(c, b)) b = c;
                 }
+                __syncthreads();
+                if (lane == 0) kred[warp] = b;
+                __syncthreads();
+                b = kred[0];
+                for (u32 w2 = 1; w2 < NW; ++w2)
+                    if (skey_better(kred[w2], b)) b = kred[w2];
+                if (threadIdx.x == 0) kout[r] = b;
+                prev = b;
+                if (!(b.hi | b.lo)) break;  // no key is left
             }
         }
         __syncthreads();
-        for (u32 t = threadIdx.x; t < nd; t += GS_BLOCK) {  // empty the node's slots for the next one
-            const u32 i = used[t];
-            keys[i] = NONE;
-            sacc[i] = 0;
+        for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) clear(i);
+        if (threadIdx.x < GS_C) {  // the candidates and a zeroed accumulator row (row = list index)
+            const SKey b = kout[threadIdx.x];
+            C.cand[(u64)u * GS_C + threadIdx.x] = (b.hi | b.lo) ? ~(u32)b.lo : NONE;
+            C.conn[(u64)idx * GS_C + threadIdx.x] = 0;
+            C.dcon[(u64)idx * GS_C + threadIdx.x] = 0;
+        }
+        if (threadIdx.x == 0) {
+            C.sacc[idx] = 0;
+            C.wacc[idx] = 0;
+            C.spos[u] = idx;
         }
         __syncthreads();
     }
@@ -3539,9 +3565,15 @@ void setup_refine_kernels(Ctx &c) {
     AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * GN_BLOCK_W * 16));
     AXC_CUDA(cudaFuncSetAttribute(k_cascade_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CB_DYN_MAX));
-    AXC_CUDA(cudaFuncSetAttribute(k_gain_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_SMEM));
-    AXC_CUDA(cudaFuncSetAttribute(k_gain_sample, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                  (int)cudaSharedmemCarveoutMaxShared));
+    const auto sample_smem = [](auto kernel, size_t bytes) {
+        AXC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        AXC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      (int)cudaSharedmemCarveoutMaxShared));
+    };
+    sample_smem(k_gain_sample<true, true>, (size_t)GS_DIRECT_UNI * 4);
+    sample_smem(k_gain_sample<true, false>, (size_t)GS_TAB * 8);
+    sample_smem(k_gain_sample<false, true>, (size_t)GS_DIRECT_GEN * 8);
+    sample_smem(k_gain_sample<false, false>, (size_t)GS_TAB * 12);
     AXC_CUDA(cudaFuncSetAttribute(k_cands_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CV_BLOCK_SMEM));
     AXC_CUDA(cudaFuncSetAttribute(k_rank_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
     AXC_CUDA(cudaFuncSetAttribute(k_copy_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
@@ -3774,7 +3806,21 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
         C.sacc = c.arena.alloc<unsigned long long>(rows);
         C.wacc = c.arena.alloc<unsigned long long>(rows);
         fill_u32(c, C.spos, NONE, L.n);
-        LAUNCH(c, k_gain_sample, std::min<u32>(rows, (u32)c.sms * GS_PER_SM), GS_BLOCK, GS_SMEM, A, lp.ntier[2], rows, C);
+        const auto sample = [&](auto uni, auto direct) {
+            constexpr bool U = decltype(uni)::value, D = decltype(direct)::value;
+            const u32 T = D ? A.K : GS_TAB;
+            const size_t smem = (size_t)T * 4 * ((U ? 1 : 2) + (D ? 0 : 1));
+            int per_sm = 1;
+            AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gain_sample<U, D>, GS_BLOCK, smem));
+            LAUNCH_AS(c, "k_gain_sample", (k_gain_sample<U, D>), std::min<u32>(rows, (u32)c.sms * (u32)std::max(per_sm, 1)),
+                      GS_BLOCK, smem, A, lp.ntier[2], rows, C, T, lp.weight);
+        };
+        const std::true_type yes;
+        const std::false_type no;
+        if (lp.uniform && A.K <= GS_DIRECT_UNI) sample(yes, yes);
+        else if (lp.uniform) sample(yes, no);
+        else if (A.K <= GS_DIRECT_GEN) sample(no, yes);
+        else sample(no, no);
         LAUNCH(c, k_cands_warp, cdiv(L.e, CV_WARPS), CV_WARPS * 32, 0, A, C, L.e);
         if (lp.n_hblock)
             LAUNCH(c, k_cands_block, lp.n_hblock, CV_BLOCK, 8 * (size_t)cs_cap(block_tier_len(lp, CV_BLOCK_LEN)), A,
