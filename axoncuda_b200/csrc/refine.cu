@@ -501,7 +501,7 @@ __device__ __forceinline__ GainArgs gain_args_now(const GainArgs &A0) {
 // sum of incident weights bounds its gain.
 __global__ void k_gain_bounds(u32 n, u32 K, const u64 *__restrict__ toff, const u32 *__restrict__ touch,
                               const u64 *__restrict__ off, const u32 *__restrict__ wfx, u64 *__restrict__ work,
-                              unsigned long long *__restrict__ wmax) {
+                              u64 *__restrict__ wsum, unsigned long long *__restrict__ wmax) {
     const u32 u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (u >= n) return;
     u64 s = 0, ws = 0;
@@ -515,6 +515,7 @@ __global__ void k_gain_bounds(u32 n, u32 K, const u64 *__restrict__ toff, const 
     ws = warp_sum(ws);
     if (lane == 0) {
         work[u] = s < K ? s : K;
+        if (wsum) wsum[u] = ws;
         atomicMax(wmax, (unsigned long long)ws);
     }
 }
@@ -1245,14 +1246,17 @@ __device__ __forceinline__ bool skey_better(const SKey &a, const SKey &b) {
     return a.hi > b.hi || (a.hi == b.hi && a.lo > b.lo);
 }
 
-// Candidates and accumulator rows of the sampled rule's exact pass (k_cands_*).
+// Candidates and sums of the sampled rule's exact pass (k_cands_*), by node. With equal weights a
+// sum is one word, the incidences holding the candidate above and the inbound ones with a
+// destination pin in it below; else conn is the weight and dcon the inbound count.
 struct CandAcc {
-    u32 *spos;                 // [n]
-    u32 *cand;                 // [n * GS_C], NONE-padded
-    unsigned long long *conn;  // [rows * GS_C]
-    u32 *dcon;                 // [rows * GS_C]
-    unsigned long long *sacc, *wacc;  // [rows]
+    u32 *cand;                 // [n * GS_C], NONE-padded; all NONE for nodes without candidates
+    unsigned long long *conn;  // [n * GS_C]
+    u32 *dcon;                 // [n * GS_C], null with equal weights
+    const u64 *wsum;           // [n] summed weights of a node's hyperedges
+    u32 weight;                // with equal weights
 };
+constexpr unsigned long long CV_ONE = 1ull << 32;
 
 // UNI: every hyperedge has the weight w. DIRECT: slots are partitions (T = K), else a hash table of
 // T = GS_TAB slots. One block per node at a time; the table is empty between nodes: the last scan
@@ -1421,7 +1425,7 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
                 Cand b = cred[0];
                 for (u32 i = 1; i < NW; ++i)
                     if (cand_better(cred[i], b)) b = cred[i];
-                write_move(A, u, b);  // spos[u] stays NONE
+                write_move(A, u, b);  // its candidates stay NONE
             }
             __syncthreads();
             continue;
@@ -1497,149 +1501,194 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
         }
         __syncthreads();
         for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) clear(i);
-        if (threadIdx.x < GS_C) {  // the candidates and a zeroed accumulator row (row = list index)
+        if (threadIdx.x < GS_C) {  // the candidates and their zeroed sums
             const SKey b = kout[threadIdx.x];
             C.cand[(u64)u * GS_C + threadIdx.x] = (b.hi | b.lo) ? ~(u32)b.lo : NONE;
-            C.conn[(u64)idx * GS_C + threadIdx.x] = 0;
-            C.dcon[(u64)idx * GS_C + threadIdx.x] = 0;
-        }
-        if (threadIdx.x == 0) {
-            C.sacc[idx] = 0;
-            C.wacc[idx] = 0;
-            C.spos[u] = idx;
+            C.conn[(u64)u * GS_C + threadIdx.x] = 0;
+            if (!UNI) C.dcon[(u64)u * GS_C + threadIdx.x] = 0;
+            // no candidate: the exact pass will not see the node
+            if (threadIdx.x == 0 && !(b.hi | b.lo)) write_move(A, u, Cand{INT64_MIN, 0});
         }
         __syncthreads();
     }
 }
 
-// The exact pass of the sampled rule, pin-centric. Each listed node u whose sample was not the
-// whole node has row r = spos[u] of the accumulators (k_gain_sample sets it and zeroes the row;
-// spos is NONE for every other node): conn[r * GS_C + i], the weight of u's hyperedges holding its
-// candidate i; dcon[r * GS_C + i], u's inbound hyperedges with a destination pin in candidate i;
-// sacc[r], u's saving from leaving its partition; wacc[r], the weight of all u's hyperedges. One
-// pass over the hyperedges fills them: a hyperedge's census goes into a hash table (partition ->
-// count, plus a has-destination bit) and each listed pin looks up its own partition and its
-// candidates. k_cands_best then takes the best feasible candidate from these integer sums, which
-// are those a scan of each node's incidences would give.
+// The exact pass of the sampled rule, pin-centric. One pass over the hyperedges fills the sums of
+// the listed nodes' candidates: a hyperedge's census goes into shared memory and each pin with
+// candidates looks them up. k_cands_best then takes the best feasible candidate from these integer
+// sums, which are those a scan of each node's incidences would give; what the node saves by
+// leaving comes from the census pass and its total weight from the level. Two forms of the census:
+//  - up to CV_BITS_K partitions two bitmaps by partition (present, with a destination pin), so a
+//    lookup is one word, and only the words that were set are cleared again;
+//  - above, a hash table (partition -> has-destination bit).
 static_assert(GS_C == 8, "k_cands_* read a node's candidates as two 16-byte words");
-constexpr u32 CV_DBIT = 0x80000000u;  // census value: the partition holds a destination pin
 constexpr u32 CV_WARPS = 4;
 constexpr u32 CV_WARP_LEN = 256;      // longer hyperedges take a block (CS_WARP_CAP)
-constexpr u32 CV_BLOCK_LEN = 4096;    // longer still: a table in device memory (CS_BLOCK_CAP)
+constexpr u32 CV_BLOCK_LEN = 4096;    // hashed, longer still: a table in device memory (CS_BLOCK_CAP)
 constexpr u32 CV_BLOCK = 256;
 constexpr size_t CV_BLOCK_SMEM = (size_t)8 * 8192;  // keys and values of cs_cap(CV_BLOCK_LEN) slots
+constexpr u32 CV_BITS_K = 16384;      // two bitmaps of 2 KB
 
-// Census entries [a, a + lm) of one hyperedge into keys/vals (mask + 1 cleared slots), threads
-// t, t + nt, ...: each partition appears once in a census, so each slot is written once.
-__device__ __forceinline__ void cv_fill(const GainArgs &A, u64 a, u32 lm, u32 *keys, u32 *vals, u32 mask, u32 t,
-                                        u32 nt) {
-    for (u32 j = t; j < lm; j += nt) {
-        const u32 slot = hash_find_or_insert(keys, mask, A.cpart[a + j]);
-        if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); continue; }
-        vals[slot] = A.ccnt[a + j] | (A.cdcnt[a + j] > 0 ? CV_DBIT : 0u);
+struct CvBits {
+    u32 *any, *dst;
+    __device__ __forceinline__ bool has(u32 q, bool &d) const {
+        const u32 bit = 1u << (q & 31u);
+        d = (dst[q >> 5] & bit) != 0;
+        return (any[q >> 5] & bit) != 0;
     }
-}
-// Listed pin v (row r) of a hyperedge of weight w; io: v is one of its destinations.
-__device__ __forceinline__ void cv_pin(const GainArgs &A, const CandAcc &C, u32 v, u32 r, bool io, u32 w,
-                                       const u32 *keys, const u32 *vals, u32 mask) {
-    const u32 sp = hash_find(keys, mask, A.part[v]);  // present: v's own partition
-    if (sp != NONE) {
-        const i64 g = leave_gain(A.encourage, w, vals[sp] & ~CV_DBIT);
-        if (g) atomicAdd(&C.sacc[r], (unsigned long long)g);
+    __device__ __forceinline__ void put(const GainArgs &A, u32 q, bool d) {
+        const u32 bit = 1u << (q & 31u);
+        atomicOr(&any[q >> 5], bit);
+        if (d) atomicOr(&dst[q >> 5], bit);
     }
-    if (w) atomicAdd(&C.wacc[r], (unsigned long long)w);
+};
+struct CvHash {
+    u32 *keys, *vals, mask;
+    __device__ __forceinline__ bool has(u32 q, bool &d) const {
+        const u32 s = hash_find(keys, mask, q);
+        d = s != NONE && vals[s];
+        return s != NONE;
+    }
+    __device__ __forceinline__ void put(const GainArgs &A, u32 q, bool d) {  // each partition once
+        const u32 s = hash_find_or_insert(keys, mask, q);
+        if (s == NONE) { atomicExch(A.status, DEV_HASH_FULL); return; }
+        vals[s] = d;
+    }
+};
+// The sums of pin v's candidates over one hyperedge of weight w; io: v is one of its destinations.
+template <class M>
+__device__ __forceinline__ void cv_pin(const CandAcc &C, u32 v, bool io, u32 w, const M &map) {
     const uint4 *cp = reinterpret_cast<const uint4 *>(C.cand + (u64)v * GS_C);
     const uint4 c0 = cp[0], c1 = cp[1];
     const u32 q[GS_C] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
     for (u32 i = 0; i < GS_C; ++i) {
         if (q[i] == NONE) break;
-        const u32 s = hash_find(keys, mask, q[i]);
-        if (s == NONE) continue;
-        if (w) atomicAdd(&C.conn[(u64)r * GS_C + i], (unsigned long long)w);
-        if (io && (vals[s] & CV_DBIT)) atomicAdd(&C.dcon[(u64)r * GS_C + i], 1u);
+        bool d;
+        if (!map.has(q[i], d)) continue;
+        const u64 at = (u64)v * GS_C + i;
+        if (!C.dcon) {
+            atomicAdd(&C.conn[at], CV_ONE | (io && d ? 1ull : 0ull));
+        } else {
+            if (w) atomicAdd(&C.conn[at], (unsigned long long)w);
+            if (io && d) atomicAdd(&C.dcon[at], 1u);
+        }
     }
 }
 
-// One warp per hyperedge of at most CV_WARP_LEN pins; skipped when it holds no listed pin.
-__global__ void __launch_bounds__(CV_WARPS * 32) k_cands_warp(GainArgs A, CandAcc C, u32 e) {
-    __shared__ u32 tk[CV_WARPS][2 * CV_WARP_LEN], tv[CV_WARPS][2 * CV_WARP_LEN];
+// One warp per hyperedge of at most CV_WARP_LEN pins; skipped when no pin has candidates. BITS: mw
+// words per bitmap.
+template <bool BITS>
+__global__ void __launch_bounds__(CV_WARPS * 32) k_cands_warp(GainArgs A, CandAcc C, u32 e, u32 mw) {
+    extern __shared__ u32 cv_dyn[];
     const u32 wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const u32 h = blockIdx.x * CV_WARPS + wp;
-    if (h >= e) return;
-    const u64 a = A.off[h], b = A.off[h + 1];
-    if (b - a > CV_WARP_LEN) return;
+    u32 *t0 = cv_dyn + wp * (BITS ? 2 * mw : 4 * CV_WARP_LEN);
+    if (BITS)
+        for (u32 i = lane; i < 2 * mw; i += 32) t0[i] = 0;
     constexpr u32 R = CV_WARP_LEN / 32;
-    u32 pv[R], pr[R];
-    bool any = false;
+    for (u32 h = blockIdx.x * CV_WARPS + wp; h < e; h += gridDim.x * CV_WARPS) {
+        const u64 a = A.off[h], b = A.off[h + 1];
+        if (b - a > CV_WARP_LEN) continue;
+        u32 pv[R];
+        bool any = false;
 #pragma unroll
-    for (u32 i = 0; i < R; ++i) {
-        const u64 k = a + lane + 32 * i;
-        pv[i] = k < b ? A.pins[k] : 0;
-        pr[i] = k < b ? C.spos[pv[i]] : NONE;
-        any |= pr[i] != NONE;
+        for (u32 i = 0; i < R; ++i) {
+            const u64 k = a + lane + 32 * i;
+            pv[i] = k < b ? A.pins[k] : NONE;
+        }
+#pragma unroll
+        for (u32 i = 0; i < R; ++i) {
+            if (pv[i] != NONE && C.cand[(u64)pv[i] * GS_C] == NONE) pv[i] = NONE;
+            any |= pv[i] != NONE;
+        }
+        if (!__any_sync(0xFFFFFFFFu, any)) continue;
+        const u32 lm = A.lam[h], w = A.wfx[h];
+        const u64 s = a + A.nsrc[h];
+        const u32 cap = cs_cap(lm);
+        if (!BITS)
+            for (u32 i = lane; i < cap; i += 32) t0[i] = NONE;
+        __syncwarp();
+        CvBits bits{t0, t0 + mw};
+        CvHash hash{t0, t0 + 2 * CV_WARP_LEN, cap - 1};
+        for (u32 j = lane; j < lm; j += 32) {
+            if (BITS) bits.put(A, A.cpart[a + j], A.cdcnt[a + j] > 0);
+            else hash.put(A, A.cpart[a + j], A.cdcnt[a + j] > 0);
+        }
+        __syncwarp();
+#pragma unroll
+        for (u32 i = 0; i < R; ++i)
+            if (pv[i] != NONE) {
+                if (BITS) cv_pin(C, pv[i], a + lane + 32 * i >= s, w, bits);
+                else cv_pin(C, pv[i], a + lane + 32 * i >= s, w, hash);
+            }
+        __syncwarp();
+        if (BITS) {
+            for (u32 j = lane; j < lm; j += 32) {
+                const u32 x = A.cpart[a + j] >> 5;
+                t0[x] = 0;
+                t0[mw + x] = 0;
+            }
+            __syncwarp();
+        }
     }
-    if (!__any_sync(0xFFFFFFFFu, any)) return;
-    const u32 lm = A.lam[h];
-    const u32 cap = cs_cap(lm);
-    u32 *keys = tk[wp], *vals = tv[wp];
-    for (u32 i = lane; i < cap; i += 32) keys[i] = NONE;
-    __syncwarp();
-    cv_fill(A, a, lm, keys, vals, cap - 1, lane, 32);
-    __syncwarp();
-    const u32 w = A.wfx[h];
-    const u64 s = a + A.nsrc[h];
-#pragma unroll
-    for (u32 i = 0; i < R; ++i)
-        if (pr[i] != NONE) cv_pin(A, C, pv[i], pr[i], a + lane + 32 * i >= s, w, keys, vals, cap - 1);
 }
 
-// One block per listed hyperedge: `list` holds those of CV_WARP_LEN < |e| <= CV_BLOCK_LEN pins
+// One block per listed hyperedge: BITS, or hashed those of CV_WARP_LEN < |e| <= CV_BLOCK_LEN pins
 // (tables in shared memory) or, with gtab set, the longer ones (tables at gtab + 2 * gtab_off[i],
 // 2 * |e| slots rounded up to a power of two, as k_tab_sizes sizes them).
+template <bool BITS>
 __global__ void __launch_bounds__(CV_BLOCK) k_cands_block(GainArgs A, CandAcc C, const u32 *__restrict__ list,
-                                                          u32 nlist, u32 *gtab, const u64 *__restrict__ gtab_off) {
+                                                          u32 nlist, u32 mw, u32 *gtab,
+                                                          const u64 *__restrict__ gtab_off) {
     extern __shared__ u32 cv_dyn[];
     if (blockIdx.x >= nlist) return;
     const u32 h = list[blockIdx.x];
     const u64 a = A.off[h], b = A.off[h + 1];
     bool any = false;
-    for (u64 k = a + threadIdx.x; k < b && !any; k += CV_BLOCK) any = C.spos[A.pins[k]] != NONE;
+    for (u64 k = a + threadIdx.x; k < b && !any; k += CV_BLOCK) any = C.cand[(u64)A.pins[k] * GS_C] != NONE;
     if (!__syncthreads_or(any)) return;
     const u32 lm = A.lam[h];
-    const u32 cap = cs_cap(lm);
-    if (!gtab && 8ull * cap > dyn_smem_bytes()) {  // launched with too small a table: refuse
+    const u32 cap = BITS ? 0 : cs_cap(lm);
+    if (!BITS && !gtab && 8ull * cap > dyn_smem_bytes()) {  // launched with too small a table: refuse
         if (threadIdx.x == 0) atomicExch(A.status, DEV_HASH_FULL);
         return;
     }
-    u32 *keys = gtab ? gtab + 2 * gtab_off[blockIdx.x] : cv_dyn;
-    u32 *vals = keys + cap;
-    for (u32 i = threadIdx.x; i < cap; i += CV_BLOCK) keys[i] = NONE;
+    u32 *t0 = !BITS && gtab ? gtab + 2 * gtab_off[blockIdx.x] : cv_dyn;
+    const u32 n0 = BITS ? 2 * mw : cap;
+    for (u32 i = threadIdx.x; i < n0; i += CV_BLOCK) t0[i] = BITS ? 0u : NONE;
     __syncthreads();
-    cv_fill(A, a, lm, keys, vals, cap - 1, threadIdx.x, CV_BLOCK);
+    CvBits bits{t0, t0 + mw};
+    CvHash hash{t0, t0 + cap, cap - 1};
+    for (u32 j = threadIdx.x; j < lm; j += CV_BLOCK) {
+        if (BITS) bits.put(A, A.cpart[a + j], A.cdcnt[a + j] > 0);
+        else hash.put(A, A.cpart[a + j], A.cdcnt[a + j] > 0);
+    }
     __syncthreads();
     const u32 w = A.wfx[h];
     const u64 s = a + A.nsrc[h];
     for (u64 k = a + threadIdx.x; k < b; k += CV_BLOCK) {
-        const u32 v = A.pins[k], r = C.spos[v];
-        if (r != NONE) cv_pin(A, C, v, r, k >= s, w, keys, vals, cap - 1);
+        if (BITS) cv_pin(C, A.pins[k], k >= s, w, bits);
+        else cv_pin(C, A.pins[k], k >= s, w, hash);
     }
 }
 
-// Each listed node with a row: its best feasible candidate (the order of gain_candidate).
+// Each node with candidates: its best feasible one (the order of gain_candidate).
 __global__ void k_cands_best(GainArgs A0, CandAcc C, const u32 *__restrict__ list, u32 nl) {
     const GainArgs A = gain_args_now(A0);
     const u32 idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= nl) return;
-    const u32 u = list[idx], r = C.spos[u];
-    if (r == NONE) return;  // settled by k_gain_sample
-    const i64 saving = (i64)C.sacc[r], wtot = (i64)C.wacc[r];
+    const u32 u = list[idx];
+    if (C.cand[(u64)u * GS_C] == NONE) return;  // settled by k_gain_sample
+    const i64 saving = A.save[u], wtot = (i64)C.wsum[u];
     Cand best{INT64_MIN, 0};
 #pragma unroll
     for (u32 i = 0; i < GS_C; ++i) {
-        const u32 q = C.cand[(u64)u * GS_C + i];
+        const u64 at = (u64)u * GS_C + i;
+        const u32 q = C.cand[at];
         if (q == NONE) break;
-        const Cand c = gain_candidate(A, u, q, C.conn[(u64)r * GS_C + i], C.dcon[(u64)r * GS_C + i], saving, wtot);
+        const u64 x = C.conn[at];
+        const u64 conn = C.dcon ? x : (x >> 32) * C.weight;
+        const Cand c = gain_candidate(A, u, q, conn, C.dcon ? C.dcon[at] : (u32)x, saving, wtot);
         if (cand_better(c, best)) best = c;
     }
     write_move(A, u, best);
@@ -3519,6 +3568,7 @@ struct LevelPrep {
     u32 *ntier[3] = {nullptr, nullptr, nullptr};
     u32 ncount[3] = {0, 0, 0};
     u64 *work = nullptr;     // per-node table bound of the gains
+    u64 *wsum = nullptr;     // K > GS_K: per-node summed weights of its hyperedges
     u64 block_work_max = 0;  // largest gain-work bound of the block tier (sizes its shared table)
     u64 gain_bound = 0;     // no gain exceeds this (sum of incident weights)
     u64 max_len = 0;         // largest hyperedge
@@ -3574,7 +3624,7 @@ void setup_refine_kernels(Ctx &c) {
     sample_smem(k_gain_sample<true, false>, (size_t)GS_TAB * 8);
     sample_smem(k_gain_sample<false, true>, (size_t)GS_DIRECT_GEN * 8);
     sample_smem(k_gain_sample<false, false>, (size_t)GS_TAB * 12);
-    AXC_CUDA(cudaFuncSetAttribute(k_cands_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CV_BLOCK_SMEM));
+    AXC_CUDA(cudaFuncSetAttribute(k_cands_block<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CV_BLOCK_SMEM));
     AXC_CUDA(cudaFuncSetAttribute(k_rank_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
     AXC_CUDA(cudaFuncSetAttribute(k_copy_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
 }
@@ -3635,8 +3685,9 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
     if (n) {
         u64 *work = c.arena.alloc<u64>(n);
         lp.work = work;
+        if (K > GS_K) lp.wsum = c.arena.alloc<u64>(n);
         LAUNCH(c, k_gain_bounds, cdiv((u64)n * 32, 256), 256, 0, n, K, L.toff, L.touch, L.off, wfx, work,
-               (unsigned long long *)(dc + 5));
+               lp.wsum, (unsigned long long *)(dc + 5));
         u32 *flag = c.arena.alloc<u32>(n);
         for (u32 t = 0; t < (kway ? 2u : 3u); ++t) {
             lp.ntier[t] = c.arena.alloc<u32>(n);
@@ -3798,14 +3849,9 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
     if (lp.ncount[2] && A.K > GS_K) {  // the sampled rule (include/axc.h AXC_SPARSE_GAIN_*)
         size_t m = c.arena.mark();
         const u32 rows = lp.ncount[2];
-        CandAcc C;
-        C.cand = c.arena.alloc<u32>((u64)L.n * GS_C);
-        C.spos = c.arena.alloc<u32>(L.n);
-        C.conn = c.arena.alloc<unsigned long long>((u64)rows * GS_C);
-        C.dcon = c.arena.alloc<u32>((u64)rows * GS_C);
-        C.sacc = c.arena.alloc<unsigned long long>(rows);
-        C.wacc = c.arena.alloc<unsigned long long>(rows);
-        fill_u32(c, C.spos, NONE, L.n);
+        CandAcc C{c.arena.alloc<u32>((u64)L.n * GS_C), c.arena.alloc<unsigned long long>((u64)L.n * GS_C),
+                  lp.uniform ? nullptr : c.arena.alloc<u32>((u64)L.n * GS_C), lp.wsum, lp.weight};
+        AXC_CUDA(cudaMemsetAsync(C.cand, 0xFF, (size_t)L.n * GS_C * 4, c.stream));  // NONE
         const auto sample = [&](auto uni, auto direct) {
             constexpr bool U = decltype(uni)::value, D = decltype(direct)::value;
             const u32 T = D ? A.K : GS_TAB;
@@ -3821,15 +3867,27 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
         else if (lp.uniform) sample(yes, no);
         else if (A.K <= GS_DIRECT_GEN) sample(no, yes);
         else sample(no, no);
-        LAUNCH(c, k_cands_warp, cdiv(L.e, CV_WARPS), CV_WARPS * 32, 0, A, C, L.e);
-        if (lp.n_hblock)
-            LAUNCH(c, k_cands_block, lp.n_hblock, CV_BLOCK, 8 * (size_t)cs_cap(block_tier_len(lp, CV_BLOCK_LEN)), A,
-                   C, lp.hblock, lp.n_hblock, (u32 *)nullptr,
-                   (const u64 *)nullptr);
-        if (lp.n_hhuge) {
-            u32 *gtab = c.arena.alloc<u32>(2 * lp.huge_tot);
-            LAUNCH(c, k_cands_block, lp.n_hhuge, CV_BLOCK, 0, A, C, lp.hhuge, lp.n_hhuge, gtab, (const u64 *)lp.huge_tab);
-        }
+        const auto exact = [&](auto bitmaps) {
+            constexpr bool B = decltype(bitmaps)::value;
+            const u32 mw = (A.K + 31) / 32;
+            const size_t ws = B ? (size_t)CV_WARPS * 2 * mw * 4 : (size_t)CV_WARPS * 4 * CV_WARP_LEN * 4;
+            int per_sm = 1;
+            AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cands_warp<B>, CV_WARPS * 32, ws));
+            LAUNCH_AS(c, "k_cands_warp", k_cands_warp<B>,
+                      std::min<u32>(cdiv(L.e, CV_WARPS), (u32)c.sms * (u32)std::max(per_sm, 1)), CV_WARPS * 32, ws, A, C,
+                      L.e, mw);
+            const size_t bs = B ? (size_t)2 * mw * 4 : 8 * (size_t)cs_cap(block_tier_len(lp, CV_BLOCK_LEN));
+            if (lp.n_hblock)
+                LAUNCH_AS(c, "k_cands_block", k_cands_block<B>, lp.n_hblock, CV_BLOCK, bs, A, C, lp.hblock, lp.n_hblock,
+                          mw, (u32 *)nullptr, (const u64 *)nullptr);
+            if (lp.n_hhuge) {
+                u32 *gtab = B ? nullptr : c.arena.alloc<u32>(2 * lp.huge_tot);
+                LAUNCH_AS(c, "k_cands_block", k_cands_block<B>, lp.n_hhuge, CV_BLOCK, B ? bs : 0, A, C, lp.hhuge,
+                          lp.n_hhuge, mw, gtab, (const u64 *)lp.huge_tab);
+            }
+        };
+        if (A.K <= CV_BITS_K) exact(yes);
+        else exact(no);
         LAUNCH(c, k_cands_best, cdiv(rows, 256), 256, 0, A, C, lp.ntier[2], rows);
         c.arena.release(m);
     }
@@ -3906,7 +3964,7 @@ static Census census_for_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, con
                                const u32 *part) {
     Census cs = alloc_census(c, L);
     const bool direct = rp.K <= GN_DIRECT_K;
-    if (direct || plane_gains(L, lp, rp.K)) {
+    if (direct || plane_gains(L, lp, rp.K) || (rp.K > GS_K && lp.ncount[2])) {
         cs.save = c.arena.alloc<i64>(L.n ? L.n : 1);
         AXC_CUDA(cudaMemsetAsync(cs.save, 0, (size_t)L.n * 8, c.stream));
         cs.wfx = wfx;
