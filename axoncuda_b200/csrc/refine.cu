@@ -411,20 +411,36 @@ __global__ void k_part_sizes(u32 n, const u32 *__restrict__ part, const u32 *__r
     if (v < n) atomicAdd(&ps[part[v]], (unsigned long long)nsize[v]);
 }
 // Few partitions (K <= PS_SMEM_K): per-block sums in shared memory, one global add per partition
-// and block, over a grid-stride range (every node's global atomic would hit the same K words).
+// and block. A size is added in 16-bit halves, each a native 32-bit add (64-bit ones would be
+// compare-and-swap loops on a few words), so a block takes at most PS_NODES nodes. Where the room
+// allows, a partition has a counter per lane (rep = 32): lanes of one partition do not collide.
 constexpr u32 PS_SMEM_K = 1024;
-__global__ void k_part_sizes_smem(u32 n, u32 K, const u32 *__restrict__ part, const u32 *__restrict__ nsize,
-                                  unsigned long long *__restrict__ ps) {
-    __shared__ unsigned long long sh[PS_SMEM_K];
-    for (u32 i = threadIdx.x; i < K; i += blockDim.x) sh[i] = 0;
+constexpr u32 PS_NODES = 65536;
+__global__ void __launch_bounds__(256) k_part_sizes_smem(u32 n, u32 K, u32 rep, u32 per_block,
+                                                         const u32 *__restrict__ part, const u32 *__restrict__ nsize,
+                                                         unsigned long long *__restrict__ ps) {
+    extern __shared__ u32 ps_sh[];  // lo[K * rep], hi[K * rep]
+    u32 *lo = ps_sh, *hi = ps_sh + K * rep;
+    for (u32 i = threadIdx.x; i < 2 * K * rep; i += blockDim.x) ps_sh[i] = 0;
     __syncthreads();
-    for (u32 v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const u32 q = part[v];
-        if (q < K) atomicAdd(&sh[q], (unsigned long long)nsize[v]);  // ids are below K by contract
+    const u32 l = threadIdx.x & (rep - 1);
+    const u64 v0 = (u64)blockIdx.x * per_block, v1 = v0 + per_block < n ? v0 + per_block : n;
+#pragma unroll 4
+    for (u64 v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+        const u32 q = part[v], s = nsize[v];
+        if (q >= K) continue;  // ids are below K by contract
+        atomicAdd(&lo[q * rep + l], s & 0xFFFFu);
+        if (s >> 16) atomicAdd(&hi[q * rep + l], s >> 16);
     }
     __syncthreads();
-    for (u32 i = threadIdx.x; i < K; i += blockDim.x)
-        if (sh[i]) atomicAdd(&ps[i], sh[i]);
+    for (u32 i = threadIdx.x; i < K; i += blockDim.x) {
+        u64 t = 0;
+        for (u32 x = 0; x < rep; ++x) {
+            const u32 y = i * rep + ((x + i) & (rep - 1));
+            t += (u64)lo[y] + ((u64)hi[y] << 16);
+        }
+        if (t) atomicAdd(&ps[i], (unsigned long long)t);
+    }
 }
 __global__ void k_part_inbound(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ lam,
                                const u32 *__restrict__ cpart, const u32 *__restrict__ cdcnt,
@@ -2916,11 +2932,12 @@ __global__ void k_best(const i64 *__restrict__ pre, u32 n, int has_vi, const u32
         if (threadIdx.x == 0) out[blockIdx.x] = x;
     }
 }
-__global__ void k_best_final(const Best *__restrict__ in, u32 nb, const i64 *__restrict__ pre, u32 n, int has_vi,
-                             Best *__restrict__ out, u32 *__restrict__ apply) {
-    Best x = in[0];
-    for (u32 i = 1; i < nb; ++i)
-        if (in[i].r != 0xFFFFFFFFu && (x.r == 0xFFFFFFFFu || best_better(in[i], x))) x = in[i];
+__global__ void __launch_bounds__(32) k_best_final(const Best *__restrict__ in, u32 nb, const i64 *__restrict__ pre,
+                                                   u32 n, int has_vi, Best *__restrict__ out, u32 *__restrict__ apply) {
+    Best x{0, 0, 0, 0xFFFFFFFFu};
+    for (u32 i = threadIdx.x; i < nb; i += 32) x = best_pick(x, in[i]);
+    x = warp_best_prefix(x);
+    if (threadIdx.x) return;
     *out = x;
     const i64 vi = (has_vi && x.r != 0xFFFFFFFFu) ? seg_prefix(pre, n, 2, x.r) : 0;
     *apply = (x.r != 0xFFFFFFFFu && x.vs <= 0 && vi <= 0 && x.g >= 0) ? 1u : 0u;
@@ -3927,10 +3944,12 @@ Census build_census(Ctx &c, const DLevel &L, const u32 *part) {
 
 void part_sizes(Ctx &c, u32 n, const u32 *part, const u32 *nsize, u64 *psize, u32 K) {
     AXC_CUDA(cudaMemsetAsync(psize, 0, (size_t)K * 8, c.stream));
-    if (n && K <= PS_SMEM_K)
-        LAUNCH(c, k_part_sizes_smem, std::min<u32>(cdiv(n, 256), (u32)c.sms * 4), 256, 0, n, K, part, nsize,
+    if (n && K <= PS_SMEM_K) {
+        const u32 rep = K <= 64 ? 32u : 1u;
+        const u32 per = std::min<u32>(PS_NODES, std::max<u32>(1024, cdiv(n, (u64)c.sms * 4)));
+        LAUNCH(c, k_part_sizes_smem, cdiv(n, per), 256, (size_t)2 * K * rep * 4, n, K, rep, per, part, nsize,
                (unsigned long long *)psize);
-    else if (n)
+    } else if (n)
         LAUNCH(c, k_part_sizes, cdiv(n, 256), 256, 0, n, part, nsize, (unsigned long long *)psize);
 }
 void part_inbound(Ctx &c, const DLevel &L, const Census &cs, u64 *pinb, u32 K) {
@@ -4438,7 +4457,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         const u32 nbk = cdiv(n, 256) < 64u ? cdiv(n, 256) : 64u;
         Best *bb = (Best *)c.arena.alloc<u64>(4 * (nbk + 1));
         LAUNCH(c, k_best, nbk, 256, 0, pre, n, track ? 1 : 0, dM, bb + 1);
-        LAUNCH(c, k_best_final, 1, 1, 0, bb + 1, nbk, pre, n, track ? 1 : 0, bb, apply);
+        LAUNCH(c, k_best_final, 1, 32, 0, bb + 1, nbk, pre, n, track ? 1 : 0, bb, apply);
         LAUNCH(c, k_apply, cdiv(n, 256), 256, 0, mv, target, bb, apply, part, ic ? ic->prev : nullptr,
                ic ? ic->stamp : nullptr, ic ? (const u32 *)ic->ctr : nullptr);
         if (kw)
