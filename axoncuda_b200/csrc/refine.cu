@@ -452,21 +452,26 @@ __global__ void k_part_inbound(u32 e, const u64 *__restrict__ off, const u32 *__
         if (cdcnt[a + j] > 0) atomicAdd(&pinb[cpart[a + j]], 1ull);
 }
 
-constexpr u32 PI_SMEM_K = 8192;
-// k_part_inbound for K <= PI_SMEM_K: warps stride over the hyperedges and count into a shared
-// histogram, which the block adds to pinb once; this avoids contended global atomics on few
-// partitions.
-__global__ void k_part_inbound_smem(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ lam,
-                                    const u32 *__restrict__ cpart, const u32 *__restrict__ cdcnt, u32 K,
-                                    unsigned long long *__restrict__ pinb) {
+constexpr u32 PI_SMEM_K = 49152;
+constexpr u32 PI_THREADS = 1024;
+// k_part_inbound for K <= PI_SMEM_K: groups of G lanes stride over the hyperedges and count into a
+// shared histogram, which the block adds to pinb once: one large block per SM, since every block
+// adds up to K words to the same places. G follows the mean length (a census has no more entries).
+template <u32 G>
+__global__ void __launch_bounds__(PI_THREADS) k_part_inbound_smem(u32 e, const u64 *__restrict__ off,
+                                                                  const u32 *__restrict__ lam,
+                                                                  const u32 *__restrict__ cpart,
+                                                                  const u32 *__restrict__ cdcnt, u32 K,
+                                                                  unsigned long long *__restrict__ pinb) {
     extern __shared__ u32 hist[];
     for (u32 i = threadIdx.x; i < K; i += blockDim.x) hist[i] = 0;
     __syncthreads();
-    const u32 lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (u32 h = blockIdx.x * nw + (threadIdx.x >> 5); h < e; h += gridDim.x * nw) {
+    const u32 gl = threadIdx.x & (G - 1);
+    constexpr u32 per = PI_THREADS / G;
+    for (u32 h = blockIdx.x * per + threadIdx.x / G; h < e; h += gridDim.x * per) {
         const u64 a = off[h];
         const u32 lm = lam[h];
-        for (u32 j = lane; j < lm; j += 32)
+        for (u32 j = gl; j < lm; j += G)
             if (cdcnt[a + j] > 0) atomicAdd(&hist[cpart[a + j]], 1u);
     }
     __syncthreads();
@@ -1043,26 +1048,27 @@ __device__ __forceinline__ void census_flat(const GainArgs &A, u32 u, u32 first,
 // partitions), so there are two forms, chosen per level by run_gains:
 //  - k_gain_table: one shared add per census entry into K-entry tables. The connectivity is one
 //    u32 where no node's incident weights pass 2^32, else a low and a high word: 64-bit shared
-//    adds would be compare-and-swap loops.
+//    adds would be compare-and-swap loops. NT threads: 64 at moderate degrees, where more nodes in
+//    flight hide the loads' latency better than more threads per node.
 //  - k_gain_planes: for equal weights and hyperedges of at least as many pins as mask words. A
 //    candidate's connectivity is then a count of incidences whose K-bit mask holds it. A lane owns
 //    one mask word and adds whole words into bit-plane counters (carry-save adders, eight
 //    incidences at a time): 32 partitions per instruction, whatever the number of entries.
-template <bool WIDE>
-__global__ void __launch_bounds__(GN_BLOCK) k_gain_table(GainArgs A0, const u32 *__restrict__ list, u32 nl) {
+template <bool WIDE, u32 NT>
+__global__ void __launch_bounds__(NT) k_gain_table(GainArgs A0, const u32 *__restrict__ list, u32 nl) {
     const GainArgs A = gain_args_now(A0);
     extern __shared__ u32 gt_dyn[];
     u32 *lo = gt_dyn, *dconn = lo + A.K, *hi = dconn + A.K;  // hi only when WIDE
-    __shared__ i64 red[2][GN_BLOCK / 32];
-    __shared__ Cand cred[GN_BLOCK / 32];
+    __shared__ i64 red[2][NT / 32];
+    __shared__ Cand cred[NT / 32];
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (u32 idx = blockIdx.x; idx < nl; idx += gridDim.x) {
         const u32 u = list[idx], p = A.part[u];
         const u32 deg = (u32)(A.toff[u + 1] - A.toff[u]);
-        for (u32 i = threadIdx.x; i < (WIDE ? 3 : 2) * A.K; i += GN_BLOCK) gt_dyn[i] = 0;
+        for (u32 i = threadIdx.x; i < (WIDE ? 3 : 2) * A.K; i += NT) gt_dyn[i] = 0;
         __syncthreads();
         i64 saving = 0, wtot = 0;
-        census_flat(A, u, 32 * warp, GN_BLOCK, deg, wtot, [&](u64 k, u32 q, u32 w, u32 io) {
+        census_flat(A, u, 32 * warp, NT, deg, wtot, [&](u64 k, u32 q, u32 w, u32 io) {
             if (q == p) { saving += leave_gain(A.encourage, w, A.ccnt[k]); return; }
             if (io && A.cdcnt[k] > 0) atomicAdd(&dconn[q], 1u);
             if (WIDE) {
@@ -1077,9 +1083,9 @@ __global__ void __launch_bounds__(GN_BLOCK) k_gain_table(GainArgs A0, const u32 
         if (lane == 0) { red[0][warp] = saving; red[1][warp] = wtot; }
         __syncthreads();
         saving = wtot = 0;
-        for (u32 i = 0; i < GN_BLOCK / 32; ++i) { saving += red[0][i]; wtot += red[1][i]; }
+        for (u32 i = 0; i < NT / 32; ++i) { saving += red[0][i]; wtot += red[1][i]; }
         Cand best{INT64_MIN, 0};
-        for (u32 q = threadIdx.x; q < A.K; q += GN_BLOCK) {
+        for (u32 q = threadIdx.x; q < A.K; q += NT) {
             const u64 conn = WIDE ? ((u64)hi[q] << 32) | lo[q] : (u64)lo[q];
             if (conn == 0) continue;  // absent, or never a positive gain
             const Cand c = gain_candidate(A, u, q, conn, dconn[q], saving, wtot);
@@ -1090,7 +1096,7 @@ __global__ void __launch_bounds__(GN_BLOCK) k_gain_table(GainArgs A0, const u32 
         __syncthreads();
         if (threadIdx.x == 0) {
             Cand b = cred[0];
-            for (u32 i = 1; i < GN_BLOCK / 32; ++i)
+            for (u32 i = 1; i < NT / 32; ++i)
                 if (cand_better(cred[i], b)) b = cred[i];
             write_move(A, u, b);
         }
@@ -1274,14 +1280,29 @@ struct CandAcc {
 };
 constexpr unsigned long long CV_ONE = 1ull << 32;
 
+// What a partition can still take, in one word: nodes (omega - size) below, inbound hyperedges
+// (delta - inbound) above, each at most RM_MORE; RM_NONE where the limit is already passed. The scans
+// of k_gain_sample read it for every partition near a node, at a quarter of the two counts' bytes.
+constexpr u32 RM_MORE = 0xFFFEu, RM_NONE = 0xFFFFu;
+static_assert(GS_SAMPLE < RM_MORE, "a sample's incidences compare exactly");
+__global__ void k_part_room(u32 K, u32 omega, u32 delta, const u64 *__restrict__ psize, const u64 *__restrict__ pinb,
+                            u32 *__restrict__ room) {
+    const u32 q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= K) return;
+    const u64 s = psize[q], b = pinb[q];
+    const u32 rs = s > omega ? RM_NONE : (u32)(omega - s < RM_MORE ? omega - s : RM_MORE);
+    const u32 rb = b > delta ? RM_NONE : (u32)(delta - b < RM_MORE ? delta - b : RM_MORE);
+    room[q] = rs | rb << 16;
+}
+
 // UNI: every hyperedge has the weight w. DIRECT: slots are partitions (T = K), else a hash table of
 // T = GS_TAB slots. One block per node at a time; the table is empty between nodes: the last scan
 // of a node clears it.
 template <bool UNI, bool DIRECT>
 __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const u32 *__restrict__ list, u32 nl, CandAcc C,
-                                                         u32 T, u32 weight) {
+                                                         u32 T, u32 weight, const u32 *__restrict__ room) {
     const GainArgs A = gain_args_now(A0);
-    extern __shared__ u32 gs_tab[];
+    extern __shared__ __align__(16) u32 gs_tab[];
     u32 *v0 = gs_tab, *v1 = UNI ? nullptr : gs_tab + T, *keys = DIRECT ? nullptr : gs_tab + (UNI ? 1 : 2) * T;
     constexpr u32 NW = GS_BLOCK / 32;
     __shared__ unsigned long long wsh[NW];
@@ -1299,21 +1320,32 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
         if (!UNI) v1[i] = 0;
         if (!DIRECT) keys[i] = NONE;
     }
-    // slot contents
-    const auto present = [&](u32 i) { return UNI ? v0[i] != 0 : (v0[i] | v1[i]) != 0; };
-    const auto conn_of = [&](u32 i) {
-        return UNI ? (u64)(v0[i] >> GS_HI) * weight : ((u64)((v1[i] & ~GS_ZERO) >> GS_HI) << 32) | v0[i];
+    // slot contents (x, y): the words of v0 and v1
+    const auto conn_of = [&](u32 x, u32 y) {
+        return UNI ? (u64)(x >> GS_HI) * weight : ((u64)((y & ~GS_ZERO) >> GS_HI) << 32) | x;
     };
-    const auto dcon_of = [&](u32 i) { return UNI ? v0[i] & GS_LOW : v1[i] & GS_LOW; };
+    const auto dcon_of = [&](u32 x, u32 y) { return (UNI ? x : y) & GS_LOW; };
     const auto part_of = [&](u32 i) { return DIRECT ? i : keys[i]; };
-    const auto clear = [&](u32 i) {
-        v0[i] = 0;
-        if (!UNI) v1[i] = 0;
-        if (!DIRECT) keys[i] = NONE;
+    const auto key_of = [&](u32 q, u64 conn) {
+        return SKey{conn, ((u64)mix32(q + A.round + A.seed) << 32) | (u64)(~q)};
     };
-    const auto key_of = [&](u32 i) {
-        const u32 q = part_of(i);
-        return SKey{conn_of(i), ((u64)mix32(q + A.round + A.seed) << 32) | (u64)(~q)};
+    // f(i, x, y) for every present slot, four slots per load (T is a multiple of 4)
+    const auto scan = [&](auto &&f) {
+        for (u32 i4 = threadIdx.x; i4 < T / 4; i4 += GS_BLOCK) {
+            const uint4 x = ((const uint4 *)v0)[i4];
+            const uint4 y = UNI ? make_uint4(0, 0, 0, 0) : ((const uint4 *)v1)[i4];
+            if (x.x | y.x) f(4 * i4, x.x, y.x);
+            if (x.y | y.y) f(4 * i4 + 1, x.y, y.y);
+            if (x.z | y.z) f(4 * i4 + 2, x.z, y.z);
+            if (x.w | y.w) f(4 * i4 + 3, x.w, y.w);
+        }
+    };
+    const auto clear_all = [&]() {
+        for (u32 i4 = threadIdx.x; i4 < T / 4; i4 += GS_BLOCK) {
+            ((uint4 *)v0)[i4] = make_uint4(0, 0, 0, 0);
+            if (!UNI) ((uint4 *)v1)[i4] = make_uint4(0, 0, 0, 0);
+            if (!DIRECT) ((uint4 *)keys)[i4] = make_uint4(NONE, NONE, NONE, NONE);
+        }
     };
     for (u32 idx = blockIdx.x; idx < nl; idx += gridDim.x) {
         const u32 u = list[idx], p = A.part[u];
@@ -1428,12 +1460,10 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
             saving = (i64)block_sum_u64((u64)saving, wsh);
             wtot = (i64)block_sum_u64((u64)wtot, wsh);
             Cand best{INT64_MIN, 0};
-            for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
-                if (!present(i)) continue;
-                const Cand c = gain_candidate(A, u, part_of(i), conn_of(i), dcon_of(i), saving, wtot);
+            scan([&](u32 i, u32 x, u32 y) {
+                const Cand c = gain_candidate(A, u, part_of(i), conn_of(x, y), dcon_of(x, y), saving, wtot);
                 if (cand_better(c, best)) best = c;
-                clear(i);
-            }
+            });
             best = warp_best(best);
             if (lane == 0) cred[warp] = best;
             __syncthreads();
@@ -1443,6 +1473,7 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
                     if (cand_better(cred[i], b)) b = cred[i];
                 write_move(A, u, b);  // its candidates stay NONE
             }
+            clear_all();
             __syncthreads();
             continue;
         }
@@ -1452,17 +1483,21 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
         // lists the keys at or above it (a few dozen), whose ranks are counted pairwise.
         const u64 in_sample = m < nin_u ? m : nin_u, need = s - s / A.discount;
         SKey best1{0, 0};
-#pragma unroll 4
-        for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
-            if (!present(i)) continue;
-            const u32 q = part_of(i);
-            if (A.psize[q] + need > A.omega || A.pinb[q] + in_sample - dcon_of(i) > A.delta) {
-                clear(i);  // (its key goes as well: nothing is inserted any more)
-                continue;
+        scan([&](u32 i, u32 x, u32 y) {
+            const u32 q = part_of(i), rm = room[q], rs = rm & 0xFFFFu, rb = rm >> 16;
+            bool out = rs == RM_NONE || rb == RM_NONE || in_sample - dcon_of(x, y) > rb;
+            // a clamped room is at least RM_MORE nodes: larger nodes look at the size itself
+            if (!out) out = rs == RM_MORE ? (need > RM_MORE && A.psize[q] + need > A.omega) : need > rs;
+            if (out) {  // the slot is emptied (a hashed key may go as well: nothing is inserted any more)
+                v0[i] = 0;
+                if (!UNI) v1[i] = 0;
+                return;
             }
-            const SKey k = key_of(i);
+            const u64 conn = conn_of(x, y);
+            if (conn < best1.hi) return;
+            const SKey k = key_of(q, conn);
             if (skey_better(k, best1)) best1 = k;
-        }
+        });
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const SKey c{__shfl_xor_sync(0xFFFFFFFFu, best1.hi, o), __shfl_xor_sync(0xFFFFFFFFu, best1.lo, o)};
@@ -1474,13 +1509,14 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
         SKey thr = kred[0];
         for (u32 w2 = 1; w2 < NW; ++w2)
             if (skey_better(thr, kred[w2])) thr = kred[w2];
-        for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
-            if (!present(i) || conn_of(i) < thr.hi) continue;
-            const SKey k = key_of(i);
-            if (skey_better(thr, k)) continue;
+        scan([&](u32 i, u32 x, u32 y) {
+            const u64 conn = conn_of(x, y);
+            if (conn < thr.hi) return;
+            const SKey k = key_of(part_of(i), conn);
+            if (skey_better(thr, k)) return;
             const u32 at = atomicAdd(&nkeys, 1u);
             if (at < GS_LIST) klist[at] = k;
-        }
+        });
         __syncthreads();
         const u32 nk = nkeys;
         if (nk <= GS_LIST) {
@@ -1494,11 +1530,10 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
             SKey prev{~0ull, ~0ull};
             for (u32 r = 0; r < GS_C; ++r) {
                 SKey b{0, 0};
-                for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
-                    if (!present(i)) continue;
-                    const SKey k = key_of(i);
+                scan([&](u32 i, u32 x, u32 y) {
+                    const SKey k = key_of(part_of(i), conn_of(x, y));
                     if (skey_better(prev, k) && skey_better(k, b)) b = k;
-                }
+                });
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     const SKey c{__shfl_xor_sync(0xFFFFFFFFu, b.hi, o), __shfl_xor_sync(0xFFFFFFFFu, b.lo, o)};
@@ -1516,7 +1551,7 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
             }
         }
         __syncthreads();
-        for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) clear(i);
+        clear_all();
         if (threadIdx.x < GS_C) {  // the candidates and their zeroed sums
             const SKey b = kout[threadIdx.x];
             C.cand[(u64)u * GS_C + threadIdx.x] = (b.hi | b.lo) ? ~(u32)b.lo : NONE;
@@ -3629,18 +3664,17 @@ static bool round_loop_enabled() {
 
 void setup_refine_kernels(Ctx &c) {
     AXC_CUDA(cudaFuncSetAttribute(k_census_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 2 * CS_BLOCK_CAP * 4));
-    AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
+    AXC_CUDA(cudaFuncSetAttribute(k_part_inbound_smem<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PI_SMEM_K * 4));
+    AXC_CUDA(cudaFuncSetAttribute(k_part_inbound_smem<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PI_SMEM_K * 4));
+    AXC_CUDA(cudaFuncSetAttribute(k_part_inbound_smem<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PI_SMEM_K * 4));
+    AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
+    AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true, GN_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * GN_BLOCK_W * 16));
     AXC_CUDA(cudaFuncSetAttribute(k_cascade_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CB_DYN_MAX));
-    const auto sample_smem = [](auto kernel, size_t bytes) {
-        AXC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-        AXC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                      (int)cudaSharedmemCarveoutMaxShared));
-    };
-    sample_smem(k_gain_sample<true, true>, (size_t)GS_DIRECT_UNI * 4);
-    sample_smem(k_gain_sample<true, false>, (size_t)GS_TAB * 8);
-    sample_smem(k_gain_sample<false, true>, (size_t)GS_DIRECT_GEN * 8);
-    sample_smem(k_gain_sample<false, false>, (size_t)GS_TAB * 12);
+    AXC_CUDA(cudaFuncSetAttribute(k_gain_sample<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_DIRECT_UNI * 4));
+    AXC_CUDA(cudaFuncSetAttribute(k_gain_sample<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_TAB * 8));
+    AXC_CUDA(cudaFuncSetAttribute(k_gain_sample<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_DIRECT_GEN * 8));
+    AXC_CUDA(cudaFuncSetAttribute(k_gain_sample<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_TAB * 12));
     AXC_CUDA(cudaFuncSetAttribute(k_cands_block<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CV_BLOCK_SMEM));
     AXC_CUDA(cudaFuncSetAttribute(k_rank_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
     AXC_CUDA(cudaFuncSetAttribute(k_copy_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
@@ -3852,12 +3886,19 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
         }
         c.arena.release(m);
     } else if (lp.ncount[1] && A.K <= GS_K) {
-        if (lp.gain_bound < (1ull << 32))
-            LAUNCH_AS(c, "k_gain_table", k_gain_table<false>, lp.ncount[1], GN_BLOCK, (size_t)A.K * 8, A, lp.ntier[1],
-                      lp.ncount[1]);
-        else
-            LAUNCH_AS(c, "k_gain_table", k_gain_table<true>, lp.ncount[1], GN_BLOCK, (size_t)A.K * 12, A, lp.ntier[1],
-                      lp.ncount[1]);
+        const auto launch = [&](auto wide, auto threads) {
+            constexpr bool W = decltype(wide)::value;
+            constexpr u32 NT = decltype(threads)::value;
+            LAUNCH_AS(c, "k_gain_table", (k_gain_table<W, NT>), lp.ncount[1], NT, (size_t)A.K * (W ? 12 : 8), A,
+                      lp.ntier[1], lp.ncount[1]);
+        };
+        const bool wide = lp.gain_bound >= (1ull << 32), small = L.P / L.n <= 256;
+        const std::integral_constant<u32, 64> t64;
+        const std::integral_constant<u32, GN_BLOCK> t256;
+        if (wide && small) launch(std::true_type(), t64);
+        else if (wide) launch(std::true_type(), t256);
+        else if (small) launch(std::false_type(), t64);
+        else launch(std::false_type(), t256);
     } else if (lp.ncount[1]) {
         // shared table sized by the tier's largest bound (16 B per slot)
         const u32 cap1 = table_cap(lp.block_work_max, 2 * GN_BLOCK_W);
@@ -3869,14 +3910,16 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
         CandAcc C{c.arena.alloc<u32>((u64)L.n * GS_C), c.arena.alloc<unsigned long long>((u64)L.n * GS_C),
                   lp.uniform ? nullptr : c.arena.alloc<u32>((u64)L.n * GS_C), lp.wsum, lp.weight};
         AXC_CUDA(cudaMemsetAsync(C.cand, 0xFF, (size_t)L.n * GS_C * 4, c.stream));  // NONE
+        u32 *room = c.arena.alloc<u32>(A.K);
+        LAUNCH(c, k_part_room, cdiv(A.K, 256), 256, 0, A.K, A.omega, A.delta, A.psize, A.pinb, room);
         const auto sample = [&](auto uni, auto direct) {
             constexpr bool U = decltype(uni)::value, D = decltype(direct)::value;
-            const u32 T = D ? A.K : GS_TAB;
+            const u32 T = D ? (A.K + 3) & ~3u : GS_TAB;
             const size_t smem = (size_t)T * 4 * ((U ? 1 : 2) + (D ? 0 : 1));
             int per_sm = 1;
             AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gain_sample<U, D>, GS_BLOCK, smem));
             LAUNCH_AS(c, "k_gain_sample", (k_gain_sample<U, D>), std::min<u32>(rows, (u32)c.sms * (u32)std::max(per_sm, 1)),
-                      GS_BLOCK, smem, A, lp.ntier[2], rows, C, T, lp.weight);
+                      GS_BLOCK, smem, A, lp.ntier[2], rows, C, T, lp.weight, room);
         };
         const std::true_type yes;
         const std::false_type no;
@@ -3955,9 +3998,16 @@ void part_sizes(Ctx &c, u32 n, const u32 *part, const u32 *nsize, u64 *psize, u3
 void part_inbound(Ctx &c, const DLevel &L, const Census &cs, u64 *pinb, u32 K) {
     AXC_CUDA(cudaMemsetAsync(pinb, 0, (size_t)K * 8, c.stream));
     if (L.e && K <= PI_SMEM_K) {  // per-block counts in shared memory, one global add per partition
-        const u32 grid = std::min<u32>(cdiv(L.e, 256 / 32), 2 * (u32)c.sms);
-        LAUNCH(c, k_part_inbound_smem, grid, 256, (size_t)K * 4, L.e, L.off, cs.lam, cs.part, cs.dcnt, K,
-               (unsigned long long *)pinb);
+        const auto launch = [&](auto g) {
+            constexpr u32 G = decltype(g)::value;
+            LAUNCH_AS(c, "k_part_inbound_smem", k_part_inbound_smem<G>,
+                      std::min<u32>(cdiv(L.e, PI_THREADS / G), (u32)c.sms), PI_THREADS, (size_t)K * 4, L.e, L.off, cs.lam,
+                      cs.part, cs.dcnt, K, (unsigned long long *)pinb);
+        };
+        const u64 len = L.P / L.e;
+        if (len <= 6) launch(std::integral_constant<u32, 4>());
+        else if (len <= 24) launch(std::integral_constant<u32, 8>());
+        else launch(std::integral_constant<u32, 32>());
     } else if (L.e)
         LAUNCH(c, k_part_inbound, cdiv((u64)L.e * 32, 256), 256, 0, L.e, L.off, cs.lam, cs.part, cs.dcnt,
                (unsigned long long *)pinb);
