@@ -160,19 +160,33 @@ __global__ void k_table_sizes(const u32 *__restrict__ list, u32 nlist, const u64
 // key = 2*pin + is_source, value = hyperedge: a stable sort by key lists, per node, its inbound
 // hyperedges ascending and then its outbound ones ascending (sources/construction.cu:17-62).
 __global__ void k_touch_keys(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ pins,
-                             const u32 *__restrict__ nsrc, u32 *__restrict__ keys, u32 *__restrict__ vals,
-                             u32 *__restrict__ deg, u32 *__restrict__ nin) {
+                             const u32 *__restrict__ nsrc, u32 *__restrict__ keys, u32 *__restrict__ vals) {
     const u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= e) return;
     const u64 a = off[w], b = off[w + 1], s = a + nsrc[w];
     for (u64 k = a + lane; k < b; k += 32) {
-        u32 v = pins[k];
-        bool src = k < s;
-        keys[k] = 2 * v + (src ? 1u : 0u);
+        keys[k] = 2 * pins[k] + (k < s ? 1u : 0u);
         vals[k] = w;
-        atomicAdd(&deg[v], 1u);
-        if (!src) atomicAdd(&nin[v], 1u);
     }
+}
+// Where a node's keys start in the sorted keys, by two binary searches: its offset, and its
+// inbound count from the start of its second key. Against counting by atomics (two per pin,
+// contended at high-degree nodes) and a scan; the searches' upper steps stay in cache.
+__device__ __forceinline__ u64 first_at_least(const u32 *__restrict__ a, u64 lo, u64 hi, u32 x) {
+    while (lo < hi) {
+        const u64 mid = (lo + hi) >> 1;
+        if (a[mid] < x) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+__global__ void k_touch_starts(u32 n, u64 P, const u32 *__restrict__ keys, u64 *__restrict__ toff,
+                               u32 *__restrict__ nin) {
+    const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v > n) return;
+    if (v == n) { toff[n] = P; return; }
+    const u64 o = first_at_least(keys, 0, P, 2 * v);
+    toff[v] = o;
+    nin[v] = (u32)(first_at_least(keys, o, P, 2 * v + 1) - o);
 }
 
 // Input validation before any id is used as an index: offsets non-decreasing, source counts within
@@ -245,12 +259,9 @@ void build_touching(Ctx &c, u32 n, u32 e, const u64 *off, const u32 *pins, const
                     u64 *toff, u32 *touch, u32 *nin) {
     size_t m = c.arena.mark();
     u32 *keys = c.arena.alloc<u32>(P ? P : 1);
-    u32 *deg = c.arena.alloc<u32>(n ? n : 1);
-    AXC_CUDA(cudaMemsetAsync(deg, 0, (size_t)n * 4, c.stream));
-    AXC_CUDA(cudaMemsetAsync(nin, 0, (size_t)n * 4, c.stream));
-    if (e) LAUNCH(c, k_touch_keys, cdiv((u64)e * 32, 256), 256, 0, e, off, pins, nsrc, keys, touch, deg, nin);
+    if (e) LAUNCH(c, k_touch_keys, cdiv((u64)e * 32, 256), 256, 0, e, off, pins, nsrc, keys, touch);
     radix_sort_pairs(c, keys, touch, P, bits_for(n ? 2ull * n - 1 : 0));
-    offsets_from_counts(c, deg, toff, n);
+    LAUNCH(c, k_touch_starts, cdiv((u64)n + 1, 256), 256, 0, n, P, keys, toff, nin);
     c.arena.release(m);
 }
 

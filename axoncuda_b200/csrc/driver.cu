@@ -311,6 +311,7 @@ int axc_create(int device, size_t arena_bytes, axc_ctx **out) {
         setup_construct_kernels();
         setup_prim_kernels();
         setup_coarsen_kernels(c);
+        setup_initpart_kernels();
         setup_refine_kernels(c);
         scan_state_create(c, 1u << 18);  // single-pass scans of up to 2^29 elements
         AXC_CUDA(cudaDeviceSynchronize());

@@ -6,6 +6,7 @@
 // balance slack (the driver caps cluster sizes in k-way mode) every chunk fits omega.
 #include "common.cuh"
 #include "kernels.h"
+#include "blocksort.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -18,28 +19,45 @@ __global__ void k_bfs_init(u32 n, u32 *__restrict__ dist, u32 root, u32 *__restr
     if (v < n) dist[v] = v == root ? 0u : NONE;
     if (v == 0) front[0] = root;
 }
-__global__ void k_bfs_expand(const u32 *__restrict__ front, u32 nf, u32 level, const u64 *__restrict__ toff,
-                             const u32 *__restrict__ touch, const u64 *__restrict__ off, const u32 *__restrict__ pins,
-                             u32 *__restrict__ hdone, u32 *__restrict__ dist, u32 *__restrict__ next, u32 *__restrict__ nn) {
-    const u32 i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= nf) return;
-    const u32 u = front[i];
-    const u64 jend = toff[u + 1];
-    // 32 incidences claimed at once (one per lane), then each claimed hyperedge expanded by the
-    // whole warp; the distances do not depend on the order
-    for (u64 jb = toff[u]; jb < jend; jb += 32) {
-        const u64 j = jb + lane;
-        const u32 h = j < jend ? touch[j] : 0;
-        const bool mine = j < jend && atomicExch(&hdone[h], 1u) == 0;
-        u32 bal = __ballot_sync(0xFFFFFFFFu, mine);
-        while (bal) {
-            const u32 t = __ffs(bal) - 1;
-            bal &= bal - 1;
-            const u32 hh = __shfl_sync(0xFFFFFFFFu, h, t);
-            for (u64 k = off[hh] + lane; k < off[hh + 1]; k += 32) {
-                const u32 v = pins[k];
-                if (atomicCAS(&dist[v], NONE, level + 1) == NONE) next[atomicAdd(nn, 1u)] = v;
-            }
+// One BFS level in two launches: the frontier's incidences claim their hyperedges into a list, and
+// each claimed hyperedge's pins are reached by a warp of its own. (One warp per frontier node would
+// walk through all pins of all its hyperedges: the first levels have one or a few nodes.) The
+// distances do not depend on the order.
+__global__ void k_bfs_claim(const u32 *__restrict__ front, u32 nf, const u64 *__restrict__ toff,
+                            const u32 *__restrict__ touch, u32 *__restrict__ hdone, u32 *__restrict__ hlist,
+                            u32 *__restrict__ nh) {
+    const u32 lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    for (u32 i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nf; i += nw) {
+        const u32 u = front[i];
+        const u64 jend = toff[u + 1];
+        for (u64 jb = toff[u]; jb < jend; jb += 32) {
+            const u64 j = jb + lane;
+            const u32 h = j < jend ? touch[j] : 0;
+            const bool mine = j < jend && !*(volatile u32 *)&hdone[h] && atomicExch(&hdone[h], 1u) == 0;
+            const u32 bal = __ballot_sync(0xFFFFFFFFu, mine);
+            u32 at = 0;
+            if (lane == 0 && bal) at = atomicAdd(nh, (u32)__popc(bal));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (mine) hlist[at + __popc(bal & ((1u << lane) - 1u))] = h;
+        }
+    }
+}
+__global__ void k_bfs_reach(const u32 *__restrict__ hlist, const u32 *__restrict__ nh, u32 level,
+                            const u64 *__restrict__ off, const u32 *__restrict__ pins, u32 *__restrict__ dist,
+                            u32 *__restrict__ next, u32 *__restrict__ nn) {
+    const u32 lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5, n = *nh;
+    for (u32 i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
+        const u32 h = hlist[i];
+        const u64 b = off[h + 1];
+        for (u64 kb = off[h]; kb < b; kb += 32) {
+            const u64 k = kb + lane;
+            const u32 v = k < b ? pins[k] : 0;
+            const bool mine = k < b && *(volatile u32 *)&dist[v] == NONE && atomicCAS(&dist[v], NONE, level + 1) == NONE;
+            const u32 bal = __ballot_sync(0xFFFFFFFFu, mine);
+            u32 at = 0;
+            if (lane == 0 && bal) at = atomicAdd(nn, (u32)__popc(bal));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (mine) next[at + __popc(bal & ((1u << lane) - 1u))] = v;
         }
     }
 }
@@ -55,13 +73,16 @@ __global__ void k_gather_w(const u32 *__restrict__ ord, u32 n, const u32 *__rest
     u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) w[i] = nsize[ord[i]];
 }
+// The chunk of a node of weight w with weight `before` ahead of it, of k equal ones in all (W).
+__device__ __forceinline__ u32 chunk_of(u64 before, u64 w, u64 W, u32 k) {
+    const unsigned __int128 x = (unsigned __int128)(2 * before + w) * k;
+    const u64 q = (u64)(x / (unsigned __int128)(2 * W));
+    return (u32)(q < k - 1 ? q : k - 1);
+}
 __global__ void k_chunk(const u32 *__restrict__ ord, u32 n, const u64 *__restrict__ before, const u64 *__restrict__ w,
                         u64 W, u32 k, u32 base, u32 *__restrict__ part) {
     u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    unsigned __int128 x = (unsigned __int128)(2 * before[i] + w[i]) * k;
-    u64 q = (u64)(x / (unsigned __int128)(2 * W));
-    part[ord[i]] = base + (u32)(q < k - 1 ? q : k - 1);
+    if (i < n) part[ord[i]] = base + chunk_of(before[i], w[i], W, k);
 }
 
 // ---- the k-way multi-start (include/axc.h AXC_KWAY_TRIES) ----------------------------------------
@@ -109,6 +130,58 @@ __global__ void k_try_keys(u32 n, u32 salt, u32 *__restrict__ key, u32 *__restri
     const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v < n) { key[v] = mix32(v ^ salt); ord[v] = v; }
 }
+// The random starts of copies of at most RSS_CAP nodes, one block each (copy blockIdx.x + 1): the
+// order by (hash, id) sorted in shared memory, the weights before each node by block scans, and the
+// weight chunks.
+__global__ void __launch_bounds__(RSS_WARPS * 32) k_copy_starts(u32 n, u32 seed, const u32 *__restrict__ nsize, u64 W,
+                                                                u32 k, u32 *__restrict__ partS) {
+    extern __shared__ u32 sm[];
+    __shared__ u64 wsum[32];
+    const u32 t = blockIdx.x + 1, salt = mix32(t * 0x9E3779B9u + seed);
+    const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    for (u32 v = threadIdx.x; v < n; v += blockDim.x) { sm[v] = mix32(v ^ salt); sm[RSS_CAP + v] = v; }
+    const u32 *ko, *vo;
+    block_radix_sort(sm, n, 32, ko, vo);
+    u64 run = 0;
+    for (u32 b = 0; b < n; b += blockDim.x) {
+        const u32 i = b + threadIdx.x, v = i < n ? vo[i] : 0;
+        const u64 s = i < n ? nsize[v] : 0;
+        u64 x = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u64 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if ((int)lane >= o) x += y;
+        }
+        __syncthreads();
+        if (lane == 31) wsum[w] = x;
+        __syncthreads();
+        u64 before = run + x - s, tot = 0;
+        for (u32 i2 = 0; i2 < RSS_WARPS; ++i2) {
+            if (i2 < w) before += wsum[i2];
+            tot += wsum[i2];
+        }
+        run += tot;
+        if (i < n) partS[(u64)t * n + v] = t * k + chunk_of(before, s, W, k);
+    }
+}
+// The incidence lists of copy 0 (n nodes, e2 hyperedges, P2 pins) repeated for the others.
+__global__ void k_copy_touch(u32 n, u32 e2, u64 P2, u32 nc, u64 *__restrict__ toff, u32 *__restrict__ touch,
+                             u32 *__restrict__ nin) {
+    const u64 i0 = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
+    for (u64 j = i0; j < P2; j += step) {
+        const u32 h = touch[j];
+        for (u32 t = 1; t < nc; ++t) touch[t * P2 + j] = t * e2 + h;
+    }
+    for (u64 v = i0; v < n; v += step) {
+        const u64 o = toff[v];
+        const u32 d = nin[v];
+        for (u32 t = 1; t < nc; ++t) {
+            toff[(u64)t * n + v] = t * P2 + o;
+            nin[(u64)t * n + v] = d;
+        }
+    }
+    if (i0 == 0) toff[(u64)nc * n] = nc * P2;
+}
 __global__ void k_pick_copy(u32 n, const u32 *__restrict__ partS, u32 best, u32 k, u32 *__restrict__ part) {
     const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v < n) part[v] = partS[(u64)best * n + v] - best * k;
@@ -119,14 +192,16 @@ u32 bfs(Ctx &c, const DLevel &L, u32 root, u32 *dist) {
     size_t m = c.arena.mark();
     const u32 n = L.n;
     u32 *fa = c.arena.alloc<u32>(n), *fb = c.arena.alloc<u32>(n), *hd = c.arena.alloc<u32>(L.e ? L.e : 1);
-    u32 *nn = c.arena.alloc<u32>(1);
+    u32 *hlist = c.arena.alloc<u32>(L.e ? L.e : 1);
+    u32 *nn = c.arena.alloc<u32>(2);  // nodes reached, hyperedges claimed
     AXC_CUDA(cudaMemsetAsync(hd, 0, (size_t)L.e * 4, c.stream));
     LAUNCH(c, k_bfs_init, cdiv(n, 256), 256, 0, n, dist, root, fa);
     u32 nf = 1, lvl = 0;
     while (nf) {
-        AXC_CUDA(cudaMemsetAsync(nn, 0, 4, c.stream));
-        LAUNCH(c, k_bfs_expand, cdiv((u64)nf * 32, 256), 256, 0, fa, nf, lvl, L.toff, L.touch, L.off, L.pins, hd, dist,
-               fb, nn);
+        AXC_CUDA(cudaMemsetAsync(nn, 0, 8, c.stream));
+        LAUNCH(c, k_bfs_claim, std::min<u32>(cdiv((u64)nf * 32, 256), (u32)c.sms * 8), 256, 0, fa, nf, L.toff, L.touch, hd,
+               hlist, nn + 1);
+        LAUNCH(c, k_bfs_reach, (u32)c.sms * 8, 256, 0, hlist, nn + 1, lvl, L.off, L.pins, dist, fb, nn);
         nf = fetch1(c, nn);
         std::swap(fa, fb);
         ++lvl;
@@ -136,6 +211,10 @@ u32 bfs(Ctx &c, const DLevel &L, u32 root, u32 *dist) {
 }
 
 }  // namespace
+
+void setup_initpart_kernels() {
+    AXC_CUDA(cudaFuncSetAttribute(k_copy_starts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
+}
 
 void kway_initial(Ctx &c, const DLevel &L, u32 k, u32 *part) {
     const u32 n = L.n;
@@ -198,8 +277,15 @@ bool kway_multistart(Ctx &c, const DLevel &L, const u32 *wfx, u32 k, u32 omega, 
     S.toff = c.arena.alloc<u64>((u64)S.n + 1);
     S.touch = c.arena.alloc<u32>(S.P);
     S.nin = c.arena.alloc<u32>(S.n);
-    build_touching(c, S.n, S.e, S.off, S.pins, S.nsrc, S.P, S.toff, S.touch, S.nin);
-    {  // the random starts: weight chunks of a hashed node order, partition ids shifted by t * k
+    // copy 0 comes first in every array: its incidence lists, repeated for the others
+    build_touching(c, n, e2, S.off, S.pins, S.nsrc, P2, S.toff, S.touch, S.nin);
+    LAUNCH(c, k_copy_touch, std::min<u32>(cdiv(std::max<u64>(P2, n), 256), (u32)c.sms * 8), 256, 0, n, e2, P2, nc, S.toff,
+           S.touch, S.nin);
+    // the random starts: weight chunks of a hashed node order, partition ids shifted by t * k
+    if (n <= (u32)RSS_CAP) {
+        const u64 W = reduce_sum_u32(c, L.nsize, n);
+        LAUNCH(c, k_copy_starts, nc - 1, RSS_WARPS * 32, RSS_SMEM, n, (u32)seed, L.nsize, W ? W : 1, k, partS);
+    } else {
         const size_t m1 = c.arena.mark();
         u32 *key = c.arena.alloc<u32>(n), *ord = c.arena.alloc<u32>(n);
         u64 *w = c.arena.alloc<u64>((u64)n + 1), *before = c.arena.alloc<u64>((u64)n + 1);

@@ -82,6 +82,7 @@ void part_sizes(Ctx &c, u32 n, const u32 *part, const u32 *nsize, u64 *psize, u3
 void part_inbound(Ctx &c, const DLevel &L, const Census &cs, u64 *pinb, u32 K);
 
 // initpart.cu
+void setup_initpart_kernels();
 void kway_initial(Ctx &c, const DLevel &L, u32 k, u32 *part);
 // the k-way multi-start on the coarsest level (include/axc.h AXC_KWAY_TRIES): refines part[n]
 // from its BFS start and random ones, keeps the best; false when fewer than 2 copies fit
