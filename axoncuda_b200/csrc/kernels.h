@@ -77,7 +77,8 @@ struct Census {
     u32 *mask = nullptr, *dmask = nullptr;  // [e * mw]
     u32 mw = 0;
 };
-Census build_census(Ctx &c, const DLevel &L, const u32 *part);
+// K: partition ids are below it
+Census build_census(Ctx &c, const DLevel &L, const u32 *part, u32 K);
 void part_sizes(Ctx &c, u32 n, const u32 *part, const u32 *nsize, u64 *psize, u32 K);
 void part_inbound(Ctx &c, const DLevel &L, const Census &cs, u64 *pinb, u32 K);
 

@@ -163,7 +163,7 @@ u32 greedy_pack(Ctx &c, const u64 *ss, const u64 *si, u32 m, u64 omega, u64 delt
 void merge_small_partitions(Ctx &c, const DLevel &L, u32 *part, u32 K, u32 omega, u32 delta) {
     if (K == 0) return;
     size_t mk = c.arena.mark();
-    Census cs = build_census(c, L, part);
+    Census cs = build_census(c, L, part, K);
     u64 *psize = c.arena.alloc<u64>(K), *pinb = c.arena.alloc<u64>(K);
     part_sizes(c, L.n, part, L.nsize, psize, K);
     part_inbound(c, L, cs, pinb, K);
@@ -209,7 +209,7 @@ void evaluate(Ctx &c, const DLevel &L, const u32 *wfx, const u32 *part, u32 omeg
               axc_stats *st) {
     size_t mk = c.arena.mark();
     const u32 K = L.n ? reduce_max_u32(c, part, L.n) + 1 : 0;
-    Census cs = build_census(c, L, part);
+    Census cs = build_census(c, L, part, K);
     u64 *psize = c.arena.alloc<u64>(K ? K : 1), *pinb = c.arena.alloc<u64>(K ? K : 1);
     // validity counts nodes (not node weights), like sources/constr.cpp:95-115
     AXC_CUDA(cudaMemsetAsync(psize, 0, (size_t)K * 8, c.stream));

@@ -86,59 +86,258 @@ __device__ __forceinline__ void cs_insert(const CensusArgs &A, u64 a, u64 b, u64
     }
 }
 
-__global__ void k_census_warp(u32 e, CensusArgs A) {
-    __shared__ u32 tk[CS_WARPS][2 * CS_WARP_CAP], tm[CS_WARPS][2 * CS_WARP_CAP], tc[CS_WARPS][2 * CS_WARP_CAP],
-        td[CS_WARPS][2 * CS_WARP_CAP];
-    const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const u32 h = blockIdx.x * CS_WARPS + w;
-    if (h >= e) return;
-    const u64 a = A.off[h], b = A.off[h + 1], s = a + A.nsrc[h];
-    const u32 len = (u32)(b - a);
-    if (len > CS_WARP_CAP) return;
-    u32 cap = 32;
-    while (cap < 2 * len) cap <<= 1;
-    u32 *keys = tk[w], *mn = tm[w], *cnt = tc[w], *dcnt = td[w];
-    for (u32 i = lane; i < cap; i += 32) { keys[i] = NONE; mn[i] = NONE; cnt[i] = 0; dcnt[i] = 0; }
-    __syncwarp();
-    cs_insert(A, a, b, s, keys, mn, cnt, dcnt, cap - 1, lane, 32);
-    __syncwarp();
-    u32 o = 0;
-    for (u64 base = a; base < b; base += 32) {
-        u64 k = base + lane;
-        u32 slot = NONE, p = 0;
-        if (k < b) {
-            p = A.part[A.pins[k]];
-            slot = hash_find(keys, cap - 1, p);
+// The hashed census by hyperedge length. Every kernel reads a pin's partition once; the entries of a
+// hyperedge come in no particular order (all consumers read them as a set).
+//  - at most CS_SHORT pins: a warp stages the partitions of consecutive hyperedges in shared memory
+//    and every pin counts its own among its hyperedge's (no table);
+//  - up to CS_WARP_CAP: one warp, a hash table of packed counts; the pin that inserts a partition
+//    writes its entry;
+//  - up to CS_BLOCK_CAP: one block, the same with the counts indexed by partition up to CS_DIRECT_K
+//    partitions, hashed above;
+//  - longer: one block, a table in device memory (k_census_block).
+constexpr u32 CS_SHORT = 32;
+constexpr u32 CS_STAGE = 512;        // pins a warp stages
+constexpr u32 CS_THREADS = 256;
+constexpr u32 CS_DIRECT_K = 16384;
+
+__global__ void __launch_bounds__(CS_THREADS) k_census_short(u32 e, CensusArgs A, u32 per_warp) {
+    constexpr u32 NW = CS_THREADS / 32;
+    __shared__ u32 sp[NW][CS_STAGE];
+    __shared__ u32 sn[NW][32];
+    const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    u32 *st = sp[w], *num = sn[w];
+    const u32 step = gridDim.x * NW * per_warp;
+    for (u32 h0 = (blockIdx.x * NW + w) * per_warp; h0 < e; h0 += step) {
+        const u32 h = h0 + lane;
+        const bool mine = lane < per_warp && h < e;
+        const u64 a = mine ? A.off[h] : 0, len64 = mine ? A.off[h + 1] - a : 0;
+        const bool take = mine && len64 <= CS_SHORT;
+        const u32 len = take ? (u32)len64 : 0u, ns = take ? A.nsrc[h] : 0u;
+        const u32 wh = take && A.save ? A.wfx[h] : 0u;
+        u32 x = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if ((int)lane >= o) x += y;
         }
-        if (A.save && slot != NONE)
-            atomicAdd(&A.save[A.pins[k]], (unsigned long long)leave_gain(A.encourage, A.wfx[h], cnt[slot]));
-        bool first = slot != NONE && mn[slot] == (u32)(k - a);
-        u32 bal = __ballot_sync(0xFFFFFFFFu, first);
-        if (first) {
-            u64 dst = a + o + __popc(bal & ((1u << lane) - 1u));
-            A.cpart[dst] = p;
-            A.ccnt[dst] = cnt[slot];
-            A.cdcnt[dst] = dcnt[slot];
+        const u32 excl = x - len;
+        num[lane] = 0;
+        for (u32 lo = 0; lo < 32;) {  // as many of the hyperedges as the stage holds at a time
+            const u32 b0 = __shfl_sync(0xFFFFFFFFu, excl, lo);
+            const u32 hi = lo + __popc(__ballot_sync(0xFFFFFFFFu, lane >= lo && x - b0 <= CS_STAGE));
+            const u32 T = __shfl_sync(0xFFFFFFFFu, x, hi - 1) - b0;
+            for (u32 pass = 0; pass < 2; ++pass) {
+                for (u32 f0 = 0; f0 < T; f0 += 32) {
+                    const u32 f = f0 + lane;
+                    u32 ol = lo, oh = hi - 1;  // owner: the last hyperedge starting at or before f
+                    for (int it = 0; it < 5; ++it) {
+                        const u32 mid = (ol + oh + 1) >> 1;
+                        const u32 em = __shfl_sync(0xFFFFFFFFu, excl, mid & 31);
+                        if (ol < oh) { if (em - b0 <= f) ol = mid; else oh = mid - 1; }
+                    }
+                    const u32 eo = __shfl_sync(0xFFFFFFFFu, excl, ol) - b0;
+                    const u64 ao = __shfl_sync(0xFFFFFFFFu, a, ol);
+                    const bool in = f < T;
+                    if (pass == 0) {
+                        if (in) st[f] = A.part[A.pins[ao + (f - eo)]];
+                        continue;
+                    }
+                    const u32 lo_len = __shfl_sync(0xFFFFFFFFu, len, ol), no = __shfl_sync(0xFFFFFFFFu, ns, ol);
+                    const u32 wo = __shfl_sync(0xFFFFFFFFu, wh, ol);
+                    u32 c = 0, dc = 0, p = 0;
+                    bool first = in;
+                    if (in) {
+                        p = st[f];
+                        for (u32 j = 0; j < lo_len; ++j) {
+                            const bool same = st[eo + j] == p;
+                            c += same;
+                            dc += same && j >= no;
+                            first = first && !(same && eo + j < f);
+                        }
+                        if (A.save) {
+                            const i64 g = leave_gain(A.encourage, wo, c);
+                            if (g) atomicAdd(&A.save[A.pins[ao + (f - eo)]], (unsigned long long)g);
+                        }
+                    }
+                    // the firsts of one hyperedge in this chunk are consecutive lanes, after those of
+                    // earlier chunks (num)
+                    const u32 bal = __ballot_sync(0xFFFFFFFFu, first);
+                    const u32 s0 = in && eo > f0 ? eo - f0 : 0;  // the owner's first lane of this chunk
+                    const u32 seg = s0 < 32 ? 0xFFFFFFFFu << s0 : 0u;
+                    const u32 had = in ? num[ol] : 0u;
+                    __syncwarp();
+                    if (first) {
+                        const u64 dst = ao + had + __popc(bal & lt & seg);
+                        A.cpart[dst] = p;
+                        A.ccnt[dst] = c;
+                        A.cdcnt[dst] = dc;
+                    }
+                    // the owner's last lane of this chunk
+                    if (in && (lane == 31 || f + 1 == eo + lo_len || f + 1 == T))
+                        num[ol] = had + __popc(bal & (lt | (1u << lane)) & seg);
+                    __syncwarp();
+                }
+                __syncwarp();
+            }
+            lo = hi;
         }
-        o += __popc(bal);
+        if (take) A.lam[h] = num[lane];
+        __syncwarp();  // num is no longer read
     }
-    if (lane == 0) A.lam[h] = o;
 }
 
+__global__ void __launch_bounds__(CS_WARPS * 32) k_census_warp(u32 e, CensusArgs A, u32 per_warp) {
+    __shared__ u32 tk[CS_WARPS][2 * CS_WARP_CAP], tv[CS_WARPS][2 * CS_WARP_CAP];
+    constexpr u32 R = CS_WARP_CAP / 32;
+    const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    const u32 h0 = (blockIdx.x * CS_WARPS + w) * per_warp;
+    u32 *keys = tk[w], *val = tv[w];
+    const u32 hl = h0 + lane;
+    const u64 al = lane < per_warp && hl < e ? A.off[hl] : 0, ll = lane < per_warp && hl < e ? A.off[hl + 1] - al : 0;
+    u32 todo = __ballot_sync(0xFFFFFFFFu, ll > CS_SHORT && ll <= CS_WARP_CAP);
+    while (todo) {
+        const u32 t = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const u32 h = h0 + t, len = (u32)__shfl_sync(0xFFFFFFFFu, ll, t);
+        const u64 a = __shfl_sync(0xFFFFFFFFu, al, t);
+        const u32 ns = A.nsrc[h], wh = A.save ? A.wfx[h] : 0u;
+        u32 cap = 64;
+        while (cap < 2 * len) cap <<= 1;
+        u32 v[R], q[R];
+#pragma unroll
+        for (u32 i = 0; i < R; ++i) v[i] = lane + 32 * i < len ? A.pins[a + lane + 32 * i] : 0;
+#pragma unroll
+        for (u32 i = 0; i < R; ++i) q[i] = lane + 32 * i < len ? A.part[v[i]] : 0;
+        for (u32 i = lane; i < cap; i += 32) { keys[i] = NONE; val[i] = 0; }
+        __syncwarp();
+        u32 fresh = 0;  // bit i: this lane's pin i inserted its partition
+#pragma unroll
+        for (u32 i = 0; i < R; ++i) {
+            if (lane + 32 * i >= len) continue;
+            bool f;
+            const u32 slot = hash_insert_fresh(keys, cap - 1, q[i], f);
+            if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); q[i] = 0; continue; }
+            atomicAdd(&val[slot], (1u << 16) | (lane + 32 * i >= ns ? 1u : 0u));
+            q[i] = slot;
+            fresh |= (u32)f << i;
+        }
+        __syncwarp();
+        u32 o = 0;
+#pragma unroll
+        for (u32 i = 0; i < R; ++i) {
+            if (32 * i >= len) break;
+            const bool in = lane + 32 * i < len;
+            const u32 c = in ? val[q[i]] : 0u;
+            if (A.save && in) {
+                const i64 g = leave_gain(A.encourage, wh, c >> 16);
+                if (g) atomicAdd(&A.save[v[i]], (unsigned long long)g);
+            }
+            const bool f = (fresh >> i) & 1u;
+            const u32 bal = __ballot_sync(0xFFFFFFFFu, f);
+            if (f) {
+                const u64 dst = a + o + __popc(bal & lt);
+                A.cpart[dst] = keys[q[i]];
+                A.ccnt[dst] = c >> 16;
+                A.cdcnt[dst] = c & 0xFFFFu;
+            }
+            o += __popc(bal);
+        }
+        if (lane == 0) A.lam[h] = o;
+        __syncwarp();  // the tables are no longer read
+    }
+}
+
+// Listed hyperedges of CS_WARP_CAP < |e| <= CS_BLOCK_CAP pins, one block at a time each. DIRECT: the
+// counts are indexed by partition (T = K words, all zero between hyperedges), else a hash table
+// sized by the hyperedge (T slots at most).
+template <bool DIRECT>
+__global__ void __launch_bounds__(CS_THREADS) k_census_mid(const u32 *__restrict__ list, u32 nlist, CensusArgs A, u32 T) {
+    extern __shared__ u32 cm_dyn[];
+    __shared__ unsigned short slot[CS_BLOCK_CAP];
+    __shared__ u32 s_n;
+    constexpr u32 FRESH = 0x8000u;
+    static_assert(CS_DIRECT_K <= FRESH && 2 * CS_BLOCK_CAP <= FRESH, "a slot and its flag fit 16 bits");
+    u32 *val = cm_dyn, *keys = cm_dyn + T;
+    const u32 lane = threadIdx.x & 31u;
+    if (DIRECT)
+        for (u32 i = threadIdx.x; i < T; i += CS_THREADS) val[i] = 0;
+    for (u32 idx = blockIdx.x; idx < nlist; idx += gridDim.x) {
+        const u32 h = list[idx];
+        const u64 a = A.off[h];
+        const u32 len = (u32)(A.off[h + 1] - a), ns = A.nsrc[h];
+        const u32 cap = DIRECT ? 0 : cs_cap(len);
+        if (!DIRECT && cap > T) {  // launched with too small a table: refuse
+            if (threadIdx.x == 0) atomicExch(A.status, DEV_HASH_FULL);
+            continue;
+        }
+        if (!DIRECT)
+            for (u32 i = threadIdx.x; i < cap; i += CS_THREADS) { keys[i] = NONE; val[i] = 0; }
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        constexpr u32 U = 4;
+        for (u32 k0 = threadIdx.x; k0 < len; k0 += U * CS_THREADS) {
+            u32 q[U];
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) q[x] = k0 + x * CS_THREADS < len ? A.pins[a + k0 + x * CS_THREADS] : 0;
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) q[x] = k0 + x * CS_THREADS < len ? A.part[q[x]] : 0;
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) {
+                const u32 k = k0 + x * CS_THREADS;
+                if (k >= len) continue;
+                u32 s = q[x];
+                bool f = false;
+                if (!DIRECT) {
+                    s = hash_insert_fresh(keys, cap - 1, q[x], f);
+                    if (s == NONE) { atomicExch(A.status, DEV_HASH_FULL); slot[k] = 0; continue; }
+                }
+                const u32 old = atomicAdd(&val[s], (1u << 16) | (k >= ns ? 1u : 0u));
+                if (DIRECT) f = old == 0;
+                slot[k] = (unsigned short)(s | (f ? FRESH : 0u));
+            }
+        }
+        __syncthreads();
+        const u32 wh = A.save ? A.wfx[h] : 0u;
+        for (u32 kb = 0; kb < len; kb += CS_THREADS) {
+            const u32 k = kb + threadIdx.x;
+            const u32 s = k < len ? slot[k] : 0u;
+            const u32 c = k < len ? val[s & (FRESH - 1)] : 0u;
+            if (A.save && k < len) {
+                const i64 g = leave_gain(A.encourage, wh, c >> 16);
+                if (g) atomicAdd(&A.save[A.pins[a + k]], (unsigned long long)g);
+            }
+            const bool f = (s & FRESH) != 0;
+            const u32 bal = __ballot_sync(0xFFFFFFFFu, f);
+            u32 at = 0;
+            if (lane == 0 && bal) at = atomicAdd(&s_n, (u32)__popc(bal));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (f) {
+                const u64 dst = a + at + __popc(bal & ((1u << lane) - 1u));
+                A.cpart[dst] = DIRECT ? (s & (FRESH - 1)) : keys[s & (FRESH - 1)];
+                A.ccnt[dst] = c >> 16;
+                A.cdcnt[dst] = c & 0xFFFFu;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) A.lam[h] = s_n;
+        if (DIRECT)
+            for (u32 k = threadIdx.x; k < len; k += CS_THREADS)
+                if (slot[k] & FRESH) val[slot[k] & (FRESH - 1)] = 0;
+        __syncthreads();
+    }
+}
+
+// Hyperedges of more than CS_BLOCK_CAP pins: one block each, the table (keys, first positions, counts)
+// in device memory.
 __global__ void k_census_block(const u32 *__restrict__ list, u32 nlist, CensusArgs A, u32 *gtab,
                                const u64 *__restrict__ gtab_off) {
-    extern __shared__ u32 dyn[];
     __shared__ u32 wsum[33];
     if (blockIdx.x >= nlist) return;
     const u32 h = list[blockIdx.x];
     const u64 a = A.off[h], b = A.off[h + 1], s = a + A.nsrc[h];
     const u32 len = (u32)(b - a);
     const u32 cap = cs_cap(len);
-    if (!gtab && 16ull * cap > dyn_smem_bytes()) {  // launched with too small a table: refuse
-        if (threadIdx.x == 0) atomicExch(A.status, DEV_HASH_FULL);
-        return;
-    }
-    u32 *keys = gtab ? gtab + 4 * gtab_off[blockIdx.x] : dyn;
+    u32 *keys = gtab + 4 * gtab_off[blockIdx.x];
     u32 *mn = keys + cap, *cnt = mn + cap, *dcnt = cnt + cap;
     for (u32 i = threadIdx.x; i < cap; i += blockDim.x) { keys[i] = NONE; mn[i] = NONE; cnt[i] = 0; dcnt[i] = 0; }
     __syncthreads();
@@ -3663,7 +3862,8 @@ static bool round_loop_enabled() {
 }
 
 void setup_refine_kernels(Ctx &c) {
-    AXC_CUDA(cudaFuncSetAttribute(k_census_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 2 * CS_BLOCK_CAP * 4));
+    AXC_CUDA(cudaFuncSetAttribute(k_census_mid<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CS_DIRECT_K * 4));
+    AXC_CUDA(cudaFuncSetAttribute(k_census_mid<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * CS_BLOCK_CAP * 8));
     AXC_CUDA(cudaFuncSetAttribute(k_part_inbound_smem<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PI_SMEM_K * 4));
     AXC_CUDA(cudaFuncSetAttribute(k_part_inbound_smem<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PI_SMEM_K * 4));
     AXC_CUDA(cudaFuncSetAttribute(k_part_inbound_smem<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PI_SMEM_K * 4));
@@ -3786,7 +3986,8 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
 // (the bound itself when the level's is not known).
 static u64 block_tier_len(const LevelPrep &lp, u64 bound) { return lp.max_len && lp.max_len < bound ? lp.max_len : bound; }
 
-static void run_census(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *part, Census &cs) {
+// K: partition ids are below it (~0 when no bound is known).
+static void run_census(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *part, u32 K, Census &cs) {
     cs.beg = L.off;
     if (L.e == 0) return;
     CensusArgs A{L.off, L.pins, L.nsrc, part, cs.part, cs.cnt, cs.dcnt, cs.lam, c.d_status,
@@ -3801,11 +4002,25 @@ static void run_census(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
             LAUNCH(c, k_census_direct_block, lp.n_hblock, 256, 0, lp.hblock, lp.n_hblock, A, lp.census_K);
         return;
     }
-    LAUNCH(c, k_census_warp, cdiv(L.e, CS_WARPS), CS_WARPS * 32, 0, L.e, A);
-    if (lp.n_hblock)
-        LAUNCH(c, k_census_block, lp.n_hblock, 256, 16 * (size_t)cs_cap(block_tier_len(lp, CS_BLOCK_CAP)),
-               lp.hblock, lp.n_hblock, A,
-               (u32 *)nullptr, (const u64 *)nullptr);
+    // hyperedges a warp looks at: fewer where the mean length leaves it many pins each
+    u32 per = 32;
+    while (per > 2 && (L.P / L.e * per > 1024 || L.e / per < (u32)c.sms * 16)) per >>= 1;
+    LAUNCH(c, k_census_short, std::min<u32>(cdiv(L.e, (CS_THREADS / 32) * per), (u32)c.sms * 8), CS_THREADS, 0, L.e, A, per);
+    if (!lp.max_len || lp.max_len > CS_SHORT)
+        LAUNCH(c, k_census_warp, cdiv(L.e, CS_WARPS * per), CS_WARPS * 32, 0, L.e, A, per);
+    if (lp.n_hblock) {
+        const bool direct = K <= CS_DIRECT_K;
+        const u32 T = direct ? K : cs_cap(block_tier_len(lp, CS_BLOCK_CAP));
+        const size_t smem = (size_t)T * (direct ? 4 : 8);
+        const auto launch = [&](auto kernel) {
+            int per_sm = 1;
+            AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, CS_THREADS, smem));
+            LAUNCH_AS(c, "k_census_mid", kernel, std::min<u32>(lp.n_hblock, (u32)c.sms * (u32)std::max(per_sm, 1)),
+                      CS_THREADS, smem, lp.hblock, lp.n_hblock, A, T);
+        };
+        if (direct) launch(k_census_mid<true>);
+        else launch(k_census_mid<false>);
+    }
     if (lp.n_hhuge) {
         size_t m = c.arena.mark();
         u32 *gtab = c.arena.alloc<u32>(4 * lp.huge_tot);
@@ -3961,7 +4176,7 @@ __global__ void k_copy_conn(u64 eS, u32 e2, const u32 *__restrict__ lam, const u
     if (l > 1) atomicAdd(&conn[h / e2], (unsigned long long)wfxS[h] * (l - 1));
 }
 
-Census build_census(Ctx &c, const DLevel &L, const u32 *part) {
+Census build_census(Ctx &c, const DLevel &L, const u32 *part, u32 K) {
     Census cs = alloc_census(c, L);
     size_t m = c.arena.mark();
     LevelPrep lp;
@@ -3980,7 +4195,7 @@ Census build_census(Ctx &c, const DLevel &L, const u32 *part) {
             lp.huge_tot = fetch1(c, lp.huge_tab + lp.n_hhuge);
         }
     }
-    run_census(c, L, lp, part, cs);
+    run_census(c, L, lp, part, K, cs);
     c.arena.release(m);
     return cs;
 }
@@ -4044,7 +4259,7 @@ static Census census_for_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, con
         cs.mask = c.arena.alloc<u32>((u64)(L.e ? L.e : 1) * cs.mw);
         cs.dmask = c.arena.alloc<u32>((u64)(L.e ? L.e : 1) * cs.mw);
     }
-    run_census(c, L, lp, part, cs);
+    run_census(c, L, lp, part, rp.K, cs);
     if (direct && L.e && !lp.census_K)  // a hashed census: masks from its entries
         LAUNCH(c, k_census_masks, cdiv((u64)L.e * 32, 256), 256, 0, L.e, L.off, cs.lam, cs.part, cs.dcnt, cs.mw,
                cs.mask, cs.dmask);
@@ -4790,7 +5005,7 @@ u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp
             AXC_CUDA(cudaGetLastError());
         });
     } else if (copy_conn) {
-        const Census cs = build_census(c, L, part);
+        const Census cs = build_census(c, L, part, rp.K);
         LAUNCH(c, k_copy_conn, cdiv((u64)L.e, 256), 256, 0, (u64)L.e, L.e / rp.copies, cs.lam, wfx, copy_conn);
     }
     c.arena.release(m);
