@@ -2098,21 +2098,20 @@ struct CascadeArgs {
 };
 
 constexpr u32 MV_DST = 0x80000000u;  // mover flag in the node field: the pin is a destination
-constexpr u32 CC_DIRECT_K = 256;
+constexpr u32 CC_DIRECT_K = 256;        // the warp kernel's tables indexed by partition
+constexpr u32 CC_DIRECT_BLOCK_K = 1024; // the block kernels'
 
-__device__ __forceinline__ bool cascade_direct(const CascadeArgs &A) { return A.K <= CC_DIRECT_K; }
 __device__ __forceinline__ u32 cascade_base(const CascadeArgs &A, u32 h) { return A.ce ? (h / A.ce) * A.K : 0u; }
 
 // The hyperedge's census into the table: partition -> (pins, destination pins). Block- or
 // warp-wide over threads [t0, t0 + nt); direct tables hold K slots, hashed ones `cap`.
 __device__ __forceinline__ void cascade_fill(const CascadeArgs &A, u32 h, u64 a, u64 b, u32 lm, u32 *tk, u32 *tc,
-                                             u32 *td, u32 cap, u32 t0, u32 nt) {
+                                             u32 *td, u32 cap, bool direct, u32 t0, u32 nt) {
     if (!A.lam) {
         const u32 base = cascade_base(A, h);
         for (u64 k = a + t0; k < b; k += nt) atomicAdd(&tc[A.state[A.pins[k]].y - base], 1u);
         return;
     }
-    const bool direct = cascade_direct(A);
     for (u32 i = t0; i < lm; i += nt) {
         const u32 q = A.cpart[a + i];
         const u32 s = direct ? q : hash_find_or_insert(tk, cap - 1, q);
@@ -2151,8 +2150,7 @@ __device__ __forceinline__ void emit_pair(const CascadeArgs &A, bool leave, u32 
 // gathered in parallel so the sequential sweep reads no global memory. Hashed tables insert the
 // partitions missing from the census (their counts stay zero); they need cap <= 65536.
 __device__ __forceinline__ void cascade_slots(const CascadeArgs &A, u32 h, const u64 *mv, u32 *sl, u32 m, u32 *tk,
-                                              u32 cap, u32 t0, u32 nt) {
-    const bool direct = cascade_direct(A);
+                                              u32 cap, bool direct, u32 t0, u32 nt) {
     const u32 base = cascade_base(A, h);
     for (u32 i = t0; i < m; i += nt) {
         const u32 v = (u32)mv[i] & ~MV_DST;
@@ -2173,9 +2171,8 @@ __device__ __forceinline__ void cascade_slots(const CascadeArgs &A, u32 h, const
 // cascade_slots; without it (hashed tables too large for 16-bit slots) they are looked up here.
 // One thread; cascade_sweep_warp is the warp-wide form used wherever the slots fit 16 bits.
 __device__ void cascade_sweep(const CascadeArgs &A, u32 h, const u64 *mv, const u32 *sl, u32 m, u32 *tk, u32 *tc,
-                              u32 *td, u32 mask) {
+                              u32 *td, u32 mask, bool direct) {
     const u32 w = A.wfx[h];
-    const bool direct = cascade_direct(A);
     for (u32 i = 0; i < m; ++i) {
         const u32 lowv = (u32)mv[i], r = (u32)(mv[i] >> 32);
         const u32 v = lowv & ~MV_DST;
@@ -2230,7 +2227,7 @@ __device__ void cascade_sweep_warp(const CascadeArgs &A, u32 h, const u64 *mv, c
                                    u32 *tc, u32 *td, u32 *lmask) {
     const u32 lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
     const u32 w = A.wfx[h];
-    const bool direct = cascade_direct(A);
+    const bool direct = lmask != nullptr;
     for (u32 base = 0; base < m; base += 32) {
         const u32 i = base + lane;
         const bool act = i < m;
@@ -2516,22 +2513,42 @@ __global__ void __launch_bounds__(CM_THREADS) k_cascade_dense(CascadeArgs A, Mov
     }
 }
 
-// The hyperedges of more than CM_LEN pins that hold a mover: every such incidence of every mover
-// flags its hyperedge (flag[] zeroed before), then the flags are compacted into the cascade's
-// list. One warp per mover.
-__global__ void k_mover_hedges(const u32 *__restrict__ mv, const u32 *__restrict__ dM, const u64 *__restrict__ toff,
-                               const u32 *__restrict__ touch, const u64 *__restrict__ off, u32 cn, u32 slots,
-                               u32 *__restrict__ flag) {
+// The hyperedges of more than CM_LEN pins that hold a mover. Few movers: every such incidence of
+// every mover flags its hyperedge (mark[]: 0, or 2 where the hyperedge is short and not to be
+// flagged, restored before), and the level's long hyperedges that are flagged form the cascade's
+// list. Many movers (cascade_dense): all of them do. One warp per mover.
+__global__ void k_mover_hedges(CascadeArgs A, MoverArgs V, uint8_t *__restrict__ mark) {
+    if (cascade_dense(V)) return;
     const u32 lane = threadIdx.x & 31u, nw = (gridDim.x * blockDim.x) >> 5;
-    const u32 end = cn ? slots : *dM;
-    for (u32 r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < end; r += nw) {
-        if (cn && r % cn >= dM[r / cn]) continue;
-        const u32 u = mv[r];
-        for (u64 j = toff[u] + lane; j < toff[u + 1]; j += 32) {
-            const u32 h = touch[j];
-            if (off[h + 1] - off[h] > CM_LEN) flag[h] = 1u;
+    const u32 end = A.cn ? V.n : *V.dM;
+    for (u32 x = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < end; x += nw) {
+        if (A.cn && x % A.cn >= V.dM[x / A.cn]) continue;
+        const u32 u = V.mv[x];
+        const u64 t1 = V.toff[u + 1];
+        for (u64 j = V.toff[u] + lane; j < t1; j += 32) {
+            const u32 h = V.touch[j];
+            if (!mark[h]) mark[h] = 1;
         }
     }
+}
+__global__ void k_long_list(MoverArgs V, const u32 *__restrict__ longs, u32 nlong, const uint8_t *__restrict__ mark,
+                            u32 *__restrict__ list, u32 *__restrict__ nlist) {
+    const bool all = cascade_dense(V);
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    const u32 h = i < nlong ? longs[i] : 0;
+    const bool f = i < nlong && (all || mark[h] == 1);
+    const u32 bal = __ballot_sync(0xFFFFFFFFu, f);
+    u32 at = 0;
+    if (lane == 0 && bal) at = atomicAdd(nlist, (u32)__popc(bal));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    if (f) list[at + __popc(bal & ((1u << lane) - 1u))] = h;
+}
+__global__ void k_long_class(u32 e, const u64 *__restrict__ off, u32 *__restrict__ flag, uint8_t *__restrict__ cls) {
+    const u32 h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h >= e) return;
+    const bool lng = off[h + 1] - off[h] > CM_LEN;
+    flag[h] = lng;
+    cls[h] = lng ? 0 : 2;
 }
 
 __global__ void k_cascade_warp(CascadeArgs A, const u32 *__restrict__ list, const u32 *__restrict__ nlist,
@@ -2568,7 +2585,7 @@ __global__ void k_cascade_warp(CascadeArgs A, const u32 *__restrict__ list, cons
             continue;
         }
         const u32 lm = A.lam ? A.lam[h] : 0;
-        const bool direct = cascade_direct(A);
+        const bool direct = A.K <= CC_DIRECT_K;
         const u32 cap = direct ? A.K : cascade_cap32(lm, m);
         if (m > CC_MOV || cap > CC_TAB) {
             if (lane == 0) big[atomicAdd(nbig, 1u)] = h;  // handled by the block kernel
@@ -2595,9 +2612,9 @@ __global__ void k_cascade_warp(CascadeArgs A, const u32 *__restrict__ list, cons
         const u32 ntk = direct ? 2 * A.K : cap;
         for (u32 i = lane; i < ntk; i += 32) tk[w][i] = direct ? 0u : NONE;
         __syncwarp();
-        cascade_fill(A, h, a, b, lm, tk[w], tc[w], td[w], cap, lane, 32);
+        cascade_fill(A, h, a, b, lm, tk[w], tc[w], td[w], cap, direct, lane, 32);
         __syncwarp();
-        cascade_slots(A, h, mvs[w], sl[w], m, tk[w], cap, lane, 32);
+        cascade_slots(A, h, mvs[w], sl[w], m, tk[w], cap, direct, lane, 32);
         __syncwarp();
         cascade_sweep_warp(A, h, mvs[w], sl[w], m, tk[w], tc[w], td[w], direct ? tk[w] : nullptr);
     }
@@ -2627,8 +2644,8 @@ constexpr u32 CB_THREADS = 128;
 constexpr u32 CB_MOV_MAX = 2048;  // movers of the block kernel, in shared memory
 constexpr u32 CB_TAB_HASH = 8192; // hashed table slots of the block kernel, at most
 constexpr size_t CB_DYN_MAX = (size_t)CB_MOV_MAX * 12 + (size_t)CB_TAB_HASH * 12;
-// The block kernel's middle tier (hashed tables): hyperedges with at most CB_MID_MOV movers and
-// CB_MID_TAB table slots take blocks small enough for several per SM; the rest go on to the
+// The block kernel's middle tier: hyperedges with at most CB_MID_MOV movers and, hashed, CB_MID_TAB
+// table slots take blocks small enough for several per SM; the rest go on to the
 // launch sized by the level's largest hyperedge.
 constexpr u32 CB_MID_MOV = 512;
 constexpr u32 CB_MID_TAB = 2048;
@@ -2666,92 +2683,99 @@ __device__ __forceinline__ u32 cascade_gather(const CascadeArgs &A, u32 h, u64 *
     return m;
 }
 
-constexpr u32 CB_SORT_R = 8;                          // keys per thread in the block radix sort
-constexpr u32 CB_RADIX_MAX = CB_SORT_R * CB_THREADS;  // more movers sort bitonically
+constexpr u32 CB_SORT_R = 8;                          // keys per thread in the block bin sort
+constexpr u32 CB_BIN_MAX = CB_SORT_R * CB_THREADS;    // more movers sort bitonically
+constexpr u32 CB_BINS = 512;
 
-// Stable LSD radix sort of buf[0, m) (m <= CB_RADIX_MAX, CB_THREADS threads) by key bits
-// [32, 32 + nbits), 2 bits per pass. Thread t holds positions [t*R, t*R + R) in registers; a
-// pass counts its keys' digits in four 16-bit fields of one u64, scans those across the block
-// (warp shuffles plus one shared word per warp) and writes each key to its digit's offset plus
-// the count of equal digits before it. About 30 instructions per key and pass, against the
-// bitonic sort's log^2 m / 2 compare-exchange stages.
-__device__ __forceinline__ void block_radix_sort_hi(u64 *buf, u32 m, u32 nbits, u64 *wsum) {
-    constexpr u32 NW = CB_THREADS / 32;
-    const u32 R = (m + CB_THREADS - 1) / CB_THREADS;
+// Sort of buf[0, m) (m <= CB_BIN_MAX, CB_THREADS threads) by the rank in the high word: ranks spread
+// over CB_BINS bins by their leading bits, and a key's place in its bin is the number of smaller
+// ranks there, one or two keys as a rule. About a tenth of a radix sort's instructions, which made
+// up most of the block kernel's. idx holds 2 * CB_BIN_MAX shorts of scratch (the slots' array).
+__device__ __forceinline__ void block_bin_sort_hi(u64 *buf, unsigned short *idx, u32 m, u32 rmax, u32 *bins, u32 *wsum) {
+    constexpr u32 NW = CB_THREADS / 32, PER = CB_BINS / CB_THREADS;
     const u32 t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const u32 nb = 32 - __clz(rmax), sh = nb > 9 ? nb - 9 : 0;  // rank >> sh < CB_BINS
+    static_assert(CB_BINS == 512, "nine leading bits");
+    for (u32 i = t; i < CB_BINS; i += CB_THREADS) bins[i] = 0;
+    __syncthreads();
     u64 key[CB_SORT_R];
+    u32 at[CB_SORT_R];
 #pragma unroll
     for (u32 r = 0; r < CB_SORT_R; ++r) {
-        const u32 i = t * R + r;
-        key[r] = (r < R && i < m) ? buf[i] : 0;
+        const u32 i = t + r * CB_THREADS;
+        if (i >= m) continue;
+        key[r] = buf[i];
+        at[r] = atomicAdd(&bins[(u32)(key[r] >> 32) >> sh], 1u);
     }
-    for (u32 sh = 0; sh < nbits; sh += 2) {
-        u64 cnt = 0, pre[CB_SORT_R];
+    __syncthreads();
+    u32 c[PER], s = 0;
 #pragma unroll
-        for (u32 r = 0; r < CB_SORT_R; ++r) {
-            pre[r] = cnt;
-            if (r < R && t * R + r < m) cnt += 1ull << (16 * ((u32)(key[r] >> (32 + sh)) & 3u));
-        }
-        u64 x = cnt;
+    for (u32 k = 0; k < PER; ++k) { c[k] = bins[t * PER + k]; s += c[k]; }
+    u32 x = s;
 #pragma unroll
-        for (u32 o = 1; o < 32; o <<= 1) {
-            const u64 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) wsum[w] = x;
-        __syncthreads();
-        u64 wpre = 0, tot = 0;
-#pragma unroll
-        for (u32 i = 0; i < NW; ++i) {
-            if (i < w) wpre += wsum[i];
-            tot += wsum[i];
-        }
-        const u64 excl = wpre + x - cnt;
-        const u32 c0 = (u32)(tot & 0xFFFFu), c1 = (u32)((tot >> 16) & 0xFFFFu), c2 = (u32)((tot >> 32) & 0xFFFFu);
-#pragma unroll
-        for (u32 r = 0; r < CB_SORT_R; ++r) {
-            if (r < R && t * R + r < m) {
-                const u32 d = (u32)(key[r] >> (32 + sh)) & 3u;
-                const u32 off = d == 0 ? 0u : d == 1 ? c0 : d == 2 ? c0 + c1 : c0 + c1 + c2;
-                buf[off + (u32)(((excl + pre[r]) >> (16 * d)) & 0xFFFFu)] = key[r];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (u32 r = 0; r < CB_SORT_R; ++r) {
-            const u32 i = t * R + r;
-            if (r < R && i < m) key[r] = buf[i];
-        }
+    for (u32 o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
     }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    u32 pre = x - s;
+#pragma unroll
+    for (u32 i = 0; i < NW; ++i)
+        if (i < w) pre += wsum[i];
+#pragma unroll
+    for (u32 k = 0; k < PER; ++k) { bins[t * PER + k] = pre; pre += c[k]; }
+    if (t == CB_THREADS - 1) bins[CB_BINS] = m;
+    __syncthreads();
+#pragma unroll
+    for (u32 r = 0; r < CB_SORT_R; ++r) {
+        const u32 i = t + r * CB_THREADS;
+        if (i < m) idx[bins[(u32)(key[r] >> 32) >> sh] + at[r]] = (unsigned short)i;
+    }
+    __syncthreads();
+#pragma unroll
+    for (u32 r = 0; r < CB_SORT_R; ++r) {
+        if (t + r * CB_THREADS >= m) continue;
+        const u32 b = (u32)(key[r] >> 32) >> sh, lo = bins[b], hi = bins[b + 1];
+        u32 p = lo;
+        for (u32 j = lo; j < hi; ++j) p += buf[idx[j]] < key[r];
+        at[r] = p;
+    }
+    __syncthreads();
+#pragma unroll
+    for (u32 r = 0; r < CB_SORT_R; ++r)
+        if (t + r * CB_THREADS < m) buf[at[r]] = key[r];
+    __syncthreads();
 }
 
 // Sort, tables, slots and sweep of one hyperedge whose m movers (largest rank rmax) are in mvs,
-// block-wide. The shared-memory kernel sorts up to CB_RADIX_MAX of them with the block radix sort
-// (wsum set); more, and the scratch kernel's, sort bitonically. Direct tables leave tk to the sweep's lane masks (2K words, zeroed).
+// block-wide. The shared-memory kernel sorts up to CB_BIN_MAX of them with the block bin sort (bins
+// set); more, and the scratch kernel's, sort bitonically. Direct tables leave tk to the sweep's lane
+// masks (2K words, zeroed).
 __device__ __forceinline__ void cascade_block_one(const CascadeArgs &A, u32 h, u64 *mvs, u32 *sl, u32 m, u32 rmax,
-                                                  u32 *tk, u32 *tc, u32 *td, u32 cap, u64 *wsum) {
-    const bool direct = cascade_direct(A);
+                                                  u32 *tk, u32 *tc, u32 *td, u32 cap, bool direct, u32 *bins,
+                                                  u32 *wsum) {
     u32 P = 1;
     while (P < m) P <<= 1;
-    const bool radix = wsum && m <= CB_RADIX_MAX;
-    if (!radix)
+    const bool binned = bins && m <= CB_BIN_MAX;
+    if (!binned)
         for (u32 i = m + threadIdx.x; i < P; i += blockDim.x) mvs[i] = ~0ull;
     for (u32 i = threadIdx.x; i < cap; i += blockDim.x) { tc[i] = 0; td[i] = 0; }
     const u32 ntk = direct ? 2 * A.K : cap;
     for (u32 i = threadIdx.x; i < ntk; i += blockDim.x) tk[i] = direct ? 0u : NONE;
     __syncthreads();
-    if (radix) block_radix_sort_hi(mvs, m, 32 - __clz(rmax), wsum);
+    if (binned) block_bin_sort_hi(mvs, (unsigned short *)sl, m, rmax, bins, wsum);
     else block_bitonic_u64(mvs, P);
-    cascade_fill(A, h, A.off[h], A.off[h + 1], A.lam ? A.lam[h] : 0, tk, tc, td, cap, threadIdx.x, blockDim.x);
+    cascade_fill(A, h, A.off[h], A.off[h + 1], A.lam ? A.lam[h] : 0, tk, tc, td, cap, direct, threadIdx.x, blockDim.x);
     __syncthreads();
     if (sl) {
-        cascade_slots(A, h, mvs, sl, m, tk, cap, threadIdx.x, blockDim.x);
+        cascade_slots(A, h, mvs, sl, m, tk, cap, direct, threadIdx.x, blockDim.x);
         __syncthreads();
     }
     if (sl) {
         if (threadIdx.x < 32) cascade_sweep_warp(A, h, mvs, sl, m, tk, tc, td, direct ? tk : nullptr);
     } else if (threadIdx.x == 0) {
-        cascade_sweep(A, h, mvs, sl, m, tk, tc, td, cap - 1);
+        cascade_sweep(A, h, mvs, sl, m, tk, tc, td, cap - 1, direct);
     }
     __syncthreads();
 }
@@ -2764,10 +2788,10 @@ __global__ void __launch_bounds__(CB_THREADS) k_cascade_block(CascadeArgs A, con
                                                               u32 *__restrict__ huge, u32 *__restrict__ nhuge) {
     extern __shared__ __align__(16) unsigned char cb_smem[];
     __shared__ u32 cntm, smax;
-    __shared__ u64 wsum[CB_THREADS / 32];
+    __shared__ u32 wsum[CB_THREADS / 32], bins[CB_BINS + 1];
     u64 *mvs = (u64 *)cb_smem;
     u32 *sl = (u32 *)(mvs + smov), *tk = sl + smov, *tc = tk + stab, *td = tc + stab;
-    const bool direct = cascade_direct(A);
+    const bool direct = A.K <= CC_DIRECT_BLOCK_K;
     for (u32 idx = blockIdx.x; idx < *nl; idx += gridDim.x) {
         const u32 h = list[idx];
         u32 rmax;
@@ -2777,7 +2801,7 @@ __global__ void __launch_bounds__(CB_THREADS) k_cascade_block(CascadeArgs A, con
             if (threadIdx.x == 0) huge[atomicAdd(nhuge, 1u)] = h;
             continue;
         }
-        cascade_block_one(A, h, mvs, sl, m, rmax, tk, tc, td, cap, wsum);
+        cascade_block_one(A, h, mvs, sl, m, rmax, tk, tc, td, cap, direct, bins, wsum);
     }
 }
 
@@ -2790,7 +2814,7 @@ __global__ void __launch_bounds__(CB_THREADS) k_cascade_huge(CascadeArgs A, cons
     __shared__ u32 cntm, smax;
     u64 *mvs = scratch_mv + (u64)blockIdx.x * mv_cap;
     u32 *tk = scratch_tab + (u64)blockIdx.x * 3 * tab_cap, *tc = tk + tab_cap, *td = tc + tab_cap;
-    const bool direct = cascade_direct(A);
+    const bool direct = A.K <= CC_DIRECT_BLOCK_K;
     for (u32 idx = blockIdx.x; idx < *nl; idx += gridDim.x) {
         const u32 h = list[idx];
         u32 rmax;
@@ -2798,7 +2822,7 @@ __global__ void __launch_bounds__(CB_THREADS) k_cascade_huge(CascadeArgs A, cons
         const u32 cap = direct ? A.K : cascade_cap32(A.lam[h], m);
         // 16-bit slots cover every direct table and hashed tables of up to 65536 slots
         u32 *sl = (direct || cap <= 65536) ? scratch_sl + (u64)blockIdx.x * mv_cap : nullptr;
-        cascade_block_one(A, h, mvs, sl, m, rmax, tk, tc, td, cap, nullptr);
+        cascade_block_one(A, h, mvs, sl, m, rmax, tk, tc, td, cap, direct, nullptr, nullptr);
     }
 }
 
@@ -3823,6 +3847,8 @@ struct LevelPrep {
     u64 block_work_max = 0;  // largest gain-work bound of the block tier (sizes its shared table)
     u64 gain_bound = 0;     // no gain exceeds this (sum of incident weights)
     u64 max_len = 0;         // largest hyperedge
+    u32 *hlong = nullptr, n_hlong = 0;         // |e| > CM_LEN
+    uint8_t *hclass = nullptr;                 // [e] 0 for those, else 2 (k_mover_hedges)
     u64 max_deg = 0;         // largest degree
     u64 short_pins = 0, short_sq = 0;  // pins of hyperedges of at most CM_LEN pins; sum of their squared lengths
     bool uniform = false;    // every hyperedge has the weight `weight`
@@ -3914,9 +3940,9 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
     // [0] census block list, [1] census huge list, [2..4] node tiers, [5] gain bound,
     // [6] largest work, [7] largest block-tier work, [8] largest degree, [9] largest hyperedge,
     // [10] destination pins, [11] largest weight, [12] complement of the smallest, [13] pins of short
-    // hyperedges, [14] the sum of their squared lengths
-    u64 *dc = c.arena.alloc<u64>(15);
-    AXC_CUDA(cudaMemsetAsync(dc, 0, 120, c.stream));
+    // hyperedges, [14] the sum of their squared lengths, [15] hyperedges above CM_LEN pins
+    u64 *dc = c.arena.alloc<u64>(16);
+    AXC_CUDA(cudaMemsetAsync(dc, 0, 128, c.stream));
     lp.census_K = K <= CD_K || kway ? K : 0;
     if (e) {
         u32 *flag = c.arena.alloc<u32>(e);
@@ -3931,6 +3957,10 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
             LAUNCH(c, k_flag_len, cdiv(e, 256), 256, 0, e, L.off, (u64)CS_BLOCK_CAP, ~0ull, flag);
             compact_indices_dn(c, flag, lp.hhuge, e, (u32 *)(dc + 1));
         }
+        lp.hlong = c.arena.alloc<u32>(e);
+        lp.hclass = c.arena.alloc<uint8_t>(e);
+        LAUNCH(c, k_long_class, cdiv(e, 256), 256, 0, e, L.off, flag, lp.hclass);
+        compact_indices_dn(c, flag, lp.hlong, e, (u32 *)(dc + 15));
         LAUNCH(c, k_level_bounds, cdiv(e, 256), 256, 0, e, L.off, L.nsrc, wfx, (unsigned long long *)(dc + 9));
     }
     if (n) {
@@ -3948,8 +3978,8 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
         LAUNCH(c, k_tier_max, cdiv(n, 256), 256, 0, n, K, work, L.toff, kway ? 1u : 0u,
                (unsigned long long *)(dc + 6));
     }
-    u64 h[15];
-    fetch(c, h, dc, 120);
+    u64 h[16];
+    fetch(c, h, dc, 128);
     lp.n_hblock = (u32)h[0];
     lp.n_hhuge = (u32)h[1];
     for (int t = 0; t < 3; ++t) lp.ncount[t] = (u32)h[2 + t];
@@ -3960,6 +3990,7 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
     lp.dst_pins = h[10];
     lp.short_pins = h[13];
     lp.short_sq = h[14];
+    lp.n_hlong = (u32)h[15];
     if (e && (u32)h[11] == ~(u32)h[12]) {
         lp.uniform = true;
         lp.weight = (u32)h[11];
@@ -4579,7 +4610,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         C.ce = kw ? kw->ce : 0;
         C.cn = slots ? kw->cn : 0;
         C.pbytes = c.profiling("k_cascade_warp") ? c.d_prof_bytes() : nullptr;
-        const bool direct = C.K <= CC_DIRECT_K;
+        const bool direct = C.K <= CC_DIRECT_BLOCK_K;
         size_t m1 = c.arena.mark();
         const bool longs = lp.max_len > CM_LEN;
         // a warp of the dense kernel looks at 32 hyperedges, or fewer where that leaves the GPU idle
@@ -4594,11 +4625,12 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         else if (lp.short_pins) run_cascade_movers<false>(c, C, V, n, L.P, lp.max_deg);
         if (longs) {
             u32 *big = c.arena.alloc<u32>(L.e), *huge = c.arena.alloc<u32>(L.e), *big2 = c.arena.alloc<u32>(L.e);
-            // only the long hyperedges that hold a mover: flagged from the movers' incidences
-            u32 *hflag = c.arena.alloc<u32>(L.e), *hlist = c.arena.alloc<u32>(L.e);
-            AXC_CUDA(cudaMemsetAsync(hflag, 0, (size_t)L.e * 4, c.stream));
-            LAUNCH(c, k_mover_hedges, (u32)c.sms * 8, 256, 0, mv, dM, L.toff, L.touch, L.off, C.cn, n, hflag);
-            compact_indices_dn(c, hflag, hlist, L.e, dHl);
+            // only the long hyperedges that hold a mover
+            u32 *hlist = c.arena.alloc<u32>(L.e);
+            uint8_t *mark = c.arena.alloc<uint8_t>(L.e);
+            AXC_CUDA(cudaMemcpyAsync(mark, lp.hclass, L.e, cudaMemcpyDeviceToDevice, c.stream));
+            LAUNCH(c, k_mover_hedges, (u32)c.sms * 8, 256, 0, C, V, mark);
+            LAUNCH(c, k_long_list, cdiv(lp.n_hlong, 256), 256, 0, V, lp.hlong, lp.n_hlong, mark, hlist, dHl);
             int per_w = 1;
             AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_w, k_cascade_warp, CC_WARPS * 32, 0));
             const u32 gw = std::min<u32>(cdiv(L.e, CC_WARPS), (u32)c.sms * (u32)std::max(per_w, 1));
@@ -4612,8 +4644,8 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
                                                                      std::min<u64>(lp.max_len, smov)),
                                                          CB_TAB_HASH);
             const u32 *blist = big, *bcount = dBig;
-            if (!direct && (smov > CB_MID_MOV || stab > CB_MID_TAB)) {  // middle tier first
-                const u32 smid = std::min(smov, CB_MID_MOV), tmid = std::min(stab, CB_MID_TAB);
+            if (smov > CB_MID_MOV || (!direct && stab > CB_MID_TAB)) {  // middle tier first
+                const u32 smid = std::min(smov, CB_MID_MOV), tmid = direct ? stab : std::min(stab, CB_MID_TAB);
                 const size_t dmid = (size_t)smid * 12 + (size_t)tmid * 12;
                 int per_mid = 1;
                 AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_mid, k_cascade_block, CB_THREADS, dmid));
