@@ -63,14 +63,20 @@ struct RateArgs {
 // calling warp takes u's incidences in batches of 32 starting at `first`, every `stride` entries.
 // A batch's hyperedge metadata loads in parallel, then its pins are flattened across the lanes
 // (each lane finds its pin's hyperedge by a 5-step search over the prefix of the batch's lengths).
-// With `ndist` set, the table is a first try: distinct keys are counted there, and once they pass
-// `limit` the node stops (the caller retries it with a larger table).
+// CM: the shared-inbound counts are kept; without an inbound limit no pair can fail it. RT_COUNT: the
+// table is a first try: distinct keys are counted in ndist, and once they pass `limit` the warps
+// stop at their next batch (the caller retries the node with a larger table). RT_DIRECT: slots are
+// node ids, a present one is never zero in both words (RT_SEEN marks a zero contribution).
+enum RateMode { RT_PLAIN, RT_COUNT, RT_DIRECT };
+constexpr u32 RT_SEEN = 0x80000000u;
+template <bool CM, RateMode MODE>
 __device__ void rate_flat(const RateArgs &A, u32 u, u32 *keys, u32 *sc, u32 *cm, u32 mask, u32 first,
                           u32 stride, u32 *ndist = nullptr, u32 limit = 0, u32 *used = nullptr) {
     const u32 lane = threadIdx.x & 31u;
     const u64 t0 = A.toff[u];
     const u32 deg = (u32)(A.toff[u + 1] - t0), nin_u = A.nin[u];
     for (u32 jb = first; jb < deg; jb += stride) {
+        if (MODE == RT_COUNT && __any_sync(0xFFFFFFFFu, *(volatile u32 *)ndist > limit)) return;
         const u32 j = jb + lane;
         const bool has = j < deg;
         const u32 h = has ? A.touch[t0 + j] : 0;
@@ -105,7 +111,9 @@ __device__ void rate_flat(const RateArgs &A, u32 u, u32 *keys, u32 *sc, u32 *cm,
             const u32 v = A.pins[ao + i];
             if (v == u) continue;
             u32 slot;
-            if (ndist) {  // counted keys: a first try gives up past `limit`; `used` lists them
+            if (MODE == RT_DIRECT) {
+                slot = v;
+            } else if (MODE == RT_COUNT) {  // counted keys; `used` lists them
                 if (*(volatile u32 *)ndist > limit) continue;
                 bool fresh = false;
                 slot = hash_insert_fresh(keys, mask, v, fresh);
@@ -123,15 +131,17 @@ __device__ void rate_flat(const RateArgs &A, u32 u, u32 *keys, u32 *sc, u32 *cm,
                 slot = hash_find_or_insert(keys, mask, v);
                 if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); continue; }
             }
-            atomicAdd(&sc[slot], cc);
-            if (ib && i >= ss) atomicAdd(&cm[slot], 1u);
+            if (MODE == RT_DIRECT && cc == 0) atomicOr(&cm[slot], RT_SEEN);
+            else atomicAdd(&sc[slot], cc);
+            if (CM && ib && i >= ss) atomicAdd(&cm[slot], 1u);
         }
     }
 }
 
+template <bool CM>
 __device__ __forceinline__ u64 cand_key(const RateArgs &A, u32 u, u32 v, u32 s, u32 shared_inb) {
     if ((u64)A.nsize[u] + A.nsize[v] > A.omega) return 0;
-    if ((u64)A.nin[u] + A.nin[v] - shared_inb > A.delta) return 0;
+    if (CM && (u64)A.nin[u] + A.nin[v] - shared_inb > A.delta) return 0;
     const u32 score = s + pair_noise(u, v);
     if (score == 0) return 0;
     return ((u64)score << 32) | v;
@@ -152,7 +162,8 @@ __device__ __forceinline__ void top_insert(u64 (&top)[TC], u64 k, u32 cnc) {
         }
 }
 // Slots [first, cap) step `step` of the table, or with `used` the listed slots used[first, cap).
-template <int TC>
+// Without keys the slots are node ids.
+template <int TC, bool CM>
 __device__ __forceinline__ void top_collect(const RateArgs &A, u32 u, const u32 *keys, const u32 *sc, const u32 *cm,
                                            u32 cap, u32 first, u32 step, u64 (&top)[TC],
                                            const u32 *used = nullptr) {
@@ -162,9 +173,17 @@ __device__ __forceinline__ void top_collect(const RateArgs &A, u32 u, const u32 
     u64 floor = 0;  // the list's last entry: a key must beat it to enter
     for (u32 t = first; t < cap; t += step) {
         const u32 s = used ? used[t] : t;
-        const u32 v = keys[s];
-        if (v == NONE) continue;
-        const u64 k = cand_key(A, u, v, sc[s], cm[s]);
+        u32 v = s, x = sc[s], y = 0;
+        if (keys) {
+            v = keys[s];
+            if (v == NONE) continue;
+            if (CM) y = cm[s];
+        } else {
+            y = cm[s];
+            if (!(x | y)) continue;
+            y &= ~RT_SEEN;
+        }
+        const u64 k = cand_key<CM>(A, u, v, x, y);
         if (k <= floor) continue;
         top_insert<TC>(top, k, cnc);
 #pragma unroll
@@ -180,7 +199,7 @@ __device__ __forceinline__ void top_pop(u64 (&top)[TC]) {
 }
 
 // TC: the length of the per-thread top lists, at least cnc (4 for cnc <= 4, else 16).
-template <int TC>
+template <int TC, bool CM>
 __global__ void __launch_bounds__(RT_WARPS * 32) k_rate_warp(RateArgs A, const u32 *__restrict__ list, u32 nlist) {
     __shared__ u32 tk[RT_WARPS][2 * RT_WARP_W], ts[RT_WARPS][2 * RT_WARP_W], tc[RT_WARPS][2 * RT_WARP_W];
     const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -191,12 +210,16 @@ __global__ void __launch_bounds__(RT_WARPS * 32) k_rate_warp(RateArgs A, const u
     const u64 W = A.work[u];  // work bound for the table size (at most RT_WARP_W in this tier)
     u32 cap = 64;
     while (cap < 2 * W) cap <<= 1;
-    for (u32 i = lane; i < cap; i += 32) { keys[i] = NONE; sc[i] = 0; cm[i] = 0; }
+    for (u32 i = lane; i < cap; i += 32) {
+        keys[i] = NONE;
+        sc[i] = 0;
+        if (CM) cm[i] = 0;
+    }
     __syncwarp();
-    rate_flat(A, u, keys, sc, cm, cap - 1, 0, 32);
+    rate_flat<CM, RT_PLAIN>(A, u, keys, sc, cm, cap - 1, 0, 32);
     __syncwarp();
     u64 top[TC];
-    top_collect<TC>(A, u, keys, sc, cm, cap, lane, 32, top);
+    top_collect<TC, CM>(A, u, keys, sc, cm, cap, lane, 32, top);
     for (u32 r = 0; r < A.cnc; ++r) {
         const u64 best = warp_max_u64(top[0]);
         if (lane == 0) {
@@ -213,12 +236,12 @@ constexpr u32 RT_SEL = (RT_BLOCK / 32) * AXC_MAX_CANDIDATES;  // shared slots of
 // Each warp reduces its lanes' lists to its own top cnc with shuffles into red[warp * cnc ..];
 // warp 0 merges those after one barrier. red holds RT_SEL entries.
 // With `used`, only the nused listed slots are read.
-template <int TC>
+template <int TC, bool CM>
 __device__ void rate_select(const RateArgs &A, u32 u, const u32 *keys, const u32 *sc, const u32 *cm, u32 cap,
                             u64 *red, const u32 *used = nullptr, u32 nused = 0) {
     const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5, nw = blockDim.x >> 5, cnc = A.cnc;
     u64 top[TC];
-    top_collect<TC>(A, u, keys, sc, cm, used ? nused : cap, threadIdx.x, blockDim.x, top, used);
+    top_collect<TC, CM>(A, u, keys, sc, cm, used ? nused : cap, threadIdx.x, blockDim.x, top, used);
     for (u32 r = 0; r < cnc; ++r) {
         const u64 best = warp_max_u64(top[0]);
         if (lane == 0) red[w * cnc + r] = best;
@@ -244,6 +267,7 @@ __device__ void rate_select(const RateArgs &A, u32 u, const u32 *keys, const u32
 // Heavy nodes of a level with few of them: `splits` blocks per node share the node's table in
 // global scratch (keys | sc | cm planes of nl * cap slots, cleared beforehand); block s of node
 // idx takes every splits-th group of its warps' incidence batches.
+template <bool CM>
 __global__ void __launch_bounds__(RT_BLOCK) k_rate_split_acc(RateArgs A, const u32 *__restrict__ list, u32 nl,
                                                             u32 cap, u32 splits, u32 *gtab) {
     const u32 idx = blockIdx.x / splits, s = blockIdx.x % splits;
@@ -251,9 +275,9 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rate_split_acc(RateArgs A, const u
     const u64 plane = (u64)nl * cap;
     u32 *keys = gtab + (u64)idx * cap, *sc = keys + plane, *cm = sc + plane;
     const u32 nw = blockDim.x >> 5;
-    rate_flat(A, list[idx], keys, sc, cm, cap - 1, 32 * (s * nw + (threadIdx.x >> 5)), 32 * nw * splits);
+    rate_flat<CM, RT_PLAIN>(A, list[idx], keys, sc, cm, cap - 1, 32 * (s * nw + (threadIdx.x >> 5)), 32 * nw * splits);
 }
-template <int TC>
+template <int TC, bool CM>
 __global__ void __launch_bounds__(RT_BLOCK) k_rate_split_select(RateArgs A, const u32 *__restrict__ list, u32 nl,
                                                                u32 cap, const u32 *gtab) {
     __shared__ u64 red[RT_SEL];
@@ -261,7 +285,7 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rate_split_select(RateArgs A, cons
     if (idx >= nl) return;
     const u64 plane = (u64)nl * cap;
     const u32 *keys = gtab + (u64)idx * cap, *sc = keys + plane, *cm = sc + plane;
-    rate_select<TC>(A, list[idx], keys, sc, cm, cap, red);
+    rate_select<TC, CM>(A, list[idx], keys, sc, cm, cap, red);
 }
 
 // One node per block iteration; table in dynamic smem (gtab == nullptr) or in this block's
@@ -270,9 +294,10 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rate_split_select(RateArgs A, cons
 // candidates from those and empties them again, so its cost follows its distinct neighbours,
 // not the slice size.
 // With `retry` set the launch is a first try on tables smaller than the nodes' work bounds: a node
-// whose distinct neighbours pass half of its table stops and is appended to retry / *d_retry.
+// whose distinct neighbours pass three quarters of its table stops and is appended to retry /
+// *d_retry.
 // With `d_nl` set the list length is read from device memory (at most nlist).
-template <int TC>
+template <int TC, bool CM>
 __global__ void __launch_bounds__(RT_BLOCK) k_rate_block(RateArgs A, const u32 *__restrict__ list, u32 nlist,
                                                         u32 cap_max, u32 *gtab, const u32 *__restrict__ d_nl,
                                                         u32 *__restrict__ retry, u32 *__restrict__ d_retry,
@@ -301,18 +326,24 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rate_block(RateArgs A, const u32 *
         if (!gtab) {
             sc = keys + cap;
             cm = sc + cap;
-            for (u32 i = threadIdx.x; i < cap; i += blockDim.x) { keys[i] = NONE; sc[i] = 0; cm[i] = 0; }
+            for (u32 i = threadIdx.x; i < cap; i += blockDim.x) {
+                keys[i] = NONE;
+                sc[i] = 0;
+                if (CM) cm[i] = 0;
+            }
         }
         if (threadIdx.x == 0) ndist = 0;
         __syncthreads();
-        const u32 limit = gtab ? cap : cap / 2;
-        rate_flat(A, u, keys, sc, cm, cap - 1, 32 * (threadIdx.x >> 5), blockDim.x,
-                  (retry || gtab) ? &ndist : nullptr, limit, used);
+        const u32 limit = gtab ? cap : cap / 4 * 3;
+        if (retry || gtab)
+            rate_flat<CM, RT_COUNT>(A, u, keys, sc, cm, cap - 1, 32 * (threadIdx.x >> 5), blockDim.x, &ndist, limit, used);
+        else
+            rate_flat<CM, RT_PLAIN>(A, u, keys, sc, cm, cap - 1, 32 * (threadIdx.x >> 5), blockDim.x);
         __syncthreads();
         if (retry && ndist > limit) {  // table too small: the retry launch redoes this node
             if (threadIdx.x == 0) retry[atomicAdd(d_retry, 1u)] = u;
         } else {
-            rate_select<TC>(A, u, keys, sc, cm, cap, red, used, ndist);
+            rate_select<TC, CM>(A, u, keys, sc, cm, cap, red, used, ndist);
         }
         if (gtab) {  // rate_select ends with a barrier: empty the listed slots
             for (u32 t = threadIdx.x; t < ndist; t += blockDim.x) {
@@ -323,6 +354,25 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rate_block(RateArgs A, const u32 *
             }
         }
         __syncthreads();
+    }
+}
+
+// The same with scores indexed by node id in shared memory, for levels of at most RT_DIRECT_N nodes:
+// no probing, no retries, whatever the node's distinct neighbours. sc and cm hold n words each (cm
+// only marks zero contributions without CM).
+constexpr u32 RT_DIRECT_N = 8192;
+template <int TC, bool CM>
+__global__ void __launch_bounds__(RT_BLOCK) k_rate_direct(RateArgs A, const u32 *__restrict__ list, u32 nlist) {
+    extern __shared__ u32 dyn[];
+    __shared__ u64 red[RT_SEL];
+    u32 *sc = dyn, *cm = dyn + A.n;
+    for (u32 idx = blockIdx.x; idx < nlist; idx += gridDim.x) {
+        const u32 u = list[idx];
+        for (u32 i = threadIdx.x; i < 2 * A.n; i += RT_BLOCK) dyn[i] = 0;
+        __syncthreads();
+        rate_flat<CM, RT_DIRECT>(A, u, nullptr, sc, cm, 0, 32 * (threadIdx.x >> 5), RT_BLOCK);
+        __syncthreads();
+        rate_select<TC, CM>(A, u, nullptr, sc, cm, A.n, red);  // ends with a barrier
     }
 }
 
@@ -533,17 +583,29 @@ __global__ void k_sum_max(const u64 *__restrict__ v, u32 n, unsigned long long *
 }
 
 void setup_coarsen_kernels(Ctx &c) {
-    AXC_CUDA(cudaFuncSetAttribute(k_rate_block<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 16384 * 4));
-    AXC_CUDA(cudaFuncSetAttribute(k_rate_block<(int)AXC_MAX_CANDIDATES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  3 * 16384 * 4));
+    const auto smem = [](auto kernel, size_t bytes) {
+        AXC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    };
+    constexpr int TC = (int)AXC_MAX_CANDIDATES;
+    smem(k_rate_block<4, false>, 3 * 16384 * 4);
+    smem(k_rate_block<4, true>, 3 * 16384 * 4);
+    smem(k_rate_block<TC, false>, 3 * 16384 * 4);
+    smem(k_rate_block<TC, true>, 3 * 16384 * 4);
+    smem(k_rate_direct<4, false>, 2 * RT_DIRECT_N * 4);
+    smem(k_rate_direct<4, true>, 2 * RT_DIRECT_N * 4);
+    smem(k_rate_direct<TC, false>, 2 * RT_DIRECT_N * 4);
+    smem(k_rate_direct<TC, true>, 2 * RT_DIRECT_N * 4);
 }
 
 // A rating kernel with per-thread top lists of 4 when cnc <= 4 (the reference scripts' -cnc 4),
 // else of AXC_MAX_CANDIDATES: shorter lists hold fewer registers, so more blocks fit an SM.
-#define RATE_LAUNCH(c, kname, cnc, grid, block, smem, ...)                                                   \
+// CM (cm): the inbound counts matter.
+#define RATE_LAUNCH(c, kname, cnc, cm, grid, block, smem, ...)                                               \
     do {                                                                                                     \
-        if ((cnc) <= 4) LAUNCH_AS(c, #kname, kname<4>, grid, block, smem, __VA_ARGS__);                      \
-        else LAUNCH_AS(c, #kname, kname<(int)AXC_MAX_CANDIDATES>, grid, block, smem, __VA_ARGS__);           \
+        if ((cnc) <= 4 && (cm)) LAUNCH_AS(c, #kname, (kname<4, true>), grid, block, smem, __VA_ARGS__);      \
+        else if ((cnc) <= 4) LAUNCH_AS(c, #kname, (kname<4, false>), grid, block, smem, __VA_ARGS__);        \
+        else if (cm) LAUNCH_AS(c, #kname, (kname<(int)AXC_MAX_CANDIDATES, true>), grid, block, smem, __VA_ARGS__); \
+        else LAUNCH_AS(c, #kname, (kname<(int)AXC_MAX_CANDIDATES, false>), grid, block, smem, __VA_ARGS__);  \
     } while (0)
 
 void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 cnc, u32 *pairs, u32 *scores,
@@ -586,9 +648,13 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
         for (int t = 0; t < 2; ++t)  // the heavy tier counts below, if it runs on k_rate_block
             if (h[1 + t]) c.prof_bytes += 4 * tier_visits[t] + 8ull * cnc * h[1 + t];
     }
+    // without an inbound limit (delta 2^31 - 1) the shared counts decide nothing while the level has
+    // fewer than 2^30 hyperedges
+    const bool cm = delta < 0x7FFFFFFFu || (u64)L.e >= (1ull << 30);
+    const u32 words = cm ? 3 : 2;  // of a hashed slot
     // tier: one warp per node, table in static smem
     u32 nl = (u32)h[0];
-    RATE_LAUNCH(c, k_rate_warp, cnc, cdiv(nl, RT_WARPS), RT_WARPS * 32, 0, A, list, nl);
+    RATE_LAUNCH(c, k_rate_warp, cnc, cm, cdiv(nl, RT_WARPS), RT_WARPS * 32, 0, A, list, nl);
     // tier: one block per node, 4096-slot table in dynamic smem
     nl = (u32)h[1];
     // shared tables sized by the largest node table the tier can need (distinct neighbours never
@@ -608,25 +674,32 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
     u32 *retry = c.arena.alloc<u32>(n), *retry2 = c.arena.alloc<u32>(n);
     u32 *d_retry = (u32 *)(dc + 4), *d_retry2 = d_retry + 1;  // dc[4] was read already
     const u32 rt_try = c.tune.rate_try, rt_mid = std::max(c.tune.rate_mid, c.tune.rate_try);
+    const auto direct_tier = [&](const u32 *lst, u32 cnt) {
+        RATE_LAUNCH(c, k_rate_direct, cnc, cm, std::min<u32>(cnt, (u32)c.sms * 8), RT_BLOCK, (size_t)2 * n * 4, A, lst, cnt);
+    };
     auto block_tier = [&](const u32 *lst, u32 cnt, u32 cap_full) {
         if (!cnt) return;
+        if (n <= RT_DIRECT_N && cap_full > rt_try) {
+            direct_tier(lst, cnt);
+            return;
+        }
         if (cap_full <= rt_try) {
-            RATE_LAUNCH(c, k_rate_block, cnc, cnt, RT_BLOCK, 3 * cap_full * 4, A, lst, cnt, cap_full, (u32 *)nullptr,
+            RATE_LAUNCH(c, k_rate_block, cnc, cm, cnt, RT_BLOCK, words * cap_full * 4, A, lst, cnt, cap_full, (u32 *)nullptr,
                    (const u32 *)nullptr, (u32 *)nullptr, (u32 *)nullptr, (u32 *)nullptr);
             return;
         }
         AXC_CUDA(cudaMemsetAsync(d_retry, 0, 8, c.stream));  // d_retry and d_retry2
-        RATE_LAUNCH(c, k_rate_block, cnc, cnt, RT_BLOCK, 3 * rt_try * 4, A, lst, cnt, rt_try, (u32 *)nullptr,
+        RATE_LAUNCH(c, k_rate_block, cnc, cm, cnt, RT_BLOCK, words * rt_try * 4, A, lst, cnt, rt_try, (u32 *)nullptr,
                (const u32 *)nullptr, retry, d_retry, (u32 *)nullptr);
         const u32 *rl = retry, *dn = d_retry;
         if (cap_full > rt_mid) {
-            RATE_LAUNCH(c, k_rate_block, cnc, std::min<u32>(cnt, (u32)c.sms * 2), RT_BLOCK, 3 * rt_mid * 4, A, rl, cnt, rt_mid,
+            RATE_LAUNCH(c, k_rate_block, cnc, cm, std::min<u32>(cnt, (u32)c.sms * 2), RT_BLOCK, words * rt_mid * 4, A, rl, cnt, rt_mid,
                    (u32 *)nullptr, dn, retry2, d_retry2, (u32 *)nullptr);
             rl = retry2;
             dn = d_retry2;
         }
         const u32 grid = std::min<u32>(cnt, (u32)c.sms * 2);
-        RATE_LAUNCH(c, k_rate_block, cnc, grid, RT_BLOCK, 3 * cap_full * 4, A, rl, cnt, cap_full, (u32 *)nullptr, dn,
+        RATE_LAUNCH(c, k_rate_block, cnc, cm, grid, RT_BLOCK, words * cap_full * 4, A, rl, cnt, cap_full, (u32 *)nullptr, dn,
                (u32 *)nullptr, (u32 *)nullptr, (u32 *)nullptr);
     };
     block_tier(list2, nl, cap1);
@@ -647,13 +720,16 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
             u32 *gtab = c.arena.alloc<u32>((u64)nl * 3 * cap);
             AXC_CUDA(cudaMemsetAsync(gtab, 0xFF, (size_t)nl * cap * 4, c.stream));
             AXC_CUDA(cudaMemsetAsync(gtab + (u64)nl * cap, 0, (size_t)nl * cap * 8, c.stream));
-            LAUNCH(c, k_rate_split_acc, nl * splits, RT_BLOCK, 0, A, list4, nl, cap, splits, gtab);
-            RATE_LAUNCH(c, k_rate_split_select, cnc, nl, RT_BLOCK, 0, A, list4, nl, cap, gtab);
+            if (cm) LAUNCH_AS(c, "k_rate_split_acc", k_rate_split_acc<true>, nl * splits, RT_BLOCK, 0, A, list4, nl, cap, splits, gtab);
+            else LAUNCH_AS(c, "k_rate_split_acc", k_rate_split_acc<false>, nl * splits, RT_BLOCK, 0, A, list4, nl, cap, splits, gtab);
+            RATE_LAUNCH(c, k_rate_split_select, cnc, cm, nl, RT_BLOCK, 0, A, list4, nl, cap, gtab);
+        } else if (n <= RT_DIRECT_N) {
+            direct_tier(list4, nl);
         } else {
             u32 grid = nl < (u32)c.sms * 2 ? nl : (u32)c.sms * 2;
             u32 *gtab = c.arena.alloc<u32>((u64)grid * 3 * cap), *gused = c.arena.alloc<u32>((u64)grid * cap);
             if (c.profiling("k_rate_block")) c.prof_bytes += 4 * tier_visits[2] + 8ull * cnc * nl;
-            RATE_LAUNCH(c, k_rate_block, cnc, grid, RT_BLOCK, 0, A, list4, nl, cap, gtab, (const u32 *)nullptr, (u32 *)nullptr,
+            RATE_LAUNCH(c, k_rate_block, cnc, cm, grid, RT_BLOCK, 0, A, list4, nl, cap, gtab, (const u32 *)nullptr, (u32 *)nullptr,
                    (u32 *)nullptr, gused);
         }
     }
