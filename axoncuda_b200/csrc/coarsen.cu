@@ -12,6 +12,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "blocksort.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -42,10 +43,26 @@ __global__ void k_rate_work(u32 n, const u64 *__restrict__ toff, const u32 *__re
     if (lane == 0) work[u] = s;
 }
 
-__global__ void k_rate_tier(u32 n, const u64 *__restrict__ work, u64 lo, u64 hi, u32 *__restrict__ flag) {
-    u32 u = blockIdx.x * blockDim.x + threadIdx.x;
-    // the first tier (lo == 0) also takes nodes without incident hyperedges
-    if (u < n) flag[u] = ((lo == 0 || work[u] > lo) && work[u] <= hi) ? 1u : 0u;
+// The four tiers' node lists by work bound (limits hi[0..3), the rest in the last), the sum of the
+// bounds (dc[4]) and their maximum (dc[5]) in one pass.
+__global__ void __launch_bounds__(1024) k_rate_tiers(u32 n, const u64 *__restrict__ work, u64 hi0, u64 hi1, u64 hi2,
+                                                     u32 *l0, u32 *l1, u32 *l2, u32 *l3, u64 *__restrict__ dc) {
+    __shared__ u32 sh[33];
+    const u32 u = blockIdx.x * blockDim.x + threadIdx.x;
+    const u64 x = u < n ? work[u] : 0;
+    const u32 t = u >= n ? 4u : x <= hi0 ? 0u : x <= hi1 ? 1u : x <= hi2 ? 2u : 3u;
+    u32 *lists[4] = {l0, l1, l2, l3};
+#pragma unroll
+    for (u32 i = 0; i < 4; ++i) {
+        if (!__syncthreads_or(t == i)) continue;
+        const u32 at = block_append(t == i, (u32 *)(dc + i), sh);
+        if (t == i) lists[i][at] = u;
+    }
+    const u64 s = warp_sum(x), m = warp_max_u64(x);
+    if ((threadIdx.x & 31) == 0) {
+        if (s) atomicAdd((unsigned long long *)&dc[4], (unsigned long long)s);
+        if (m) atomicMax((unsigned long long *)&dc[5], (unsigned long long)m);
+    }
 }
 
 struct RateArgs {
@@ -520,6 +537,109 @@ __global__ void k_group_assign(u32 n, const u32 *__restrict__ mate, const u32 *_
     groups[v] = gid[(m == NONE || v < m) ? v : m];
 }
 
+// Everything after the matching rounds on levels of at most RSS_CAP nodes, in one block: the two-hop
+// pass, the orphans (paired from both ends of their order by (size, id)) and the group numbers in
+// order of the smallest member, as the launches for larger levels do. out: the group count.
+__global__ void __launch_bounds__(RSS_WARPS * 32) k_match_tail_small(u32 n, u32 cnc, const u32 *__restrict__ pairs,
+                                                                     const u32 *__restrict__ nsize,
+                                                                     const u32 *__restrict__ nin, u32 omega, u32 delta,
+                                                                     u32 idbits, u32 *__restrict__ mate,
+                                                                     u32 *__restrict__ groups, u32 *__restrict__ out) {
+    extern __shared__ u32 sm[];
+    __shared__ u32 ws[33], s_max;
+    const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5, T = blockDim.x;
+    // exclusive prefix of v over the block, and the total
+    const auto scan = [&](u32 v, u32 &tot) {
+        u32 x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if ((int)lane >= o) x += y;
+        }
+        __syncthreads();
+        if (lane == 31) ws[w] = x;
+        __syncthreads();
+        u32 before = 0;
+        tot = 0;
+        for (u32 i = 0; i < RSS_WARPS; ++i) {
+            if (i < w) before += ws[i];
+            tot += ws[i];
+        }
+        return before + x - v;
+    };
+    // the nodes with f, ascending, into the sort buffer with their keys; returns their number
+    const auto gather = [&](auto &&f, auto &&key) {
+        u32 m = 0;
+        for (u32 b = 0; b < n; b += T) {
+            const u32 v = b + threadIdx.x;
+            const bool in = v < n && f(v);
+            u32 tot;
+            const u32 at = m + scan(in ? 1u : 0u, tot);
+            if (in) {
+                sm[at] = key(v);
+                sm[RSS_CAP + at] = v;
+            }
+            m += tot;
+        }
+        return m;
+    };
+    const auto fits = [&](u32 x, u32 y) {
+        return (u64)nsize[x] + nsize[y] <= omega && (u64)nin[x] + nin[y] <= delta;
+    };
+    const u32 *ko, *vo;
+    // two-hop: unmatched nodes by (best candidate, id), paired at even and odd places of each bucket
+    u32 m = gather([&](u32 v) { return mate[v] == NONE && pairs[(u64)v * cnc] != NONE; },
+                   [&](u32 v) { return pairs[(u64)v * cnc]; });
+    block_radix_sort(sm, m, idbits, ko, vo);
+    for (u32 i = threadIdx.x; i + 1 < m; i += T) {
+        const u32 k = ko[i];
+        if (ko[i + 1] != k) continue;
+        u32 lo = 0, hi = i;  // the bucket's first place
+        while (lo < hi) {
+            const u32 mid = (lo + hi) >> 1;
+            if (ko[mid] < k) lo = mid + 1; else hi = mid;
+        }
+        const u32 x = vo[i], y = vo[i + 1];
+        if (((i - lo) & 1u) || !fits(x, y)) continue;
+        mate[x] = y;
+        mate[y] = x;
+    }
+    __syncthreads();
+    // orphans: no candidate at all
+    if (threadIdx.x == 0) s_max = 0;
+    m = gather([&](u32 v) { return pairs[(u64)v * cnc] == NONE; }, [&](u32 v) { return nsize[v]; });
+    u32 mx = 0;
+    __syncthreads();
+    for (u32 i = threadIdx.x; i < m; i += T) mx = sm[i] > mx ? sm[i] : mx;
+    mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+    if (lane == 0 && mx) atomicMax(&s_max, mx);
+    __syncthreads();
+    block_radix_sort(sm, m, 32 - __clz(s_max), ko, vo);
+    for (u32 k = threadIdx.x; k < m / 2; k += T) {
+        const u32 x = vo[k], y = vo[m - 1 - k];
+        if (!fits(x, y)) continue;
+        mate[x] = y;
+        mate[y] = x;
+    }
+    __syncthreads();
+    // group numbers: sm[v] for the heads
+    u32 ng = 0;
+    for (u32 b = 0; b < n; b += T) {
+        const u32 v = b + threadIdx.x;
+        const bool head = v < n && (mate[v] == NONE || v < mate[v]);
+        u32 tot;
+        const u32 at = ng + scan(head ? 1u : 0u, tot);
+        if (head) sm[v] = at;
+        ng += tot;
+    }
+    __syncthreads();
+    for (u32 v = threadIdx.x; v < n; v += T) {
+        const u32 x = mate[v];
+        groups[v] = sm[x == NONE || v < x ? v : x];
+    }
+    if (threadIdx.x == 0) *out = ng;
+}
+
 // ---------------------------------------------------------------- greedy merge (-ipm)
 __global__ void k_group_sums(u32 n, const u32 *__restrict__ groups, const u32 *__restrict__ nsize,
                              const u32 *__restrict__ nin, u32 *__restrict__ gs, unsigned long long *__restrict__ gi) {
@@ -571,22 +691,12 @@ __global__ void k_list_sum(const u32 *__restrict__ list, u32 nl, const u64 *__re
     if ((threadIdx.x & 31) == 0 && s) atomicAdd(out, (unsigned long long)s);
 }
 
-// out[0] += sum of v[0, n), out[1] = max(out[1], max of v[0, n))
-__global__ void k_sum_max(const u64 *__restrict__ v, u32 n, unsigned long long *__restrict__ out) {
-    u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    u64 x = i < n ? v[i] : 0;
-    const u64 s = warp_sum(x), m = warp_max_u64(x);
-    if ((threadIdx.x & 31) == 0) {
-        if (s) atomicAdd(&out[0], (unsigned long long)s);
-        if (m) atomicMax(&out[1], (unsigned long long)m);
-    }
-}
-
 void setup_coarsen_kernels(Ctx &c) {
     const auto smem = [](auto kernel, size_t bytes) {
         AXC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     };
     constexpr int TC = (int)AXC_MAX_CANDIDATES;
+    smem(k_match_tail_small, RSS_SMEM);
     smem(k_rate_block<4, false>, 3 * 16384 * 4);
     smem(k_rate_block<4, true>, 3 * 16384 * 4);
     smem(k_rate_block<TC, false>, 3 * 16384 * 4);
@@ -609,14 +719,13 @@ void setup_coarsen_kernels(Ctx &c) {
     } while (0)
 
 void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 cnc, u32 *pairs, u32 *scores,
-            u64 *pin_visits) {
+            u64 *pin_visits, bool check) {
     const u32 n = L.n;
     if (n == 0) return;
     size_t m = c.arena.mark();
     u64 *work = c.arena.alloc<u64>(n);
     RateArgs A{n, cnc, omega, delta, L.off, L.pins, L.nsrc, wfx, L.toff, L.touch, L.nin, L.nsize, pairs, scores,
                c.d_status, work};
-    u32 *flag = c.arena.alloc<u32>(n);
     u32 *lists[4];
     for (auto &l : lists) l = c.arena.alloc<u32>(n);
     // device counters, read back in one round trip: [0..3] tier sizes, [4] work sum, [5] work max
@@ -624,12 +733,8 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
     AXC_CUDA(cudaMemsetAsync(dc, 0, 48, c.stream));
     fill_u32(c, pairs, NONE, (u64)n * cnc);
     LAUNCH(c, k_rate_work, cdiv((u64)n * 32, 256), 256, 0, n, L.toff, L.touch, L.off, work);
-    LAUNCH(c, k_sum_max, cdiv(n, 256), 256, 0, work, n, (unsigned long long *)(dc + 4));
-    const u64 lim[5] = {0, RT_WARP_W, RT_BLK1_W, RT_BLK2_W, ~0ull};
-    for (int t = 0; t < 4; ++t) {
-        LAUNCH(c, k_rate_tier, cdiv(n, 256), 256, 0, n, work, lim[t], lim[t + 1], flag);
-        compact_indices_dn(c, flag, lists[t], n, (u32 *)(dc + t));
-    }
+    LAUNCH(c, k_rate_tiers, cdiv(n, 1024), 1024, 0, n, work, (u64)RT_WARP_W, (u64)RT_BLK1_W, (u64)RT_BLK2_W, lists[0],
+           lists[1], lists[2], lists[3], dc);
     u64 h[6];
     fetch(c, h, dc, 48);
     if (pin_visits) *pin_visits = h[4];
@@ -733,7 +838,7 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
                    (u32 *)nullptr, gused);
         }
     }
-    check_status(c);
+    if (check) check_status(c);
     c.arena.release(m);
 }
 
@@ -766,6 +871,17 @@ u32 matching(Ctx &c, u32 n, u32 cnc, const u32 *pairs, const u32 *scores, const 
         u32 grid = cdiv(n, 256);
         for (u32 r = 0; r < rounds; ++r)
             for (int ph = 0; ph < 3; ++ph) LAUNCH(c, k_match_phase, grid, 256, 0, A, r, ph);
+    }
+    if (n <= (u32)RSS_CAP) {
+        u32 *out = c.arena.alloc<u32>(2);  // the group count and the status word
+        LAUNCH(c, k_match_tail_small, 1, RSS_WARPS * 32, RSS_SMEM, n, cnc, pairs, nsize, nin, omega, delta, bits_for(n - 1),
+               mate, groups, out);
+        AXC_CUDA(cudaMemcpyAsync(out + 1, c.d_status, 4, cudaMemcpyDeviceToDevice, c.stream));
+        u64 res;
+        fetch(c, &res, out, 8);
+        if (res >> 32) check_status(c);
+        c.arena.release(m);
+        return (u32)res;
     }
     // two-hop pass
     {
@@ -800,12 +916,14 @@ u32 matching(Ctx &c, u32 n, u32 cnc, const u32 *pairs, const u32 *scores, const 
     scan_excl_u32(c, head, gid, n);
     u64 tail[2];
     {
-        u32 *d = c.arena.alloc<u32>(2);
+        u32 *d = c.arena.alloc<u32>(4);
         AXC_CUDA(cudaMemcpyAsync(d, gid + n - 1, 4, cudaMemcpyDeviceToDevice, c.stream));
         AXC_CUDA(cudaMemcpyAsync(d + 1, head + n - 1, 4, cudaMemcpyDeviceToDevice, c.stream));
-        fetch(c, tail, d, 8);
+        AXC_CUDA(cudaMemcpyAsync(d + 2, c.d_status, 4, cudaMemcpyDeviceToDevice, c.stream));
+        fetch(c, tail, d, 12);
     }
     const u32 *t32 = (const u32 *)tail;
+    if (t32[2] != DEV_OK) check_status(c);
     u32 ng = t32[0] + t32[1];
     LAUNCH(c, k_group_assign, cdiv(n, 256), 256, 0, n, mate, gid, groups);
     c.arena.release(m);

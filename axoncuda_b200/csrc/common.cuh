@@ -225,6 +225,28 @@ __device__ __forceinline__ u64 warp_max_u64(u64 v) {
     return v;
 }
 
+// The place of the calling thread, when f, in a list counted by *count: one add per block (every
+// thread of the block calls it; sh holds 33 words). The order among blocks is arbitrary, for lists
+// whose order decides nothing but the schedule.
+__device__ __forceinline__ u32 block_append(bool f, u32 *count, u32 *sh) {
+    const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    const u32 bal = __ballot_sync(0xFFFFFFFFu, f);
+    __syncthreads();  // sh is no longer read by an earlier call
+    if (lane == 0) sh[w] = __popc(bal);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        u32 tot = 0;
+        for (u32 i = 0; i < nw; ++i) {
+            const u32 c = sh[i];
+            sh[i] = tot;
+            tot += c;
+        }
+        sh[32] = tot ? atomicAdd(count, tot) : 0;
+    }
+    __syncthreads();
+    return sh[32] + sh[w] + __popc(bal & ((1u << lane) - 1u));
+}
+
 // Symmetric noise in [0, 63] of an unordered id pair: the same integer mixing sequence as the
 // reference's deterministic_noise (headers/utils.cuh:159-171), so ratings agree with it.
 __host__ __device__ __forceinline__ u32 pair_noise(u32 a, u32 b) {

@@ -9,6 +9,8 @@
 // Contraction (kernels/construction.cu:304-489): cls = 1 for sources, 0 for destinations, so a
 // group that is both keeps its destination occurrence. Survivors are compacted in position order,
 // so the output keeps sources first and is deterministic.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -24,7 +26,8 @@ __global__ void k_wfx(const float *__restrict__ w, u32 *__restrict__ wfx, u32 e)
 }
 
 constexpr u32 UQ_WARP_CAP = 256;      // hyperedges up to this size: one warp, table in smem
-constexpr u32 UQ_BLOCK_CAP = 8192;    // up to this size: one block, table in dynamic smem
+constexpr u32 UQ_MID_CAP = 2048;      // up to this size: one block, 32 KB of table (several per SM)
+constexpr u32 UQ_BLOCK_CAP = 8192;    // up to this size: one block, 128 KB of table
 constexpr u32 UQ_WARPS = 8;
 
 __device__ __forceinline__ u32 uq_key(const u32 *pins, const u32 *groups, u64 k) {
@@ -83,42 +86,40 @@ __global__ void k_uniq_warp(u32 e, const u64 *__restrict__ off, const u32 *__res
     if (lane == 0) { cnt[h] = kept; cnt_src[h] = ks; }
 }
 
-__global__ void k_uniq_block(const u32 *__restrict__ list, u32 nlist, const u64 *__restrict__ off,
+// One block per listed hyperedge (the count in device memory when d_n is set).
+__global__ void k_uniq_block(const u32 *__restrict__ list, u32 nlist, const u32 *__restrict__ d_n,
+                             const u64 *__restrict__ off,
                              const u32 *__restrict__ pins, const u32 *__restrict__ nsrc,
                              const u32 *__restrict__ groups, int dst_wins, uint8_t *__restrict__ keep,
                              u32 *__restrict__ cnt, u32 *__restrict__ cnt_src, u32 *gtab,
                              const u64 *__restrict__ gtab_off, u32 *status) {
     extern __shared__ u32 dyn[];
     __shared__ u32 red[2][32];
-    if (blockIdx.x >= nlist) return;
-    const u32 h = list[blockIdx.x];
-    const u64 a = off[h], b = off[h + 1], s = a + nsrc[h];
-    const u32 len = (u32)(b - a);
-    u32 cap = 64;
-    while (cap < 2 * len) cap <<= 1;
-    u32 *keys, *vals;
-    if (gtab) {
-        keys = gtab + 2 * gtab_off[blockIdx.x];
-        vals = keys + cap;
-    } else {
-        keys = dyn;
-        vals = dyn + cap;
-    }
-    for (u32 i = threadIdx.x; i < cap; i += blockDim.x) { keys[i] = NONE; vals[i] = NONE; }
-    __syncthreads();
-    uq_insert(pins, groups, a, b, s, dst_wins, keys, vals, cap - 1, threadIdx.x, blockDim.x, status);
-    __syncthreads();
-    u32 kept = 0, ks = 0;
-    uq_mark(pins, groups, a, b, s, dst_wins, keys, vals, cap - 1, threadIdx.x, blockDim.x, keep, kept, ks);
-    kept = warp_sum(kept);
-    ks = warp_sum(ks);
-    if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = kept; red[1][threadIdx.x >> 5] = ks; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        u32 t0 = 0, t1 = 0;
-        for (u32 i = 0; i < blockDim.x / 32; ++i) { t0 += red[0][i]; t1 += red[1][i]; }
-        cnt[h] = t0;
-        cnt_src[h] = t1;
+    if (d_n) nlist = *d_n;
+    for (u32 idx = blockIdx.x; idx < nlist; idx += gridDim.x) {
+        const u32 h = list[idx];
+        const u64 a = off[h], b = off[h + 1], s = a + nsrc[h];
+        const u32 len = (u32)(b - a);
+        u32 cap = 64;
+        while (cap < 2 * len) cap <<= 1;
+        u32 *keys = gtab ? gtab + 2 * gtab_off[idx] : dyn, *vals = keys + cap;
+        for (u32 i = threadIdx.x; i < cap; i += blockDim.x) { keys[i] = NONE; vals[i] = NONE; }
+        __syncthreads();
+        uq_insert(pins, groups, a, b, s, dst_wins, keys, vals, cap - 1, threadIdx.x, blockDim.x, status);
+        __syncthreads();
+        u32 kept = 0, ks = 0;
+        uq_mark(pins, groups, a, b, s, dst_wins, keys, vals, cap - 1, threadIdx.x, blockDim.x, keep, kept, ks);
+        kept = warp_sum(kept);
+        ks = warp_sum(ks);
+        if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = kept; red[1][threadIdx.x >> 5] = ks; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            u32 t0 = 0, t1 = 0;
+            for (u32 i = 0; i < blockDim.x / 32; ++i) { t0 += red[0][i]; t1 += red[1][i]; }
+            cnt[h] = t0;
+            cnt_src[h] = t1;
+        }
+        __syncthreads();  // the table and red are no longer read
     }
 }
 
@@ -139,11 +140,21 @@ __global__ void k_uniq_compact(u32 e, const u64 *__restrict__ off, const u32 *__
     }
 }
 
-__global__ void k_flag_big(u32 e, const u64 *__restrict__ off, u32 lo, u32 hi, u32 *__restrict__ flag) {
-    u32 h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= e) return;
-    u64 len = off[h + 1] - off[h];
-    flag[h] = (len > lo && len <= hi) ? 1u : 0u;
+// The hyperedges beyond a warp's table by length: up to UQ_MID_CAP, up to UQ_BLOCK_CAP, longer.
+__global__ void __launch_bounds__(1024) k_uniq_lists(u32 e, const u64 *__restrict__ off, u32 *mid, u32 *big, u32 *huge,
+                                                     u32 *__restrict__ n) {
+    __shared__ u32 sh[33];
+    const u32 h = blockIdx.x * blockDim.x + threadIdx.x;
+    const u64 len = h < e ? off[h + 1] - off[h] : 0;
+    const u32 t = len <= UQ_WARP_CAP ? 3u : len <= UQ_MID_CAP ? 0u : len <= UQ_BLOCK_CAP ? 1u : 2u;
+    if (!__syncthreads_or(t < 3)) return;
+    u32 *lists[3] = {mid, big, huge};
+#pragma unroll
+    for (u32 i = 0; i < 3; ++i) {
+        if (!__syncthreads_or(t == i)) continue;
+        const u32 at = block_append(t == i, n + i, sh);
+        if (t == i) lists[i][at] = h;
+    }
 }
 __global__ void k_table_sizes(const u32 *__restrict__ list, u32 nlist, const u64 *__restrict__ off,
                               u64 *__restrict__ sz) {
@@ -227,30 +238,39 @@ u64 hedge_unique(Ctx &c, u32 e, const u64 *off, const u32 *pins, const u32 *nsrc
     u32 *cnt = c.arena.alloc<u32>(e);
     LAUNCH(c, k_uniq_warp, cdiv(e, UQ_WARPS), UQ_WARPS * 32, 0, e, off, pins, nsrc, groups,
            (int)dst_wins, keep, cnt, new_nsrc, c.d_status);
-    // hyperedges larger than a warp's table
-    u32 *flag = c.arena.alloc<u32>(e), *list = c.arena.alloc<u32>(e);
-    LAUNCH(c, k_flag_big, cdiv(e, 256), 256, 0, e, off, UQ_WARP_CAP, UQ_BLOCK_CAP, flag);
-    u32 nb = compact_indices(c, flag, list, e);
-    if (nb) {
-        size_t smem = 2 * 16384 * sizeof(u32);
-        LAUNCH(c, k_uniq_block, nb, 512, smem, list, nb, off, pins, nsrc, groups, (int)dst_wins, keep,
-               cnt, new_nsrc, (u32 *)nullptr, (const u64 *)nullptr, c.d_status);
-    }
-    LAUNCH(c, k_flag_big, cdiv(e, 256), 256, 0, e, off, UQ_BLOCK_CAP, 0xFFFFFFFFu, flag);
-    u32 nh = compact_indices(c, flag, list, e);
+    // hyperedges larger than a warp's table: their lists and counts stay on the device, except for
+    // those that need tables in device memory, which are rare and sized by the host
+    u32 *mid = c.arena.alloc<u32>(e), *big = c.arena.alloc<u32>(e), *huge = c.arena.alloc<u32>(e);
+    u64 *res = c.arena.alloc<u64>(4);  // list counts (three words), then the total and the status
+    u32 *ln = (u32 *)res;
+    AXC_CUDA(cudaMemsetAsync(res, 0, 32, c.stream));
+    LAUNCH(c, k_uniq_lists, cdiv(e, 1024), 1024, 0, e, off, mid, big, huge, ln);
+    if (pins_in > UQ_WARP_CAP)
+        LAUNCH(c, k_uniq_block, std::min<u32>(cdiv(pins_in, UQ_WARP_CAP), (u32)c.sms * 6), 256, 2 * 2 * UQ_MID_CAP * 4, mid, 0u,
+               ln, off, pins, nsrc, groups, (int)dst_wins, keep, cnt, new_nsrc, (u32 *)nullptr, (const u64 *)nullptr,
+               c.d_status);
+    if (pins_in > UQ_MID_CAP)
+        LAUNCH(c, k_uniq_block, std::min<u32>(cdiv(pins_in, UQ_MID_CAP), (u32)c.sms), 512, 2 * 2 * UQ_BLOCK_CAP * 4, big, 0u,
+               ln + 1, off, pins, nsrc, groups, (int)dst_wins, keep, cnt, new_nsrc, (u32 *)nullptr, (const u64 *)nullptr,
+               c.d_status);
+    const u32 nh = pins_in > UQ_BLOCK_CAP ? fetch1(c, ln + 2) : 0;
     if (nh) {
         u64 *tsz = c.arena.alloc<u64>(nh + 1);
-        LAUNCH(c, k_table_sizes, cdiv(nh + 1, 256), 256, 0, list, nh, off, tsz);
+        LAUNCH(c, k_table_sizes, cdiv(nh + 1, 256), 256, 0, huge, nh, off, tsz);
         scan_excl_u64(c, tsz, tsz, nh + 1);
         u64 tot = fetch1(c, tsz + nh);  // sum of table capacities
         u32 *gtab = c.arena.alloc<u32>(2 * tot);
-        LAUNCH(c, k_uniq_block, nh, 512, 0, list, nh, off, pins, nsrc, groups, (int)dst_wins, keep, cnt,
+        LAUNCH(c, k_uniq_block, nh, 512, 0, huge, nh, (const u32 *)nullptr, off, pins, nsrc, groups, (int)dst_wins, keep, cnt,
                new_nsrc, gtab, (const u64 *)tsz, c.d_status);
     }
     offsets_from_counts(c, cnt, new_off, e);
     LAUNCH(c, k_uniq_compact, cdiv((u64)e * 32, 256), 256, 0, e, off, pins, groups, keep, new_off, new_pins);
-    u64 total = fetch1(c, new_off + e);
-    check_status(c);
+    AXC_CUDA(cudaMemcpyAsync(res + 2, new_off + e, 8, cudaMemcpyDeviceToDevice, c.stream));
+    AXC_CUDA(cudaMemcpyAsync(res + 3, c.d_status, 4, cudaMemcpyDeviceToDevice, c.stream));
+    u64 fin[2];
+    fetch(c, fin, res + 2, 16);
+    const u64 total = fin[0];
+    if ((u32)fin[1] != DEV_OK) check_status(c);
     c.arena.release(m);
     return total;
 }
@@ -280,7 +300,7 @@ void group_sizes(Ctx &c, u32 n, const u32 *groups, const u32 *nsize, u32 *gsize,
 }
 
 void setup_construct_kernels() {
-    cudaFuncSetAttribute(k_uniq_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 16384 * 4);
+    cudaFuncSetAttribute(k_uniq_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 2 * UQ_BLOCK_CAP * 4);
 }
 
 }  // namespace axc

@@ -153,7 +153,8 @@ static u32 partition_core(Ctx &c, u32 n, u32 e, const u64 *d_off, const u32 *d_p
         const size_t tmp = c.arena.mark();
         u32 *pairs = c.arena.alloc<u32>((u64)cur.n * R.cnc), *scores = c.arena.alloc<u32>((u64)cur.n * R.cnc);
         u64 visits = 0;
-        rating(c, cur, wfx, R.kway ? R.omega_c : R.omega, R.delta, R.cnc, pairs, scores, st ? &visits : nullptr);
+        rating(c, cur, wfx, R.kway ? R.omega_c : R.omega, R.delta, R.cnc, pairs, scores, st ? &visits : nullptr,
+               false);
         if (st) st->rating_pin_visits += visits;
         log("level %u rated", l);
         u32 ng = matching(c, cur.n, R.cnc, pairs, scores, cur.nsize, cur.nin, R.kway ? R.omega_c : R.omega, R.delta, 32,

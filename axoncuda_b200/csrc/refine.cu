@@ -587,12 +587,19 @@ __global__ void k_round_tick(u32 *ctr) {
     if (threadIdx.x == 0 && blockIdx.x == 0) ctr[0] += 1;
 }
 
-__global__ void k_flag_len(u32 e, const u64 *__restrict__ off, u64 lo, u64 hi, u32 *__restrict__ flag) {
-    u32 h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h < e) {
-        u64 l = off[h + 1] - off[h];
-        flag[h] = (l > lo && l <= hi) ? 1u : 0u;
-    }
+// The hashed census's block (n[0]) and device-table (n[1]) hyperedges.
+__global__ void __launch_bounds__(1024) k_census_lists(u32 e, const u64 *__restrict__ off, u32 *mid, u32 *huge,
+                                                       u32 *__restrict__ n) {
+    __shared__ u32 sh[33];
+    const u32 h = blockIdx.x * blockDim.x + threadIdx.x;
+    const u64 len = h < e ? off[h + 1] - off[h] : 0;
+    if (!__syncthreads_or(len > CS_WARP_CAP)) return;
+    const bool m = len > CS_WARP_CAP && len <= CS_BLOCK_CAP, g = len > CS_BLOCK_CAP;
+    const u32 am = block_append(m, n, sh);
+    if (m) mid[am] = h;
+    if (!__syncthreads_or(g)) return;
+    const u32 ag = block_append(g, n + 1, sh);
+    if (g) huge[ag] = h;
 }
 __global__ void k_tab_sizes(const u32 *__restrict__ list, u32 nl, const u64 *__restrict__ off, u64 *__restrict__ sz) {
     u32 i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1962,11 +1969,36 @@ __device__ __forceinline__ u32 gain_tier(u32 n, u32 K, u64 wk, u64 deg, u32 kway
     if (wk > GN_BLOCK_W) return 2u;
     return (n > GN_SMALL_LEVEL && wk <= GN_WARP_W && deg <= GN_WARP_DEG) ? 0u : 1u;
 }
-__global__ void k_tier(u32 n, u32 K, const u64 *__restrict__ work, const u64 *__restrict__ toff, u32 tier, u32 kway,
-                       u32 *__restrict__ flag) {
-    u32 u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= n) return;
-    flag[u] = gain_tier(n, K, work[u], toff[u + 1] - toff[u], kway) == tier ? 1u : 0u;
+// The tiers' node lists, the largest work bound over all nodes (out[0]) and over the block tier
+// (out[1]), and the largest degree (out[2]); cnt: three list counts in u64 words.
+__global__ void __launch_bounds__(1024) k_tier_lists(u32 n, u32 K, const u64 *__restrict__ work,
+                                                     const u64 *__restrict__ toff, u32 kway, u32 *l0, u32 *l1, u32 *l2,
+                                                     u64 *__restrict__ cnt, unsigned long long *__restrict__ out) {
+    __shared__ u32 sh[33];
+    const u32 u = blockIdx.x * blockDim.x + threadIdx.x;
+    u64 all = 0, blk = 0, deg = 0;
+    u32 t = 3;
+    if (u < n) {
+        all = work[u];
+        deg = toff[u + 1] - toff[u];
+        t = gain_tier(n, K, all, deg, kway);
+        if (t == 1u) blk = all;
+    }
+    u32 *lists[3] = {l0, l1, l2};
+#pragma unroll
+    for (u32 i = 0; i < 3; ++i) {
+        if (!__syncthreads_or(t == i)) continue;
+        const u32 at = block_append(t == i, (u32 *)(cnt + i), sh);
+        if (t == i) lists[i][at] = u;
+    }
+    all = warp_max_u64(all);
+    blk = warp_max_u64(blk);
+    deg = warp_max_u64(deg);
+    if ((threadIdx.x & 31) == 0) {
+        if (all) atomicMax(&out[0], (unsigned long long)all);
+        if (blk) atomicMax(&out[1], (unsigned long long)blk);
+        if (deg) atomicMax(&out[2], (unsigned long long)deg);
+    }
 }
 
 // ------------------------------------------------------------------ ranking
@@ -2543,14 +2575,6 @@ __global__ void k_long_list(MoverArgs V, const u32 *__restrict__ longs, u32 nlon
     at = __shfl_sync(0xFFFFFFFFu, at, 0);
     if (f) list[at + __popc(bal & ((1u << lane) - 1u))] = h;
 }
-__global__ void k_long_class(u32 e, const u64 *__restrict__ off, u32 *__restrict__ flag, uint8_t *__restrict__ cls) {
-    const u32 h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= e) return;
-    const bool lng = off[h + 1] - off[h] > CM_LEN;
-    flag[h] = lng;
-    cls[h] = lng ? 0 : 2;
-}
-
 __global__ void k_cascade_warp(CascadeArgs A, const u32 *__restrict__ list, const u32 *__restrict__ nlist,
                                u32 *__restrict__ big, u32 *__restrict__ nbig) {
     __shared__ u64 mvs[CC_WARPS][CC_MOV];
@@ -3906,28 +3930,51 @@ void setup_refine_kernels(Ctx &c) {
     AXC_CUDA(cudaFuncSetAttribute(k_copy_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
 }
 
-__global__ void k_level_bounds(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ nsrc,
-                               const u32 *__restrict__ wfx, unsigned long long *__restrict__ out);
-
-// Largest gain-work bound over all nodes (out[0]) and over the block tier (out[1]); the largest
-// degree (out[2]).
-__global__ void k_tier_max(u32 n, u32 K, const u64 *__restrict__ work, const u64 *__restrict__ toff, u32 kway,
-                           unsigned long long *__restrict__ out) {
-    u32 u = blockIdx.x * blockDim.x + threadIdx.x;
-    u64 all = 0, blk = 0, deg = 0;
-    if (u < n) {
-        const u64 wk = work[u];
-        deg = toff[u + 1] - toff[u];
-        all = wk;
-        if (gain_tier(n, K, wk, deg, kway) == 1u) blk = wk;
+// The level's hyperedge lists and bounds in one pass; dc as in prepare_level: the lists of lo < |e| <=
+// hi pins ([0]), longer ones ([1]) and those above CM_LEN ([15]), with cls their class
+// (k_mover_hedges); the longest, the destination pins, the extreme weights, and the pins and squared
+// lengths of the short ones ([9] to [14]).
+__global__ void __launch_bounds__(1024) k_level_hedges(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ nsrc,
+                                                       const u32 *__restrict__ wfx, u64 lo, u64 hi, u32 *mid, u32 *huge,
+                                                       u32 *lng, uint8_t *__restrict__ cls, u64 *__restrict__ dc) {
+    __shared__ u32 sh[33];
+    const u32 h = blockIdx.x * blockDim.x + threadIdx.x;
+    u64 len = 0, dst = 0, sp = 0, sq = 0;
+    u32 w = 0, nw = 0;
+    if (h < e) {
+        len = off[h + 1] - off[h];
+        dst = len - nsrc[h];
+        w = wfx[h];
+        nw = ~w;
+        cls[h] = len > CM_LEN ? 0 : 2;
+        if (len <= CM_LEN) { sp = len; sq = len * len; }
     }
-    all = warp_max_u64(all);
-    blk = warp_max_u64(blk);
-    deg = warp_max_u64(deg);
+    if (__syncthreads_or(len > CM_LEN)) {
+        const u32 at = block_append(len > CM_LEN, (u32 *)(dc + 15), sh);
+        if (len > CM_LEN) lng[at] = h;
+    }
+    if (__syncthreads_or(len > lo)) {
+        const u32 at = block_append(len > lo && len <= hi, (u32 *)(dc + 0), sh);
+        if (len > lo && len <= hi) mid[at] = h;
+        if (__syncthreads_or(len > hi)) {
+            const u32 ah = block_append(len > hi, (u32 *)(dc + 1), sh);
+            if (len > hi) huge[ah] = h;
+        }
+    }
+    len = warp_max_u64(len);
+    dst = warp_sum(dst);
+    sp = warp_sum(sp);
+    sq = warp_sum(sq);
+    w = __reduce_max_sync(0xFFFFFFFFu, w);
+    nw = __reduce_max_sync(0xFFFFFFFFu, nw);
     if ((threadIdx.x & 31) == 0) {
-        if (all) atomicMax(&out[0], (unsigned long long)all);
-        if (blk) atomicMax(&out[1], (unsigned long long)blk);
-        if (deg) atomicMax(&out[2], (unsigned long long)deg);
+        unsigned long long *out = (unsigned long long *)dc;
+        if (len) atomicMax(&out[9], (unsigned long long)len);
+        if (dst) atomicAdd(&out[10], (unsigned long long)dst);
+        if (w) atomicMax(&out[11], (unsigned long long)w);
+        if (nw) atomicMax(&out[12], (unsigned long long)nw);
+        if (sp) atomicAdd(&out[13], (unsigned long long)sp);
+        if (sq) atomicAdd(&out[14], (unsigned long long)sq);
     }
 }
 
@@ -3945,23 +3992,14 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
     AXC_CUDA(cudaMemsetAsync(dc, 0, 128, c.stream));
     lp.census_K = K <= CD_K || kway ? K : 0;
     if (e) {
-        u32 *flag = c.arena.alloc<u32>(e);
+        // census: a warp, a block above CD_WARP_LEN pins (partition-indexed) or CS_WARP_CAP (hashed),
+        // and hashed above CS_BLOCK_CAP a table in device memory
         lp.hblock = c.arena.alloc<u32>(e);
-        if (lp.census_K) {  // partition-indexed census: a warp, or a block above CD_WARP_LEN pins
-            LAUNCH(c, k_flag_len, cdiv(e, 256), 256, 0, e, L.off, (u64)CD_WARP_LEN, ~0ull, flag);
-            compact_indices_dn(c, flag, lp.hblock, e, (u32 *)(dc + 0));
-        } else {
-            lp.hhuge = c.arena.alloc<u32>(e);
-            LAUNCH(c, k_flag_len, cdiv(e, 256), 256, 0, e, L.off, (u64)CS_WARP_CAP, (u64)CS_BLOCK_CAP, flag);
-            compact_indices_dn(c, flag, lp.hblock, e, (u32 *)(dc + 0));
-            LAUNCH(c, k_flag_len, cdiv(e, 256), 256, 0, e, L.off, (u64)CS_BLOCK_CAP, ~0ull, flag);
-            compact_indices_dn(c, flag, lp.hhuge, e, (u32 *)(dc + 1));
-        }
+        if (!lp.census_K) lp.hhuge = c.arena.alloc<u32>(e);
         lp.hlong = c.arena.alloc<u32>(e);
         lp.hclass = c.arena.alloc<uint8_t>(e);
-        LAUNCH(c, k_long_class, cdiv(e, 256), 256, 0, e, L.off, flag, lp.hclass);
-        compact_indices_dn(c, flag, lp.hlong, e, (u32 *)(dc + 15));
-        LAUNCH(c, k_level_bounds, cdiv(e, 256), 256, 0, e, L.off, L.nsrc, wfx, (unsigned long long *)(dc + 9));
+        LAUNCH(c, k_level_hedges, cdiv(e, 1024), 1024, 0, e, L.off, L.nsrc, wfx, lp.census_K ? (u64)CD_WARP_LEN : (u64)CS_WARP_CAP,
+               lp.census_K ? ~0ull : (u64)CS_BLOCK_CAP, lp.hblock, lp.hhuge, lp.hlong, lp.hclass, dc);
     }
     if (n) {
         u64 *work = c.arena.alloc<u64>(n);
@@ -3969,14 +4007,9 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
         if (K > GS_K) lp.wsum = c.arena.alloc<u64>(n);
         LAUNCH(c, k_gain_bounds, cdiv((u64)n * 32, 256), 256, 0, n, K, L.toff, L.touch, L.off, wfx, work,
                lp.wsum, (unsigned long long *)(dc + 5));
-        u32 *flag = c.arena.alloc<u32>(n);
-        for (u32 t = 0; t < (kway ? 2u : 3u); ++t) {
-            lp.ntier[t] = c.arena.alloc<u32>(n);
-            LAUNCH(c, k_tier, cdiv(n, 256), 256, 0, n, K, work, L.toff, t, kway ? 1u : 0u, flag);
-            compact_indices_dn(c, flag, lp.ntier[t], n, (u32 *)(dc + 2 + t));
-        }
-        LAUNCH(c, k_tier_max, cdiv(n, 256), 256, 0, n, K, work, L.toff, kway ? 1u : 0u,
-               (unsigned long long *)(dc + 6));
+        for (u32 t = 0; t < (kway ? 2u : 3u); ++t) lp.ntier[t] = c.arena.alloc<u32>(n);
+        LAUNCH(c, k_tier_lists, cdiv(n, 1024), 1024, 0, n, K, work, L.toff, kway ? 1u : 0u, lp.ntier[0], lp.ntier[1],
+               lp.ntier[2], dc + 2, (unsigned long long *)(dc + 6));
     }
     u64 h[16];
     fetch(c, h, dc, 128);
@@ -4212,13 +4245,15 @@ Census build_census(Ctx &c, const DLevel &L, const u32 *part, u32 K) {
     size_t m = c.arena.mark();
     LevelPrep lp;
     if (L.e) {
-        u32 *flag = c.arena.alloc<u32>(L.e);
         lp.hblock = c.arena.alloc<u32>(L.e);
-        LAUNCH(c, k_flag_len, cdiv(L.e, 256), 256, 0, L.e, L.off, (u64)CS_WARP_CAP, (u64)CS_BLOCK_CAP, flag);
-        lp.n_hblock = compact_indices(c, flag, lp.hblock, L.e);
         lp.hhuge = c.arena.alloc<u32>(L.e);
-        LAUNCH(c, k_flag_len, cdiv(L.e, 256), 256, 0, L.e, L.off, (u64)CS_BLOCK_CAP, ~0ull, flag);
-        lp.n_hhuge = compact_indices(c, flag, lp.hhuge, L.e);
+        u32 *cnt = c.arena.alloc<u32>(2);
+        AXC_CUDA(cudaMemsetAsync(cnt, 0, 8, c.stream));
+        LAUNCH(c, k_census_lists, cdiv(L.e, 1024), 1024, 0, L.e, L.off, lp.hblock, lp.hhuge, cnt);
+        u64 h;
+        fetch(c, &h, cnt, 8);
+        lp.n_hblock = (u32)h;
+        lp.n_hhuge = (u32)(h >> 32);
         if (lp.n_hhuge) {
             lp.huge_tab = c.arena.alloc<u64>(lp.n_hhuge + 1);
             LAUNCH(c, k_tab_sizes, cdiv(lp.n_hhuge + 1, 256), 256, 0, lp.hhuge, lp.n_hhuge, L.off, lp.huge_tab);
@@ -4841,36 +4876,6 @@ __global__ void k_round_next(cudaGraphConditionalHandle h, u32 *__restrict__ rs,
         dyn[1] = r;
     }
     cudaGraphSetConditional(h, go ? 1u : 0u);
-}
-
-// level bounds over the hyperedges: the longest, the destination pin count, the largest weight and
-// the largest complement of a weight (the smallest weight)
-__global__ void k_level_bounds(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ nsrc,
-                               const u32 *__restrict__ wfx, unsigned long long *__restrict__ out) {
-    u32 h = blockIdx.x * blockDim.x + threadIdx.x;
-    u64 len = 0, dst = 0, sp = 0, sq = 0;
-    u32 w = 0, nw = 0;
-    if (h < e) {
-        len = off[h + 1] - off[h];
-        dst = len - nsrc[h];
-        w = wfx[h];
-        nw = ~w;
-        if (len <= CM_LEN) { sp = len; sq = len * len; }
-    }
-    sp = warp_sum(sp);
-    sq = warp_sum(sq);
-    len = warp_max_u64(len);
-    dst = warp_sum(dst);
-    w = __reduce_max_sync(0xFFFFFFFFu, w);
-    nw = __reduce_max_sync(0xFFFFFFFFu, nw);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(&out[0], (unsigned long long)len);
-        atomicAdd(&out[1], (unsigned long long)dst);
-        atomicMax(&out[2], (unsigned long long)w);
-        atomicMax(&out[3], (unsigned long long)nw);
-        if (sp) atomicAdd(&out[4], (unsigned long long)sp);
-        if (sq) atomicAdd(&out[5], (unsigned long long)sq);
-    }
 }
 
 // All rounds of a level in one graph launch: a conditional WHILE node whose body is one round
