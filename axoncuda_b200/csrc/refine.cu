@@ -23,9 +23,13 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "blocksort.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace axc {
 namespace {
@@ -923,8 +927,8 @@ struct MaskAcc {
 // batch stages its masks in the warp's shared slots (sm, sd, sw: 32 entries), which every lane
 // then reads as broadcasts.
 template <u32 MW>
-__device__ __forceinline__ void gain_mask_acc(const GainArgs &A, const u32 *__restrict__ mask,
-                                              const u32 *__restrict__ dmask, u32 u, u32 first, u32 stride,
+__device__ __forceinline__ void gain_mask_acc(const GainArgs &A, const u32 *mask,
+                                              const u32 *dmask, u32 u, u32 first, u32 stride,
                                               u32 (*sm)[MW], u32 (*sd)[MW], u32 *sw, MaskAcc<MW> &acc, i64 &wtot) {
     const u32 lane = threadIdx.x & 31u;
     const u64 t0 = A.toff[u];
@@ -2448,17 +2452,13 @@ __global__ void __launch_bounds__(CM_THREADS) k_cascade_movers_heavy(CascadeArgs
 
 // A staged pin: its rank, and partition | target << 15 | destination << 31 (target 0 without a
 // rank); its node beside it.
-template <bool TRACK>
-__global__ void __launch_bounds__(CM_THREADS) k_cascade_dense(CascadeArgs A, MoverArgs V) {
-    constexpr u32 NW = CM_THREADS / 32;
-    __shared__ uint2 ss[NW][CD_STAGE];
-    __shared__ u32 sn[NW][CD_STAGE];
-    if (!cascade_dense(V)) return;
-    const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    uint2 *st = ss[w];
-    u32 *nd = sn[w];
-    const u32 step = gridDim.x * NW * V.per_warp;
-    for (u32 h0 = (blockIdx.x * NW + w) * V.per_warp; h0 < A.e; h0 += step) {
+// Warp `warp` of `warps`; st and nd hold STAGE staged pins of this warp.
+template <bool TRACK, u32 STAGE>
+__device__ __forceinline__ void cascade_dense_body(const CascadeArgs &A, const MoverArgs &V, u32 warp, u32 warps, uint2 *st,
+                                                   u32 *nd) {
+    const u32 lane = threadIdx.x & 31u;
+    const u32 step = warps * V.per_warp;
+    for (u32 h0 = warp * V.per_warp; h0 < A.e; h0 += step) {
         const u32 h = h0 + lane;
         const bool mine = lane < V.per_warp && h < A.e;
         const u64 a = mine ? A.off[h] : 0, len64 = mine ? A.off[h + 1] - a : 0;
@@ -2474,7 +2474,7 @@ __global__ void __launch_bounds__(CM_THREADS) k_cascade_dense(CascadeArgs A, Mov
         // as many of the hyperedges as the stage holds at a time
         for (u32 lo = 0; lo < 32;) {
             const u32 b0 = __shfl_sync(0xFFFFFFFFu, excl, lo);
-            const u32 hi = lo + __popc(__ballot_sync(0xFFFFFFFFu, lane >= lo && x - b0 <= CD_STAGE));
+            const u32 hi = lo + __popc(__ballot_sync(0xFFFFFFFFu, lane >= lo && x - b0 <= STAGE));
             const u32 T = __shfl_sync(0xFFFFFFFFu, x, hi - 1) - b0;
             bool movers = false;
             for (u32 f0 = 0; f0 < T; f0 += 32) {
@@ -2543,6 +2543,16 @@ __global__ void __launch_bounds__(CM_THREADS) k_cascade_dense(CascadeArgs A, Mov
             lo = hi;
         }
     }
+}
+
+template <bool TRACK>
+__global__ void __launch_bounds__(CM_THREADS) k_cascade_dense(CascadeArgs A, MoverArgs V) {
+    constexpr u32 NW = CM_THREADS / 32;
+    __shared__ uint2 ss[NW][CD_STAGE];
+    __shared__ u32 sn[NW][CD_STAGE];
+    if (!cascade_dense(V)) return;
+    const u32 w = threadIdx.x >> 5;
+    cascade_dense_body<TRACK, CD_STAGE>(A, V, blockIdx.x * NW + w, gridDim.x * NW, ss[w], sn[w]);
 }
 
 // The hyperedges of more than CM_LEN pins that hold a mover. Few movers: every such incidence of
@@ -2985,13 +2995,13 @@ __device__ __forceinline__ i64 block_incl_scan_i64(i64 v, i64 *sh, i64 &total) {
     total = sh[(blockDim.x >> 5) - 1];
     return v + (w ? sh[w - 1] : 0);
 }
-__global__ void __launch_bounds__(VS_THREADS) k_validity_small(
-    const u32 *__restrict__ mv, const u32 *__restrict__ dM, const u32 *__restrict__ part,
-    const u32 *__restrict__ target, const u32 *__restrict__ nsize, const u64 *__restrict__ psize, u64 omega,
-    unsigned long long *__restrict__ Vs, int track, const unsigned long long *__restrict__ tdense, u32 stride,
-    const u64 *__restrict__ pinb, u64 delta, unsigned long long *__restrict__ Vi) {
+// Partition p by the calling block of VS_THREADS threads. CLEAR: the transitions read are zeroed.
+template <bool CLEAR>
+__device__ __forceinline__ void validity_small_body(u32 p, u32 M, const u32 *mv, const u32 *part, const u32 *target,
+                                                    const u32 *nsize, const u64 *psize, u64 omega, unsigned long long *Vs,
+                                                    int track, unsigned long long *tdense, u32 stride, const u64 *pinb,
+                                                    u64 delta, unsigned long long *Vi) {
     __shared__ i64 sh[32];
-    const u32 p = blockIdx.x, M = *dM;
     i64 run = (i64)psize[p];
     const i64 om = (i64)omega;
     for (u32 base = 0; base < M; base += VS_THREADS) {
@@ -3018,6 +3028,7 @@ __global__ void __launch_bounds__(VS_THREADS) k_validity_small(
     for (u32 base = 0; base < M; base += VS_THREADS) {
         const u32 r = base + threadIdx.x;
         const unsigned long long x = r < M ? tdense[(u64)p * stride + r] : 0ull;
+        if (CLEAR && x) tdense[(u64)p * stride + r] = 0;
         const bool has = (u32)x != 0u;
         const i64 D = has ? (i64)(int32_t)(u32)(x >> 32) : 0;
         i64 tot, htot;
@@ -3032,6 +3043,14 @@ __global__ void __launch_bounds__(VS_THREADS) k_validity_small(
         run2 += tot;
         seen = seen || htot > 0;
     }
+}
+__global__ void __launch_bounds__(VS_THREADS) k_validity_small(
+    const u32 *__restrict__ mv, const u32 *__restrict__ dM, const u32 *__restrict__ part,
+    const u32 *__restrict__ target, const u32 *__restrict__ nsize, const u64 *__restrict__ psize, u64 omega,
+    unsigned long long *__restrict__ Vs, int track, unsigned long long *__restrict__ tdense, u32 stride,
+    const u64 *__restrict__ pinb, u64 delta, unsigned long long *__restrict__ Vi) {
+    validity_small_body<false>(blockIdx.x, *dM, mv, part, target, nsize, psize, omega, Vs, track, tdense, stride, pinb, delta,
+                               Vi);
 }
 
 // best prefix (best_move_functor): inbound-valid first, then fewer size violations, then larger
@@ -3070,13 +3089,9 @@ __device__ __forceinline__ Best warp_best_prefix(Best b) {
 // radix sort of the descending gain keys (a second pass over the high words when the gain bound
 // needs more than 32 bits), then the ranks. Also resets every node's rank and cascaded gain and
 // writes the mover count and the size-event count, as k_move_flags ... k_set_rank do.
-__global__ void __launch_bounds__(RSS_WARPS * 32) k_rank_small(u32 n, const u32 *__restrict__ target,
-                                                              const i64 *__restrict__ gain, u64 gbound, u32 kb,
-                                                              const u32 *__restrict__ part, u32 *__restrict__ mv,
-                                                              uint2 *__restrict__ state,
-                                                              unsigned long long *__restrict__ g2, u32 *__restrict__ dM,
-                                                              u32 *__restrict__ twice) {
-    extern __shared__ u32 sm[];
+// sm: RSS_SMEM bytes. Returns the mover count.
+__device__ __forceinline__ u32 rank_small_body(u32 *sm, u32 n, const u32 *target, const i64 *gain, u64 gbound, u32 kb,
+                                               const u32 *part, u32 *mv, uint2 *state, unsigned long long *g2) {
     __shared__ i64 sh[32];
     u32 M = 0;
     for (u32 b = 0; b < n; b += blockDim.x) {
@@ -3115,6 +3130,16 @@ __global__ void __launch_bounds__(RSS_WARPS * 32) k_rank_small(u32 n, const u32 
         mv[i] = v;
         state[v].x = i;
     }
+    return M;
+}
+__global__ void __launch_bounds__(RSS_WARPS * 32) k_rank_small(u32 n, const u32 *__restrict__ target,
+                                                              const i64 *__restrict__ gain, u64 gbound, u32 kb,
+                                                              const u32 *__restrict__ part, u32 *__restrict__ mv,
+                                                              uint2 *__restrict__ state,
+                                                              unsigned long long *__restrict__ g2, u32 *__restrict__ dM,
+                                                              u32 *__restrict__ twice) {
+    extern __shared__ u32 sm[];
+    const u32 M = rank_small_body(sm, n, target, gain, gbound, kb, part, mv, state, g2);
     if (threadIdx.x == 0) {
         *dM = M;
         *twice = 2 * M;
@@ -3124,17 +3149,15 @@ __global__ void __launch_bounds__(RSS_WARPS * 32) k_rank_small(u32 n, const u32 
 // The inclusive prefix sums by rank of the cascaded gains, size violations (Vs) and inbound
 // violations (Vi), the best prefix by best_better, and its application when it is valid with a
 // non-negative gain: k_gather_g2, the 3n scan, k_best, k_best_final and k_apply in one block.
-__global__ void __launch_bounds__(1024) k_tail_small(const u32 *__restrict__ mv, const u32 *__restrict__ dM,
-                                                     const unsigned long long *__restrict__ g2,
-                                                     const i64 *__restrict__ Vs, const i64 *__restrict__ Vi, int has_vi,
-                                                     const u32 *__restrict__ target, u32 *__restrict__ part,
-                                                     u32 *__restrict__ apply) {
+// The block's best prefix: the number of movers to apply (0: none).
+__device__ __forceinline__ u32 tail_small_body(u32 M, const u32 *mv, const unsigned long long *g2, const i64 *Vs,
+                                               const i64 *Vi, int has_vi) {
     __shared__ i64 sh[32];
     __shared__ Best bsh[32];
     __shared__ i64 vsh[32];
     __shared__ Best s_best;
     __shared__ i64 s_vi;
-    const u32 M = *dM, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x == 0) { s_best = Best{0, 0, 0, 0xFFFFFFFFu}; s_vi = 0; }
     i64 rg = 0, rs = 0, ri = 0;
     for (u32 base = 0; base < M; base += blockDim.x) {
@@ -3179,9 +3202,16 @@ __global__ void __launch_bounds__(1024) k_tail_small(const u32 *__restrict__ mv,
     const Best x = s_best;
     const i64 vi = has_vi ? s_vi : 0;
     const bool ok = x.r != 0xFFFFFFFFu && x.vs <= 0 && vi <= 0 && x.g >= 0;
-    if (threadIdx.x == 0) *apply = ok ? 1u : 0u;
-    if (!ok) return;
-    for (u32 i = threadIdx.x; i <= x.r; i += blockDim.x) {
+    return ok ? x.r + 1 : 0u;
+}
+__global__ void __launch_bounds__(1024) k_tail_small(const u32 *__restrict__ mv, const u32 *__restrict__ dM,
+                                                     const unsigned long long *__restrict__ g2,
+                                                     const i64 *__restrict__ Vs, const i64 *__restrict__ Vi, int has_vi,
+                                                     const u32 *__restrict__ target, u32 *__restrict__ part,
+                                                     u32 *__restrict__ apply) {
+    const u32 end = tail_small_body(*dM, mv, g2, Vs, Vi, has_vi);
+    if (threadIdx.x == 0) *apply = end ? 1u : 0u;
+    for (u32 i = threadIdx.x; i < end; i += blockDim.x) {
         const u32 v = mv[i];
         part[v] = target[v];
     }
@@ -3842,6 +3872,185 @@ __global__ void __launch_bounds__(1024) k_copy_tail(CopyArgs A) {
         A.psize[base + i] = (u64)((i64)A.psize[base + i] + (i64)dlo[i] + ((i64)dhi[i] << 16));
 }
 
+// ------------------------------------------------------------------ all rounds of a small level
+// Inbound-constrained levels of at most RSS_CAP nodes, VS_MAX_K partitions and CM_LEN pins per
+// hyperedge: every round of the level in one cooperative launch. Such a round is a handful of
+// microseconds per phase, and as launches it was bound by their number and by capturing and
+// instantiating a graph per level. The phases are those of round_body on a small level, a grid
+// barrier apart; ranking and the best prefix run on block 0. What a phase accumulates into is
+// cleared by the phase that reads it last.
+constexpr u32 SR_THREADS = 1024;
+constexpr u32 SR_STAGE = 256;  // pins a warp of the cascade stages
+constexpr size_t SR_SMEM = RSS_SMEM;
+static_assert(SR_SMEM >= (size_t)SR_THREADS / 32 * SR_STAGE * 12 && SR_SMEM >= (size_t)SR_THREADS / 32 * 2 * CD_K * 4 &&
+                  SR_SMEM >= (size_t)SR_THREADS / 32 * 32 * (2 * 8 + 1) * 4 + 8 * 32 * 12 + 1024 && CM_LEN <= SR_STAGE &&
+                  VS_THREADS == SR_THREADS,
+              "every phase's shared state fits the launch");
+struct SmallArgs {
+    CensusArgs C;
+    GainArgs G;
+    CascadeArgs D;
+    MoverArgs V;
+    u32 R, kb;
+    u64 gbound;
+    u32 *mv, *dM;
+    uint2 *state;
+    unsigned long long *Vs, *Vi;
+    u32 *part;
+    u64 *psize, *pinb;
+    i64 *save;
+    u32 *rs;     // [0] round, [1] rounds done, [2] go on
+    int track;
+};
+
+template <u32 MW>
+__global__ void __launch_bounds__(SR_THREADS) k_small_rounds(SmallArgs S) {
+    cg::grid_group grid = cg::this_grid();
+    extern __shared__ __align__(16) u32 sr_sm[];
+    __shared__ u32 s_pinb[CD_K];
+    constexpr u32 NW = SR_THREADS / 32;
+    const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31u, K = S.G.K, n = S.G.n;
+    const u32 warp = blockIdx.x * NW + w, warps = gridDim.x * NW;
+    const u32 R = S.R;
+    for (u32 round = 0;;) {
+        // 1. census, savings and masks; the partitions' inbound counts
+        for (u32 i = threadIdx.x; i < K; i += SR_THREADS) s_pinb[i] = 0;
+        __syncthreads();
+        {
+            u32 *cnt = sr_sm + w * 2 * CD_K, *dcnt = cnt + CD_K;
+            for (u32 h = warp; h < S.D.e; h += warps) {
+                const u64 a = S.C.off[h], b = S.C.off[h + 1], s = a + S.C.nsrc[h];
+                for (u32 i = lane; i < K; i += 32) { cnt[i] = 0; dcnt[i] = 0; }
+                __syncwarp();
+                cd_count(S.C, a, b, s, cnt, dcnt, lane, 32);
+                __syncwarp();
+                cd_save(S.C, h, a, b, cnt, lane, 32);
+                cd_emit(S.C, h, a, cnt, dcnt, K);
+                for (u32 q = lane; q < K; q += 32)
+                    if (dcnt[q]) atomicAdd(&s_pinb[q], 1u);
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        for (u32 i = threadIdx.x; i < K; i += SR_THREADS)
+            if (s_pinb[i]) atomicAdd((unsigned long long *)&S.pinb[i], (unsigned long long)s_pinb[i]);
+        grid.sync();
+        // 2. gains: a warp per node, or a block per node where the nodes are few
+        GainArgs A = S.G;
+        A.discount = round < R / 3 ? 1u : (round < 2 * R / 3 ? 2u : 0xFFFFFFFFu);
+        A.round = round;
+        {
+            u32(*sm)[MW] = (u32(*)[MW])(sr_sm + w * 32 * (2 * MW + 1)), (*sd)[MW] = sm + 32;
+            u32 *sw = (u32 *)(sd + 32);
+            u32 *rest = sr_sm + NW * 32 * (2 * MW + 1);
+            if (n > warps / 2) {
+                for (u32 u = warp; u < n; u += warps) {
+                    MaskAcc<MW> acc;
+#pragma unroll
+                    for (u32 k = 0; k < MW; ++k) { acc.conn[k] = 0; acc.dconn[k] = 0; acc.pres[k] = 0; }
+                    i64 wtot = 0;
+                    gain_mask_acc<MW>(A, S.C.mask, S.C.dmask, u, 0, 32, sm, sd, sw, acc, wtot);
+                    wtot = warp_sum(wtot);
+                    const Cand best = mask_best<MW>(A, u, S.part[u], acc, S.save[u], wtot);
+                    if (lane == 0) {
+                        write_move(A, u, best);
+                        S.save[u] = 0;
+                    }
+                }
+            } else {
+                unsigned long long *rc = (unsigned long long *)rest;  // [MW * 32]
+                u32 *rd = (u32 *)(rc + MW * 32), *rp = rd + MW * 32;  // [MW * 32], [MW]
+                i64 *rw = (i64 *)(rp + 8);                            // [NW]
+                for (u32 u = blockIdx.x; u < n; u += gridDim.x) {
+                    for (u32 i = threadIdx.x; i < MW * 32; i += SR_THREADS) { rc[i] = 0; rd[i] = 0; }
+                    if (threadIdx.x < MW) rp[threadIdx.x] = 0;
+                    __syncthreads();
+                    MaskAcc<MW> acc;
+#pragma unroll
+                    for (u32 k = 0; k < MW; ++k) { acc.conn[k] = 0; acc.dconn[k] = 0; acc.pres[k] = 0; }
+                    i64 wtot = 0;
+                    gain_mask_acc<MW>(A, S.C.mask, S.C.dmask, u, 32 * w, SR_THREADS, sm, sd, sw, acc, wtot);
+                    wtot = warp_sum(wtot);
+#pragma unroll
+                    for (u32 k = 0; k < MW; ++k) {
+                        if (acc.conn[k]) atomicAdd(&rc[k * 32 + lane], acc.conn[k]);
+                        if (acc.dconn[k]) atomicAdd(&rd[k * 32 + lane], acc.dconn[k]);
+                        if (lane == 0 && acc.pres[k]) atomicOr(&rp[k], acc.pres[k]);
+                    }
+                    if (lane == 0) rw[w] = wtot;
+                    __syncthreads();
+                    if (w == 0) {
+#pragma unroll
+                        for (u32 k = 0; k < MW; ++k) {
+                            acc.conn[k] = rc[k * 32 + lane];
+                            acc.dconn[k] = rd[k * 32 + lane];
+                            acc.pres[k] = rp[k];
+                        }
+                        wtot = 0;
+                        for (u32 i = 0; i < NW; ++i) wtot += rw[i];
+                        const Cand best = mask_best<MW>(A, u, S.part[u], acc, S.save[u], wtot);
+                        if (lane == 0) {
+                            write_move(A, u, best);
+                            S.save[u] = 0;
+                        }
+                    }
+                    __syncthreads();
+                }
+            }
+        }
+        grid.sync();
+        // 3. ranks
+        if (blockIdx.x == 0) {
+            const u32 M = rank_small_body(sr_sm, n, A.target, A.gain, S.gbound, S.kb, S.part, S.mv, S.state, S.D.g2);
+            for (u32 i = threadIdx.x; i < M; i += SR_THREADS) S.Vs[i] = S.Vi[i] = 0;
+            if (threadIdx.x == 0) *S.dM = M;
+        }
+        grid.sync();
+        const u32 M = *(volatile u32 *)S.dM;
+        if (M) {
+            // 4. the cascade
+            {
+                uint2 *st = (uint2 *)sr_sm + w * SR_STAGE;
+                u32 *nd = sr_sm + NW * SR_STAGE * 2 + w * SR_STAGE;
+                if (S.track) cascade_dense_body<true, SR_STAGE>(S.D, S.V, warp, warps, st, nd);
+                else cascade_dense_body<false, SR_STAGE>(S.D, S.V, warp, warps, st, nd);
+            }
+            grid.sync();
+            // 5. size and inbound validity of every prefix
+            for (u32 p = blockIdx.x; p < K; p += gridDim.x)
+                validity_small_body<true>(p, M, S.mv, S.part, A.target, A.nsize, S.psize, A.omega, S.Vs, S.track, S.D.tdense, n,
+                                          S.pinb, A.delta, S.Vi);
+            grid.sync();
+        }
+        // 6. the best prefix, its application, and the schedule (k_round_next)
+        if (blockIdx.x == 0) {
+            const u32 end = M ? tail_small_body(M, S.mv, S.D.g2, (const i64 *)S.Vs, (const i64 *)S.Vi, S.track) : 0u;
+            for (u32 i = threadIdx.x; i < end; i += SR_THREADS) {
+                const u32 v = S.mv[i], p = S.part[v], q = A.target[v];
+                atomicAdd((unsigned long long *)&S.psize[p], 0ull - (unsigned long long)A.nsize[v]);
+                atomicAdd((unsigned long long *)&S.psize[q], (unsigned long long)A.nsize[v]);
+                S.part[v] = q;
+            }
+            for (u32 i = threadIdx.x; i < K; i += SR_THREADS) S.pinb[i] = 0;
+            if (threadIdx.x == 0) {
+                u32 x = round;
+                if (!end) {
+                    if (x < R / 3) x = R / 2;
+                    else if (x < 2 * R / 3) x = 2 * R / 3;
+                    else x = R;
+                }
+                x += 1;
+                S.rs[0] = x;
+                S.rs[1] += 1;
+                S.rs[2] = x < R && *(volatile const u32 *)S.C.status == 0;
+            }
+        }
+        grid.sync();
+        if (!*(volatile u32 *)&S.rs[2]) return;
+        round = *(volatile u32 *)&S.rs[0];
+    }
+}
+
 GainArgs make_gain_args(const DLevel &L, const u32 *wfx, const RefineParams &rp, const Census &cs, const u32 *part,
                         const u64 *psize, const u64 *pinb, u32 discount, u32 round, u32 *target, i64 *gain,
                         u32 *status) {
@@ -3928,6 +4137,10 @@ void setup_refine_kernels(Ctx &c) {
     AXC_CUDA(cudaFuncSetAttribute(k_cands_block<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CV_BLOCK_SMEM));
     AXC_CUDA(cudaFuncSetAttribute(k_rank_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
     AXC_CUDA(cudaFuncSetAttribute(k_copy_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RSS_SMEM));
+    AXC_CUDA(cudaFuncSetAttribute(k_small_rounds<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SR_SMEM));
+    AXC_CUDA(cudaFuncSetAttribute(k_small_rounds<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SR_SMEM));
+    AXC_CUDA(cudaFuncSetAttribute(k_small_rounds<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SR_SMEM));
+    AXC_CUDA(cudaFuncSetAttribute(k_small_rounds<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SR_SMEM));
 }
 
 // The level's hyperedge lists and bounds in one pass; dc as in prepare_level: the lists of lo < |e| <=
@@ -4944,6 +5157,67 @@ static u32 refine_level_loop(Ctx &c, const DLevel &L, const LevelPrep &lp, const
     return done;
 }
 
+// Levels whose rounds run in one launch (k_small_rounds).
+static bool small_rounds_eligible(const Ctx &c, const DLevel &L, const LevelPrep &lp, const RefineParams &rp) {
+    return rp.encourage && rp.copies == 1 && rp.K <= VS_MAX_K && L.n <= (u32)RSS_CAP && L.e && lp.max_len <= CM_LEN &&
+           c.coop_supported && !c.prof_on && round_loop_enabled();
+}
+
+static u32 small_rounds(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *wfx, const RefineParams &rp, u32 *part) {
+    const u32 n = L.n, K = rp.K;
+    Census cs = alloc_census(c, L);
+    cs.save = c.arena.alloc<i64>(n);
+    AXC_CUDA(cudaMemsetAsync(cs.save, 0, (size_t)n * 8, c.stream));
+    cs.wfx = wfx;
+    cs.encourage = 1;
+    cs.mw = mask_words(K);
+    cs.mask = c.arena.alloc<u32>((u64)L.e * cs.mw);
+    cs.dmask = c.arena.alloc<u32>((u64)L.e * cs.mw);
+    u64 *psize = c.arena.alloc<u64>(K), *pinb = c.arena.alloc<u64>(K);
+    part_sizes(c, n, part, L.nsize, psize, K);
+    AXC_CUDA(cudaMemsetAsync(pinb, 0, (size_t)K * 8, c.stream));
+    const bool track = rp.delta < 0x7FFFFFFFu && lp.dst_pins;
+    unsigned long long *tdense = nullptr;
+    if (track) {
+        tdense = c.arena.alloc<unsigned long long>((u64)K * n);
+        AXC_CUDA(cudaMemsetAsync(tdense, 0, (size_t)K * n * 8, c.stream));
+    }
+    u32 *target = c.arena.alloc<u32>(n);
+    i64 *gain = c.arena.alloc<i64>(n);
+    u32 *ctl = c.arena.alloc<u32>(8);  // [0, 3) schedule, [3] movers, [4] transitions (unused: summed)
+    AXC_CUDA(cudaMemsetAsync(ctl, 0, 32, c.stream));
+    SmallArgs S{};
+    S.C = CensusArgs{L.off, L.pins, L.nsrc, part, cs.part, cs.cnt, cs.dcnt, cs.lam, c.d_status,
+                     (unsigned long long *)cs.save, wfx, 1, cs.mask, cs.dmask, cs.mw, nullptr};
+    S.G = make_gain_args(L, wfx, rp, cs, part, psize, pinb, 1, 0, target, gain, c.d_status);
+    S.mv = c.arena.alloc<u32>(n);
+    S.dM = ctl + 3;
+    S.state = (uint2 *)c.arena.alloc<u64>(n);
+    S.D.e = L.e; S.D.encourage = 1; S.D.off = L.off; S.D.pins = L.pins; S.D.nsrc = L.nsrc; S.D.wfx = wfx;
+    S.D.part = part; S.D.target = target; S.D.state = S.state;
+    S.D.g2 = c.arena.alloc<unsigned long long>(n);
+    S.D.track = track ? 1 : 0; S.D.dT = ctl + 4; S.D.tdense = tdense; S.D.dense_stride = n; S.D.status = c.d_status;
+    S.D.K = K;
+    S.Vs = c.arena.alloc<unsigned long long>(n);
+    S.Vi = c.arena.alloc<unsigned long long>(n);
+    S.R = rp.rounds; S.kb = bits_for(lp.gain_bound); S.gbound = lp.gain_bound;
+    S.part = part; S.psize = psize; S.pinb = pinb; S.save = cs.save; S.rs = ctl; S.track = track ? 1 : 0;
+    // a warp per two or so hyperedges and per node, at most one block per SM
+    const u32 grid = std::max(1u, std::min<u32>((u32)c.sms, cdiv(std::max<u64>(L.e, n), 2 * (SR_THREADS / 32))));
+    S.V.per_warp = 32;
+    while (S.V.per_warp > 2 && L.e / S.V.per_warp < grid * (SR_THREADS / 32)) S.V.per_warp >>= 1;
+    const void *k = cs.mw == 1 ? (const void *)k_small_rounds<1> : cs.mw == 2 ? (const void *)k_small_rounds<2>
+                  : cs.mw == 4 ? (const void *)k_small_rounds<4> : (const void *)k_small_rounds<8>;
+    void *args[] = {(void *)&S};
+    AXC_CUDA(cudaLaunchCooperativeKernel(k, grid, SR_THREADS, args, SR_SMEM, c.stream));
+    c.launches++;
+    u64 res[3];
+    AXC_CUDA(cudaMemcpyAsync(ctl + 5, c.d_status, 4, cudaMemcpyDeviceToDevice, c.stream));
+    fetch(c, res, ctl, 24);
+    if ((u32)(res[2] >> 32) != DEV_OK) check_status(c);
+    return (u32)(res[0] >> 32);
+}
+
 static u32 refine_rounds(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *wfx, const RefineParams &rp, u32 *part,
                          IncCensus *ic, const KwayLevel *kw) {
     const u32 R = rp.rounds;
@@ -5029,6 +5303,11 @@ u32 refine_level(Ctx &c, const DLevel &L, const u32 *wfx, const RefineParams &rp
     KwayLevel kw;
     IncCensus ic;
     const bool inc = !kway && inc_census_eligible(L, lp, rp) && inc_census_enabled();
+    if (!kway && small_rounds_eligible(c, L, lp, rp)) {
+        const u32 done = small_rounds(c, L, lp, wfx, rp, part);
+        c.arena.release(m);
+        return done;
+    }
     if (kway) kway_init(c, L, rp, part, kw);
     if (inc) inc_census_init(c, L, wfx, rp, ic);
     const u32 done = refine_rounds(c, L, lp, wfx, rp, part, inc ? &ic : nullptr, kway ? &kw : nullptr);
