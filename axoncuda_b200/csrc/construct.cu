@@ -200,19 +200,20 @@ __global__ void k_touch_starts(u32 n, u64 P, const u32 *__restrict__ keys, u64 *
     nin[v] = (u32)(first_at_least(keys, o, P, 2 * v + 1) - o);
 }
 
-// Input validation before any id is used as an index: offsets non-decreasing, source counts within
-// their hyperedge, pin ids below n. Failures set the status word (no trap).
-__global__ void k_check_input(u32 n, u32 e, const u64 *__restrict__ off, const u32 *__restrict__ pins,
+// Input validation before any id is used as an index: offsets non-decreasing and within the P pins,
+// source counts within their hyperedge, pin ids below n. Failures set the status word (no trap).
+// The pins are read in order, whatever the hyperedges' lengths.
+__global__ void k_check_input(u32 n, u32 e, u64 P, const u64 *__restrict__ off, const u32 *__restrict__ pins,
                               const u32 *__restrict__ nsrc, u32 *status) {
-    const u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= e) return;
-    const u64 a = off[w], b = off[w + 1];
-    if (b < a || nsrc[w] > b - a) {
-        if (lane == 0) atomicExch(status, DEV_BAD_INDEX);
-        return;
+    const u64 i0 = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
+    bool bad = false;
+    for (u64 h = i0; h < e; h += step) {
+        const u64 a = off[h], b = off[h + 1];
+        bad |= b < a || b > P || nsrc[h] > b - a;
     }
-    for (u64 k = a + lane; k < b; k += 32)
-        if (pins[k] >= n) atomicExch(status, DEV_BAD_INDEX);
+#pragma unroll 4
+    for (u64 k = off[0] + i0; k < P; k += step) bad |= pins[k] >= n;
+    if (bad) atomicExch(status, DEV_BAD_INDEX);
 }
 
 __global__ void k_group_sizes(u32 n, const u32 *__restrict__ groups, const u32 *__restrict__ nsize,
@@ -285,8 +286,10 @@ void build_touching(Ctx &c, u32 n, u32 e, const u64 *off, const u32 *pins, const
     c.arena.release(m);
 }
 
-void check_input(Ctx &c, u32 n, u32 e, const u64 *off, const u32 *pins, const u32 *nsrc) {
-    if (e) LAUNCH(c, k_check_input, cdiv((u64)e * 32, 256), 256, 0, n, e, off, pins, nsrc, c.d_status);
+void check_input(Ctx &c, u32 n, u32 e, u64 P, const u64 *off, const u32 *pins, const u32 *nsrc) {
+    if (e)
+        LAUNCH(c, k_check_input, std::min<u32>(cdiv(std::max<u64>(P, e), 256), (u32)c.sms * 16), 256, 0, n, e, P, off, pins, nsrc,
+               c.d_status);
     u32 s = fetch1(c, c.d_status);
     if (s != DEV_OK) {
         AXC_CUDA(cudaMemsetAsync(c.d_status, 0, 4, c.stream));

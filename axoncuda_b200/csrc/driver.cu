@@ -83,7 +83,7 @@ static int resolve(const axc_params *p, u32 n, Resolved &r) {
 // Allocate and build level 0 from a raw device hypergraph (dedupe + incidence CSR).
 static DLevel build_level0(Ctx &c, u32 n, u32 e, const u64 *off, const u32 *pins, const u32 *nsrc, u64 P_in) {
     DLevel L;
-    check_input(c, n, e, off, pins, nsrc);
+    check_input(c, n, e, P_in, off, pins, nsrc);
     L.arena_mark = c.arena.mark();
     L.n = n;
     L.e = e;
@@ -451,7 +451,7 @@ static axc_hgraph upload(Ctx &c, const axc_hgraph *g, u64 &P) {
     d.pins = pins;
     d.src_count = ns;
     d.hedge_w = w;
-    check_input(c, g->n, g->e, off, pins, ns);
+    check_input(c, g->n, g->e, P, off, pins, ns);
     return d;
 }
 

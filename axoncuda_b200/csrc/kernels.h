@@ -30,7 +30,8 @@ void build_touching(Ctx &c, u32 n, u32 e, const u64 *off, const u32 *pins, const
                     u64 *toff, u32 *touch, u32 *nin);
 void group_sizes(Ctx &c, u32 n, const u32 *groups, const u32 *nsize, u32 *gsize, u32 ng);
 // rejects (AXC_EINVAL) offsets that decrease, source counts beyond their hyperedge, pins >= n
-void check_input(Ctx &c, u32 n, u32 e, const u64 *off, const u32 *pins, const u32 *nsrc);
+// (P = off[e], read by the caller)
+void check_input(Ctx &c, u32 n, u32 e, u64 P, const u64 *off, const u32 *pins, const u32 *nsrc);
 
 // coarsen.cu
 void setup_coarsen_kernels(Ctx &c);
@@ -79,6 +80,7 @@ struct Census {
 };
 // K: partition ids are below it
 Census build_census(Ctx &c, const DLevel &L, const u32 *part, u32 K);
+// nsize null: every node counts 1
 void part_sizes(Ctx &c, u32 n, const u32 *part, const u32 *nsize, u64 *psize, u32 K);
 void part_inbound(Ctx &c, const DLevel &L, const Census &cs, u64 *pinb, u32 K);
 

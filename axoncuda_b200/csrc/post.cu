@@ -115,11 +115,6 @@ __global__ void k_part_stats(u32 K, const u64 *__restrict__ psize, const u64 *__
         atomicMax(&acc[5], (unsigned long long)mi);
     }
 }
-__global__ void k_count_nodes(u32 n, const u32 *__restrict__ part, unsigned long long *__restrict__ cnt) {
-    u32 v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < n) atomicAdd(&cnt[part[v]], 1ull);
-}
-
 }  // namespace
 
 void uncoarsen(Ctx &c, u32 n, const u32 *groups, const u32 *coarse_part, u32 *part) {
@@ -212,8 +207,7 @@ void evaluate(Ctx &c, const DLevel &L, const u32 *wfx, const u32 *part, u32 omeg
     Census cs = build_census(c, L, part, K);
     u64 *psize = c.arena.alloc<u64>(K ? K : 1), *pinb = c.arena.alloc<u64>(K ? K : 1);
     // validity counts nodes (not node weights), like sources/constr.cpp:95-115
-    AXC_CUDA(cudaMemsetAsync(psize, 0, (size_t)K * 8, c.stream));
-    if (L.n) LAUNCH(c, k_count_nodes, cdiv(L.n, 256), 256, 0, L.n, part, (unsigned long long *)psize);
+    if (K) part_sizes(c, L.n, part, nullptr, psize, K);
     part_inbound(c, L, cs, pinb, K);
     unsigned long long *acc = c.arena.alloc<unsigned long long>(6);
     AXC_CUDA(cudaMemsetAsync(acc, 0, 48, c.stream));

@@ -618,7 +618,7 @@ __global__ void k_tab_sizes(const u32 *__restrict__ list, u32 nl, const u64 *__r
 __global__ void k_part_sizes(u32 n, const u32 *__restrict__ part, const u32 *__restrict__ nsize,
                              unsigned long long *__restrict__ ps) {
     u32 v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < n) atomicAdd(&ps[part[v]], (unsigned long long)nsize[v]);
+    if (v < n) atomicAdd(&ps[part[v]], (unsigned long long)(nsize ? nsize[v] : 1u));
 }
 // Few partitions (K <= PS_SMEM_K): per-block sums in shared memory, one global add per partition
 // and block. A size is added in 16-bit halves, each a native 32-bit add (64-bit ones would be
@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(256) k_part_sizes_smem(u32 n, u32 K, u32 rep, 
     const u64 v0 = (u64)blockIdx.x * per_block, v1 = v0 + per_block < n ? v0 + per_block : n;
 #pragma unroll 4
     for (u64 v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-        const u32 q = part[v], s = nsize[v];
+        const u32 q = part[v], s = nsize ? nsize[v] : 1u;
         if (q >= K) continue;  // ids are below K by contract
         atomicAdd(&lo[q * rep + l], s & 0xFFFFu);
         if (s >> 16) atomicAdd(&hi[q * rep + l], s >> 16);
@@ -1348,18 +1348,19 @@ __device__ __forceinline__ void csa(u32 &h, u32 &l, u32 a, u32 b, u32 c) {
     h = (a & b) | (x & c);
     l = x ^ c;
 }
-// Bit-plane counters of mask word `wl` over the incidences slot, slot + S, ... below jend of the
-// node's list t: plane b of bit i counts 2^b incidences whose word has bit i.
-__device__ __forceinline__ void plane_count(const u32 *__restrict__ t, u32 jend, const u32 *__restrict__ mask, u32 MW,
-                                            u32 wl, u32 slot, u32 S, u32 (&pl)[GP_PLANES]) {
+// Bit-plane counters of mask word `wl` (of MW, pitch words apart) over the incidences slot, slot + S,
+// ... below jend of the node's list t: plane b of bit i counts 2^b incidences whose word has bit i.
+template <u32 NP>
+__device__ __forceinline__ void plane_count(const u32 *__restrict__ t, u32 jend, const u32 *__restrict__ mask, u32 pitch,
+                                            u32 MW, u32 wl, u32 slot, u32 S, u32 (&pl)[NP]) {
 #pragma unroll
-    for (u32 b = 0; b < GP_PLANES; ++b) pl[b] = 0;
+    for (u32 b = 0; b < NP; ++b) pl[b] = 0;
     for (u32 j = slot; j < jend; j += 8 * S) {
         u32 x[8];
 #pragma unroll
         for (u32 r = 0; r < 8; ++r) x[r] = j + r * S < jend ? t[j + r * S] : NONE;
 #pragma unroll
-        for (u32 r = 0; r < 8; ++r) x[r] = x[r] != NONE && wl < MW ? mask[(u64)x[r] * MW + wl] : 0u;
+        for (u32 r = 0; r < 8; ++r) x[r] = x[r] != NONE && wl < MW ? mask[(u64)x[r] * pitch + wl] : 0u;
         u32 t0, t1, f0, f1, e0;
         csa(t0, pl[0], pl[0], x[0], x[1]);
         csa(t1, pl[0], pl[0], x[2], x[3]);
@@ -1369,7 +1370,7 @@ __device__ __forceinline__ void plane_count(const u32 *__restrict__ t, u32 jend,
         csa(f1, pl[1], pl[1], t0, t1);
         csa(e0, pl[2], pl[2], f0, f1);
 #pragma unroll
-        for (u32 b = 3; b < GP_PLANES; ++b) {
+        for (u32 b = 3; b < NP; ++b) {
             const u32 c = pl[b] & e0;
             pl[b] ^= e0;
             e0 = c;
@@ -1377,10 +1378,11 @@ __device__ __forceinline__ void plane_count(const u32 *__restrict__ t, u32 jend,
     }
 }
 // The counters of lanes l and l ^ o added (both get the sum).
-__device__ __forceinline__ void plane_merge(u32 (&pl)[GP_PLANES], u32 o) {
+template <u32 NP>
+__device__ __forceinline__ void plane_merge(u32 (&pl)[NP], u32 o) {
     u32 c = 0;
 #pragma unroll
-    for (u32 b = 0; b < GP_PLANES; ++b) {
+    for (u32 b = 0; b < NP; ++b) {
         const u32 y = __shfl_xor_sync(0xFFFFFFFFu, pl[b], o);
         u32 h;
         csa(h, pl[b], pl[b], y, c);
@@ -1410,7 +1412,7 @@ __global__ void __launch_bounds__(GN_BLOCK) k_gain_planes(GainArgs A0, const u32
 #pragma unroll 1
         for (u32 pass = 0; pass < 2; ++pass) {
             u32 pl[GP_PLANES];
-            plane_count(A.touch + t0, pass ? nin : deg, pass ? dmask : mask, MW, wl, slot, S, pl);
+            plane_count(A.touch + t0, pass ? nin : deg, pass ? dmask : mask, MW, MW, wl, slot, S, pl);
             if (MWP < 32)
 #pragma unroll
                 for (u32 o = 16; o >= MWP; o >>= 1) plane_merge(pl, o);
@@ -3460,6 +3462,8 @@ struct KwGain {
     u32 k, cn;  // partitions and nodes of one copy
     const u32 *list;
     u32 nl;
+    int uni;     // every hyperedge has the weight `weight`
+    u32 weight;
 };
 
 // Best target of node u from the lanes' connectivities: lane `own` of a group of G holds those of
@@ -3509,7 +3513,7 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain(GainArgs A0, KwGain V)
     for (u32 x = 0; x < C; ++x) conn[x] = 0;
 #pragma unroll 4
     for (u32 j = 0; j < deg; ++j) {
-        const u32 h = A.touch[t0 + j], w = A.wfx[h];
+        const u32 h = A.touch[t0 + j], w = V.uni ? V.weight : A.wfx[h];
         const u32 *r = V.rec + (u64)h * (2 * MW);
         u32 any[MW];
         u32 sg;
@@ -3545,7 +3549,7 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain_few(GainArgs A0, KwGai
     T conn[4] = {0, 0, 0, 0}, saving = 0, wtot = 0;
 #pragma unroll 2
     for (u32 j = own; j < deg; j += G) {
-        const u32 h = A.touch[t0 + j], w = A.wfx[h];
+        const u32 h = A.touch[t0 + j], w = V.uni ? V.weight : A.wfx[h];
         const uint2 r = *(const uint2 *)(V.rec + (u64)h * 2);
         wtot += w;
         if ((r.y >> pl) & 1u) saving += w;
@@ -3581,7 +3585,7 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain_block(GainArgs A0, KwG
         for (u32 x = 0; x < MW; ++x) conn[x] = 0;
 #pragma unroll 4
         for (u64 j = w; j < deg; j += NW) {
-            const u32 h = A.touch[t0 + j], wh = A.wfx[h];
+            const u32 h = A.touch[t0 + j], wh = V.uni ? V.weight : A.wfx[h];
             const u32 *r = V.rec + (u64)h * (2 * MW);
             u32 any[MW];
             load_words<MW>(r, any);
@@ -3607,6 +3611,66 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain_block(GainArgs A0, KwG
             kw_move<32, MW, T>(A, u, base, pl, V.k, lane, 0xFFFFFFFFu, conn, saving, wtot);
         }
         __syncthreads();  // warp 0 has read the sums
+    }
+}
+
+// Equal weights and many incidences per node: connectivity as a count, by bit planes (k_gain_planes)
+// over the records' present words. A lane owns one word of an incidence, so 32 / MW incidences go
+// side by side and an incidence costs a lane a few bit operations for 32 partitions, against one
+// test and add per partition. A warp per node, or with BLOCK a block of KW_THREADS whose warps split
+// the incidences. NP: planes, enough for a warp's incidences.
+constexpr u32 KP_PLANES = 11, KP_PLANES_BLOCK = 14;
+static_assert(KW_WARP_DEG < (1u << KP_PLANES), "a warp's counters hold its node's incidences");
+template <u32 MW, bool BLOCK>
+__global__ void __launch_bounds__(KW_THREADS) k_kway_planes(GainArgs A0, KwGain V) {
+    constexpr u32 NP = BLOCK ? KP_PLANES_BLOCK : KP_PLANES, NW = KW_THREADS / 32, S = 32 / MW;
+    const GainArgs A = gain_args_now(A0);
+    __shared__ u32 sc[BLOCK ? NW : 1][MW * 32], ss[NW];
+    const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5, wl = lane & (MW - 1), slot = lane / MW;
+    const u32 first = BLOCK ? blockIdx.x : blockIdx.x * NW + w, step = BLOCK ? gridDim.x : gridDim.x * NW;
+    for (u32 idx = first; idx < V.nl; idx += step) {
+        const u32 u = V.list[idx], base = (u / V.cn) * V.k, pl = A.part[u] - base;
+        const u64 t0 = A.toff[u];
+        const u32 deg = (u32)(A.toff[u + 1] - t0);
+        // BLOCK: warp w takes incidences [j0, j1)
+        const u32 share = BLOCK ? (deg + NW - 1) / NW : deg, j0 = BLOCK ? min(deg, w * share) : 0;
+        const u32 cnt = BLOCK ? min(share, deg - j0) : deg;
+        const u32 *t = A.touch + t0 + j0;
+        u32 pc[NP];
+        plane_count<NP>(t, cnt, V.rec, 2 * MW, MW, wl, slot, S, pc);
+#pragma unroll
+        for (u32 o = 16; o >= MW; o >>= 1) plane_merge<NP>(pc, o);
+        u32 one = 0;  // incidences whose only pin in u's partition is u
+        for (u32 j = lane; j < cnt; j += 32)
+            one += (V.rec[(u64)t[j] * (2 * MW) + MW + (pl >> 5)] >> (pl & 31u)) & 1u;
+        one = __reduce_add_sync(0xFFFFFFFFu, one);
+        unsigned long long conn[MW];
+#pragma unroll
+        for (u32 x = 0; x < MW; ++x) {
+            u32 c = 0;
+#pragma unroll
+            for (u32 b = 0; b < NP; ++b) c += ((__shfl_sync(0xFFFFFFFFu, pc[b], x) >> lane) & 1u) << b;
+            if (BLOCK) sc[w][x * 32 + lane] = c;
+            else conn[x] = (unsigned long long)c * V.weight;
+        }
+        if (BLOCK) {
+            if (lane == 0) ss[w] = one;
+            __syncthreads();
+            if (w == 0) {
+                one = 0;
+                for (u32 i = 0; i < NW; ++i) one += ss[i];
+#pragma unroll
+                for (u32 x = 0; x < MW; ++x) {
+                    u32 c = 0;
+                    for (u32 i = 0; i < NW; ++i) c += sc[i][x * 32 + lane];
+                    conn[x] = (unsigned long long)c * V.weight;
+                }
+            }
+        }
+        if (!BLOCK || w == 0)
+            kw_move<32, MW, unsigned long long>(A, u, base, pl, V.k, lane, 0xFFFFFFFFu, conn,
+                                                (unsigned long long)one * V.weight, (unsigned long long)deg * V.weight);
+        if (BLOCK) __syncthreads();  // warp 0 has read the sums
     }
 }
 
@@ -4695,7 +4759,9 @@ static void kway_records(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32
 // degree fills); heavy nodes and small levels: a block per node.
 template <class T>
 static void kway_gains_t(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainArgs &A, const KwayLevel &kw) {
-    KwGain V{kw.rec, kw.k, kw.cn, lp.ntier[0], lp.ncount[0]};
+    KwGain V{kw.rec, kw.k, kw.cn, lp.ntier[0], lp.ncount[0], lp.uniform ? 1 : 0, lp.weight};
+    // planes: merging a warp's counters costs as much as a few dozen incidences the other way
+    const bool planes = lp.uniform && kw.k > 8 && L.P / L.n >= 48;
     const auto grid = [&](u32 G) { return cdiv((u64)lp.ncount[0] * G, KW_THREADS); };
     if (lp.ncount[0] && kw.k <= 4) {
         const u64 deg = L.P / L.n;
@@ -4703,6 +4769,11 @@ static void kway_gains_t(Ctx &c, const DLevel &L, const LevelPrep &lp, const Gai
         else if (deg < 24) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain_few<8, T>), grid(8), KW_THREADS, 0, A, V);
         else if (deg < 64) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain_few<16, T>), grid(16), KW_THREADS, 0, A, V);
         else LAUNCH_AS(c, "k_kway_gain", (k_kway_gain_few<32, T>), grid(32), KW_THREADS, 0, A, V);
+    } else if (lp.ncount[0] && planes) {
+        kway_words(kw.mw, [&](auto mw) {
+            LAUNCH_AS(c, "k_kway_planes", (k_kway_planes<decltype(mw)::value, false>), cdiv(lp.ncount[0], KW_THREADS / 32),
+                      KW_THREADS, 0, A, V);
+        });
     } else if (lp.ncount[0]) {
         if (kw.k <= 8) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain<1, 8, T>), grid(8), KW_THREADS, 0, A, V);
         else if (kw.k <= 16) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain<1, 16, T>), grid(16), KW_THREADS, 0, A, V);
@@ -4714,7 +4785,12 @@ static void kway_gains_t(Ctx &c, const DLevel &L, const LevelPrep &lp, const Gai
     if (lp.ncount[1]) {
         V.list = lp.ntier[1];
         V.nl = lp.ncount[1];
+        const bool wide = planes && lp.max_deg / (KW_THREADS / 32) + 1 < (1u << KP_PLANES_BLOCK);
         kway_words(kw.mw, [&](auto mw) {
+            if (wide)
+                LAUNCH_AS(c, "k_kway_planes_block", (k_kway_planes<decltype(mw)::value, true>), lp.ncount[1], KW_THREADS, 0, A,
+                          V);
+            else
             LAUNCH_AS(c, "k_kway_gain_block", (k_kway_gain_block<decltype(mw)::value, T>), lp.ncount[1], KW_THREADS, 0, A,
                       V);
         });
