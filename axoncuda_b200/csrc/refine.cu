@@ -1496,6 +1496,7 @@ constexpr unsigned long long CV_ONE = 1ull << 32;
 // (delta - inbound) above, each at most RM_MORE; RM_NONE where the limit is already passed. The scans
 // of k_gain_sample read it for every partition near a node, at a quarter of the two counts' bytes.
 constexpr u32 RM_MORE = 0xFFFEu, RM_NONE = 0xFFFFu;
+static_assert(GS_BLOCK == 256, "32 groups of 8 threads");
 static_assert(GS_SAMPLE < RM_MORE, "a sample's incidences compare exactly");
 __global__ void k_part_room(u32 K, u32 omega, u32 delta, const u64 *__restrict__ psize, const u64 *__restrict__ pinb,
                             u32 *__restrict__ room) {
@@ -1520,7 +1521,7 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
     __shared__ unsigned long long wsh[NW];
     __shared__ unsigned long long s_acc;
     __shared__ Cand cred[NW];
-    __shared__ SKey kred[NW], kout[GS_C], klist[GS_LIST];
+    __shared__ SKey kred[32], kout[GS_C], klist[GS_LIST];
     __shared__ u32 nkeys;
     // the first GS_BLOCK incidences: exclusive census prefix (entry m = the sample's total when m is
     // at most GS_BLOCK), census offset and weight
@@ -1690,9 +1691,11 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
             continue;
         }
         // 3b. the GS_C best by (sampled connectivity, tie hash, -id) among the keys the size limit and
-        // the inbound bound do not rule out. Pass 1 empties the ruled-out slots and takes each warp's
-        // best key; the least of those NW >= GS_C keys is no better than the GS_C-th best, so pass 2
-        // lists the keys at or above it (a few dozen), whose ranks are counted pairwise.
+        // the inbound bound do not rule out. Pass 1 empties the ruled-out slots and takes the best key
+        // of each group of 8 threads; the GS_C-th of those 32 keys is no better than the GS_C-th of
+        // all, so pass 2 lists the keys at or above it (a dozen or so), whose ranks are counted
+        // pairwise. (The least of the warps' best keys listed hundreds where a warp's slots, a range
+        // of partitions, lie away from the node's.)
         const u64 in_sample = m < nin_u ? m : nin_u, need = s - s / A.discount;
         SKey best1{0, 0};
         scan([&](u32 i, u32 x, u32 y) {
@@ -1711,16 +1714,21 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
             if (skey_better(k, best1)) best1 = k;
         });
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+        for (int o = 4; o > 0; o >>= 1) {  // 32 groups of 8 threads
             const SKey c{__shfl_xor_sync(0xFFFFFFFFu, best1.hi, o), __shfl_xor_sync(0xFFFFFFFFu, best1.lo, o)};
             if (skey_better(c, best1)) best1 = c;
         }
-        if (lane == 0) kred[warp] = best1;
+        if ((lane & 7u) == 0) kred[threadIdx.x / 8] = best1;
         if (threadIdx.x < GS_C) kout[threadIdx.x] = SKey{0, 0};
         __syncthreads();
-        SKey thr = kred[0];
-        for (u32 w2 = 1; w2 < NW; ++w2)
-            if (skey_better(thr, kred[w2])) thr = kred[w2];
+        SKey thr{0, 0};
+        {
+            const SKey mine = kred[lane];
+            u32 rank = 0;
+            for (u32 j = 0; j < 32; ++j) rank += skey_better(kred[j], mine);
+            const u32 bal = __ballot_sync(0xFFFFFFFFu, rank == GS_C - 1 && (mine.hi | mine.lo));
+            if (bal) thr = kred[__ffs(bal) - 1];  // keys are unique: one lane
+        }
         scan([&](u32 i, u32 x, u32 y) {
             const u64 conn = conn_of(x, y);
             if (conn < thr.hi) return;
@@ -1738,7 +1746,7 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
                 for (u32 j = 0; j < nk && rank < GS_C; ++j) rank += skey_better(klist[j], k);
                 if (rank < GS_C) kout[rank] = k;
             }
-        } else {  // a warp without keys leaves a threshold that lists too many: GS_C block-wide maxima
+        } else {  // fewer than GS_C groups hold a key and some hold very many: GS_C block-wide maxima
             SKey prev{~0ull, ~0ull};
             for (u32 r = 0; r < GS_C; ++r) {
                 SKey b{0, 0};
@@ -2101,9 +2109,6 @@ __global__ void k_pair_gain_high(const u32 *__restrict__ mv, const u32 *__restri
 }
 
 // ------------------------------------------------------------------ cascade
-constexpr u32 CC_WARPS = 4;
-constexpr u32 CC_MOV = 128;    // movers per hyperedge handled by the warp kernel
-constexpr u32 CC_TAB = 512;    // partition table slots of the warp kernel
 
 struct CascadeArgs {
     u32 e;
@@ -2131,13 +2136,10 @@ struct CascadeArgs {
     // movers in slots (k-way copies ranked by one block each): copy t's from slot t * cn, dM[t] of
     // them; 0: ranks [0, *dM)
     u32 cn;
-    // when set (kernel timer on k_cascade_warp): each hyperedge's algorithmic bytes are added here
-    unsigned long long *pbytes;
 };
 
 constexpr u32 MV_DST = 0x80000000u;  // mover flag in the node field: the pin is a destination
-constexpr u32 CC_DIRECT_K = 256;        // the warp kernel's tables indexed by partition
-constexpr u32 CC_DIRECT_BLOCK_K = 1024; // the block kernels'
+constexpr u32 CC_DIRECT_BLOCK_K = 1024;  // tables indexed by partition up to this many
 
 __device__ __forceinline__ u32 cascade_base(const CascadeArgs &A, u32 h) { return A.ce ? (h / A.ce) * A.K : 0u; }
 
@@ -2587,74 +2589,208 @@ __global__ void k_long_list(MoverArgs V, const u32 *__restrict__ longs, u32 nlon
     at = __shfl_sync(0xFFFFFFFFu, at, 0);
     if (f) list[at + __popc(bal & ((1u << lane) - 1u))] = h;
 }
-__global__ void k_cascade_warp(CascadeArgs A, const u32 *__restrict__ list, const u32 *__restrict__ nlist,
-                               u32 *__restrict__ big, u32 *__restrict__ nbig) {
-    __shared__ u64 mvs[CC_WARPS][CC_MOV];
-    __shared__ u32 sl[CC_WARPS][CC_MOV];
-    __shared__ u32 tk[CC_WARPS][CC_TAB], tc[CC_WARPS][CC_TAB], td[CC_WARPS][CC_TAB];
-    const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const u32 nl = *nlist;
-    u64 bytes = 0;  // algorithmic bytes of this warp's hyperedges (kernel timer)
-    for (u32 idx = blockIdx.x * CC_WARPS + w; idx < nl; idx += gridDim.x * CC_WARPS) {
-        __syncwarp();  // the previous hyperedge's shared state is no longer read
-        const u32 h = list[idx];
-        const u64 a = A.off[h], b = A.off[h + 1], d0 = a + A.nsrc[h];
-        // collect movers (rank << 32 | dst flag | node)
-        u32 m = 0;
-        for (u64 base = a; base < b; base += 32) {
-            u64 k = base + lane;
-            u32 v = k < b ? A.pins[k] : 0, r = k < b ? A.state[v].x : NONE;
-            bool mvr = r != NONE;
-            u32 bal = __ballot_sync(0xFFFFFFFFu, mvr);
-            if (mvr) {
-                u32 pos = m + __popc(bal & ((1u << lane) - 1u));
-                if (pos < CC_MOV) mvs[w][pos] = ((u64)r << 32) | (k >= d0 ? MV_DST : 0u) | v;
-            }
-            m += __popc(bal);
-        }
-        // algorithmic bytes (kernel timer): the list entry, offsets and source count, each pin's id
-        // and rank, the census size, then the hand-off to the block kernel or the census entries,
-        // each mover's partition, target and cascaded gain, and the weight (transitions not counted)
-        const u64 bytes_read = 24 + 8 * (b - a);
-        if (m == 0) {  // (a listed hyperedge always has a mover)
-            bytes += bytes_read;
-            continue;
-        }
-        const u32 lm = A.lam ? A.lam[h] : 0;
-        const bool direct = A.K <= CC_DIRECT_K;
-        const u32 cap = direct ? A.K : cascade_cap32(lm, m);
-        if (m > CC_MOV || cap > CC_TAB) {
-            if (lane == 0) big[atomicAdd(nbig, 1u)] = h;  // handled by the block kernel
-            bytes += bytes_read + 8;
-            continue;
-        }
-        bytes += bytes_read + 8 + 12ull * lm + 16ull * m;
-        __syncwarp();
-        // sort movers by rank: each key's position is the number of smaller keys (keys are unique)
-        u64 mine[CC_MOV / 32];
-        u32 posv[CC_MOV / 32];
-        for (u32 i = 0; i < CC_MOV / 32; ++i) mine[i] = (lane + 32 * i < m) ? mvs[w][lane + 32 * i] : ~0ull;
-        for (u32 i = 0; i < CC_MOV / 32; ++i) {
-            posv[i] = 0;
-            if (lane + 32 * i >= m) continue;
-            for (u32 j = 0; j < m; ++j) posv[i] += mvs[w][j] < mine[i];
-        }
-        __syncwarp();
-        for (u32 i = 0; i < CC_MOV / 32; ++i)
-            if (lane + 32 * i < m) mvs[w][posv[i]] = mine[i];
-        // table of partition counts from the census, then the movers' slots; direct tables leave
-        // tk to the sweep's lane masks (2K <= CC_TAB words, zeroed)
-        for (u32 i = lane; i < cap; i += 32) { tc[w][i] = 0; td[w][i] = 0; }
-        const u32 ntk = direct ? 2 * A.K : cap;
-        for (u32 i = lane; i < ntk; i += 32) tk[w][i] = direct ? 0u : NONE;
-        __syncwarp();
-        cascade_fill(A, h, a, b, lm, tk[w], tc[w], td[w], cap, direct, lane, 32);
-        __syncwarp();
-        cascade_slots(A, h, mvs[w], sl[w], m, tk[w], cap, direct, lane, 32);
-        __syncwarp();
-        cascade_sweep_warp(A, h, mvs[w], sl[w], m, tk[w], tc[w], td[w], direct ? tk[w] : nullptr);
+// Long hyperedges with at most MV movers, one warp each: the gather, the order by rank and the sweep
+// are chains of dependent loads, so what counts is the hyperedges in flight, and a warp needs no
+// block barrier between its phases. Everything a mover needs is loaded in the gather.
+//  - DIRECT (partitions of one copy up to CC_DIRECT_BLOCK_K): a counter word per partition (pins
+//    below, destination pins above), counted from the pins themselves;
+//  - hashed: only the movers' sources and targets are keys (at most 2 MV of them, 4 MV slots), and the
+//    hyperedge's census entries fill in the counts of those.
+// Hyperedges with more movers, or too many pins for 16-bit counts, go on to the block kernel.
+constexpr u32 CL_WARPS = 4;
+constexpr u32 CL_BINS = 256;
+constexpr u32 CL_MAX_LEN = 65535;
+// Bytes of one warp's shared memory.
+__host__ __device__ __forceinline__ u32 cl_bytes(bool direct, u32 K, u32 MV) {
+    const u32 common = MV * 8 + MV * 4 + 2 * MV * 2 + CL_BINS * 4 + 16;
+    return (common + (direct ? 3 * K * 4 : MV * 4 + 4 * MV * 8) + 15) & ~15u;
+}
+
+// Places of the m movers by rank (the high word of mv): ord[i] is the index of the i-th. Ranks spread
+// over CL_BINS bins by their leading bits; a mover's place in its bin is the number of smaller ranks.
+__device__ __forceinline__ void warp_rank_order(const u64 *mv, u32 m, u32 rmax, u32 *bins, unsigned short *idx,
+                                                unsigned short *ord) {
+    const u32 lane = threadIdx.x & 31u;
+    const u32 nb = 32 - __clz(rmax), sh = nb > 8 ? nb - 8 : 0;
+    static_assert(CL_BINS == 256, "eight leading bits");
+    for (u32 i = lane; i < CL_BINS; i += 32) bins[i] = 0;
+    __syncwarp();
+    // arrival places are kept in ord until the movers are listed by bin in idx
+    for (u32 i = lane; i < m; i += 32) ord[i] = (unsigned short)atomicAdd(&bins[(u32)(mv[i] >> 32) >> sh], 1u);
+    __syncwarp();
+    u32 c[8], s = 0;
+#pragma unroll
+    for (u32 k = 0; k < 8; ++k) { c[k] = bins[lane * 8 + k]; s += c[k]; }
+    u32 x = s;
+#pragma unroll
+    for (u32 o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
     }
-    if (A.pbytes && lane == 0 && bytes) prof_add(A.pbytes, blockIdx.x * CC_WARPS + w, bytes);
+    u32 pre = x - s;
+#pragma unroll
+    for (u32 k = 0; k < 8; ++k) { bins[lane * 8 + k] = pre; pre += c[k]; }
+    if (lane == 31) bins[CL_BINS] = m;
+    __syncwarp();
+    for (u32 i = lane; i < m; i += 32) idx[bins[(u32)(mv[i] >> 32) >> sh] + ord[i]] = (unsigned short)i;
+    __syncwarp();
+    for (u32 i0 = 0; i0 < m; i0 += 32) {
+        const u32 i = i0 + lane;
+        u32 p = 0;
+        if (i < m) {
+            const u64 key = mv[i];
+            const u32 b = (u32)(key >> 32) >> sh, lo = bins[b], hi = bins[b + 1];
+            p = lo;
+            for (u32 j = lo; j < hi; ++j) p += mv[idx[j]] < key;
+        }
+        __syncwarp();
+        if (i < m) ord[p] = (unsigned short)i;  // arrival places are no longer read
+    }
+    __syncwarp();
+}
+
+template <bool DIRECT>
+__global__ void __launch_bounds__(CL_WARPS * 32) k_cascade_long(CascadeArgs A, const u32 *__restrict__ list,
+                                                               const u32 *__restrict__ nlist, u32 MV, u32 per,
+                                                               u32 *__restrict__ big, u32 *__restrict__ nbig) {
+    extern __shared__ __align__(16) unsigned char cl_smem[];
+    const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, nl = *nlist;
+    u64 *mv = (u64 *)(cl_smem + w * per);
+    u32 *sl = (u32 *)(mv + MV);
+    unsigned short *idx = (unsigned short *)(sl + MV), *ord = idx + MV;
+    u32 *bins = (u32 *)(ord + MV), *rest = bins + CL_BINS + 4;
+    u32 *tc = rest, *pm = tc + A.K, *qm = pm + A.K;                     // DIRECT
+    u32 *sq = rest, *keys = sq + MV, *hc = keys + 4 * MV;               // hashed
+    if (DIRECT)
+        for (u32 i = lane; i < 2 * A.K; i += 32) pm[i] = 0;
+    for (u32 li = blockIdx.x * CL_WARPS + w; li < nl; li += gridDim.x * CL_WARPS) {
+        __syncwarp();  // the previous hyperedge's shared state is no longer read
+        const u32 h = list[li];
+        const u64 a = A.off[h], len64 = A.off[h + 1] - a;
+        const u32 len = len64 <= CL_MAX_LEN ? (u32)len64 : 0u, ns = A.nsrc[h], base = cascade_base(A, h);
+        if (DIRECT)
+            for (u32 i = lane; i < A.K; i += 32) tc[i] = 0;
+        __syncwarp();
+        u32 m = 0, rmax = 0;
+        constexpr u32 U = 4;
+        for (u32 k0 = 0; k0 < len; k0 += 32 * U) {
+            u32 v[U], q[U];
+            uint2 st[U];
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) v[x] = k0 + 32 * x + lane < len ? A.pins[a + k0 + 32 * x + lane] : NONE;
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) st[x] = v[x] != NONE ? A.state[v[x]] : make_uint2(NONE, 0);
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) q[x] = st[x].x != NONE ? A.target[v[x]] : 0;
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) {
+                const bool in = v[x] != NONE, dst = in && k0 + 32 * x + lane >= ns, mover = st[x].x != NONE;
+                if (DIRECT && in) atomicAdd(&tc[st[x].y - base], dst ? 0x10001u : 1u);
+                const u32 bal = __ballot_sync(0xFFFFFFFFu, mover);
+                const u32 at = m + __popc(bal & lt);
+                if (mover && at < MV) {
+                    mv[at] = ((u64)st[x].x << 32) | (dst ? MV_DST : 0u) | v[x];
+                    if (DIRECT) {
+                        sl[at] = (st[x].y - base) | (q[x] - base) << 16;
+                    } else {
+                        sl[at] = st[x].y;
+                        sq[at] = q[x];
+                    }
+                    rmax = st[x].x > rmax ? st[x].x : rmax;
+                }
+                m += __popc(bal);
+            }
+        }
+        if (m > MV || len64 > CL_MAX_LEN) {
+            if (lane == 0) big[atomicAdd(nbig, 1u)] = h;
+            continue;
+        }
+        if (m == 0) continue;
+        rmax = __reduce_max_sync(0xFFFFFFFFu, rmax);
+        u32 cap = 32;
+        if (!DIRECT) {
+            while (cap < 4 * m) cap <<= 1;  // at most 4 * MV
+            for (u32 i = lane; i < cap; i += 32) { keys[i] = NONE; hc[i] = 0; }
+        }
+        __syncwarp();
+        if (!DIRECT) {
+            for (u32 i = lane; i < m; i += 32) {
+                const u32 sp = hash_find_or_insert(keys, cap - 1, sl[i]), st = hash_find_or_insert(keys, cap - 1, sq[i]);
+                if (sp == NONE || st == NONE) atomicExch(A.status, DEV_HASH_FULL);
+                sl[i] = (sp & 0xFFFFu) | st << 16;
+            }
+            __syncwarp();
+            const u32 lm = A.lam[h];
+            for (u32 j = lane; j < lm; j += 32) {  // each partition once
+                const u32 s = hash_find(keys, cap - 1, A.cpart[a + j]);
+                if (s != NONE) hc[s] = A.ccnt[a + j] | A.cdcnt[a + j] << 16;
+            }
+        }
+        warp_rank_order(mv, m, rmax, bins, idx, ord);
+        // the sweep, 32 movers at a time (cascade_sweep_warp)
+        u32 *cnt = DIRECT ? tc : hc;
+        const u32 wh = A.wfx[h];
+        for (u32 b0 = 0; b0 < m; b0 += 32) {
+            const bool act = b0 + lane < m;
+            const u32 i = act ? ord[b0 + lane] : 0;
+            const u64 e = act ? mv[i] : 0;
+            const u32 pq = sl[i];
+            const u32 sp = act ? pq & 0xFFFFu : 0x10000u + lane, sqx = act ? pq >> 16 : 0x20000u + lane;
+            const bool dst = act && ((u32)e & MV_DST);
+            const u32 dmask = __ballot_sync(0xFFFFFFFFu, dst);
+            u32 m_pp, m_qq, m_qp = 0, m_pq = 0;  // lanes with my source / my target as source / target
+            if (DIRECT) {
+                if (act) {
+                    atomicOr(&pm[sp], 1u << lane);
+                    atomicOr(&qm[sqx], 1u << lane);
+                }
+                __syncwarp();
+                m_pp = act ? pm[sp] : 0u;
+                m_qq = act ? qm[sqx] : 0u;
+                m_qp = act ? qm[sp] : 0u;
+                m_pq = act ? pm[sqx] : 0u;
+                __syncwarp();
+                if (act) {
+                    pm[sp] = 0;
+                    qm[sqx] = 0;
+                }
+            } else {
+                m_pp = __match_any_sync(0xFFFFFFFFu, sp);
+                m_qq = __match_any_sync(0xFFFFFFFFu, sqx);
+#pragma unroll 8
+                for (u32 j = 0; j < 32; ++j) {
+                    const u32 spj = __shfl_sync(0xFFFFFFFFu, sp, j), sqj = __shfl_sync(0xFFFFFFFFu, sqx, j);
+                    m_qp |= (u32)(sqj == sp) << j;
+                    m_pq |= (u32)(spj == sqx) << j;
+                }
+            }
+            const u32 cP = act ? cnt[sp] : 0, cQ = act ? cnt[sqx] : 0;
+            if (act) {
+                const u32 cp = (u32)((int)(cP & 0xFFFFu) + __popc(m_qp & lt) - __popc(m_pp & lt));
+                const u32 cq = (u32)((int)(cQ & 0xFFFFu) + __popc(m_qq & lt) - __popc(m_pq & lt));
+                const i64 d = leave_gain(A.encourage, wh, cp) - (cq == 0 ? (i64)wh : 0);
+                if (d) atomicAdd(&A.g2[(u32)e & ~MV_DST], (unsigned long long)d);
+            }
+            if (A.track) {  // warp-uniform
+                bool ep = false, eq = false;
+                if (dst) {
+                    ep = (int)(cP >> 16) + __popc(m_qp & lt & dmask) - __popc(m_pp & lt & dmask) == 1;
+                    eq = (int)(cQ >> 16) + __popc(m_qq & lt & dmask) - __popc(m_pq & lt & dmask) == 0;
+                }
+                const u32 r = (u32)(e >> 32);
+                const u32 pid = DIRECT ? sp + base : ep ? keys[sp] : 0, qid = DIRECT ? sqx + base : eq ? keys[sqx] : 0;
+                __syncwarp();
+                emit_pair(A, ep, pid, eq, qid, r);
+            }
+            __syncwarp();
+            if (act) {  // counts stay within their halves once the whole chunk is in
+                const u32 one = dst ? 0x10001u : 1u;
+                atomicSub(&cnt[sp], one);
+                atomicAdd(&cnt[sqx], one);
+            }
+            __syncwarp();
+        }
+    }
 }
 
 // Block-wide bitonic sort of buf[0, P) ascending (P a power of two).
@@ -4193,6 +4329,10 @@ void setup_refine_kernels(Ctx &c) {
     AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true, GN_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * GN_BLOCK_W * 16));
+    AXC_CUDA(cudaFuncSetAttribute(k_cascade_long<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(CL_WARPS * cl_bytes(true, CC_DIRECT_BLOCK_K, 512))));
+    AXC_CUDA(cudaFuncSetAttribute(k_cascade_long<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(CL_WARPS * cl_bytes(false, 0, 256))));
     AXC_CUDA(cudaFuncSetAttribute(k_cascade_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CB_DYN_MAX));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_sample<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_DIRECT_UNI * 4));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_sample<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_TAB * 8));
@@ -4933,7 +5073,6 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         C.K = kw ? kw->k : rp.K;
         C.ce = kw ? kw->ce : 0;
         C.cn = slots ? kw->cn : 0;
-        C.pbytes = c.profiling("k_cascade_warp") ? c.d_prof_bytes() : nullptr;
         const bool direct = C.K <= CC_DIRECT_BLOCK_K;
         size_t m1 = c.arena.mark();
         const bool longs = lp.max_len > CM_LEN;
@@ -4955,10 +5094,20 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
             AXC_CUDA(cudaMemcpyAsync(mark, lp.hclass, L.e, cudaMemcpyDeviceToDevice, c.stream));
             LAUNCH(c, k_mover_hedges, (u32)c.sms * 8, 256, 0, C, V, mark);
             LAUNCH(c, k_long_list, cdiv(lp.n_hlong, 256), 256, 0, V, lp.hlong, lp.n_hlong, mark, hlist, dHl);
-            int per_w = 1;
-            AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_w, k_cascade_warp, CC_WARPS * 32, 0));
-            const u32 gw = std::min<u32>(cdiv(L.e, CC_WARPS), (u32)c.sms * (u32)std::max(per_w, 1));
-            LAUNCH(c, k_cascade_warp, gw, CC_WARPS * 32, 0, C, hlist, dHl, big, dBig);
+            // a warp per hyperedge: as many movers as 512 (hashed 256) leave room for
+            u32 mvs = 64;
+            while (mvs < (direct ? 512u : 256u) && mvs < lp.max_len) mvs <<= 1;
+            mvs = std::min(mvs, cascade_block_movers(c));
+            const u32 per = cl_bytes(direct, C.K, mvs);
+            const auto lng = [&](auto kernel) {
+                int per_w = 1;
+                AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_w, kernel, CL_WARPS * 32, CL_WARPS * per));
+                LAUNCH_AS(c, "k_cascade_long", kernel,
+                          std::min<u32>(cdiv(lp.n_hlong, CL_WARPS), (u32)c.sms * (u32)std::max(per_w, 1)), CL_WARPS * 32,
+                          CL_WARPS * per, C, hlist, dHl, mvs, per, big, dBig);
+            };
+            if (direct) lng(k_cascade_long<true>);
+            else lng(k_cascade_long<false>);
             // block kernel: shared memory sized by the level's largest hyperedge, all resident blocks
             u32 smov = 128;
             while (smov < lp.max_len && smov < cascade_block_movers(c)) smov <<= 1;
