@@ -739,7 +739,9 @@ void radix_sort_pairs_dn(Ctx &c, u32 *keys, u32 *vals, const u32 *d_n, u64 n, u3
         return;
     }
     const size_t m = c.arena.mark();
-    const u32 tile = RS_WARPS * 32 * (n <= RS_SMALL_N ? RS_ITEMS_SMALL : RS_ITEMS_LARGE);
+    // a count in device memory is usually a fraction of its capacity
+    const bool few = n <= (d_n ? 8 * RS_SMALL_N : RS_SMALL_N);
+    const u32 tile = RS_WARPS * 32 * (few ? RS_ITEMS_SMALL : RS_ITEMS_LARGE);
     const u64 tiles = (n + tile - 1) / tile;
     SortState S{keys, vals, c.arena.alloc<u32>(n), c.arena.alloc<u32>(n), n, d_n, (u32)RSS_CAP, (bits + 7) / 8};
     const bool wide = n >= (1ull << 30);
@@ -758,7 +760,7 @@ void radix_sort_pairs_dn(Ctx &c, u32 *keys, u32 *vals, const u32 *d_n, u64 n, u3
             LAUNCH_AS(c, "k_rs_pass", kernel, grid, RS_WARPS * 32, (size_t)tile * 8, S, p, c.d_status);
         };
         if (wide) pass(k_rs_pass<unsigned long long, RS_ITEMS_LARGE>);
-        else if (n <= RS_SMALL_N) pass(k_rs_pass<u32, RS_ITEMS_SMALL>);
+        else if (few) pass(k_rs_pass<u32, RS_ITEMS_SMALL>);
         else pass(k_rs_pass<u32, RS_ITEMS_LARGE>);
     }
     LAUNCH(c, k_rs_home, std::min<u32>(cdiv(n, 256), (u32)c.sms * 8), 256, 0, S);
