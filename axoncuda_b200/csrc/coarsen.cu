@@ -86,12 +86,41 @@ struct RateArgs {
 // node ids, a present one is never zero in both words (RT_SEEN marks a zero contribution).
 enum RateMode { RT_PLAIN, RT_COUNT, RT_DIRECT };
 constexpr u32 RT_SEEN = 0x80000000u;
+constexpr u32 RT_LONG = 16;  // mean rated pins per incidence from which a batch is read hyperedge by hyperedge
 template <bool CM, RateMode MODE>
 __device__ void rate_flat(const RateArgs &A, u32 u, u32 *keys, u32 *sc, u32 *cm, u32 mask, u32 first,
                           u32 stride, u32 *ndist = nullptr, u32 limit = 0, u32 *used = nullptr) {
     const u32 lane = threadIdx.x & 31u;
     const u64 t0 = A.toff[u];
     const u32 deg = (u32)(A.toff[u + 1] - t0), nin_u = A.nin[u];
+    // pin v of a hyperedge of contribution cc; inb: it shares an inbound hyperedge with u
+    const auto put = [&](u32 v, u32 cc, bool inb) {
+            if (v == u) return;
+            u32 slot;
+            if (MODE == RT_DIRECT) {
+                slot = v;
+            } else if (MODE == RT_COUNT) {  // counted keys; `used` lists them
+                if (*(volatile u32 *)ndist > limit) return;
+                bool fresh = false;
+                slot = hash_insert_fresh(keys, mask, v, fresh);
+                if (slot == NONE) {  // full: a first try overflows, a sized table is an error
+                    if (used) atomicExch(A.status, DEV_HASH_FULL);
+                    else atomicExch(ndist, limit + 1);
+                    return;
+                }
+                if (fresh) {
+                    const u32 idx = atomicAdd(ndist, 1u);
+                    if (used) used[idx] = slot;
+                    if (idx + 1 > limit) return;
+                }
+            } else {
+                slot = hash_find_or_insert(keys, mask, v);
+                if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); return; }
+            }
+            if (MODE == RT_DIRECT && cc == 0) atomicOr(CM ? &cm[slot] : &cm[slot >> 5], CM ? RT_SEEN : 1u << (slot & 31u));
+            else atomicAdd(&sc[slot], cc);
+            if (CM && inb) atomicAdd(&cm[slot], 1u);
+    };
     for (u32 jb = first; jb < deg; jb += stride) {
         if (MODE == RT_COUNT && __any_sync(0xFFFFFFFFu, *(volatile u32 *)ndist > limit)) return;
         const u32 j = jb + lane;
@@ -110,6 +139,21 @@ __device__ void rate_flat(const RateArgs &A, u32 u, u32 *keys, u32 *sc, u32 *cm,
         }
         const u32 total = __shfl_sync(0xFFFFFFFFu, x, 31), excl = x - len;
         const u32 chunk = (deg - jb) < 32 ? (deg - jb) : 32;
+        if (total >= 32 * RT_LONG) {  // long hyperedges: the warp reads one at a time, no search
+            for (u32 t = 0; t < chunk; ++t) {
+                const u64 ao = __shfl_sync(0xFFFFFFFFu, a, t);
+                const u32 lt = __shfl_sync(0xFFFFFFFFu, len, t), cc = __shfl_sync(0xFFFFFFFFu, c, t);
+                const u32 ss = __shfl_sync(0xFFFFFFFFu, s_end, t), ib = __shfl_sync(0xFFFFFFFFu, inb, t);
+                constexpr u32 U = AXC_RATE_MAX_LEN / 32;
+                u32 v[U];
+#pragma unroll
+                for (u32 x = 0; x < U; ++x) v[x] = lane + 32 * x < lt ? A.pins[ao + lane + 32 * x] : u;
+#pragma unroll
+                for (u32 x = 0; x < U; ++x)
+                    if (lane + 32 * x < lt) put(v[x], cc, ib && lane + 32 * x >= ss);
+            }
+            continue;
+        }
         for (u32 fb = 0; fb < total; fb += 32) {
             const u32 f = fb + lane;
             u32 lo = 0, hi = chunk - 1;  // owner: largest o < chunk with excl_o <= f
@@ -125,32 +169,7 @@ __device__ void rate_flat(const RateArgs &A, u32 u, u32 *keys, u32 *sc, u32 *cm,
             const u32 eo = __shfl_sync(0xFFFFFFFFu, excl, lo);
             if (f >= total) continue;
             const u32 i = f - eo;  // position inside the owner hyperedge
-            const u32 v = A.pins[ao + i];
-            if (v == u) continue;
-            u32 slot;
-            if (MODE == RT_DIRECT) {
-                slot = v;
-            } else if (MODE == RT_COUNT) {  // counted keys; `used` lists them
-                if (*(volatile u32 *)ndist > limit) continue;
-                bool fresh = false;
-                slot = hash_insert_fresh(keys, mask, v, fresh);
-                if (slot == NONE) {  // full: a first try overflows, a sized table is an error
-                    if (used) atomicExch(A.status, DEV_HASH_FULL);
-                    else atomicExch(ndist, limit + 1);
-                    continue;
-                }
-                if (fresh) {
-                    const u32 idx = atomicAdd(ndist, 1u);
-                    if (used) used[idx] = slot;
-                    if (idx + 1 > limit) continue;
-                }
-            } else {
-                slot = hash_find_or_insert(keys, mask, v);
-                if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); continue; }
-            }
-            if (MODE == RT_DIRECT && cc == 0) atomicOr(&cm[slot], RT_SEEN);
-            else atomicAdd(&sc[slot], cc);
-            if (CM && ib && i >= ss) atomicAdd(&cm[slot], 1u);
+            put(A.pins[ao + i], cc, ib && i >= ss);
         }
     }
 }
@@ -196,7 +215,7 @@ __device__ __forceinline__ void top_collect(const RateArgs &A, u32 u, const u32 
             if (v == NONE) continue;
             if (CM) y = cm[s];
         } else {
-            y = cm[s];
+            y = CM ? cm[s] : (cm[s >> 5] >> (s & 31u)) & 1u;
             if (!(x | y)) continue;
             y &= ~RT_SEEN;
         }
@@ -375,9 +394,11 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rate_block(RateArgs A, const u32 *
 }
 
 // The same with scores indexed by node id in shared memory, for levels of at most RT_DIRECT_N nodes:
-// no probing, no retries, whatever the node's distinct neighbours. sc and cm hold n words each (cm
-// only marks zero contributions without CM).
-constexpr u32 RT_DIRECT_N = 8192;
+// no probing, no retries, whatever the node's distinct neighbours. sc holds n words, cm as many, or
+// without CM a bit per node that marks zero contributions: 64 KB at most, three blocks per SM.
+template <bool CM>
+constexpr u32 RT_DIRECT_N = CM ? 8192 : 16384;
+__host__ __device__ __forceinline__ u32 rate_direct_words(bool cm, u32 n) { return n + (cm ? n : (n + 31) / 32); }
 template <int TC, bool CM>
 __global__ void __launch_bounds__(RT_BLOCK) k_rate_direct(RateArgs A, const u32 *__restrict__ list, u32 nlist) {
     extern __shared__ u32 dyn[];
@@ -385,7 +406,7 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rate_direct(RateArgs A, const u32 
     u32 *sc = dyn, *cm = dyn + A.n;
     for (u32 idx = blockIdx.x; idx < nlist; idx += gridDim.x) {
         const u32 u = list[idx];
-        for (u32 i = threadIdx.x; i < 2 * A.n; i += RT_BLOCK) dyn[i] = 0;
+        for (u32 i = threadIdx.x; i < rate_direct_words(CM, A.n); i += RT_BLOCK) dyn[i] = 0;
         __syncthreads();
         rate_flat<CM, RT_DIRECT>(A, u, nullptr, sc, cm, 0, 32 * (threadIdx.x >> 5), RT_BLOCK);
         __syncthreads();
@@ -701,10 +722,10 @@ void setup_coarsen_kernels(Ctx &c) {
     smem(k_rate_block<4, true>, 3 * 16384 * 4);
     smem(k_rate_block<TC, false>, 3 * 16384 * 4);
     smem(k_rate_block<TC, true>, 3 * 16384 * 4);
-    smem(k_rate_direct<4, false>, 2 * RT_DIRECT_N * 4);
-    smem(k_rate_direct<4, true>, 2 * RT_DIRECT_N * 4);
-    smem(k_rate_direct<TC, false>, 2 * RT_DIRECT_N * 4);
-    smem(k_rate_direct<TC, true>, 2 * RT_DIRECT_N * 4);
+    smem(k_rate_direct<4, false>, rate_direct_words(false, RT_DIRECT_N<false>) * 4);
+    smem(k_rate_direct<4, true>, rate_direct_words(true, RT_DIRECT_N<true>) * 4);
+    smem(k_rate_direct<TC, false>, rate_direct_words(false, RT_DIRECT_N<false>) * 4);
+    smem(k_rate_direct<TC, true>, rate_direct_words(true, RT_DIRECT_N<true>) * 4);
 }
 
 // A rating kernel with per-thread top lists of 4 when cnc <= 4 (the reference scripts' -cnc 4),
@@ -779,12 +800,14 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
     u32 *retry = c.arena.alloc<u32>(n), *retry2 = c.arena.alloc<u32>(n);
     u32 *d_retry = (u32 *)(dc + 4), *d_retry2 = d_retry + 1;  // dc[4] was read already
     const u32 rt_try = c.tune.rate_try, rt_mid = std::max(c.tune.rate_mid, c.tune.rate_try);
+    const bool by_node = n <= (cm ? RT_DIRECT_N<true> : RT_DIRECT_N<false>);
     const auto direct_tier = [&](const u32 *lst, u32 cnt) {
-        RATE_LAUNCH(c, k_rate_direct, cnc, cm, std::min<u32>(cnt, (u32)c.sms * 8), RT_BLOCK, (size_t)2 * n * 4, A, lst, cnt);
+        RATE_LAUNCH(c, k_rate_direct, cnc, cm, std::min<u32>(cnt, (u32)c.sms * 8), RT_BLOCK,
+                    (size_t)rate_direct_words(cm, n) * 4, A, lst, cnt);
     };
     auto block_tier = [&](const u32 *lst, u32 cnt, u32 cap_full) {
         if (!cnt) return;
-        if (n <= RT_DIRECT_N && cap_full > rt_try) {
+        if (by_node && cap_full > rt_try) {
             direct_tier(lst, cnt);
             return;
         }
@@ -828,7 +851,7 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
             if (cm) LAUNCH_AS(c, "k_rate_split_acc", k_rate_split_acc<true>, nl * splits, RT_BLOCK, 0, A, list4, nl, cap, splits, gtab);
             else LAUNCH_AS(c, "k_rate_split_acc", k_rate_split_acc<false>, nl * splits, RT_BLOCK, 0, A, list4, nl, cap, splits, gtab);
             RATE_LAUNCH(c, k_rate_split_select, cnc, cm, nl, RT_BLOCK, 0, A, list4, nl, cap, gtab);
-        } else if (n <= RT_DIRECT_N) {
+        } else if (by_node) {
             direct_tier(list4, nl);
         } else {
             u32 grid = nl < (u32)c.sms * 2 ? nl : (u32)c.sms * 2;
