@@ -761,8 +761,9 @@ __host__ __device__ __forceinline__ u32 table_cap(u64 work, u32 cap_max) {
 // `stride` entries. A batch's hyperedge metadata loads in parallel; its census entries are then
 // flattened across the lanes (each lane finds its entry's hyperedge by a 5-step search over the
 // prefix of the batch's lambdas). saving and wtot are per-lane partial sums.
-__device__ __forceinline__ void gain_flat(const GainArgs &A, u32 u, u32 p, u32 *keys, unsigned long long *conn,
-                                          u32 *dconn, u32 mask, u32 first, u32 stride, i64 &saving, i64 &wtot) {
+template <bool WIDE>
+__device__ __forceinline__ void gain_flat(const GainArgs &A, u32 u, u32 p, u32 *keys, u32 *conn, u32 *high, u32 *dconn,
+                                          u32 mask, u32 first, u32 stride, i64 &saving, i64 &wtot) {
     const u32 lane = threadIdx.x & 31u;
     const u64 t0 = A.toff[u];
     const u32 deg = (u32)(A.toff[u + 1] - t0), nin_u = A.nin[u];
@@ -804,7 +805,8 @@ __device__ __forceinline__ void gain_flat(const GainArgs &A, u32 u, u32 p, u32 *
             }
             const u32 slot = hash_find_or_insert(keys, mask, q);
             if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); continue; }
-            atomicAdd(&conn[slot], (unsigned long long)wo);
+            const u32 old = atomicAdd(&conn[slot], wo);
+            if (WIDE && old + wo < old) atomicAdd(&high[slot], 1u);
             if (io && A.cdcnt[k] > 0) atomicAdd(&dconn[slot], 1u);
         }
     }
@@ -1065,84 +1067,42 @@ __global__ void __launch_bounds__(GN_BLOCK) k_gain_mask_block(GainArgs A0, const
     }
 }
 
+// WIDE: some node's incident weights pass 2^32, and a connectivity is a low and a high word (64-bit
+// shared adds would be compare-and-swap loops).
+template <bool WIDE>
 __global__ void __launch_bounds__(GN_WARPS * 32) k_gain_warp(GainArgs A0, const u32 *__restrict__ list, u32 nl,
                                                              const u64 *__restrict__ work) {
     const GainArgs A = gain_args_now(A0);
-    __shared__ u32 tk[GN_WARPS][2 * GN_WARP_W], td[GN_WARPS][2 * GN_WARP_W];
-    __shared__ unsigned long long tcw[GN_WARPS][2 * GN_WARP_W];
+    __shared__ u32 tk[GN_WARPS][2 * GN_WARP_W], td[GN_WARPS][2 * GN_WARP_W], tl[GN_WARPS][2 * GN_WARP_W],
+        th[WIDE ? GN_WARPS : 1][WIDE ? 2 * GN_WARP_W : 1];
     const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const u32 idx = blockIdx.x * GN_WARPS + w;
     if (idx >= nl) return;
     const u32 u = list[idx], p = A.part[u];
-    u32 *keys = tk[w], *dconn = td[w];
-    unsigned long long *conn = tcw[w];
+    u32 *keys = tk[w], *dconn = td[w], *lo = tl[w], *hi = th[WIDE ? w : 0];
     const u32 cap = gain_cap(work[u], 2 * GN_WARP_W);
-    for (u32 i = lane; i < cap; i += 32) { keys[i] = NONE; dconn[i] = 0; conn[i] = 0; }
+    for (u32 i = lane; i < cap; i += 32) {
+        keys[i] = NONE;
+        dconn[i] = 0;
+        lo[i] = 0;
+        if (WIDE) hi[i] = 0;
+    }
     __syncwarp();
     i64 saving = 0, wtot = 0;
-    gain_flat(A, u, p, keys, conn, dconn, cap - 1, 0, 32, saving, wtot);
+    gain_flat<WIDE>(A, u, p, keys, lo, hi, dconn, cap - 1, 0, 32, saving, wtot);
     saving = warp_sum(saving);
     wtot = warp_sum(wtot);
     __syncwarp();
     Cand best{INT64_MIN, 0};
     for (u32 i = lane; i < cap; i += 32) {
         if (keys[i] == NONE) continue;
-        Cand c = gain_candidate(A, u, keys[i], conn[i], dconn[i], saving, wtot);
+        const u64 conn = WIDE ? ((u64)hi[i] << 32) | lo[i] : (u64)lo[i];
+        if (saving - (wtot - (i64)conn) <= 0) continue;  // no move
+        const Cand c = gain_candidate(A, u, keys[i], conn, dconn[i], saving, wtot);
         if (cand_better(c, best)) best = c;
     }
     best = warp_best(best);
-    if (lane == 0) {
-        if (best.g != INT64_MIN && best.g > 0) {
-            A.target[u] = ~(u32)best.tie;
-            A.gain[u] = best.g;
-        } else {
-            A.target[u] = NONE;
-            A.gain[u] = 0;
-        }
-    }
-}
-
-// One block per node, for nodes of the block tier when K > GS_K: a shared table sized by the node's
-// bound.
-__global__ void __launch_bounds__(GN_BLOCK) k_gain_block(GainArgs A0, const u32 *__restrict__ list, u32 nl, u32 cap_max,
-                                                        const u64 *__restrict__ work) {
-    const GainArgs A = gain_args_now(A0);
-    extern __shared__ unsigned long long dyn64[];
-    __shared__ i64 red[2][32];
-    __shared__ Cand cred[32];
-    for (u32 idx = blockIdx.x; idx < nl; idx += gridDim.x) {
-        const u32 u = list[idx], p = A.part[u];
-        const u32 cap = gain_cap(work[u], cap_max);
-        unsigned long long *conn = dyn64;
-        u32 *keys = (u32 *)(dyn64 + cap), *dconn = keys + cap;
-        for (u32 i = threadIdx.x; i < cap; i += blockDim.x) { keys[i] = NONE; dconn[i] = 0; conn[i] = 0; }
-        __syncthreads();
-        i64 saving = 0, wtot = 0;
-        gain_flat(A, u, p, keys, conn, dconn, cap - 1, 32 * (threadIdx.x >> 5), blockDim.x, saving, wtot);
-        saving = warp_sum(saving);
-        wtot = warp_sum(wtot);
-        if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = saving; red[1][threadIdx.x >> 5] = wtot; }
-        __syncthreads();
-        saving = 0;
-        wtot = 0;
-        for (u32 i = 0; i < blockDim.x / 32; ++i) { saving += red[0][i]; wtot += red[1][i]; }
-        Cand best{INT64_MIN, 0};
-        for (u32 i = threadIdx.x; i < cap; i += blockDim.x) {
-            if (keys[i] == NONE) continue;
-            const Cand c = gain_candidate(A, u, keys[i], conn[i], dconn[i], saving, wtot);
-            if (cand_better(c, best)) best = c;
-        }
-        best = warp_best(best);
-        if ((threadIdx.x & 31) == 0) cred[threadIdx.x >> 5] = best;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            Cand b = cred[0];
-            for (u32 i = 1; i < blockDim.x / 32; ++i)
-                if (cand_better(cred[i], b)) b = cred[i];
-            write_move(A, u, b);
-        }
-        __syncthreads();
-    }
+    if (lane == 0) write_move(A, u, best);
 }
 
 // ------------------------------------------------------------------ sampled gains (K > AXC_SPARSE_GAIN_K)
@@ -1297,7 +1257,7 @@ __global__ void __launch_bounds__(NT) k_gain_table(GainArgs A0, const u32 *__res
         Cand best{INT64_MIN, 0};
         for (u32 q = threadIdx.x; q < A.K; q += NT) {
             const u64 conn = WIDE ? ((u64)hi[q] << 32) | lo[q] : (u64)lo[q];
-            if (conn == 0) continue;  // absent, or never a positive gain
+            if (saving - (wtot - (i64)conn) <= 0) continue;  // absent, or no move
             const Cand c = gain_candidate(A, u, q, conn, dconn[q], saving, wtot);
             if (cand_better(c, best)) best = c;
         }
@@ -1409,41 +1369,55 @@ __global__ void __launch_bounds__(GN_BLOCK) k_gain_planes(GainArgs A0, const u32
         // planes that can be set: the bits of the most incidences one counter sees
         u32 nb = 32 - __clz((deg + S - 1) / S * (MWP < 32 ? 32 / MWP : 1));
         nb = nb < GP_PLANES ? nb : GP_PLANES;
-#pragma unroll 1
-        for (u32 pass = 0; pass < 2; ++pass) {
+        const auto count = [&](u32 jend, const u32 *m, u32 (&out)[GP_PLANES][ROWS * MWP]) {
             u32 pl[GP_PLANES];
-            plane_count(A.touch + t0, pass ? nin : deg, pass ? dmask : mask, MW, MW, wl, slot, S, pl);
+            plane_count<GP_PLANES>(A.touch + t0, jend, m, MW, MW, wl, slot, S, pl);
             if (MWP < 32)
 #pragma unroll
-                for (u32 o = 16; o >= MWP; o >>= 1) plane_merge(pl, o);
+                for (u32 o = 16; o >= MWP; o >>= 1) plane_merge<GP_PLANES>(pl, o);
             const u32 row = MWP < 32 ? warp * MWP + wl : threadIdx.x;
             if (MWP >= 32 || lane < MWP)
 #pragma unroll
                 for (u32 b = 0; b < GP_PLANES; ++b)
-                    if (b < nb) (pass ? pd : pc)[b][row] = pl[b];
-        }
-        __syncthreads();
-        const i64 saving = A.save[u], wtot = (i64)((u64)deg * w);
-        Cand best{INT64_MIN, 0};
-        for (u32 q = threadIdx.x; q < A.K; q += GN_BLOCK) {
+                    if (b < nb) out[b][row] = pl[b];
+        };
+        const auto total = [&](const u32 (&in)[GP_PLANES][ROWS * MWP], u32 q) {
             const u32 wd = q >> 5, sh = q & 31u;
             u32 cnt = 0;
             for (u32 b = 0; b < nb; ++b) {
                 u32 c = 0;
 #pragma unroll
-                for (u32 r = 0; r < ROWS; ++r) c += (pc[b][r * MWP + wd] >> sh) & 1u;
+                for (u32 r = 0; r < ROWS; ++r) c += (in[b][r * MWP + wd] >> sh) & 1u;
                 cnt += c << b;
             }
-            if (cnt == 0 || q == p) continue;
-            u32 dc = 0;
-            for (u32 b = 0; b < nb; ++b) {
-                u32 c = 0;
-#pragma unroll
-                for (u32 r = 0; r < ROWS; ++r) c += (pd[b][r * MWP + wd] >> sh) & 1u;
-                dc += c << b;
+            return cnt;
+        };
+        count(deg, mask, pc);
+        __syncthreads();
+        // A partition whose connectivity does not outweigh what the node pays, or that has no room, is
+        // no target whatever its inbound count: the destination planes are counted only where some
+        // partition is left (bit k of pos: this thread's k-th), which late rounds rarely have.
+        const i64 saving = A.save[u], wtot = (i64)((u64)deg * w);
+        const u64 s = A.nsize[u], need = s - s / A.discount;
+        u32 pos = 0;
+        {
+            u32 k = 0;
+            for (u32 q = threadIdx.x; q < A.K; q += GN_BLOCK, ++k) {
+                const i64 conn = (i64)((u64)total(pc, q) * w);
+                if (q != p && saving - (wtot - conn) > 0 && A.psize[q] + need <= A.omega) pos |= 1u << k;
             }
-            const Cand c = gain_candidate(A, u, q, (u64)cnt * w, dc, saving, wtot);
-            if (cand_better(c, best)) best = c;
+        }
+        static_assert(GS_K / GN_BLOCK <= 32, "a thread's partitions fit its mask");
+        Cand best{INT64_MIN, 0};
+        if (__syncthreads_or(pos)) {
+            count(nin, dmask, pd);
+            __syncthreads();
+            for (u32 k = 0; pos >> k; ++k) {
+                if (!((pos >> k) & 1u)) continue;
+                const u32 q = threadIdx.x + k * GN_BLOCK;
+                const Cand c = gain_candidate(A, u, q, (u64)total(pc, q) * w, total(pd, q), saving, wtot);
+                if (cand_better(c, best)) best = c;
+            }
         }
         best = warp_best(best);
         if (lane == 0) cred[warp] = best;
@@ -4328,7 +4302,6 @@ void setup_refine_kernels(Ctx &c) {
     AXC_CUDA(cudaFuncSetAttribute(k_part_inbound_smem<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PI_SMEM_K * 4));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true, GN_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
-    AXC_CUDA(cudaFuncSetAttribute(k_gain_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * GN_BLOCK_W * 16));
     AXC_CUDA(cudaFuncSetAttribute(k_cascade_long<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(CL_WARPS * cl_bytes(true, CC_DIRECT_BLOCK_K, 512))));
     AXC_CUDA(cudaFuncSetAttribute(k_cascade_long<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -4563,8 +4536,12 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
     }
     fill_u32(c, A.target, NONE, L.n);
     if (c.profiling("k_gain_warp") && lp.ncount[0]) c.prof_bytes += gain_bytes(lp, 0);
-    if (c.profiling("k_gain_block")) c.prof_bytes += gain_bytes(lp, 1) + gain_bytes(lp, 2);
-    LAUNCH(c, k_gain_warp, cdiv(lp.ncount[0], GN_WARPS), GN_WARPS * 32, 0, A, lp.ntier[0], lp.ncount[0], lp.work);
+    if (lp.gain_bound < (1ull << 32))
+        LAUNCH_AS(c, "k_gain_warp", k_gain_warp<false>, cdiv(lp.ncount[0], GN_WARPS), GN_WARPS * 32, 0, A, lp.ntier[0],
+                  lp.ncount[0], lp.work);
+    else
+        LAUNCH_AS(c, "k_gain_warp", k_gain_warp<true>, cdiv(lp.ncount[0], GN_WARPS), GN_WARPS * 32, 0, A, lp.ntier[0],
+                  lp.ncount[0], lp.work);
     if (lp.ncount[1] && plane_gains(L, lp, A.K)) {
         const size_t m = c.arena.mark();
         const u32 MW = (A.K + 31) / 32;
@@ -4595,12 +4572,8 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
         else if (wide) launch(std::true_type(), t256);
         else if (small) launch(std::false_type(), t64);
         else launch(std::false_type(), t256);
-    } else if (lp.ncount[1]) {
-        // shared table sized by the tier's largest bound (16 B per slot)
-        const u32 cap1 = table_cap(lp.block_work_max, 2 * GN_BLOCK_W);
-        LAUNCH(c, k_gain_block, lp.ncount[1], GN_BLOCK, cap1 * 16, A, lp.ntier[1], lp.ncount[1], cap1, lp.work);
     }
-    if (lp.ncount[2] && A.K > GS_K) {  // the sampled rule (include/axc.h AXC_SPARSE_GAIN_*)
+    if (A.K > GS_K && lp.ncount[1] + lp.ncount[2]) {  // the sampled rule (include/axc.h AXC_SPARSE_GAIN_*)
         size_t m = c.arena.mark();
         const u32 rows = lp.ncount[2];
         CandAcc C{c.arena.alloc<u32>((u64)L.n * GS_C), c.arena.alloc<unsigned long long>((u64)L.n * GS_C),
@@ -4614,8 +4587,11 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
             const size_t smem = (size_t)T * 4 * ((U ? 1 : 2) + (D ? 0 : 1));
             int per_sm = 1;
             AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gain_sample<U, D>, GS_BLOCK, smem));
-            LAUNCH_AS(c, "k_gain_sample", (k_gain_sample<U, D>), std::min<u32>(rows, (u32)c.sms * (u32)std::max(per_sm, 1)),
-                      GS_BLOCK, smem, A, lp.ntier[2], rows, C, T, lp.weight, room);
+            // tier 1: nodes whose bound fits the sample are settled exactly
+            for (u32 t = 1; t <= 2; ++t)
+                LAUNCH_AS(c, "k_gain_sample", (k_gain_sample<U, D>),
+                          std::min<u32>(lp.ncount[t], (u32)c.sms * (u32)std::max(per_sm, 1)), GS_BLOCK, smem, A, lp.ntier[t],
+                          lp.ncount[t], C, T, lp.weight, room);
         };
         const std::true_type yes;
         const std::false_type no;
@@ -4642,8 +4618,8 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
                           lp.n_hhuge, mw, gtab, (const u64 *)lp.huge_tab);
             }
         };
-        if (A.K <= CV_BITS_K) exact(yes);
-        else exact(no);
+        if (rows && A.K <= CV_BITS_K) exact(yes);
+        else if (rows) exact(no);
         LAUNCH(c, k_cands_best, cdiv(rows, 256), 256, 0, A, C, lp.ntier[2], rows);
         c.arena.release(m);
     }
@@ -4731,7 +4707,7 @@ static Census census_for_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, con
                                const u32 *part) {
     Census cs = alloc_census(c, L);
     const bool direct = rp.K <= GN_DIRECT_K;
-    if (direct || plane_gains(L, lp, rp.K) || (rp.K > GS_K && lp.ncount[2])) {
+    if (direct || plane_gains(L, lp, rp.K) || (rp.K > GS_K && lp.ncount[1] + lp.ncount[2])) {
         cs.save = c.arena.alloc<i64>(L.n ? L.n : 1);
         AXC_CUDA(cudaMemsetAsync(cs.save, 0, (size_t)L.n * 8, c.stream));
         cs.wfx = wfx;
