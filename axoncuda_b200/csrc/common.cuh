@@ -90,6 +90,8 @@ struct Tune {
     u32 cascade_movers = 0;
 };
 
+constexpr size_t STAGE_BYTES = 4u << 20;
+
 struct Ctx {
     int device = 0;
     Tune tune;
@@ -99,6 +101,8 @@ struct Ctx {
     Arena arena;
     u32 *d_status = nullptr;       // device status word
     u64 *h_pinned = nullptr;       // small pinned staging buffer for scalars (4 KiB)
+    char *h_stage = nullptr;       // pinned staging of large uploads (2 * STAGE_BYTES), made at the first
+    cudaEvent_t stage_free[2] = {nullptr, nullptr};  // a half's last copy has read it
     u32 launches = 0;
     std::string last_error;
     int coop_supported = 0;
