@@ -1122,6 +1122,9 @@ constexpr u32 GS_C = AXC_SPARSE_GAIN_CANDIDATES;
 constexpr u32 GS_TAB = 2 * GS_SAMPLE;  // hashed sample table: at most half full
 constexpr u32 GS_BLOCK = 256;
 constexpr u32 GS_LIST = 256;           // keys the final selection of the candidates looks at
+constexpr u32 GS_HIST = 32;            // equal weights: slots are counted by incidences from GS_BAND up ...
+constexpr u32 GS_BAND = 3;             // (nearly every slot reaches one or two)
+constexpr u32 GS_BAND_MIN = 16;        // ... and looked at in bands of at least so many
 // A slot of the sample table holds a partition's sampled connectivity and inbound count in 32-bit
 // words (64-bit shared adds would be compare-and-swap loops). Equal weights: one word, incidences
 // holding the partition above, inbound ones with a destination pin in it below. Else the low word
@@ -1501,6 +1504,8 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
     // at most GS_BLOCK), census offset and weight
     __shared__ u32 s_ex[GS_BLOCK + 1], s_w[GS_BLOCK];
     __shared__ u64 s_off[GS_BLOCK];
+    __shared__ u32 hist[UNI ? GS_HIST : 1];  // [c]: slots of at least c incidences, c >= GS_BAND
+    if (UNI && threadIdx.x < GS_HIST) hist[threadIdx.x] = 0;
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (u32 i = threadIdx.x; i < T; i += GS_BLOCK) {
         v0[i] = 0;
@@ -1528,6 +1533,7 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
         }
     };
     const auto clear_all = [&]() {
+        if (UNI && threadIdx.x < GS_HIST) hist[threadIdx.x] = 0;
         for (u32 i4 = threadIdx.x; i4 < T / 4; i4 += GS_BLOCK) {
             ((uint4 *)v0)[i4] = make_uint4(0, 0, 0, 0);
             if (!UNI) ((uint4 *)v1)[i4] = make_uint4(0, 0, 0, 0);
@@ -1603,7 +1609,8 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
                 if (slot == NONE) { atomicExch(A.status, DEV_HASH_FULL); return; }
             }
             if (UNI) {
-                atomicAdd(&v0[slot], (1u << GS_HI) | (dst ? 1u : 0u));
+                const u32 cnt = (atomicAdd(&v0[slot], (1u << GS_HI) | (dst ? 1u : 0u)) >> GS_HI) + 1;
+                if (cnt >= GS_BAND && cnt < GS_HIST) atomicAdd(&hist[cnt], 1u);
             } else {
                 const u32 old = atomicAdd(&v0[slot], w);
                 const u32 up = (old + w < old ? 1u << GS_HI : 0u) | (dst ? 1u : 0u);
@@ -1664,55 +1671,86 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
             __syncthreads();
             continue;
         }
-        // 3b. the GS_C best by (sampled connectivity, tie hash, -id) among the keys the size limit and
-        // the inbound bound do not rule out. Pass 1 empties the ruled-out slots and takes the best key
+        // 3b. with equal weights the histogram says where the few dozen best connected slots lie: slots are
+        // looked at in bands of falling counts until GS_C keys stand that the size limit and the inbound
+        // bound do not rule out, so only a band's slots look up their partition's room. A band with more
+        // keys than the list holds, and other weights, take the general selection.
+        const u64 in_sample = m < nin_u ? m : nin_u, need = s - s / A.discount;
+        const auto ruled_out = [&](u32 q, u32 dcon) {
+            const u32 rm = room[q], rs = rm & 0xFFFFu, rb = rm >> 16;
+            if (rs == RM_NONE || rb == RM_NONE || in_sample - dcon > rb) return true;
+            // a clamped room is at least RM_MORE nodes: larger nodes look at the size itself
+            return rs == RM_MORE ? (need > RM_MORE && A.psize[q] + need > A.omega) : need > rs;
+        };
+        u32 nk = GS_LIST + 1;
+        if (threadIdx.x < GS_C) kout[threadIdx.x] = SKey{0, 0};
+        if (UNI && weight) {
+            u32 top = NONE, seen = 0;  // the seen slots of count top and more were looked at
+            do {
+                u32 c = (top < GS_HIST ? top : GS_HIST) - 1;
+                while (c >= GS_BAND && hist[c] < seen + GS_BAND_MIN) --c;
+                seen = c >= GS_BAND ? hist[c] : 0;
+                const u32 x0 = c << GS_HI, x1 = top < GS_HIST ? (top << GS_HI) - 1 : NONE;
+                scan([&](u32 i, u32 x, u32) {
+                    if (x < x0 || x > x1) return;
+                    const u32 q = part_of(i);
+                    if (ruled_out(q, dcon_of(x, 0))) return;
+                    const u32 at = atomicAdd(&nkeys, 1u);
+                    if (at < GS_LIST) klist[at] = key_of(q, conn_of(x, 0));
+                });
+                __syncthreads();
+                nk = nkeys;
+                __syncthreads();  // read before the next band, or the reset below
+                top = c;
+            } while (nk < GS_C && top > 1);
+        }
+        // The general selection: the GS_C best by (sampled connectivity, tie hash, -id) among the keys
+        // that are not ruled out. Pass 1 empties the ruled-out slots and takes the best key
         // of each group of 8 threads; the GS_C-th of those 32 keys is no better than the GS_C-th of
         // all, so pass 2 lists the keys at or above it (a dozen or so), whose ranks are counted
         // pairwise. (The least of the warps' best keys listed hundreds where a warp's slots, a range
         // of partitions, lie away from the node's.)
-        const u64 in_sample = m < nin_u ? m : nin_u, need = s - s / A.discount;
-        SKey best1{0, 0};
-        scan([&](u32 i, u32 x, u32 y) {
-            const u32 q = part_of(i), rm = room[q], rs = rm & 0xFFFFu, rb = rm >> 16;
-            bool out = rs == RM_NONE || rb == RM_NONE || in_sample - dcon_of(x, y) > rb;
-            // a clamped room is at least RM_MORE nodes: larger nodes look at the size itself
-            if (!out) out = rs == RM_MORE ? (need > RM_MORE && A.psize[q] + need > A.omega) : need > rs;
-            if (out) {  // the slot is emptied (a hashed key may go as well: nothing is inserted any more)
-                v0[i] = 0;
-                if (!UNI) v1[i] = 0;
-                return;
-            }
-            const u64 conn = conn_of(x, y);
-            if (conn < best1.hi) return;
-            const SKey k = key_of(q, conn);
-            if (skey_better(k, best1)) best1 = k;
-        });
+        if (nk > GS_LIST) {
+            if (threadIdx.x == 0) nkeys = 0;
+            SKey best1{0, 0};
+            scan([&](u32 i, u32 x, u32 y) {
+                const u32 q = part_of(i);
+                if (ruled_out(q, dcon_of(x, y))) {  // the slot is emptied (its key may stay: nothing is inserted any more)
+                    v0[i] = 0;
+                    if (!UNI) v1[i] = 0;
+                    return;
+                }
+                const u64 conn = conn_of(x, y);
+                if (conn < best1.hi) return;
+                const SKey k = key_of(q, conn);
+                if (skey_better(k, best1)) best1 = k;
+            });
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) {  // 32 groups of 8 threads
-            const SKey c{__shfl_xor_sync(0xFFFFFFFFu, best1.hi, o), __shfl_xor_sync(0xFFFFFFFFu, best1.lo, o)};
-            if (skey_better(c, best1)) best1 = c;
+            for (int o = 4; o > 0; o >>= 1) {  // 32 groups of 8 threads
+                const SKey c{__shfl_xor_sync(0xFFFFFFFFu, best1.hi, o), __shfl_xor_sync(0xFFFFFFFFu, best1.lo, o)};
+                if (skey_better(c, best1)) best1 = c;
+            }
+            if ((lane & 7u) == 0) kred[threadIdx.x / 8] = best1;
+            __syncthreads();
+            SKey thr{0, 0};
+            {
+                const SKey mine = kred[lane];
+                u32 rank = 0;
+                for (u32 j = 0; j < 32; ++j) rank += skey_better(kred[j], mine);
+                const u32 bal = __ballot_sync(0xFFFFFFFFu, rank == GS_C - 1 && (mine.hi | mine.lo));
+                if (bal) thr = kred[__ffs(bal) - 1];  // keys are unique: one lane
+            }
+            scan([&](u32 i, u32 x, u32 y) {
+                const u64 conn = conn_of(x, y);
+                if (conn < thr.hi) return;
+                const SKey k = key_of(part_of(i), conn);
+                if (skey_better(thr, k)) return;
+                const u32 at = atomicAdd(&nkeys, 1u);
+                if (at < GS_LIST) klist[at] = k;
+            });
+            __syncthreads();
+            nk = nkeys;
         }
-        if ((lane & 7u) == 0) kred[threadIdx.x / 8] = best1;
-        if (threadIdx.x < GS_C) kout[threadIdx.x] = SKey{0, 0};
-        __syncthreads();
-        SKey thr{0, 0};
-        {
-            const SKey mine = kred[lane];
-            u32 rank = 0;
-            for (u32 j = 0; j < 32; ++j) rank += skey_better(kred[j], mine);
-            const u32 bal = __ballot_sync(0xFFFFFFFFu, rank == GS_C - 1 && (mine.hi | mine.lo));
-            if (bal) thr = kred[__ffs(bal) - 1];  // keys are unique: one lane
-        }
-        scan([&](u32 i, u32 x, u32 y) {
-            const u64 conn = conn_of(x, y);
-            if (conn < thr.hi) return;
-            const SKey k = key_of(part_of(i), conn);
-            if (skey_better(thr, k)) return;
-            const u32 at = atomicAdd(&nkeys, 1u);
-            if (at < GS_LIST) klist[at] = k;
-        });
-        __syncthreads();
-        const u32 nk = nkeys;
         if (nk <= GS_LIST) {
             if (threadIdx.x < nk) {
                 const SKey k = klist[threadIdx.x];

@@ -72,3 +72,10 @@ def test_incidence_lists_at_sort_tile_bounds(ctx, pins):
     np.testing.assert_array_equal(toff, o_toff)
     np.testing.assert_array_equal(touch, o_touch)
     np.testing.assert_array_equal(nin, o_nin)
+
+
+@pytest.mark.parametrize("K,omega,delta", [(4097, 3, 1 << 20), (5000, 4, 200), (8000, 3, 110), (12289, 5, 110),
+                                           (16385, 2, 1 << 20)])
+def test_sampled_candidate_bands_match_oracle(ctx, K, omega, delta):
+    g = weigh(ax.gen_snn(4, 1200, 120, 0.5, 400, 0.7, K), "unit", K)
+    check_gains(ctx, g, K, omega, delta, 1, 2, K)
