@@ -2493,28 +2493,40 @@ __device__ __forceinline__ void cascade_dense_body(const CascadeArgs &A, const M
             const u32 hi = lo + __popc(__ballot_sync(0xFFFFFFFFu, lane >= lo && x - b0 <= STAGE));
             const u32 T = __shfl_sync(0xFFFFFFFFu, x, hi - 1) - b0;
             bool movers = false;
-            for (u32 f0 = 0; f0 < T; f0 += 32) {
-                const u32 f = f0 + lane;
-                u32 ol = lo, oh = hi - 1;  // owner: the last hyperedge starting at or before f
-                for (int it = 0; it < 5; ++it) {
-                    const u32 mid = (ol + oh + 1) >> 1;
-                    const u32 em = __shfl_sync(0xFFFFFFFFu, excl, mid & 31);
-                    if (ol < oh) { if (em - b0 <= f) ol = mid; else oh = mid - 1; }
+            // pin, state and target are a chain of loads: U pins of a lane go through it together
+            constexpr u32 U = 4;
+            for (u32 f0 = 0; f0 < T; f0 += 32 * U) {
+                u32 v[U], q[U], dst = 0;
+                uint2 s[U];
+#pragma unroll
+                for (u32 x = 0; x < U; ++x) {
+                    v[x] = NONE;
+                    if (f0 + 32 * x >= T) continue;  // uniform over the warp
+                    const u32 f = f0 + 32 * x + lane;
+                    u32 ol = lo, oh = hi - 1;  // owner: the last hyperedge starting at or before f
+                    for (int it = 0; it < 5; ++it) {
+                        const u32 mid = (ol + oh + 1) >> 1;
+                        const u32 em = __shfl_sync(0xFFFFFFFFu, excl, mid & 31);
+                        if (ol < oh) { if (em - b0 <= f) ol = mid; else oh = mid - 1; }
+                    }
+                    const u32 eo = __shfl_sync(0xFFFFFFFFu, excl, ol) - b0;
+                    const u64 ao = __shfl_sync(0xFFFFFFFFu, a, ol);
+                    const u32 no = TRACK ? __shfl_sync(0xFFFFFFFFu, ns, ol) : 0u;
+                    if (f < T) v[x] = A.pins[ao + (f - eo)];
+                    if (TRACK && f - eo >= no) dst |= 1u << x;
                 }
-                const u32 eo = __shfl_sync(0xFFFFFFFFu, excl, ol) - b0;
-                const u64 ao = __shfl_sync(0xFFFFFFFFu, a, ol);
-                const u32 no = TRACK ? __shfl_sync(0xFFFFFFFFu, ns, ol) : 0u;
-                if (f >= T) continue;
-                const u32 v = A.pins[ao + (f - eo)];
-                const uint2 s = A.state[v];
-                u32 y = s.y;
-                if (s.x != NONE) {
-                    movers = true;
-                    y |= A.target[v] << 15;
+#pragma unroll
+                for (u32 x = 0; x < U; ++x) s[x] = v[x] != NONE ? A.state[v[x]] : make_uint2(NONE, 0);
+#pragma unroll
+                for (u32 x = 0; x < U; ++x) q[x] = s[x].x != NONE ? A.target[v[x]] : 0;
+#pragma unroll
+                for (u32 x = 0; x < U; ++x) {
+                    if (v[x] == NONE) continue;
+                    const u32 f = f0 + 32 * x + lane;
+                    movers |= s[x].x != NONE;
+                    st[f] = make_uint2(s[x].x, s[x].y | q[x] << 15 | (TRACK ? (dst >> x) << 31 : 0u));
+                    nd[f] = v[x];
                 }
-                if (TRACK && f - eo >= no) y |= 1u << 31;
-                st[f] = make_uint2(s.x, y);
-                nd[f] = v;
             }
             __syncwarp();
             if (__any_sync(0xFFFFFFFFu, movers)) {
@@ -3659,25 +3671,37 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain(GainArgs A0, KwGain V)
     T conn[C], saving = 0, wtot = 0;
 #pragma unroll
     for (u32 x = 0; x < C; ++x) conn[x] = 0;
-#pragma unroll 4
-    for (u32 j = 0; j < deg; ++j) {
-        const u32 h = A.touch[t0 + j], w = V.uni ? V.weight : A.wfx[h];
-        const u32 *r = V.rec + (u64)h * (2 * MW);
-        u32 any[MW];
-        u32 sg;
-        if constexpr (MW == 1) {
-            const uint2 v = *(const uint2 *)r;
-            any[0] = v.x;
-            sg = v.y;
-        } else {
-            load_words<MW>(r, any);
-            sg = r[MW + (pl >> 5)];
-        }
-        wtot += w;
-        if ((sg >> (pl & 31u)) & 1u) saving += w;
+    // batches of U incidences, the last one's remainder included, with their loads in flight together
+    constexpr u32 U = MW <= 2 ? 4 : 2;
+    for (u32 j = 0; j < deg; j += U) {
+        u32 h[U], w[U], any[U][MW], sg[U];
 #pragma unroll
-        for (u32 x = 0; x < C; ++x)
-            if ((any[x] >> own) & 1u) conn[x] += w;
+        for (u32 i = 0; i < U; ++i) h[i] = j + i < deg ? A.touch[t0 + j + i] : NONE;
+#pragma unroll
+        for (u32 i = 0; i < U; ++i) {
+            w[i] = h[i] == NONE ? 0u : V.uni ? V.weight : A.wfx[h[i]];
+            sg[i] = 0;
+#pragma unroll
+            for (u32 x = 0; x < MW; ++x) any[i][x] = 0;
+            if (h[i] == NONE) continue;
+            const u32 *r = V.rec + (u64)h[i] * (2 * MW);
+            if constexpr (MW == 1) {
+                const uint2 v = *(const uint2 *)r;
+                any[i][0] = v.x;
+                sg[i] = v.y;
+            } else {
+                load_words<MW>(r, any[i]);
+                sg[i] = r[MW + (pl >> 5)];
+            }
+        }
+#pragma unroll
+        for (u32 i = 0; i < U; ++i) {
+            wtot += w[i];
+            if ((sg[i] >> (pl & 31u)) & 1u) saving += w[i];
+#pragma unroll
+            for (u32 x = 0; x < C; ++x)
+                if ((any[i][x] >> own) & 1u) conn[x] += w[i];
+        }
     }
     kw_move<G, C, T>(A, u, base, pl, V.k, own, gmask, conn, saving, wtot);
 }
@@ -3695,15 +3719,25 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain_few(GainArgs A0, KwGai
     const u64 t0 = A.toff[u];
     const u32 deg = (u32)(A.toff[u + 1] - t0);
     T conn[4] = {0, 0, 0, 0}, saving = 0, wtot = 0;
-#pragma unroll 2
-    for (u32 j = own; j < deg; j += G) {
-        const u32 h = A.touch[t0 + j], w = V.uni ? V.weight : A.wfx[h];
-        const uint2 r = *(const uint2 *)(V.rec + (u64)h * 2);
-        wtot += w;
-        if ((r.y >> pl) & 1u) saving += w;
+    constexpr u32 U = 4;  // incidences of a lane whose loads are in flight together
+    for (u32 j = own; j < deg; j += G * U) {
+        u32 h[U], w[U];
+        uint2 r[U];
 #pragma unroll
-        for (u32 x = 0; x < 4; ++x)
-            if ((r.x >> x) & 1u) conn[x] += w;
+        for (u32 i = 0; i < U; ++i) h[i] = j + G * i < deg ? A.touch[t0 + j + G * i] : NONE;
+#pragma unroll
+        for (u32 i = 0; i < U; ++i) {
+            w[i] = h[i] == NONE ? 0u : V.uni ? V.weight : A.wfx[h[i]];
+            r[i] = h[i] == NONE ? make_uint2(0, 0) : *(const uint2 *)(V.rec + (u64)h[i] * 2);
+        }
+#pragma unroll
+        for (u32 i = 0; i < U; ++i) {
+            wtot += w[i];
+            if ((r[i].y >> pl) & 1u) saving += w[i];
+#pragma unroll
+            for (u32 x = 0; x < 4; ++x)
+                if ((r[i].x >> x) & 1u) conn[x] += w[i];
+        }
     }
     __syncwarp(gmask);
 #pragma unroll
