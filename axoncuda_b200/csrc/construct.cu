@@ -61,29 +61,93 @@ __device__ __forceinline__ void uq_mark(const u32 *pins, const u32 *groups, u64 
     }
 }
 
-__global__ void k_uniq_warp(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ pins,
-                            const u32 *__restrict__ nsrc, const u32 *__restrict__ groups, int dst_wins,
-                            uint8_t *__restrict__ keep, u32 *__restrict__ cnt, u32 *__restrict__ cnt_src,
-                            u32 *status) {
+// A warp's consecutive hyperedges: 32 where most have a handful of pins, fewer where they are long or
+// few. A warp per hyperedge left seven lanes in eight idle on a netlist.
+static u32 hedges_per_warp(const Ctx &c, u32 e, u64 P) {
+    u32 per = P <= 16ull * e ? 32u : P <= 64ull * e ? 8u : 1u;
+    while (per > 1 && e / per < (u32)c.sms * 16) per >>= 1;
+    return per;
+}
+// The lane l whose item holds position f, given the items' exclusive prefix sums less b0 (lanes
+// [lo, hi)): the last that starts at or before f. All lanes take part.
+__device__ __forceinline__ u32 owner_lane(u32 excl, u32 b0, u32 lo, u32 hi, u32 f) {
+    u32 l = lo, h = hi - 1;
+    for (int it = 0; it < 5; ++it) {
+        const u32 mid = (l + h + 1) >> 1;
+        const u32 em = __shfl_sync(0xFFFFFFFFu, excl, mid & 31);
+        if (l < h) { if (em - b0 <= f) l = mid; else h = mid - 1; }
+    }
+    return l;
+}
+__device__ __forceinline__ u32 warp_incl(u32 x, u32 lane) {
+#pragma unroll
+    for (u32 o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    return x;
+}
+
+// One warp per `per` consecutive hyperedges. Those of at most 32 pins are packed into the warp's
+// lanes, a pin each: the lanes holding the same pin of the same hyperedge find each other by a match,
+// no table. Then those up to UQ_WARP_CAP, one after the other, by a table in shared memory.
+__global__ void __launch_bounds__(UQ_WARPS * 32) k_uniq_warp(u32 e, const u64 *__restrict__ off,
+                                                             const u32 *__restrict__ pins, const u32 *__restrict__ nsrc,
+                                                             const u32 *__restrict__ groups, int dst_wins, u32 per,
+                                                             uint8_t *__restrict__ keep, u32 *__restrict__ cnt,
+                                                             u32 *__restrict__ cnt_src, u32 *status) {
     __shared__ u32 tk[UQ_WARPS][2 * UQ_WARP_CAP], tv[UQ_WARPS][2 * UQ_WARP_CAP];
     const u32 w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const u32 h = blockIdx.x * UQ_WARPS + w;
-    if (h >= e) return;
-    const u64 a = off[h], b = off[h + 1], s = a + nsrc[h];
-    const u32 len = (u32)(b - a);
-    if (len > UQ_WARP_CAP) return;  // handled by the block kernel
-    u32 cap = 64;
-    while (cap < 2 * len) cap <<= 1;
+    const u64 h0 = ((u64)blockIdx.x * UQ_WARPS + w) * per;
+    if (h0 >= e) return;
+    const u32 nh = (u32)(e - h0 < per ? e - h0 : per), h = (u32)h0 + lane;
+    const bool mine = lane < nh;
+    const u64 a = mine ? off[h] : 0, len64 = mine ? off[h + 1] - a : 0;
+    const u32 ns = mine ? nsrc[h] : 0, few = len64 <= 32 ? (u32)len64 : 0u;
+    const u32 x = warp_incl(few, lane), excl = x - few;
+    for (u32 lo = 0; lo < nh;) {
+        const u32 b0 = __shfl_sync(0xFFFFFFFFu, excl, lo);
+        const u32 hi = lo + __popc(__ballot_sync(0xFFFFFFFFu, lane >= lo && lane < nh && x - b0 <= 32));
+        const u32 T = __shfl_sync(0xFFFFFFFFu, x, hi - 1) - b0;
+        if (T == 0) {  // only longer or empty ones (uniform over the warp)
+            if (lane >= lo && lane < hi && len64 == 0) cnt[h] = cnt_src[h] = 0;
+            lo = hi;
+            continue;
+        }
+        const u32 ol = owner_lane(excl, b0, lo, hi, lane);
+        const u32 at = lane - (__shfl_sync(0xFFFFFFFFu, excl, ol) - b0);  // in the hyperedge
+        const u64 k = __shfl_sync(0xFFFFFFFFu, a, ol) + at;
+        const bool in = lane < T, src = at < __shfl_sync(0xFFFFFFFFu, ns, ol);
+        const u64 key = in ? (u64)ol << 32 | uq_key(pins, groups, k) : (u64)(32 + lane) << 32;
+        const u32 same = __match_any_sync(0xFFFFFFFFu, key), dsts = __ballot_sync(0xFFFFFFFFu, in && !src);
+        const u32 from = dst_wins && (same & dsts) ? same & dsts : same;
+        const bool kp = in && (u32)__ffs(from) == lane + 1;
+        if (in) keep[k] = kp;
+        const u32 kb = __ballot_sync(0xFFFFFFFFu, kp), sb = __ballot_sync(0xFFFFFFFFu, kp && src);
+        if (lane >= lo && lane < hi && len64 <= 32) {
+            const u32 run = few ? (0xFFFFFFFFu >> (32 - few)) << (excl - b0) : 0u;
+            cnt[h] = __popc(kb & run);
+            cnt_src[h] = __popc(sb & run);
+        }
+        lo = hi;
+    }
     u32 *keys = tk[w], *vals = tv[w];
-    for (u32 i = lane; i < cap; i += 32) { keys[i] = NONE; vals[i] = NONE; }
-    __syncwarp();
-    uq_insert(pins, groups, a, b, s, dst_wins, keys, vals, cap - 1, lane, 32, status);
-    __syncwarp();
-    u32 kept = 0, ks = 0;
-    uq_mark(pins, groups, a, b, s, dst_wins, keys, vals, cap - 1, lane, 32, keep, kept, ks);
-    kept = warp_sum(kept);
-    ks = warp_sum(ks);
-    if (lane == 0) { cnt[h] = kept; cnt_src[h] = ks; }
+    for (u32 left = __ballot_sync(0xFFFFFFFFu, len64 > 32 && len64 <= UQ_WARP_CAP); left; left &= left - 1) {
+        const u32 i = __ffs(left) - 1, len = (u32)__shfl_sync(0xFFFFFFFFu, len64, i);
+        const u64 ai = __shfl_sync(0xFFFFFFFFu, a, i), bi = ai + len, si = ai + __shfl_sync(0xFFFFFFFFu, ns, i);
+        u32 cap = 64;
+        while (cap < 2 * len) cap <<= 1;
+        for (u32 j = lane; j < cap; j += 32) { keys[j] = NONE; vals[j] = NONE; }
+        __syncwarp();
+        uq_insert(pins, groups, ai, bi, si, dst_wins, keys, vals, cap - 1, lane, 32, status);
+        __syncwarp();
+        u32 kept = 0, ks = 0;
+        uq_mark(pins, groups, ai, bi, si, dst_wins, keys, vals, cap - 1, lane, 32, keep, kept, ks);
+        kept = warp_sum(kept);
+        ks = warp_sum(ks);
+        if (lane == i) { cnt[h] = kept; cnt_src[h] = ks; }
+        __syncwarp();  // the table is no longer read
+    }
 }
 
 // One block per listed hyperedge (the count in device memory when d_n is set).
@@ -123,20 +187,35 @@ __global__ void k_uniq_block(const u32 *__restrict__ list, u32 nlist, const u32 
     }
 }
 
-// Stable compaction of survivors, one warp per hyperedge.
+// Stable compaction of survivors: a warp per `per` consecutive hyperedges, whose pins follow one
+// another before and after.
 __global__ void k_uniq_compact(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ pins,
-                               const u32 *__restrict__ groups, const uint8_t *__restrict__ keep,
+                               const u32 *__restrict__ groups, const uint8_t *__restrict__ keep, u32 per,
                                const u64 *__restrict__ new_off, u32 *__restrict__ new_pins) {
-    const u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= e) return;
-    const u64 a = off[w], b = off[w + 1];
-    u64 o = new_off[w];
-    for (u64 base = a; base < b; base += 32) {
-        u64 k = base + lane;
-        bool kp = k < b && keep[k];
-        u32 bal = __ballot_sync(0xFFFFFFFFu, kp);
-        if (kp) new_pins[o + __popc(bal & ((1u << lane) - 1u))] = uq_key(pins, groups, k);
-        o += __popc(bal);
+    const u32 lane = threadIdx.x & 31;
+    const u64 h0 = (((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
+    if (h0 >= e) return;
+    const u64 a = off[h0], b = off[h0 + per < e ? h0 + per : e];
+    u64 o = new_off[h0];
+    constexpr u32 U = 4;
+    for (u64 base = a; base < b; base += 32 * U) {
+        bool kp[U];
+        u32 v[U];
+#pragma unroll
+        for (u32 r = 0; r < U; ++r) {
+            const u64 k = base + 32 * r + lane;
+            kp[r] = k < b && keep[k];
+            v[r] = k < b ? pins[k] : 0;
+        }
+#pragma unroll
+        for (u32 r = 0; r < U; ++r)
+            if (kp[r] && groups) v[r] = groups[v[r]];
+#pragma unroll
+        for (u32 r = 0; r < U; ++r) {
+            const u32 bal = __ballot_sync(0xFFFFFFFFu, kp[r]);
+            if (kp[r]) new_pins[o + __popc(bal & ((1u << lane) - 1u))] = v[r];
+            o += __popc(bal);
+        }
     }
 }
 
@@ -170,14 +249,46 @@ __global__ void k_table_sizes(const u32 *__restrict__ list, u32 nlist, const u64
 // ---------------------------------------------------------------- transpose
 // key = 2*pin + is_source, value = hyperedge: a stable sort by key lists, per node, its inbound
 // hyperedges ascending and then its outbound ones ascending (sources/construction.cu:17-62).
+// A warp per `per` consecutive hyperedges, their pins side by side.
 __global__ void k_touch_keys(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ pins,
-                             const u32 *__restrict__ nsrc, u32 *__restrict__ keys, u32 *__restrict__ vals) {
-    const u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= e) return;
-    const u64 a = off[w], b = off[w + 1], s = a + nsrc[w];
-    for (u64 k = a + lane; k < b; k += 32) {
-        keys[k] = 2 * pins[k] + (k < s ? 1u : 0u);
-        vals[k] = w;
+                             const u32 *__restrict__ nsrc, u32 per, u32 *__restrict__ keys, u32 *__restrict__ vals) {
+    const u32 lane = threadIdx.x & 31;
+    const u64 h0 = (((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
+    if (h0 >= e) return;
+    const u32 nh = (u32)(e - h0 < per ? e - h0 : per);
+    const u64 a = off[h0], P = off[h0 + nh] - a;
+    const u32 h = (u32)h0 + (lane < nh ? lane : nh - 1);
+    const u64 at = off[h] - a;
+    const u32 ns = nsrc[h];
+    if (nh == 1 || P >> 31) {  // one by one (positions below are 32-bit)
+        for (u32 i = 0; i < nh; ++i) {
+            const u64 s0 = a + __shfl_sync(0xFFFFFFFFu, at, i), s = s0 + __shfl_sync(0xFFFFFFFFu, ns, i);
+            const u64 s1 = i + 1 < nh ? a + __shfl_sync(0xFFFFFFFFu, at, (i + 1) & 31) : a + P;
+            for (u64 k = s0 + lane; k < s1; k += 32) {
+                keys[k] = 2 * pins[k] + (k < s ? 1u : 0u);
+                vals[k] = (u32)h0 + i;
+            }
+        }
+        return;
+    }
+    constexpr u32 U = 4;
+    for (u32 f0 = 0; f0 < (u32)P; f0 += 32 * U) {
+        u32 v[U], ol[U];
+#pragma unroll
+        for (u32 r = 0; r < U; ++r) {
+            const u32 f = f0 + 32 * r + lane;
+            v[r] = f < (u32)P ? pins[a + f] : 0;
+        }
+#pragma unroll
+        for (u32 r = 0; r < U; ++r) {
+            const u32 f = f0 + 32 * r + lane;
+            ol[r] = owner_lane((u32)at, 0, 0, nh, f);
+            const u32 src = f < __shfl_sync(0xFFFFFFFFu, (u32)at + ns, ol[r]) ? 1u : 0u;
+            if (f < (u32)P) {
+                keys[a + f] = 2 * v[r] + src;
+                vals[a + f] = (u32)h0 + ol[r];
+            }
+        }
     }
 }
 // Where a node's keys start in the sorted keys, by two binary searches: its offset, and its
@@ -237,8 +348,9 @@ u64 hedge_unique(Ctx &c, u32 e, const u64 *off, const u32 *pins, const u32 *nsrc
     size_t m = c.arena.mark();
     uint8_t *keep = c.arena.alloc<uint8_t>(pins_in ? pins_in : 1);
     u32 *cnt = c.arena.alloc<u32>(e);
-    LAUNCH(c, k_uniq_warp, cdiv(e, UQ_WARPS), UQ_WARPS * 32, 0, e, off, pins, nsrc, groups,
-           (int)dst_wins, keep, cnt, new_nsrc, c.d_status);
+    const u32 per = hedges_per_warp(c, e, pins_in);
+    LAUNCH(c, k_uniq_warp, cdiv(e, UQ_WARPS * per), UQ_WARPS * 32, 0, e, off, pins, nsrc, groups,
+           (int)dst_wins, per, keep, cnt, new_nsrc, c.d_status);
     // hyperedges larger than a warp's table: their lists and counts stay on the device, except for
     // those that need tables in device memory, which are rare and sized by the host
     u32 *mid = c.arena.alloc<u32>(e), *big = c.arena.alloc<u32>(e), *huge = c.arena.alloc<u32>(e);
@@ -265,7 +377,7 @@ u64 hedge_unique(Ctx &c, u32 e, const u64 *off, const u32 *pins, const u32 *nsrc
                new_nsrc, gtab, (const u64 *)tsz, c.d_status);
     }
     offsets_from_counts(c, cnt, new_off, e);
-    LAUNCH(c, k_uniq_compact, cdiv((u64)e * 32, 256), 256, 0, e, off, pins, groups, keep, new_off, new_pins);
+    LAUNCH(c, k_uniq_compact, cdiv(e, 8 * per), 256, 0, e, off, pins, groups, keep, per, new_off, new_pins);
     AXC_CUDA(cudaMemcpyAsync(res + 2, new_off + e, 8, cudaMemcpyDeviceToDevice, c.stream));
     AXC_CUDA(cudaMemcpyAsync(res + 3, c.d_status, 4, cudaMemcpyDeviceToDevice, c.stream));
     u64 fin[2];
@@ -280,7 +392,8 @@ void build_touching(Ctx &c, u32 n, u32 e, const u64 *off, const u32 *pins, const
                     u64 *toff, u32 *touch, u32 *nin) {
     size_t m = c.arena.mark();
     u32 *keys = c.arena.alloc<u32>(P ? P : 1);
-    if (e) LAUNCH(c, k_touch_keys, cdiv((u64)e * 32, 256), 256, 0, e, off, pins, nsrc, keys, touch);
+    const u32 per = e ? hedges_per_warp(c, e, P) : 1;
+    if (e) LAUNCH(c, k_touch_keys, cdiv(e, 8 * per), 256, 0, e, off, pins, nsrc, per, keys, touch);
     radix_sort_pairs(c, keys, touch, P, bits_for(n ? 2ull * n - 1 : 0));
     LAUNCH(c, k_touch_starts, cdiv((u64)n + 1, 256), 256, 0, n, P, keys, toff, nin);
     c.arena.release(m);

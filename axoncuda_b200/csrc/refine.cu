@@ -730,24 +730,40 @@ __device__ __forceinline__ GainArgs gain_args_now(const GainArgs &A0) {
 // Per-level bounds of a node's gain work: the partitions adjacent to it in any round number at
 // most min(sum over incident hyperedges of min(|e|, K), K), which sizes its accumulator table; the
 // sum of incident weights bounds its gain.
-__global__ void k_gain_bounds(u32 n, u32 K, const u64 *__restrict__ toff, const u32 *__restrict__ touch,
-                              const u64 *__restrict__ off, const u32 *__restrict__ wfx, u64 *__restrict__ work,
-                              u64 *__restrict__ wsum, unsigned long long *__restrict__ wmax) {
-    const u32 u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (u >= n) return;
+template <u32 G>
+__global__ void __launch_bounds__(256) k_gain_bounds(u32 n, u32 K, const u64 *__restrict__ toff,
+                                                     const u32 *__restrict__ touch, const u64 *__restrict__ off,
+                                                     const u32 *__restrict__ wfx, u64 *__restrict__ work,
+                                                     u64 *__restrict__ wsum, unsigned long long *__restrict__ wmax) {
+    __shared__ u64 top[8];
+    const u32 u = (blockIdx.x * 256 + threadIdx.x) / G, own = threadIdx.x & (G - 1);
     u64 s = 0, ws = 0;
-    for (u64 j = toff[u] + lane; j < toff[u + 1]; j += 32) {
-        u32 h = touch[j];
-        u64 len = off[h + 1] - off[h];
-        s += len < K ? len : K;
-        ws += wfx[h];
+    if (u < n) {
+        const u64 t1 = toff[u + 1];
+        for (u64 j = toff[u] + own; j < t1; j += G) {
+            const u32 h = touch[j];
+            const u64 len = off[h + 1] - off[h];
+            s += len < K ? len : K;
+            ws += wfx[h];
+        }
     }
-    s = warp_sum(s);
-    ws = warp_sum(ws);
-    if (lane == 0) {
+#pragma unroll
+    for (u32 o = G / 2; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+        ws += __shfl_xor_sync(0xFFFFFFFFu, ws, o);
+    }
+    if (u < n && own == 0) {
         work[u] = s < K ? s : K;
         if (wsum) wsum[u] = ws;
-        atomicMax(wmax, (unsigned long long)ws);
+    }
+    // the largest of the block in one atomic: one per node met at a single address
+    ws = warp_max_u64(ws);
+    if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = ws;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (u32 i = 1; i < 8; ++i) ws = top[i] > ws ? top[i] : ws;
+        if (ws) atomicMax(wmax, (unsigned long long)ws);
     }
 }
 __host__ __device__ __forceinline__ u32 table_cap(u64 work, u32 cap_max) {
@@ -4423,13 +4439,36 @@ __global__ void __launch_bounds__(1024) k_level_hedges(u32 e, const u64 *__restr
             if (len > hi) huge[ah] = h;
         }
     }
-    len = warp_max_u64(len);
-    dst = warp_sum(dst);
-    sp = warp_sum(sp);
-    sq = warp_sum(sq);
-    w = __reduce_max_sync(0xFFFFFFFFu, w);
-    nw = __reduce_max_sync(0xFFFFFFFFu, nw);
-    if ((threadIdx.x & 31) == 0) {
+    // one atomic per block and word: one per warp met at six addresses
+    __shared__ u64 red[6][32];
+    const u32 lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const auto reduce = [&]() {
+        len = warp_max_u64(len);
+        dst = warp_sum(dst);
+        sp = warp_sum(sp);
+        sq = warp_sum(sq);
+        w = __reduce_max_sync(0xFFFFFFFFu, w);
+        nw = __reduce_max_sync(0xFFFFFFFFu, nw);
+    };
+    reduce();
+    if (lane == 0) {
+        red[0][wp] = len;
+        red[1][wp] = dst;
+        red[2][wp] = sp;
+        red[3][wp] = sq;
+        red[4][wp] = w;
+        red[5][wp] = nw;
+    }
+    __syncthreads();
+    if (wp) return;
+    len = red[0][lane];  // 32 warps
+    dst = red[1][lane];
+    sp = red[2][lane];
+    sq = red[3][lane];
+    w = (u32)red[4][lane];
+    nw = (u32)red[5][lane];
+    reduce();
+    if (lane == 0) {
         unsigned long long *out = (unsigned long long *)dc;
         if (len) atomicMax(&out[9], (unsigned long long)len);
         if (dst) atomicAdd(&out[10], (unsigned long long)dst);
@@ -4467,8 +4506,14 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
         u64 *work = c.arena.alloc<u64>(n);
         lp.work = work;
         if (K > GS_K) lp.wsum = c.arena.alloc<u64>(n);
-        LAUNCH(c, k_gain_bounds, cdiv((u64)n * 32, 256), 256, 0, n, K, L.toff, L.touch, L.off, wfx, work,
-               lp.wsum, (unsigned long long *)(dc + 5));
+        const auto bounds = [&](auto g) {  // lanes per node: as many as a mean node has incidences
+            constexpr u32 G = decltype(g)::value;
+            LAUNCH_AS(c, "k_gain_bounds", k_gain_bounds<G>, cdiv((u64)n * G, 256), 256, 0, n, K, L.toff, L.touch, L.off, wfx,
+                      work, lp.wsum, (unsigned long long *)(dc + 5));
+        };
+        if (L.P < 8ull * n) bounds(std::integral_constant<u32, 4>());
+        else if (L.P < 32ull * n) bounds(std::integral_constant<u32, 8>());
+        else bounds(std::integral_constant<u32, 32>());
         for (u32 t = 0; t < (kway ? 2u : 3u); ++t) lp.ntier[t] = c.arena.alloc<u32>(n);
         LAUNCH(c, k_tier_lists, cdiv(n, 1024), 1024, 0, n, K, work, L.toff, kway ? 1u : 0u, lp.ntier[0], lp.ntier[1],
                lp.ntier[2], dc + 2, (unsigned long long *)(dc + 6));
