@@ -2640,6 +2640,10 @@ __global__ void k_long_list(MoverArgs V, const u32 *__restrict__ longs, u32 nlon
 constexpr u32 CL_WARPS = 4;
 constexpr u32 CL_BINS = 256;
 constexpr u32 CL_MAX_LEN = 65535;
+// Movers a warp takes. Hashed, a mover's slots are most of the warp's shared memory, and the warps in
+// flight count for more than the hyperedges that go on to the wide kernel (20 x 5000 network: 456 ms
+// with 256, 424 with 128, 413 with 64); by index 512 (128 parts: 156 ms, with 256 165).
+constexpr u32 CL_MOV_DIRECT = 512, CL_MOV_HASH = 64;
 // Bytes of one warp's shared memory.
 __host__ __device__ __forceinline__ u32 cl_bytes(bool direct, u32 K, u32 MV) {
     const u32 common = MV * 8 + MV * 4 + 2 * MV * 2 + CL_BINS * 4 + 16;
@@ -2687,6 +2691,74 @@ __device__ __forceinline__ void warp_rank_order(const u64 *mv, u32 m, u32 rmax, 
         if (i < m) ord[p] = (unsigned short)i;  // arrival places are no longer read
     }
     __syncwarp();
+}
+
+// The sweep of one warp over its hyperedge's movers [i0, i1) in rank order, 32 at a time
+// (cascade_sweep_warp). cnt: pins below, destination pins above, as the first of them finds them.
+template <bool DIRECT>
+__device__ __forceinline__ void cl_sweep(const CascadeArgs &A, const u64 *mv, const u32 *sl, const unsigned short *ord,
+                                         u32 i0, u32 i1, u32 *cnt, u32 *pm, u32 *qm, const u32 *keys, u32 wh, u32 base) {
+    const u32 lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    for (u32 b0 = i0; b0 < i1; b0 += 32) {
+        const bool act = b0 + lane < i1;
+        const u32 i = act ? ord[b0 + lane] : 0;
+        const u64 e = act ? mv[i] : 0;
+        const u32 pq = sl[i];
+        const u32 sp = act ? pq & 0xFFFFu : 0x10000u + lane, sqx = act ? pq >> 16 : 0x20000u + lane;
+        const bool dst = act && ((u32)e & MV_DST);
+        const u32 dmask = __ballot_sync(0xFFFFFFFFu, dst);
+        u32 m_pp, m_qq, m_qp = 0, m_pq = 0;  // lanes with my source / my target as source / target
+        if (DIRECT) {
+            if (act) {
+                atomicOr(&pm[sp], 1u << lane);
+                atomicOr(&qm[sqx], 1u << lane);
+            }
+            __syncwarp();
+            m_pp = act ? pm[sp] : 0u;
+            m_qq = act ? qm[sqx] : 0u;
+            m_qp = act ? qm[sp] : 0u;
+            m_pq = act ? pm[sqx] : 0u;
+            __syncwarp();
+            if (act) {
+                pm[sp] = 0;
+                qm[sqx] = 0;
+            }
+        } else {
+            m_pp = __match_any_sync(0xFFFFFFFFu, sp);
+            m_qq = __match_any_sync(0xFFFFFFFFu, sqx);
+#pragma unroll 8
+            for (u32 j = 0; j < 32; ++j) {
+                const u32 spj = __shfl_sync(0xFFFFFFFFu, sp, j), sqj = __shfl_sync(0xFFFFFFFFu, sqx, j);
+                m_qp |= (u32)(sqj == sp) << j;
+                m_pq |= (u32)(spj == sqx) << j;
+            }
+        }
+        const u32 cP = act ? cnt[sp] : 0, cQ = act ? cnt[sqx] : 0;
+        if (act) {
+            const u32 cp = (u32)((int)(cP & 0xFFFFu) + __popc(m_qp & lt) - __popc(m_pp & lt));
+            const u32 cq = (u32)((int)(cQ & 0xFFFFu) + __popc(m_qq & lt) - __popc(m_pq & lt));
+            const i64 d = leave_gain(A.encourage, wh, cp) - (cq == 0 ? (i64)wh : 0);
+            if (d) atomicAdd(&A.g2[(u32)e & ~MV_DST], (unsigned long long)d);
+        }
+        if (A.track) {  // warp-uniform
+            bool ep = false, eq = false;
+            if (dst) {
+                ep = (int)(cP >> 16) + __popc(m_qp & lt & dmask) - __popc(m_pp & lt & dmask) == 1;
+                eq = (int)(cQ >> 16) + __popc(m_qq & lt & dmask) - __popc(m_pq & lt & dmask) == 0;
+            }
+            const u32 r = (u32)(e >> 32);
+            const u32 pid = DIRECT ? sp + base : ep ? keys[sp] : 0, qid = DIRECT ? sqx + base : eq ? keys[sqx] : 0;
+            __syncwarp();
+            emit_pair(A, ep, pid, eq, qid, r);
+        }
+        __syncwarp();
+        if (act) {  // counts stay within their halves once the whole chunk is in
+            const u32 one = dst ? 0x10001u : 1u;
+            atomicSub(&cnt[sp], one);
+            atomicAdd(&cnt[sqx], one);
+        }
+        __syncwarp();
+    }
 }
 
 template <bool DIRECT>
@@ -2767,68 +2839,251 @@ __global__ void __launch_bounds__(CL_WARPS * 32) k_cascade_long(CascadeArgs A, c
             }
         }
         warp_rank_order(mv, m, rmax, bins, idx, ord);
-        // the sweep, 32 movers at a time (cascade_sweep_warp)
         u32 *cnt = DIRECT ? tc : hc;
-        const u32 wh = A.wfx[h];
-        for (u32 b0 = 0; b0 < m; b0 += 32) {
-            const bool act = b0 + lane < m;
-            const u32 i = act ? ord[b0 + lane] : 0;
-            const u64 e = act ? mv[i] : 0;
-            const u32 pq = sl[i];
-            const u32 sp = act ? pq & 0xFFFFu : 0x10000u + lane, sqx = act ? pq >> 16 : 0x20000u + lane;
-            const bool dst = act && ((u32)e & MV_DST);
-            const u32 dmask = __ballot_sync(0xFFFFFFFFu, dst);
-            u32 m_pp, m_qq, m_qp = 0, m_pq = 0;  // lanes with my source / my target as source / target
-            if (DIRECT) {
-                if (act) {
-                    atomicOr(&pm[sp], 1u << lane);
-                    atomicOr(&qm[sqx], 1u << lane);
-                }
-                __syncwarp();
-                m_pp = act ? pm[sp] : 0u;
-                m_qq = act ? qm[sqx] : 0u;
-                m_qp = act ? qm[sp] : 0u;
-                m_pq = act ? pm[sqx] : 0u;
-                __syncwarp();
-                if (act) {
-                    pm[sp] = 0;
-                    qm[sqx] = 0;
-                }
-            } else {
-                m_pp = __match_any_sync(0xFFFFFFFFu, sp);
-                m_qq = __match_any_sync(0xFFFFFFFFu, sqx);
-#pragma unroll 8
-                for (u32 j = 0; j < 32; ++j) {
-                    const u32 spj = __shfl_sync(0xFFFFFFFFu, sp, j), sqj = __shfl_sync(0xFFFFFFFFu, sqx, j);
-                    m_qp |= (u32)(sqj == sp) << j;
-                    m_pq |= (u32)(spj == sqx) << j;
+        cl_sweep<DIRECT>(A, mv, sl, ord, 0, m, cnt, pm, qm, keys, A.wfx[h], base);
+    }
+}
+
+// Hyperedges with more movers than a warp takes, a block each; everything a mover needs is loaded in one
+// gather. The counts a mover finds come in one of two ways:
+//  - CW_SWEEP, up to CW_SWEEP_K partitions by index: the movers are ordered by rank, and each warp sweeps
+//    over its share of them with a table of its own, which holds the counts its first mover finds
+//    (the hyperedge's, plus what the earlier shares did). The block kernel has one warp sweep over all.
+//  - CW_EVENTS by index and CW_HASH, more partitions: the movers' leave and join events are dealt out by
+//    partition, and a mover counts those of smaller rank in its source and its target: no order and no
+//    chain at all. With m movers over K partitions a list holds about 2m / K events; a hyperedge whose
+//    lists hold more than CW_PAIRS events per mover goes on to the block kernel.
+// So do those with more movers than MV or too many pins for 16-bit counts.
+enum WideForm { CW_SWEEP, CW_EVENTS, CW_HASH };
+constexpr u32 CW_SWEEP_K = 256;
+constexpr u32 CW_PAIRS = 256;
+constexpr u32 CW_BINS = 1024;
+__host__ __device__ constexpr u32 cw_threads(WideForm f) { return f == CW_SWEEP ? 256u : 512u; }
+constexpr u32 cw_movers(WideForm f) { return f == CW_SWEEP ? 2048u : f == CW_EVENTS ? 4096u : 1024u; }
+// Words of the events, or of the sweep's order (two shorts per mover, then the bins).
+__host__ __device__ constexpr u32 cw_event_words(WideForm f, u32 MV) {
+    return f == CW_SWEEP ? MV + CW_BINS + 1 : 2 * MV;
+}
+__host__ __device__ constexpr u32 cw_bytes(WideForm f, u32 K, u32 MV) {
+    return (MV * 12 + cw_event_words(f, MV) * 4 +
+            (f == CW_SWEEP ? (1 + 3 * (cw_threads(f) / 32)) * K : f == CW_EVENTS ? 2 * K : 12 * MV) * 4 + 15) & ~15u;
+}
+// Counts c[0, S) into exclusive prefix sums; returns the sum of the counts' squares.
+template <u32 NT>
+__device__ __forceinline__ u32 cw_starts(u32 *c, u32 S, u32 *wsum) {
+    constexpr u32 NW = NT / 32;
+    const u32 lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    u32 carry = 0, sq = 0;
+    for (u32 base = 0; base < S; base += NT) {
+        const u32 i = base + threadIdx.x, v = i < S ? c[i] : 0;
+        sq += v * v;
+        u32 x = v;
+#pragma unroll
+        for (u32 o = 1; o < 32; o <<= 1) {
+            const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[w] = x;
+        __syncthreads();
+        u32 tot = 0;
+        for (u32 k = 0; k < NW; ++k) {
+            if (k == w) x += tot;
+            tot += wsum[k];
+        }
+        __syncthreads();
+        if (i < S) c[i] = carry + x - v;
+        carry += tot;
+    }
+    sq = __reduce_add_sync(0xFFFFFFFFu, sq);
+    if (lane == 0) wsum[w] = sq;
+    __syncthreads();
+    sq = 0;
+    for (u32 k = 0; k < NW; ++k) sq += wsum[k];
+    return sq;
+}
+
+// Places of the m movers by rank, block-wide (warp_rank_order).
+template <u32 NT>
+__device__ __forceinline__ void cw_rank_order(const u64 *mv, u32 m, u32 rmax, u32 *bins, unsigned short *idx,
+                                              unsigned short *ord, u32 *wsum) {
+    const u32 t = threadIdx.x, nb = 32 - __clz(rmax), sh = nb > 10 ? nb - 10 : 0;
+    static_assert(CW_BINS == 1024, "ten leading bits");
+    for (u32 i = t; i <= CW_BINS; i += NT) bins[i] = 0;
+    __syncthreads();
+    // arrival places are kept in ord until the movers are listed by bin in idx
+    for (u32 i = t; i < m; i += NT) ord[i] = (unsigned short)atomicAdd(&bins[(u32)(mv[i] >> 32) >> sh], 1u);
+    __syncthreads();
+    cw_starts<NT>(bins, CW_BINS + 1, wsum);
+    __syncthreads();
+    for (u32 i = t; i < m; i += NT) idx[bins[(u32)(mv[i] >> 32) >> sh] + ord[i]] = (unsigned short)i;
+    __syncthreads();
+    for (u32 i = t; i < m; i += NT) {
+        const u64 key = mv[i];
+        const u32 b = (u32)(key >> 32) >> sh, lo = bins[b], hi = bins[b + 1];
+        u32 p = lo;
+        for (u32 j = lo; j < hi; ++j) p += mv[idx[j]] < key;
+        ord[p] = (unsigned short)i;  // arrival places are no longer read
+    }
+    __syncthreads();
+}
+
+template <WideForm FORM>
+__global__ void __launch_bounds__(cw_threads(FORM)) k_cascade_wide(CascadeArgs A, const u32 *__restrict__ list,
+                                                            const u32 *__restrict__ nlist, u32 MV,
+                                                            u32 *__restrict__ big, u32 *__restrict__ nbig) {
+    extern __shared__ __align__(16) unsigned char cw_smem[];
+    constexpr bool DIRECT = FORM != CW_HASH;
+    constexpr u32 NT = cw_threads(FORM), NW = NT / 32;
+    __shared__ u32 wsum[NW], cm, smax;
+    const u32 t = threadIdx.x, lane = t & 31u, lt = (1u << lane) - 1u, nl = *nlist;
+    u64 *mv = (u64 *)cw_smem;
+    u32 *sl = (u32 *)(mv + MV), *ev = sl + MV, *tc = ev + cw_event_words(FORM, MV);
+    u32 *ec = tc + (DIRECT ? A.K : 4 * MV);  // events per partition; the sweep: tables per warp
+    u32 *keys = ec + 4 * MV, *sq = ev;  // hashed
+    for (u32 li = blockIdx.x; li < nl; li += gridDim.x) {
+        __syncthreads();  // the previous hyperedge's shared state is no longer read
+        const u32 h = list[li];
+        const u64 a = A.off[h], len64 = A.off[h + 1] - a;
+        const u32 len = len64 <= CL_MAX_LEN ? (u32)len64 : 0u, ns = A.nsrc[h], base = cascade_base(A, h);
+        if (DIRECT)
+            for (u32 i = t; i < (FORM == CW_SWEEP ? 1 + 3 * NW : 2) * A.K; i += NT) tc[i] = 0;  // and ec
+        if (t == 0) cm = smax = 0;
+        __syncthreads();
+        u32 rmax = 0;
+        constexpr u32 U = 4;
+        for (u32 k0 = 0; k0 < len; k0 += NT * U) {
+            u32 v[U], q[U];
+            uint2 st[U];
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) v[x] = k0 + NT * x + t < len ? A.pins[a + k0 + NT * x + t] : NONE;
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) st[x] = v[x] != NONE ? A.state[v[x]] : make_uint2(NONE, 0);
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) q[x] = st[x].x != NONE ? A.target[v[x]] : 0;
+#pragma unroll
+            for (u32 x = 0; x < U; ++x) {
+                const bool in = v[x] != NONE, dst = in && k0 + NT * x + t >= ns, mover = st[x].x != NONE;
+                if (DIRECT && in) atomicAdd(&tc[st[x].y - base], dst ? 0x10001u : 1u);
+                const u32 bal = __ballot_sync(0xFFFFFFFFu, mover);
+                u32 at = 0;
+                if (lane == 0 && bal) at = atomicAdd(&cm, (u32)__popc(bal));
+                at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(bal & lt);
+                if (mover && at < MV) {
+                    mv[at] = ((u64)st[x].x << 32) | (dst ? MV_DST : 0u) | v[x];
+                    if (DIRECT) {
+                        const u32 p = st[x].y - base, to = q[x] - base;
+                        sl[at] = p | to << 16;
+                        if (FORM == CW_EVENTS) {
+                            atomicAdd(&ec[p], 1u);
+                            atomicAdd(&ec[to], 1u);
+                        }
+                        rmax = st[x].x > rmax ? st[x].x : rmax;
+                    } else {
+                        sl[at] = st[x].y;
+                        sq[at] = q[x];
+                    }
                 }
             }
-            const u32 cP = act ? cnt[sp] : 0, cQ = act ? cnt[sqx] : 0;
+        }
+        if (FORM == CW_SWEEP) {
+            rmax = __reduce_max_sync(0xFFFFFFFFu, rmax);
+            if (lane == 0) atomicMax(&smax, rmax);
+        }
+        __syncthreads();
+        const u32 m = cm;
+        if (m > MV || len64 > CL_MAX_LEN) {
+            if (t == 0) big[atomicAdd(nbig, 1u)] = h;
+            continue;
+        }
+        if (FORM == CW_SWEEP) {
+            unsigned short *idx = (unsigned short *)ev, *ord = idx + MV;
+            cw_rank_order<NT>(mv, m, smax, ev + MV, idx, ord, wsum);
+            // what each share of the movers changes, then the counts its first one finds
+            const u32 w = t >> 5, per = (m + 32 * NW - 1) / (32 * NW) * 32;
+            const u32 i0 = w * per < m ? w * per : m, i1 = i0 + per < m ? i0 + per : m;
+            u32 *cnt = ec + w * A.K, *pm = ec + (NW + 2 * w) * A.K;
+            for (u32 i = i0 + lane; i < i1; i += 32) {
+                const u32 pq = sl[ord[i]], one = (u32)mv[ord[i]] & MV_DST ? 0x10001u : 1u;
+                atomicSub(&cnt[pq & 0xFFFFu], one);
+                atomicAdd(&cnt[pq >> 16], one);
+            }
+            __syncthreads();
+            for (u32 q = t; q < A.K; q += NT) {
+                u32 run = tc[q];
+#pragma unroll
+                for (u32 k = 0; k < NW; ++k) {
+                    const u32 d = ec[k * A.K + q];
+                    ec[k * A.K + q] = run;
+                    run += d;
+                }
+            }
+            __syncthreads();
+            cl_sweep<true>(A, mv, sl, ord, i0, i1, cnt, pm, pm + A.K, nullptr, A.wfx[h], base);
+            continue;
+        }
+        u32 cap = 32;
+        if (!DIRECT) {
+            while (cap < 4 * m) cap <<= 1;  // at most 4 * MV
+            for (u32 i = t; i < cap; i += NT) {
+                keys[i] = NONE;
+                tc[i] = 0;
+                ec[i] = 0;
+            }
+            __syncthreads();
+            for (u32 i = t; i < m; i += NT) {
+                const u32 sp = hash_find_or_insert(keys, cap - 1, sl[i]), st = hash_find_or_insert(keys, cap - 1, sq[i]);
+                if (sp == NONE || st == NONE) {
+                    atomicExch(A.status, DEV_HASH_FULL);
+                    sl[i] = 0;
+                    continue;
+                }
+                sl[i] = sp | st << 16;
+                atomicAdd(&ec[sp], 1u);
+                atomicAdd(&ec[st], 1u);
+            }
+            __syncthreads();
+            const u32 lm = A.lam[h];
+            for (u32 j = t; j < lm; j += NT) {  // each partition once
+                const u32 s = hash_find(keys, cap - 1, A.cpart[a + j]);
+                if (s != NONE) tc[s] = A.ccnt[a + j] | A.cdcnt[a + j] << 16;
+            }
+        }
+        if (cw_starts<NT>(ec, DIRECT ? A.K : cap, wsum) > CW_PAIRS * m) {
+            if (t == 0) big[atomicAdd(nbig, 1u)] = h;
+            continue;
+        }
+        // events: rank, join, destination pin; ec[b] becomes the end of partition b's
+        for (u32 i = t; i < m; i += NT) {
+            const u64 e = mv[i];
+            const u32 pq = sl[i], x = (u32)(e >> 32) << 2 | ((u32)e & MV_DST ? 1u : 0u);
+            ev[atomicAdd(&ec[pq & 0xFFFFu], 1u)] = x;
+            ev[atomicAdd(&ec[pq >> 16], 1u)] = x | 2u;
+        }
+        __syncthreads();
+        const u32 wh = A.wfx[h];
+        for (u32 b0 = 0; b0 < m; b0 += NT) {
+            const bool act = b0 + t < m;
+            const u64 e = act ? mv[b0 + t] : 0;
+            const u32 pq = act ? sl[b0 + t] : 0, sp = pq & 0xFFFFu, st = pq >> 16, r4 = (u32)(e >> 32) << 2;
+            const auto found = [&](u32 b) {  // pins below, destination pins above
+                u32 x = tc[b];
+                for (u32 j = b ? ec[b - 1] : 0, end = ec[b]; j < end; ++j) {
+                    const u32 y = ev[j];
+                    if (y < r4) x += ((y & 2u) - 1u) * ((y & 1u) << 16 | 1u);
+                }
+                return x;
+            };
+            const u32 cP = act ? found(sp) : 0, cQ = act ? found(st) : 0;
             if (act) {
-                const u32 cp = (u32)((int)(cP & 0xFFFFu) + __popc(m_qp & lt) - __popc(m_pp & lt));
-                const u32 cq = (u32)((int)(cQ & 0xFFFFu) + __popc(m_qq & lt) - __popc(m_pq & lt));
-                const i64 d = leave_gain(A.encourage, wh, cp) - (cq == 0 ? (i64)wh : 0);
+                const i64 d = leave_gain(A.encourage, wh, cP & 0xFFFFu) - ((cQ & 0xFFFFu) == 0 ? (i64)wh : 0);
                 if (d) atomicAdd(&A.g2[(u32)e & ~MV_DST], (unsigned long long)d);
             }
-            if (A.track) {  // warp-uniform
-                bool ep = false, eq = false;
-                if (dst) {
-                    ep = (int)(cP >> 16) + __popc(m_qp & lt & dmask) - __popc(m_pp & lt & dmask) == 1;
-                    eq = (int)(cQ >> 16) + __popc(m_qq & lt & dmask) - __popc(m_pq & lt & dmask) == 0;
-                }
-                const u32 r = (u32)(e >> 32);
-                const u32 pid = DIRECT ? sp + base : ep ? keys[sp] : 0, qid = DIRECT ? sqx + base : eq ? keys[sqx] : 0;
+            if (A.track) {  // uniform over the grid
+                const bool dst = act && ((u32)e & MV_DST), ep = dst && cP >> 16 == 1, eq = dst && cQ >> 16 == 0;
+                const u32 pid = DIRECT ? sp + base : ep ? keys[sp] : 0, qid = DIRECT ? st + base : eq ? keys[st] : 0;
                 __syncwarp();
-                emit_pair(A, ep, pid, eq, qid, r);
+                emit_pair(A, ep, pid, eq, qid, (u32)(e >> 32));
             }
-            __syncwarp();
-            if (act) {  // counts stay within their halves once the whole chunk is in
-                const u32 one = dst ? 0x10001u : 1u;
-                atomicSub(&cnt[sp], one);
-                atomicAdd(&cnt[sqx], one);
-            }
-            __syncwarp();
         }
     }
 }
@@ -4391,9 +4646,15 @@ void setup_refine_kernels(Ctx &c) {
     AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_table<true, GN_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_K * 12));
     AXC_CUDA(cudaFuncSetAttribute(k_cascade_long<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(CL_WARPS * cl_bytes(true, CC_DIRECT_BLOCK_K, 512))));
+                                  (int)(CL_WARPS * cl_bytes(true, CC_DIRECT_BLOCK_K, CL_MOV_DIRECT))));
     AXC_CUDA(cudaFuncSetAttribute(k_cascade_long<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(CL_WARPS * cl_bytes(false, 0, 256))));
+                                  (int)(CL_WARPS * cl_bytes(false, 0, CL_MOV_HASH))));
+    AXC_CUDA(cudaFuncSetAttribute(k_cascade_wide<CW_SWEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)cw_bytes(CW_SWEEP, CW_SWEEP_K, cw_movers(CW_SWEEP))));
+    AXC_CUDA(cudaFuncSetAttribute(k_cascade_wide<CW_EVENTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)cw_bytes(CW_EVENTS, CC_DIRECT_BLOCK_K, cw_movers(CW_EVENTS))));
+    AXC_CUDA(cudaFuncSetAttribute(k_cascade_wide<CW_HASH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)cw_bytes(CW_HASH, 0, cw_movers(CW_HASH))));
     AXC_CUDA(cudaFuncSetAttribute(k_cascade_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CB_DYN_MAX));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_sample<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_DIRECT_UNI * 4));
     AXC_CUDA(cudaFuncSetAttribute(k_gain_sample<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_TAB * 8));
@@ -5071,12 +5332,12 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     if (kw) kway_gains(c, L, lp, A, *kw);
     else run_gains(c, L, lp, A, cs);
     // counters on the device: [0] M movers, [1] 2M size events, [2] inbound transitions,
-    // [3] cascade hyperedges for the block kernel, [4] for the scratch kernel, [5] for the block
-    // kernel's full-size launch after its middle tier, [6] hyperedges holding a mover
+    // [3] cascade hyperedges left by the warp kernel, [4] for the scratch kernel, [5] for the block
+    // kernel's full-size launch after its middle tier, [6] holding a mover, [7] left by the wide kernel
     u32 *cnt = c.arena.alloc<u32>(8);
     AXC_CUDA(cudaMemsetAsync(cnt, 0, 32, c.stream));
     u32 *dM = cnt, *dSE = cnt + 1, *dT = cnt + 2, *dBig = cnt + 3, *dHuge = cnt + 4, *dBig2 = cnt + 5;
-    u32 *dHl = cnt + 6;  // hyperedges holding a mover
+    u32 *dHl = cnt + 6, *dBigW = cnt + 7;  // hyperedges holding a mover; the wide kernel's leftovers
     // small levels: ranking, validity and the best prefix in one block each (SMALL_*)
     const bool small = !slots && rp.K <= VS_MAX_K && n <= (u32)RSS_CAP && rp.copies == 1;
     CopyArgs ca{};
@@ -5187,10 +5448,11 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
             AXC_CUDA(cudaMemcpyAsync(mark, lp.hclass, L.e, cudaMemcpyDeviceToDevice, c.stream));
             LAUNCH(c, k_mover_hedges, (u32)c.sms * 8, 256, 0, C, V, mark);
             LAUNCH(c, k_long_list, cdiv(lp.n_hlong, 256), 256, 0, V, lp.hlong, lp.n_hlong, mark, hlist, dHl);
-            // a warp per hyperedge: as many movers as 512 (hashed 256) leave room for
+            const u32 lim = cascade_block_movers(c);
+            // a warp per hyperedge: as many movers as 512 (hashed 64) leave room for
             u32 mvs = 64;
-            while (mvs < (direct ? 512u : 256u) && mvs < lp.max_len) mvs <<= 1;
-            mvs = std::min(mvs, cascade_block_movers(c));
+            while (mvs < (direct ? CL_MOV_DIRECT : CL_MOV_HASH) && mvs < lp.max_len) mvs <<= 1;
+            mvs = std::min(mvs, lim);
             const u32 per = cl_bytes(direct, C.K, mvs);
             const auto lng = [&](auto kernel) {
                 int per_w = 1;
@@ -5201,21 +5463,42 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
             };
             if (direct) lng(k_cascade_long<true>);
             else lng(k_cascade_long<false>);
+            const u32 *blist = big, *bcount = dBig;
+            const auto wide = [&](auto form) {
+                constexpr WideForm F = decltype(form)::value;
+                u32 mvw = mvs;
+                while (mvw < cw_movers(F) && mvw < lp.max_len) mvw <<= 1;
+                if (lim < CB_MOV_MAX) mvw = std::min(mvw, lim);
+                if (mvw <= mvs) return;  // no hyperedge has more movers than a warp takes
+                u32 *bigw = c.arena.alloc<u32>(L.e);
+                const u32 bytes = cw_bytes(F, C.K, mvw);
+                int per_w = 1;
+                AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_w, k_cascade_wide<F>, cw_threads(F), bytes));
+                LAUNCH_AS(c, "k_cascade_wide", k_cascade_wide<F>,
+                          std::min<u32>(lp.n_hlong, (u32)c.sms * (u32)std::max(per_w, 1)), cw_threads(F), bytes, C, blist,
+                          bcount, mvw, bigw, dBigW);
+                blist = bigw;
+                bcount = dBigW;
+            };
+            if (C.K <= CW_SWEEP_K) wide(std::integral_constant<WideForm, CW_SWEEP>());
+            else if (n < (1u << 30)) {  // an event holds 30 bits of rank
+                if (direct) wide(std::integral_constant<WideForm, CW_EVENTS>());
+                else wide(std::integral_constant<WideForm, CW_HASH>());
+            }
             // block kernel: shared memory sized by the level's largest hyperedge, all resident blocks
             u32 smov = 128;
-            while (smov < lp.max_len && smov < cascade_block_movers(c)) smov <<= 1;
+            while (smov < lp.max_len && smov < lim) smov <<= 1;
             // hashed tables: sized for the level's largest hyperedge within the block's limit
             const u32 stab = direct ? std::max(2 * C.K, 32u)  // tk: the sweep's 2K lane masks
                                     : (u32)std::min<u64>(cascade_cap(std::min<u64>(lp.max_len, rp.K),
                                                                      std::min<u64>(lp.max_len, smov)),
                                                          CB_TAB_HASH);
-            const u32 *blist = big, *bcount = dBig;
             if (smov > CB_MID_MOV || (!direct && stab > CB_MID_TAB)) {  // middle tier first
                 const u32 smid = std::min(smov, CB_MID_MOV), tmid = direct ? stab : std::min(stab, CB_MID_TAB);
                 const size_t dmid = (size_t)smid * 12 + (size_t)tmid * 12;
                 int per_mid = 1;
                 AXC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_mid, k_cascade_block, CB_THREADS, dmid));
-                LAUNCH(c, k_cascade_block, (u32)c.sms * (u32)std::max(per_mid, 1), CB_THREADS, dmid, C, big, dBig, smid,
+                LAUNCH(c, k_cascade_block, (u32)c.sms * (u32)std::max(per_mid, 1), CB_THREADS, dmid, C, blist, bcount, smid,
                        tmid, big2, dBig2);
                 blist = big2;
                 bcount = dBig2;
