@@ -1567,6 +1567,7 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
         {
             const u32 h = lane < deg ? A.touch[t0 + lane] : 0;
             const u32 lm = lane < deg ? A.lam[h] : 0;
+            const u64 ah = warp == 0 && lane < deg ? A.off[h] : 0;  // in flight with lam
             u64 x = lm;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -1576,7 +1577,7 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
             m = __popc(__ballot_sync(0xFFFFFFFFu, lane < deg && x <= GS_SAMPLE));
             if (m) acc = __shfl_sync(0xFFFFFFFFu, x, m - 1);
             if (warp == 0 && lane < m) {
-                s_off[lane] = A.off[h];
+                s_off[lane] = ah;
                 s_w[lane] = UNI ? weight : A.wfx[h];
                 s_ex[lane] = (u32)(x - lm);
                 if (lane == m - 1) s_ex[m] = (u32)x;
@@ -1637,10 +1638,9 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
         if (m <= GS_BLOCK) {
             // the sample's acc entries split evenly over the block: thread t takes entries t,
             // t + GS_BLOCK, ..., finding each one's incidence with a cursor over s_ex
-            constexpr u32 U = 4;
+            constexpr u32 U = 8;
             u32 j = 0;
             for (u32 f0 = threadIdx.x; f0 < acc; f0 += U * GS_BLOCK) {
-                u64 kk[U];
                 u32 xx[U], jj[U], dd[U];
 #pragma unroll
                 for (u32 r = 0; r < U; ++r) {
@@ -1649,14 +1649,15 @@ __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const 
                     if (f < acc) {
                         while (s_ex[j + 1] <= f) ++j;  // s_ex[m] = acc > f ends it below m
                         jj[r] = j;
-                        kk[r] = s_off[j] + (f - s_ex[j]);
-                        xx[r] = A.cpart[kk[r]];
-                        dd[r] = j < nin_u ? A.cdcnt[kk[r]] : 0;
+                        const u64 k = s_off[j] + (f - s_ex[j]);
+                        xx[r] = A.cpart[k];
+                        dd[r] = j < nin_u ? A.cdcnt[k] : 0;
                     }
                 }
 #pragma unroll
                 for (u32 r = 0; r < U; ++r)
-                    if (jj[r] != NONE) put(kk[r], xx[r], s_w[jj[r]], dd[r] > 0);
+                    if (jj[r] != NONE)
+                        put(s_off[jj[r]] + (f0 + r * GS_BLOCK - s_ex[jj[r]]), xx[r], UNI ? weight : s_w[jj[r]], dd[r] > 0);
             }
             if (threadIdx.x < m) wtot = s_w[threadIdx.x];
         } else {
