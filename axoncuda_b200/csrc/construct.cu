@@ -91,7 +91,7 @@ __device__ __forceinline__ u32 warp_incl(u32 x, u32 lane) {
 // One warp per `per` consecutive hyperedges. Those of at most 32 pins are packed into the warp's
 // lanes, a pin each: the lanes holding the same pin of the same hyperedge find each other by a match,
 // no table. Then those up to UQ_WARP_CAP, one after the other, by a table in shared memory.
-__global__ void __launch_bounds__(UQ_WARPS * 32) k_uniq_warp(u32 e, const u64 *__restrict__ off,
+__global__ void __launch_bounds__(UQ_WARPS * 32, 7) k_uniq_warp(u32 e, const u64 *__restrict__ off,
                                                              const u32 *__restrict__ pins, const u32 *__restrict__ nsrc,
                                                              const u32 *__restrict__ groups, int dst_wins, u32 per,
                                                              uint8_t *__restrict__ keep, u32 *__restrict__ cnt,

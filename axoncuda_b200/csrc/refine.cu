@@ -2045,16 +2045,21 @@ __global__ void __launch_bounds__(1024) k_tier_lists(u32 n, u32 K, const u64 *__
 }
 
 // ------------------------------------------------------------------ ranking
-// A node's state in the cascade: {rank, partition}, rank NONE unless it moves. One 8-byte gather
-// tells a hyperedge's pin apart from an earlier mover.
+// A node's state in the cascade: {rank, place}, rank NONE unless it moves. One 8-byte gather tells a
+// hyperedge's pin apart from an earlier mover: the place is the node's partition, and up to
+// STATE_PACK_K partitions a mover's target above it, which larger levels gather besides (scattered
+// loads and adds were three quarters of the long hyperedges' kernel).
+constexpr u32 STATE_PACK_K = 65536;
+__device__ __forceinline__ u32 state_place(u32 part, u32 target, int packed) { return packed ? part | target << 16 : part; }
 // Mover flags, and every node's state without a rank (k_set_rank then ranks the movers) and
 // cascaded gain zeroed.
 __global__ void k_move_flags(u32 n, const u32 *__restrict__ target, const u32 *__restrict__ part,
-                             u32 *__restrict__ flag, uint2 *__restrict__ state, unsigned long long *__restrict__ g2) {
+                             u32 *__restrict__ flag, uint2 *__restrict__ state, unsigned long long *__restrict__ g2,
+                             int packed) {
     u32 v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v < n) {
         flag[v] = target[v] != NONE ? 1u : 0u;
-        state[v] = make_uint2(NONE, part[v]);
+        state[v] = make_uint2(NONE, state_place(part[v], target[v], packed));
         g2[v] = 0;
     }
 }
@@ -2144,7 +2149,8 @@ struct CascadeArgs {
     int encourage;
     const u64 *off;
     const u32 *pins, *nsrc, *wfx, *lam, *cpart, *ccnt, *cdcnt, *part, *target;
-    const uint2 *state;  // [n] {rank, partition}
+    const uint2 *state;  // [n] {rank, place}
+    int packed;          // places hold targets
     unsigned long long *g2;
     // inbound-set transitions (INCC): a (partition, hyperedge) destination count going 0 -> 1 or
     // 1 -> 0 at a move's rank; appended as (partition, rank, +-1)
@@ -2170,6 +2176,11 @@ struct CascadeArgs {
 constexpr u32 MV_DST = 0x80000000u;  // mover flag in the node field: the pin is a destination
 constexpr u32 CC_DIRECT_BLOCK_K = 1024;  // tables indexed by partition up to this many
 
+// The partition of a node and the target of mover v, from its state.
+__device__ __forceinline__ u32 state_part(const CascadeArgs &A, const uint2 &s) { return A.packed ? s.y & 0xFFFFu : s.y; }
+__device__ __forceinline__ u32 state_target(const CascadeArgs &A, const uint2 &s, u32 v) {
+    return A.packed ? s.y >> 16 : A.target[v];
+}
 __device__ __forceinline__ u32 cascade_base(const CascadeArgs &A, u32 h) { return A.ce ? (h / A.ce) * A.K : 0u; }
 
 // The hyperedge's census into the table: partition -> (pins, destination pins). Block- or
@@ -2178,7 +2189,7 @@ __device__ __forceinline__ void cascade_fill(const CascadeArgs &A, u32 h, u64 a,
                                              u32 *td, u32 cap, bool direct, u32 t0, u32 nt) {
     if (!A.lam) {
         const u32 base = cascade_base(A, h);
-        for (u64 k = a + t0; k < b; k += nt) atomicAdd(&tc[A.state[A.pins[k]].y - base], 1u);
+        for (u64 k = a + t0; k < b; k += nt) atomicAdd(&tc[state_part(A, A.state[A.pins[k]]) - base], 1u);
         return;
     }
     for (u32 i = t0; i < lm; i += nt) {
@@ -2382,7 +2393,8 @@ __device__ void cascade_sweep_warp(const CascadeArgs &A, u32 h, const u64 *mv, c
 constexpr u32 CM_LEN = 128;
 constexpr u32 CM_THREADS = 256;
 constexpr u32 CD_STAGE = 512;        // pins a warp of the dense kernel stages at a time
-constexpr u32 CD_MAX_K = 32768;      // partitions its packed states hold
+constexpr u32 CD_MAX_K = 32768;      // partitions its staged words hold
+static_assert(CD_MAX_K <= STATE_PACK_K, "its nodes' places hold targets");
 static_assert(CM_LEN <= CD_STAGE, "every short hyperedge fits the stage");
 
 struct MoverArgs {
@@ -2423,7 +2435,7 @@ __device__ __forceinline__ i64 cascade_incidence(const CascadeArgs &A, u32 h, u3
 #pragma unroll
         for (u32 x = 0; x < U; ++x)
             if (i0 + x < len) {
-                const u32 s = st[x].x < r ? A.target[v[x]] : st[x].y;
+                const u32 s = st[x].x < r ? state_target(A, st[x], v[x]) : state_part(A, st[x]);
                 cp += s == p;
                 cq += s == q;
                 if (TRACK && i0 + x >= ns) {
@@ -2510,10 +2522,10 @@ __device__ __forceinline__ void cascade_dense_body(const CascadeArgs &A, const M
             const u32 hi = lo + __popc(__ballot_sync(0xFFFFFFFFu, lane >= lo && x - b0 <= STAGE));
             const u32 T = __shfl_sync(0xFFFFFFFFu, x, hi - 1) - b0;
             bool movers = false;
-            // pin, state and target are a chain of loads: U pins of a lane go through it together
+            // a pin and its state are a chain of loads: U pins of a lane go through it together
             constexpr u32 U = 4;
             for (u32 f0 = 0; f0 < T; f0 += 32 * U) {
-                u32 v[U], q[U], dst = 0;
+                u32 v[U], dst = 0;
                 uint2 s[U];
 #pragma unroll
                 for (u32 x = 0; x < U; ++x) {
@@ -2535,13 +2547,12 @@ __device__ __forceinline__ void cascade_dense_body(const CascadeArgs &A, const M
 #pragma unroll
                 for (u32 x = 0; x < U; ++x) s[x] = v[x] != NONE ? A.state[v[x]] : make_uint2(NONE, 0);
 #pragma unroll
-                for (u32 x = 0; x < U; ++x) q[x] = s[x].x != NONE ? A.target[v[x]] : 0;
-#pragma unroll
                 for (u32 x = 0; x < U; ++x) {
                     if (v[x] == NONE) continue;
                     const u32 f = f0 + 32 * x + lane;
                     movers |= s[x].x != NONE;
-                    st[f] = make_uint2(s[x].x, s[x].y | q[x] << 15 | (TRACK ? (dst >> x) << 31 : 0u));
+                    const u32 q = s[x].x != NONE ? s[x].y >> 16 : 0u;
+                    st[f] = make_uint2(s[x].x, (s[x].y & 0xFFFFu) | q << 15 | (TRACK ? (dst >> x) << 31 : 0u));
                     nd[f] = v[x];
                 }
             }
@@ -2794,7 +2805,10 @@ __global__ void __launch_bounds__(CL_WARPS * 32) k_cascade_long(CascadeArgs A, c
 #pragma unroll
             for (u32 x = 0; x < U; ++x) st[x] = v[x] != NONE ? A.state[v[x]] : make_uint2(NONE, 0);
 #pragma unroll
-            for (u32 x = 0; x < U; ++x) q[x] = st[x].x != NONE ? A.target[v[x]] : 0;
+            for (u32 x = 0; x < U; ++x) {
+                q[x] = st[x].x != NONE ? state_target(A, st[x], v[x]) : 0;
+                st[x].y = state_part(A, st[x]);
+            }
 #pragma unroll
             for (u32 x = 0; x < U; ++x) {
                 const bool in = v[x] != NONE, dst = in && k0 + 32 * x + lane >= ns, mover = st[x].x != NONE;
@@ -2960,7 +2974,10 @@ __global__ void __launch_bounds__(cw_threads(FORM)) k_cascade_wide(CascadeArgs A
 #pragma unroll
             for (u32 x = 0; x < U; ++x) st[x] = v[x] != NONE ? A.state[v[x]] : make_uint2(NONE, 0);
 #pragma unroll
-            for (u32 x = 0; x < U; ++x) q[x] = st[x].x != NONE ? A.target[v[x]] : 0;
+            for (u32 x = 0; x < U; ++x) {
+                q[x] = st[x].x != NONE ? state_target(A, st[x], v[x]) : 0;
+                st[x].y = state_part(A, st[x]);
+            }
 #pragma unroll
             for (u32 x = 0; x < U; ++x) {
                 const bool in = v[x] != NONE, dst = in && k0 + NT * x + t >= ns, mover = st[x].x != NONE;
@@ -3526,12 +3543,13 @@ __device__ __forceinline__ Best warp_best_prefix(Best b) {
 // sm: RSS_SMEM bytes. Returns the mover count.
 __device__ __forceinline__ u32 rank_small_body(u32 *sm, u32 n, const u32 *target, const i64 *gain, u64 gbound, u32 kb,
                                                const u32 *part, u32 *mv, uint2 *state, unsigned long long *g2) {
+    static_assert(VS_MAX_K <= STATE_PACK_K, "places hold targets");
     __shared__ i64 sh[32];
     u32 M = 0;
     for (u32 b = 0; b < n; b += blockDim.x) {
         const u32 v = b + threadIdx.x;
         const bool f = v < n && target[v] != NONE;
-        if (v < n) { state[v] = make_uint2(NONE, part[v]); g2[v] = 0; }
+        if (v < n) { state[v] = make_uint2(NONE, state_place(part[v], target[v], 1)); g2[v] = 0; }
         i64 tot;
         const i64 incl = block_incl_scan_i64(f ? 1 : 0, sh, tot);
         if (f) {
@@ -4182,6 +4200,7 @@ struct CopyArgs {
     u32 *applied;               // [copies]
     u32 *apply;                 // any copy moved
     u64 omega;
+    int packed;                 // states hold targets
 };
 
 // Stable sort of the block's (key, node) pairs by a 64-bit key of `bits` bits: the low words are in
@@ -4215,7 +4234,7 @@ __global__ void __launch_bounds__(RSS_WARPS * 32) k_copy_rank(CopyArgs A) {
         const u32 i = b + threadIdx.x, v = v0 + i;
         const bool f = i < A.cn && A.target[v] != NONE;
         if (i < A.cn) {
-            A.state[v] = make_uint2(NONE, A.part[v]);
+            A.state[v] = make_uint2(NONE, state_place(A.part[v], A.target[v], A.packed));
             A.g2[v] = 0;
             A.vs[v] = 0;
         }
@@ -5348,19 +5367,20 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     unsigned long long *g2 = c.arena.alloc<unsigned long long>(n);  // cascaded gains, zeroed here
     const u32 kb = bits_for(lp.gain_bound);
     u32 *khi = flag, *klo = c.arena.alloc<u32>(n);  // the flags are spent when the keys are made
+    const int packed = rp.K <= STATE_PACK_K ? 1 : 0;
     if (slots) {
         const u64 pbound = 2 * lp.gain_bound;
         u32 *dMc = c.arena.alloc<u32>(2 * (u64)rp.copies);
         ca = CopyArgs{kw->cn, kw->k, n, target, L.nsize, gain, part, lp.gain_bound, pbound, kb, bits_for(pbound),
                       bits_for(2 * (u64)kw->k * kw->k), mv, dMc, state, g2, c.arena.alloc<i64>(n),
-                      c.arena.alloc<i64>(n), psize, dMc + rp.copies, apply, rp.omega};
+                      c.arena.alloc<i64>(n), psize, dMc + rp.copies, apply, rp.omega, packed};
         dM = dMc;
         LAUNCH(c, k_copy_rank, rp.copies, RSS_WARPS * 32, RSS_SMEM, ca);
     } else if (small) {
         LAUNCH(c, k_rank_small, 1, RSS_WARPS * 32, RSS_SMEM, n, target, gain, lp.gain_bound, kb, part, mv, state,
                g2, dM, dSE);
     } else {
-    LAUNCH(c, k_move_flags, cdiv(n, 256), 256, 0, n, target, part, flag, state, g2);
+    LAUNCH(c, k_move_flags, cdiv(n, 256), 256, 0, n, target, part, flag, state, g2, packed);
     compact_indices_dn(c, flag, mv, n, dM);
     LAUNCH(c, k_move_keys, cdiv(n, 256), 256, 0, mv, dM, gain, lp.gain_bound, khi, klo);
     if (kb > 32) {
@@ -5420,7 +5440,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     {
         CascadeArgs C;
         C.e = L.e; C.encourage = rp.encourage ? 1 : 0; C.off = L.off; C.pins = L.pins; C.nsrc = L.nsrc;
-        C.wfx = wfx; C.lam = cs.lam; C.cpart = cs.part; C.ccnt = cs.cnt; C.cdcnt = cs.dcnt; C.state = state;
+        C.wfx = wfx; C.lam = cs.lam; C.cpart = cs.part; C.ccnt = cs.cnt; C.cdcnt = cs.dcnt; C.state = state; C.packed = packed;
         C.part = part; C.target = target; C.g2 = g2;
         C.track = track ? 1 : 0; C.tp = tp; C.tr = tr; C.tdv = tdv; C.dT = dT; C.tcap = tcap;
         C.tdense = tdense; C.dense_stride = n;
@@ -5431,9 +5451,12 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
         const bool direct = C.K <= CC_DIRECT_BLOCK_K;
         size_t m1 = c.arena.mark();
         const bool longs = lp.max_len > CM_LEN;
-        // a warp of the dense kernel looks at 32 hyperedges, or fewer where that leaves the GPU idle
+        // a warp of the dense kernel looks at 32 hyperedges, or fewer where that leaves the GPU idle or
+        // gives some warps several times the work of others (at 60 pins a hyperedge and 32 to a warp a
+        // fifth of the warps were busy on average)
         u32 per_warp = 32;
         while (per_warp > 4 && L.e / per_warp < (u32)c.sms * 16) per_warp >>= 1;
+        while (per_warp > 2 && per_warp * lp.short_pins > 192ull * L.e) per_warp >>= 1;
         // few nodes of many short incidences: a lane of the mover kernel would walk through several
         // of them one after the other while the dense kernel reads the whole level in a few microseconds
         const bool always = L.P / n > 128 && lp.short_pins <= (2u << 20);
@@ -5796,7 +5819,7 @@ static u32 small_rounds(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 
     S.dM = ctl + 3;
     S.state = (uint2 *)c.arena.alloc<u64>(n);
     S.D.e = L.e; S.D.encourage = 1; S.D.off = L.off; S.D.pins = L.pins; S.D.nsrc = L.nsrc; S.D.wfx = wfx;
-    S.D.part = part; S.D.target = target; S.D.state = S.state;
+    S.D.part = part; S.D.target = target; S.D.state = S.state; S.D.packed = 1;
     S.D.g2 = c.arena.alloc<unsigned long long>(n);
     S.D.track = track ? 1 : 0; S.D.dT = ctl + 4; S.D.tdense = tdense; S.D.dense_stride = n; S.D.status = c.d_status;
     S.D.K = K;
