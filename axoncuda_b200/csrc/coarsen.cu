@@ -29,6 +29,9 @@ constexpr u32 RT_BLK2_W = 8192;    // block tier 2: table 16384 slots (192 KiB)
 // second try of the larger tier (c.tune.rate_mid, 8192: 96 KiB, two blocks per SM) are tunable.
 constexpr u32 RT_WARPS = 4;
 constexpr u32 RT_BLOCK = 256;
+// Threads for the tables that leave room for one to three blocks per SM: the shared adds' latency wants
+// more warps than 256 threads give (20 x 5000 network, 128 parts: 40.9 ms of rating, 33.5 with 512).
+constexpr u32 RT_WIDE = 512;
 
 __global__ void k_rate_work(u32 n, const u64 *__restrict__ toff, const u32 *__restrict__ touch,
                             const u64 *__restrict__ off, u64 *__restrict__ work) {
@@ -266,7 +269,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) k_rate_warp(RateArgs A, const u
     }
 }
 
-constexpr u32 RT_SEL = (RT_BLOCK / 32) * AXC_MAX_CANDIDATES;  // shared slots of the block selection
+constexpr u32 RT_SEL = (RT_WIDE / 32) * AXC_MAX_CANDIDATES;  // shared slots of the block selection
 
 // The top-cnc candidates of node u from its table (keys, sc, cm) of `cap` slots; block-wide.
 // Each warp reduces its lanes' lists to its own top cnc with shuffles into red[warp * cnc ..];
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(RT_BLOCK) k_rate_split_select(RateArgs A, cons
 // *d_retry.
 // With `d_nl` set the list length is read from device memory (at most nlist).
 template <int TC, bool CM>
-__global__ void __launch_bounds__(RT_BLOCK) k_rate_block(RateArgs A, const u32 *__restrict__ list, u32 nlist,
+__global__ void __launch_bounds__(RT_WIDE) k_rate_block(RateArgs A, const u32 *__restrict__ list, u32 nlist,
                                                         u32 cap_max, u32 *gtab, const u32 *__restrict__ d_nl,
                                                         u32 *__restrict__ retry, u32 *__restrict__ d_retry,
                                                         u32 *gused) {
@@ -795,7 +798,7 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
     // Nodes' work bounds count pins with multiplicity; their distinct neighbours are usually far
     // fewer. A first launch tries rt_try-slot tables (more blocks per SM); nodes that outgrow
     // theirs are redone by a second launch with the tier's full tables.
-    // A node that outgrows an rt_try table retries at rt_mid slots (two blocks per SM) when the
+    // A node that outgrows an rt_try table retries at rt_mid slots (two or three blocks per SM) when the
     // tier's tables are larger still, and only past that at the tier's full size.
     u32 *retry = c.arena.alloc<u32>(n), *retry2 = c.arena.alloc<u32>(n);
     u32 *d_retry = (u32 *)(dc + 4), *d_retry2 = d_retry + 1;  // dc[4] was read already
@@ -821,13 +824,13 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
                (const u32 *)nullptr, retry, d_retry, (u32 *)nullptr);
         const u32 *rl = retry, *dn = d_retry;
         if (cap_full > rt_mid) {
-            RATE_LAUNCH(c, k_rate_block, cnc, cm, std::min<u32>(cnt, (u32)c.sms * 2), RT_BLOCK, words * rt_mid * 4, A, rl, cnt, rt_mid,
+            RATE_LAUNCH(c, k_rate_block, cnc, cm, std::min<u32>(cnt, (u32)c.sms * 3), RT_WIDE, words * rt_mid * 4, A, rl, cnt, rt_mid,
                    (u32 *)nullptr, dn, retry2, d_retry2, (u32 *)nullptr);
             rl = retry2;
             dn = d_retry2;
         }
         const u32 grid = std::min<u32>(cnt, (u32)c.sms * 2);
-        RATE_LAUNCH(c, k_rate_block, cnc, cm, grid, RT_BLOCK, words * cap_full * 4, A, rl, cnt, cap_full, (u32 *)nullptr, dn,
+        RATE_LAUNCH(c, k_rate_block, cnc, cm, grid, RT_WIDE, words * cap_full * 4, A, rl, cnt, cap_full, (u32 *)nullptr, dn,
                (u32 *)nullptr, (u32 *)nullptr, (u32 *)nullptr);
     };
     block_tier(list2, nl, cap1);
