@@ -3919,7 +3919,10 @@ struct KwGain {
 // Best target of node u from the lanes' connectivities: lane `own` of a group of G holds those of
 // its partitions own, own + G, ... (conn[x]); the group's lane 0 writes the move. A partition
 // without connectivity gains at most saving - wtot <= 0, so presence needs no test.
-template <u32 G, u32 C, class T>
+// EARLY: a partition's gain is looked at before its size, and a group without a gain skips the
+// reduction, as most do in the later rounds (the plane kernels, which come here once per hundreds of
+// incidences, got slower by it: 110 -> 130 us a launch).
+template <u32 G, u32 C, class T, bool EARLY = false>
 __device__ __forceinline__ void kw_move(const GainArgs &A, u32 u, u32 base, u32 pl, u32 k, u32 own, u32 gmask,
                                         const T (&conn)[C], T saving, T wtot) {
     Cand best{INT64_MIN, 0};
@@ -3927,11 +3930,15 @@ __device__ __forceinline__ void kw_move(const GainArgs &A, u32 u, u32 base, u32 
 #pragma unroll
     for (u32 x = 0; x < C; ++x) {
         const u32 q = own + G * x;
-        if (q >= k || q == pl || conn[x] == 0) continue;
+        const i64 g = (i64)saving - ((i64)wtot - (i64)conn[x]);
+        if (q >= k || q == pl || (EARLY ? g <= 0 : conn[x] == 0)) continue;
         if (A.psize[base + q] + need > A.omega) continue;
-        const Cand c{(i64)saving - ((i64)wtot - (i64)conn[x]),
-                     ((u64)mix32(base + q + A.round + A.seed) << 32) | (u64)(~(base + q))};
+        const Cand c{g, ((u64)mix32(base + q + A.round + A.seed) << 32) | (u64)(~(base + q))};
         if (cand_better(c, best)) best = c;
+    }
+    if (EARLY && !__any_sync(gmask, best.g > 0)) {
+        if (own == 0) write_move(A, u, best);
+        return;
     }
 #pragma unroll
     for (u32 o = G / 2; o > 0; o >>= 1) {
@@ -3961,39 +3968,27 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain(GainArgs A0, KwGain V)
     T conn[C], saving = 0, wtot = 0;
 #pragma unroll
     for (u32 x = 0; x < C; ++x) conn[x] = 0;
-    // batches of U incidences, the last one's remainder included, with their loads in flight together
-    constexpr u32 U = MW <= 2 ? 4 : 2;
-    for (u32 j = 0; j < deg; j += U) {
-        u32 h[U], w[U], any[U][MW], sg[U];
-#pragma unroll
-        for (u32 i = 0; i < U; ++i) h[i] = j + i < deg ? A.touch[t0 + j + i] : NONE;
-#pragma unroll
-        for (u32 i = 0; i < U; ++i) {
-            w[i] = h[i] == NONE ? 0u : V.uni ? V.weight : A.wfx[h[i]];
-            sg[i] = 0;
-#pragma unroll
-            for (u32 x = 0; x < MW; ++x) any[i][x] = 0;
-            if (h[i] == NONE) continue;
-            const u32 *r = V.rec + (u64)h[i] * (2 * MW);
-            if constexpr (MW == 1) {
-                const uint2 v = *(const uint2 *)r;
-                any[i][0] = v.x;
-                sg[i] = v.y;
-            } else {
-                load_words<MW>(r, any[i]);
-                sg[i] = r[MW + (pl >> 5)];
-            }
+#pragma unroll 4
+    for (u32 j = 0; j < deg; ++j) {
+        const u32 h = A.touch[t0 + j], w = V.uni ? V.weight : A.wfx[h];
+        const u32 *r = V.rec + (u64)h * (2 * MW);
+        u32 any[MW];
+        u32 sg;
+        if constexpr (MW == 1) {
+            const uint2 v = *(const uint2 *)r;
+            any[0] = v.x;
+            sg = v.y;
+        } else {
+            load_words<MW>(r, any);
+            sg = r[MW + (pl >> 5)];
         }
+        wtot += w;
+        if ((sg >> (pl & 31u)) & 1u) saving += w;
 #pragma unroll
-        for (u32 i = 0; i < U; ++i) {
-            wtot += w[i];
-            if ((sg[i] >> (pl & 31u)) & 1u) saving += w[i];
-#pragma unroll
-            for (u32 x = 0; x < C; ++x)
-                if ((any[i][x] >> own) & 1u) conn[x] += w[i];
-        }
+        for (u32 x = 0; x < C; ++x)
+            if ((any[x] >> own) & 1u) conn[x] += w;
     }
-    kw_move<G, C, T>(A, u, base, pl, V.k, own, gmask, conn, saving, wtot);
+    kw_move<G, C, T, true>(A, u, base, pl, V.k, own, gmask, conn, saving, wtot);
 }
 
 // At most 4 partitions: a group of G lanes per node takes the incidences side by side, each lane
@@ -4009,25 +4004,15 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain_few(GainArgs A0, KwGai
     const u64 t0 = A.toff[u];
     const u32 deg = (u32)(A.toff[u + 1] - t0);
     T conn[4] = {0, 0, 0, 0}, saving = 0, wtot = 0;
-    constexpr u32 U = 4;  // incidences of a lane whose loads are in flight together
-    for (u32 j = own; j < deg; j += G * U) {
-        u32 h[U], w[U];
-        uint2 r[U];
+#pragma unroll 2
+    for (u32 j = own; j < deg; j += G) {
+        const u32 h = A.touch[t0 + j], w = V.uni ? V.weight : A.wfx[h];
+        const uint2 r = *(const uint2 *)(V.rec + (u64)h * 2);
+        wtot += w;
+        if ((r.y >> pl) & 1u) saving += w;
 #pragma unroll
-        for (u32 i = 0; i < U; ++i) h[i] = j + G * i < deg ? A.touch[t0 + j + G * i] : NONE;
-#pragma unroll
-        for (u32 i = 0; i < U; ++i) {
-            w[i] = h[i] == NONE ? 0u : V.uni ? V.weight : A.wfx[h[i]];
-            r[i] = h[i] == NONE ? make_uint2(0, 0) : *(const uint2 *)(V.rec + (u64)h[i] * 2);
-        }
-#pragma unroll
-        for (u32 i = 0; i < U; ++i) {
-            wtot += w[i];
-            if ((r[i].y >> pl) & 1u) saving += w[i];
-#pragma unroll
-            for (u32 x = 0; x < 4; ++x)
-                if ((r[i].x >> x) & 1u) conn[x] += w[i];
-        }
+        for (u32 x = 0; x < 4; ++x)
+            if ((r.x >> x) & 1u) conn[x] += w;
     }
     __syncwarp(gmask);
 #pragma unroll
@@ -4038,7 +4023,7 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain_few(GainArgs A0, KwGai
         for (u32 x = 0; x < 4; ++x) conn[x] += __shfl_xor_sync(gmask, conn[x], o);
     }
     T mine[1] = {own == 0 ? conn[0] : own == 1 ? conn[1] : own == 2 ? conn[2] : own == 3 ? conn[3] : (T)0};
-    kw_move<G, 1, T>(A, u, base, pl, V.k, own, gmask, mine, saving, wtot);
+    kw_move<G, 1, T, true>(A, u, base, pl, V.k, own, gmask, mine, saving, wtot);
 }
 
 // One block per node (heavy nodes and small levels): each warp takes every eighth incidence with a
