@@ -47,9 +47,10 @@ __global__ void k_rate_work(u32 n, const u64 *__restrict__ toff, const u32 *__re
 }
 
 // The four tiers' node lists by work bound (limits hi[0..3), the rest in the last), the sum of the
-// bounds (dc[4]) and their maximum (dc[5]) in one pass.
-__global__ void __launch_bounds__(1024) k_rate_tiers(u32 n, const u64 *__restrict__ work, u64 hi0, u64 hi1, u64 hi2,
-                                                     u32 *l0, u32 *l1, u32 *l2, u32 *l3, u64 *__restrict__ dc) {
+// bounds (dc[4]), their maximum (dc[5]) and the largest inbound count (dc[6]) in one pass.
+__global__ void __launch_bounds__(1024) k_rate_tiers(u32 n, const u64 *__restrict__ work, const u32 *__restrict__ nin,
+                                                     u64 hi0, u64 hi1, u64 hi2, u32 *l0, u32 *l1, u32 *l2, u32 *l3,
+                                                     u64 *__restrict__ dc) {
     __shared__ u32 sh[33];
     const u32 u = blockIdx.x * blockDim.x + threadIdx.x;
     const u64 x = u < n ? work[u] : 0;
@@ -62,7 +63,9 @@ __global__ void __launch_bounds__(1024) k_rate_tiers(u32 n, const u64 *__restric
         if (t == i) lists[i][at] = u;
     }
     const u64 s = warp_sum(x), m = warp_max_u64(x);
+    const u32 in = __reduce_max_sync(0xFFFFFFFFu, u < n ? nin[u] : 0u);
     if ((threadIdx.x & 31) == 0) {
+        if (in > *(volatile u64 *)&dc[6]) atomicMax((unsigned long long *)&dc[6], (unsigned long long)in);
         if (s) atomicAdd((unsigned long long *)&dc[4], (unsigned long long)s);
         if (m) atomicMax((unsigned long long *)&dc[5], (unsigned long long)m);
     }
@@ -753,14 +756,14 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
     u32 *lists[4];
     for (auto &l : lists) l = c.arena.alloc<u32>(n);
     // device counters, read back in one round trip: [0..3] tier sizes, [4] work sum, [5] work max
-    u64 *dc = c.arena.alloc<u64>(6);
-    AXC_CUDA(cudaMemsetAsync(dc, 0, 48, c.stream));
+    u64 *dc = c.arena.alloc<u64>(7);
+    AXC_CUDA(cudaMemsetAsync(dc, 0, 56, c.stream));
     fill_u32(c, pairs, NONE, (u64)n * cnc);
     LAUNCH(c, k_rate_work, cdiv((u64)n * 32, 256), 256, 0, n, L.toff, L.touch, L.off, work);
-    LAUNCH(c, k_rate_tiers, cdiv(n, 1024), 1024, 0, n, work, (u64)RT_WARP_W, (u64)RT_BLK1_W, (u64)RT_BLK2_W, lists[0],
+    LAUNCH(c, k_rate_tiers, cdiv(n, 1024), 1024, 0, n, work, L.nin, (u64)RT_WARP_W, (u64)RT_BLK1_W, (u64)RT_BLK2_W, lists[0],
            lists[1], lists[2], lists[3], dc);
-    u64 h[6];
-    fetch(c, h, dc, 48);
+    u64 h[7];
+    fetch(c, h, dc, 56);
     if (pin_visits) *pin_visits = h[4];
     const u32 *list = lists[0], *list2 = lists[1], *list3 = lists[2], *list4 = lists[3];
     // Kernel timer: algorithmic bytes of the block tiers, 4 per pin visit (the pin id) and 8 per
@@ -777,9 +780,9 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
         for (int t = 0; t < 2; ++t)  // the heavy tier counts below, if it runs on k_rate_block
             if (h[1 + t]) c.prof_bytes += 4 * tier_visits[t] + 8ull * cnc * h[1 + t];
     }
-    // without an inbound limit (delta 2^31 - 1) the shared counts decide nothing while the level has
-    // fewer than 2^30 hyperedges
-    const bool cm = delta < 0x7FFFFFFFu || (u64)L.e >= (1ull << 30);
+    // the shared counts decide nothing where no pair's inbound counts add up to more than the limit, as
+    // on the first levels (a third of a slot's bytes, and an atomic per inbound pin)
+    const bool cm = 2 * h[6] > delta && (delta < 0x7FFFFFFFu || (u64)L.e >= (1ull << 30));
     const u32 words = cm ? 3 : 2;  // of a hashed slot
     // tier: one warp per node, table in static smem
     u32 nl = (u32)h[0];
