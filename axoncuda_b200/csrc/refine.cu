@@ -2,17 +2,16 @@
 // integer arithmetic and a sparse per-hyperedge census instead of the dense E x K table).
 //
 // One round:
-//  1. census: for every hyperedge the partitions among its pins with (pins, destination pins),
-//     in first-occurrence order (hashed) or ascending order (partition-indexed, K <= 256);
-//     partition sizes and distinct-inbound counts.
+//  1. census: for every hyperedge the partitions among its pins with (pins, destination pins), a
+//     set in no particular order; partition sizes and distinct-inbound counts. k-way rounds without
+//     an inbound limit keep two masks per hyperedge instead (k_kway_records).
 //  2. gains: every node's best feasible target among the partitions adjacent to it; only moves
-//     with positive gain are proposed. With K <= 256 from per-hyperedge partition bitmasks
-//     (O(K/32) per incidence and lane), else from hash tables (O(lambda) per incidence).
-//  3. rank by (gain desc, id asc).
-//  4. cascade: each move's gain recomputed assuming every better-ranked move is applied, by a
-//     sweep over each hyperedge's movers in rank order (O(pins) instead of the reference's
-//     per-move re-read of every incident hyperedge), 32 movers at a time per warp with exact
-//     prefix counts.
+//     with positive gain are proposed. From per-hyperedge partition masks (O(K/32) per incidence
+//     and lane) or from sums by partition or hash (O(lambda) per incidence).
+//  3. rank by (gain desc, id asc), k-way in pairs.
+//  4. cascade: each move's gain recomputed assuming every better-ranked move is applied. Hyperedges
+//     of at most CM_LEN pins compare ranks pin by pin; longer ones gather their movers once and
+//     sweep over them in rank order with exact prefix counts, or count events by partition.
 //  5. prefix sums of cascaded gains; size-excess and inbound-validity of every prefix from sorted
 //     event streams (sources/refinement.cu:239-491); best prefix by best_move_functor
 //     (headers/data_types.cuh:113-136); apply when valid with non-negative prefix gain.
@@ -104,6 +103,7 @@ constexpr u32 CS_STAGE = 512;        // pins a warp stages
 constexpr u32 CS_THREADS = 256;
 constexpr u32 CS_DIRECT_K = 16384;
 
+// Bound by the partitions' gathers. Measured: 1M nets 651 us by a warp and a table per net, 92.
 __global__ void __launch_bounds__(CS_THREADS) k_census_short(u32 e, CensusArgs A, u32 per_warp) {
     constexpr u32 NW = CS_THREADS / 32;
     __shared__ u32 sp[NW][CS_STAGE];
@@ -190,6 +190,8 @@ __global__ void __launch_bounds__(CS_THREADS) k_census_short(u32 e, CensusArgs A
     }
 }
 
+// Measured with k_census_mid: 20 x 5000 network at some 10k partitions 1060 us by hash tables sized
+// by the hyperedge, 185 + 338 (34M gathers).
 __global__ void __launch_bounds__(CS_WARPS * 32) k_census_warp(u32 e, CensusArgs A, u32 per_warp) {
     __shared__ u32 tk[CS_WARPS][2 * CS_WARP_CAP], tv[CS_WARPS][2 * CS_WARP_CAP];
     constexpr u32 R = CS_WARP_CAP / 32;
@@ -381,7 +383,7 @@ __global__ void k_census_block(const u32 *__restrict__ list, u32 nlist, CensusAr
 
 // Partition-indexed census for K <= CD_K: the counters are K-slot arrays indexed by partition id,
 // so a hyperedge of any length fits in shared memory and needs no hashing. Entries are emitted in
-// ascending partition order (the hashed census emits them in order of first occurrence; every
+// ascending partition order (the hashed census emits them in no order; every
 // consumer reads them as a set). With A.save set, every pin then adds its saving from the count
 // of its own partition.
 constexpr u32 CD_K = 256;
@@ -667,6 +669,8 @@ constexpr u32 PI_THREADS = 1024;
 // k_part_inbound for K <= PI_SMEM_K: groups of G lanes stride over the hyperedges and count into a
 // shared histogram, which the block adds to pinb once: one large block per SM, since every block
 // adds up to K words to the same places. G follows the mean length (a census has no more entries).
+// Measured: 1M nets 495 us with a warp per net, 44; 20 x 5000 network 292 us by global atomics, 159
+// in shared memory.
 template <u32 G>
 __global__ void __launch_bounds__(PI_THREADS) k_part_inbound_smem(u32 e, const u64 *__restrict__ off,
                                                                   const u32 *__restrict__ lam,
@@ -730,6 +734,7 @@ __device__ __forceinline__ GainArgs gain_args_now(const GainArgs &A0) {
 // Per-level bounds of a node's gain work: the partitions adjacent to it in any round number at
 // most min(sum over incident hyperedges of min(|e|, K), K), which sizes its accumulator table; the
 // sum of incident weights bounds its gain.
+// Measured: 1M nodes 169 us a level, 664 at the first (an atomic per node at one address), 45.
 template <u32 G>
 __global__ void __launch_bounds__(256) k_gain_bounds(u32 n, u32 K, const u64 *__restrict__ toff,
                                                      const u32 *__restrict__ touch, const u64 *__restrict__ off,
@@ -1085,6 +1090,7 @@ __global__ void __launch_bounds__(GN_BLOCK) k_gain_mask_block(GainArgs A0, const
 
 // WIDE: some node's incident weights pass 2^32, and a connectivity is a low and a high word (64-bit
 // shared adds would be compare-and-swap loops).
+// Bound by latency (touch list, census offsets, entries). Measured: 120k-node netlist 57 us, 46.
 template <bool WIDE>
 __global__ void __launch_bounds__(GN_WARPS * 32) k_gain_warp(GainArgs A0, const u32 *__restrict__ list, u32 nl,
                                                              const u64 *__restrict__ work) {
@@ -1127,7 +1133,7 @@ __global__ void __launch_bounds__(GN_WARPS * 32) k_gain_warp(GainArgs A0, const 
 // include/axc.h in two kernels:
 //  - k_gain_sample (one block per node, the sample table in shared memory) finds the sample
 //    prefix, accumulates the sampled connectivity and, when the prefix is the whole node, settles
-//    the node exactly as k_gain_block would; otherwise it writes the node's candidates;
+//    the node exactly; otherwise it writes the node's candidates;
 //  - k_cands_warp / k_cands_block (one warp or block per hyperedge holding such a node) put the
 //    hyperedge's census in a hash table and add, for each such pin, the hyperedge's weight to its
 //    candidates' sums, and k_cands_best picks each node's best feasible candidate. A node's exact
@@ -1243,6 +1249,7 @@ __device__ __forceinline__ void census_flat(const GainArgs &A, u32 u, u32 first,
 //    candidate's connectivity is then a count of incidences whose K-bit mask holds it. A lane owns
 //    one mask word and adds whole words into bit-plane counters (carry-save adders, eight
 //    incidences at a time): 32 partitions per instruction, whatever the number of entries.
+// Measured: 120k-node netlist 134 us hashed, 64 (64 threads) and 68 (256).
 template <bool WIDE, u32 NT>
 __global__ void __launch_bounds__(NT) k_gain_table(GainArgs A0, const u32 *__restrict__ list, u32 nl) {
     const GainArgs A = gain_args_now(A0);
@@ -1370,6 +1377,8 @@ __device__ __forceinline__ void plane_merge(u32 (&pl)[NP], u32 o) {
 }
 
 // One block per node; MWP, the power of two from MW up, lanes per incidence. w: the level's weight.
+// Bound by issue: about five instructions per mask word. Measured: 20 x 500 network, 10k nodes of
+// some 340 incidences at 500 partitions, 3056 us hashed, 107.
 template <u32 MWP>
 __global__ void __launch_bounds__(GN_BLOCK) k_gain_planes(GainArgs A0, const u32 *__restrict__ list, u32 nl,
                                                          const u32 *__restrict__ mask, const u32 *__restrict__ dmask,
@@ -1504,6 +1513,8 @@ __global__ void k_part_room(u32 K, u32 omega, u32 delta, const u64 *__restrict__
 // UNI: every hyperedge has the weight w. DIRECT: slots are partitions (T = K), else a hash table of
 // T = GS_TAB slots. One block per node at a time; the table is empty between nodes: the last scan
 // of a node clears it.
+// Bound by the shared adds and the block's barriers. Measured: 20 x 5000 network 1422 us (and 315
+// for the middling nodes' own kernel), 529 a launch, two launches a round.
 template <bool UNI, bool DIRECT>
 __global__ void __launch_bounds__(GS_BLOCK, 4) k_gain_sample(GainArgs A0, const u32 *__restrict__ list, u32 nl, CandAcc C,
                                                          u32 T, u32 weight, const u32 *__restrict__ room) {
@@ -1878,6 +1889,8 @@ __device__ __forceinline__ void cv_pin(const CandAcc &C, u32 v, bool io, u32 w, 
 
 // One warp per hyperedge of at most CV_WARP_LEN pins; skipped when no pin has candidates. BITS: mw
 // words per bitmap.
+// Bound by the candidates' 32-byte gathers and the 64-bit atomics. Measured with k_cands_block: 20
+// x 5000 network 5060 us with nine hash probes and up to eighteen atomics per pin, 159 + 297.
 template <bool BITS>
 __global__ void __launch_bounds__(CV_WARPS * 32) k_cands_warp(GainArgs A, CandAcc C, u32 e, u32 mw) {
     extern __shared__ u32 cv_dyn[];
@@ -2014,6 +2027,7 @@ __device__ __forceinline__ u32 gain_tier(u32 n, u32 K, u64 wk, u64 deg, u32 kway
 }
 // The tiers' node lists, the largest work bound over all nodes (out[0]) and over the block tier
 // (out[1]), and the largest degree (out[2]); cnt: three list counts in u64 words.
+// Measured: 1M nodes 12 us, in place of a launch and a scan per list.
 __global__ void __launch_bounds__(1024) k_tier_lists(u32 n, u32 K, const u64 *__restrict__ work,
                                                      const u64 *__restrict__ toff, u32 kway, u32 *l0, u32 *l1, u32 *l2,
                                                      u64 *__restrict__ cnt, unsigned long long *__restrict__ out) {
@@ -2451,6 +2465,8 @@ __device__ __forceinline__ i64 cascade_incidence(const CascadeArgs &A, u32 h, u3
 // Movers of at most CM_HEAVY * G incidences (a lane's share stays bounded); the others take a block
 // each (k_cascade_movers_heavy).
 constexpr u32 CM_HEAVY = 128;
+// Bound by latency; its cost follows the movers. Measured with the dense kernel, per round: 200k
+// nodes 64 parts 658 us by a sorted sweep per net, 67; 1M nodes 16 parts 656, 93.
 template <u32 G, bool TRACK>
 __global__ void __launch_bounds__(CM_THREADS) k_cascade_movers(CascadeArgs A, MoverArgs V) {
     const u32 lane = threadIdx.x & 31u, gl = lane & (G - 1);
@@ -2601,6 +2617,8 @@ __device__ __forceinline__ void cascade_dense_body(const CascadeArgs &A, const M
     }
 }
 
+// Bound by issue on nets of a few pins (about 170 instructions per 32 pins, then ten per pin and
+// mover). Measured: 20 x 5000 network 75 us (137 with up to 32 hyperedges a warp).
 template <bool TRACK>
 __global__ void __launch_bounds__(CM_THREADS) k_cascade_dense(CascadeArgs A, MoverArgs V) {
     constexpr u32 NW = CM_THREADS / 32;
@@ -2629,6 +2647,8 @@ __global__ void k_mover_hedges(CascadeArgs A, MoverArgs V, uint8_t *__restrict__
         }
     }
 }
+// Measured: 100k hyperedges 4 us; with k_mover_hedges 190 before, when every incidence's flag was
+// stored.
 __global__ void k_long_list(MoverArgs V, const u32 *__restrict__ longs, u32 nlong, const uint8_t *__restrict__ mark,
                             u32 *__restrict__ list, u32 *__restrict__ nlist) {
     const bool all = cascade_dense(V);
@@ -2773,6 +2793,9 @@ __device__ __forceinline__ void cl_sweep(const CascadeArgs &A, const u64 *mv, co
     }
 }
 
+// Bound by scattered loads and adds (L1 at 82% of its peak). Measured per round, short hyperedges
+// included: 20 x 5000 network, 128 parts 353 us in a warp and 1710 in a block kernel, now 500, 248
+// in the wide and 120 in the dense one; 20 x 500 595, now 105, 56 and 64.
 template <bool DIRECT>
 __global__ void __launch_bounds__(CL_WARPS * 32) k_cascade_long(CascadeArgs A, const u32 *__restrict__ list,
                                                                const u32 *__restrict__ nlist, u32 MV, u32 per,
@@ -2942,6 +2965,8 @@ __device__ __forceinline__ void cw_rank_order(const u64 *mv, u32 m, u32 rmax, u3
     __syncthreads();
 }
 
+// Measured: 20 x 5000 network, 128 parts, 248 us where the block kernel took 693; 20 x 500 (500
+// partitions) 56 a round by events, 155 by the block and scratch kernels.
 template <WideForm FORM>
 __global__ void __launch_bounds__(cw_threads(FORM)) k_cascade_wide(CascadeArgs A, const u32 *__restrict__ list,
                                                             const u32 *__restrict__ nlist, u32 MV,
@@ -3818,6 +3843,8 @@ __device__ __forceinline__ void kw_store(u32 *rec, const u32 (&any)[MW], const u
 
 // The records of the flagged hyperedges, which are unflagged. A warp looks at per_warp hyperedges:
 // a lane does its own when it has at most KW_SHORT pins, the warp the others one by one.
+// Measured: the multi-start of 200k nodes, 64 parts, 896 partitions in all: 1074 us a hashed
+// census, 8 with only the moved nodes' hyperedges rewritten.
 template <u32 MW>
 __global__ void __launch_bounds__(KW_THREADS) k_kway_records(KwArgs A) {
     const u32 lane = threadIdx.x & 31u;
@@ -3953,6 +3980,8 @@ __device__ __forceinline__ void kw_move(const GainArgs &A, u32 u, u32 base, u32 
 // One group of G lanes per node (G a power of two, at least k for one word): lane l owns
 // partitions l, l + G, ... (C of them) and reads every incidence's record, the same addresses across the group. T: u32 when
 // no node's incident weights pass 2^32, else u64.
+// Bound by issue and the records' L2 reads. Measured: the same multi-start 1970 us hashed, 46 to
+// 70; 1M nodes 16 parts 218 from the census' masks, 101.
 template <u32 MW, u32 G, class T>
 __global__ void __launch_bounds__(KW_THREADS) k_kway_gain(GainArgs A0, KwGain V) {
     static_assert(MW == 1 || G == 32, "one word: a lane per partition; more: a lane per bit of each");
@@ -4078,6 +4107,8 @@ __global__ void __launch_bounds__(KW_THREADS) k_kway_gain_block(GainArgs A0, KwG
 // the incidences. NP: planes, enough for a warp's incidences.
 constexpr u32 KP_PLANES = 11, KP_PLANES_BLOCK = 14;
 static_assert(KW_WARP_DEG < (1u << KP_PLANES), "a warp's counters hold its node's incidences");
+// Measured: 20 x 5000 network, 128 parts 1069 us from the census' masks, 109 and 155 (light and
+// heavy nodes).
 template <u32 MW, bool BLOCK>
 __global__ void __launch_bounds__(KW_THREADS) k_kway_planes(GainArgs A0, KwGain V) {
     constexpr u32 NP = BLOCK ? KP_PLANES_BLOCK : KP_PLANES, NW = KW_THREADS / 32, S = 32 / MW;
@@ -4210,6 +4241,8 @@ __device__ __forceinline__ void copy_sort64(u32 *sm, u32 M, u32 bits, const u32 
     block_radix_sort(sm, M, bits - 32, ko, vo);
 }
 
+// Bound by one block's latency per copy. Measured: 14 copies 66 us, with k_copy_sizes 38 and
+// k_copy_tail 22, in place of about 60 launches a round.
 __global__ void __launch_bounds__(RSS_WARPS * 32) k_copy_rank(CopyArgs A) {
     extern __shared__ u32 sm[];
     __shared__ i64 sh[32];
@@ -4425,6 +4458,8 @@ struct SmallArgs {
     int track;
 };
 
+// Bound by its grid barriers. Measured: 8 x 512 network 12.0 ms with a graph of some 40 launches a
+// round, 10.0; 4 x 64 6.5 and 3.5.
 template <u32 MW>
 __global__ void __launch_bounds__(SR_THREADS) k_small_rounds(SmallArgs S) {
     cg::grid_group grid = cg::this_grid();
@@ -4678,6 +4713,7 @@ void setup_refine_kernels(Ctx &c) {
 // hi pins ([0]), longer ones ([1]) and those above CM_LEN ([15]), with cls their class
 // (k_mover_hedges); the longest, the destination pins, the extreme weights, and the pins and squared
 // lengths of the short ones ([9] to [14]).
+// Measured: 1M nets 138 us, 16.
 __global__ void __launch_bounds__(1024) k_level_hedges(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ nsrc,
                                                        const u32 *__restrict__ wfx, u64 lo, u64 hi, u32 *mid, u32 *huge,
                                                        u32 *lng, uint8_t *__restrict__ cls, u64 *__restrict__ dc) {
@@ -4808,7 +4844,7 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
         lp.huge_tot = fetch1(c, lp.huge_tab + lp.n_hhuge);
     }
     if (n) {
-        if (c.profiling("k_gain_warp") || c.profiling("k_gain_block")) {
+        if (c.prof_on && c.prof_name.find("gain") != std::string::npos) {
             unsigned long long *dg = c.arena.alloc<unsigned long long>(3);
             AXC_CUDA(cudaMemsetAsync(dg, 0, 24, c.stream));
             for (int t = 0; t < 3; ++t)
@@ -5296,8 +5332,10 @@ static void kway_gains_t(Ctx &c, const DLevel &L, const LevelPrep &lp, const Gai
     }
 }
 static void kway_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainArgs &A, const KwayLevel &kw) {
-    if (c.profiling("k_kway_gain")) c.prof_bytes += gain_bytes(lp, 0);
-    if (c.profiling("k_kway_gain_block")) c.prof_bytes += gain_bytes(lp, 1);
+    // per incidence: hyperedge id, a word of single pins, the present words, the weight where unequal
+    for (int t = 0; t < 2; ++t)
+        if (c.profiling(t ? "k_kway_gain_block" : "k_kway_gain"))
+            c.prof_bytes += (8 + 4 * kw.mw + (lp.uniform ? 0 : 4)) * lp.tier_deg[t] + 16 * (u64)lp.ncount[t];
     if (lp.gain_bound < (1ull << 32)) kway_gains_t<u32>(c, L, lp, A, kw);
     else kway_gains_t<unsigned long long>(c, L, lp, A, kw);
 }
