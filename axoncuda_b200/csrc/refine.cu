@@ -771,11 +771,6 @@ __global__ void __launch_bounds__(256) k_gain_bounds(u32 n, u32 K, const u64 *__
         if (ws) atomicMax(wmax, (unsigned long long)ws);
     }
 }
-__host__ __device__ __forceinline__ u32 table_cap(u64 work, u32 cap_max) {
-    u32 cap = 32;
-    while (cap < 2 * work && cap < cap_max) cap <<= 1;
-    return cap;
-}
 
 // Accumulate node u's adjacency to other partitions into (keys, conn, dconn). Warp-cooperative:
 // the calling warp takes the node's incidences in batches of 32 starting at `first`, every
@@ -4634,7 +4629,6 @@ struct LevelPrep {
     u32 ncount[3] = {0, 0, 0};
     u64 *work = nullptr;     // per-node table bound of the gains
     u64 *wsum = nullptr;     // K > GS_K: per-node summed weights of its hyperedges
-    u64 block_work_max = 0;  // largest gain-work bound of the block tier (sizes its shared table)
     u64 gain_bound = 0;     // no gain exceeds this (sum of incident weights)
     u64 max_len = 0;         // largest hyperedge
     u32 *hlong = nullptr, n_hlong = 0;         // |e| > CM_LEN
@@ -4826,7 +4820,6 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
     lp.n_hhuge = (u32)h[1];
     for (int t = 0; t < 3; ++t) lp.ncount[t] = (u32)h[2 + t];
     lp.gain_bound = h[5];
-    lp.block_work_max = h[7];
     lp.max_deg = h[8];
     lp.max_len = h[9];
     lp.dst_pins = h[10];
