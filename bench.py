@@ -218,19 +218,17 @@ def barrier(world):
 
 
 # the kernel with the largest share of device time (ncu launch lists in profiles/) per workload
-ROOFLINE_KERNELS = {"circuit-200k-k2": "k_census_inc_warp", "circuit-200k-k64": "k_census_inc_warp",
+ROOFLINE_KERNELS = {"circuit-200k-k2": "k_kway_gain", "circuit-200k-k64": "k_kway_gain",
                     "snn-8x512": "k_rate_block", "snn-1m-k128": "k_rate_block"}
 # algorithmic bytes per launch of the kernels the library's timer has a byte model for
 BYTE_MODELS = {
     "k_rate_block": "4 B per pin visit of the listed nodes (the pin id) + 8 B per candidate slot written",
     "k_gain_warp": "8 B per incidence entry of the listed nodes + 16 B per listed node",
-    "k_gain_block": "8 B per incidence entry of the listed nodes + 16 B per listed node",
+    "k_kway_gain": "per incidence of the listed nodes 8 B (hyperedge id, one word of single pins) + 4 B per word of "
+                   "present partitions (one per 32) + 4 B (weight) where unequal; + 16 B per listed node",
+    "k_kway_gain_block": "as k_kway_gain",
     "k_gain_mask_warp": "8 B per incidence entry of the listed nodes + 16 B per listed node",
     "k_gain_mask_block": "8 B per incidence entry of the listed nodes + 16 B per listed node",
-    "k_cascade_warp": "per listed hyperedge (those holding a mover), counted by the kernel: 24 B (list entry, "
-                      "offsets, source count) + 8 B per pin (id, rank) + 4 B (census size), then 4 B (hand-off "
-                      "to the block kernel) or 12 B per census entry + 16 B per mover (partition, target, "
-                      "cascaded gain) + 4 B (weight); inbound transitions not counted",
     "k_census_direct_warp": "per hyperedge, counted by the kernel: 20 B (offsets, source count) + 8 B per pin (id, "
                             "partition) + 12 B per census entry written + 4 B (its count) + 8 B per mask word pair "
                             "+ 4 B (weight) + 8 B per nonzero saving added to a pin's node",
@@ -242,7 +240,7 @@ BYTE_MODELS = {
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch from one ncu capture of the
 # kernel on the workload, recorded with its capture command in profiles/<kernel>-<workload>.md
 PROFILED_TRAFFIC = {("k_rate_block", "snn-8x512"): 616456, ("k_census_direct_warp", "circuit-200k-k2"): 67656819,
-                    ("k_census_inc_warp", "circuit-200k-k2"): 22632375}
+                    ("k_census_inc_warp", "circuit-200k-k2"): 22632375, ("k_kway_gain", "circuit-200k-k2"): 17986452}
 STEP_MODEL = ("construction 8P+8(n+E); per rated level 4 B per rating pin visit + 4P_l + 16 n_l C (matching); "
               "per contraction 8P_l + 12P_(l+1); per refinement round 16P_l + 16n_l (moves not counted)")
 
