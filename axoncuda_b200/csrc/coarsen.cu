@@ -783,9 +783,9 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
     if (pin_visits) *pin_visits = h[4];
     const u32 *list = lists[0], *list2 = lists[1], *list3 = lists[2], *list4 = lists[3];
     // Kernel timer: algorithmic bytes of the block tiers, 4 per pin visit (the pin id) and 8 per
-    // candidate slot written (pair and score), per launch.
+    // candidate slot written (pair and score), added where the kernel they belong to is launched.
     u64 tier_visits[3] = {0, 0, 0};
-    if (c.profiling("k_rate_block")) {
+    if (c.profiling("k_rate_block") || c.profiling("k_rate_direct")) {
         u64 *dv = c.arena.alloc<u64>(3);
         AXC_CUDA(cudaMemsetAsync(dv, 0, 24, c.stream));
         for (int t = 0; t < 3; ++t)
@@ -793,9 +793,10 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
                 LAUNCH(c, k_list_sum, cdiv(h[1 + t], 256), 256, 0, lists[1 + t], (u32)h[1 + t], work,
                        (unsigned long long *)(dv + t));
         fetch(c, tier_visits, dv, 24);
-        for (int t = 0; t < 2; ++t)  // the heavy tier counts below, if it runs on k_rate_block
-            if (h[1 + t]) c.prof_bytes += 4 * tier_visits[t] + 8ull * cnc * h[1 + t];
     }
+    const auto add_bytes = [&](const char *kernel, int t) {
+        if (c.profiling(kernel)) c.prof_bytes += 4 * tier_visits[t] + 8ull * cnc * h[1 + t];
+    };
     // the shared counts decide nothing where no pair's inbound counts add up to more than the limit, as
     // on the first levels (a third of a slot's bytes, and an atomic per inbound pin)
     const bool cm = 2 * h[6] > delta && (delta < 0x7FFFFFFFu || (u64)L.e >= (1ull << 30));
@@ -823,16 +824,18 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
     u32 *d_retry = (u32 *)(dc + 4), *d_retry2 = d_retry + 1;  // dc[4] was read already
     const u32 rt_try = c.tune.rate_try, rt_mid = std::max(c.tune.rate_mid, c.tune.rate_try);
     const bool by_node = n <= (cm ? RT_DIRECT_N<true> : RT_DIRECT_N<false>);
-    const auto direct_tier = [&](const u32 *lst, u32 cnt) {
+    const auto direct_tier = [&](int t, const u32 *lst, u32 cnt) {
+        add_bytes("k_rate_direct", t);
         RATE_LAUNCH(c, k_rate_direct, cnc, cm, std::min<u32>(cnt, (u32)c.sms * 8), RT_BLOCK,
                     (size_t)rate_direct_words(cm, n) * 4, A, lst, cnt);
     };
-    auto block_tier = [&](const u32 *lst, u32 cnt, u32 cap_full) {
+    auto block_tier = [&](int t, const u32 *lst, u32 cnt, u32 cap_full) {
         if (!cnt) return;
         if (by_node && cap_full > rt_try) {
-            direct_tier(lst, cnt);
+            direct_tier(t, lst, cnt);
             return;
         }
+        add_bytes("k_rate_block", t);  // once for all tries
         if (cap_full <= rt_try) {
             RATE_LAUNCH(c, k_rate_block, cnc, cm, cnt, RT_BLOCK, words * cap_full * 4, A, lst, cnt, cap_full, (u32 *)nullptr,
                    (const u32 *)nullptr, (u32 *)nullptr, (u32 *)nullptr, (u32 *)nullptr);
@@ -852,10 +855,10 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
         RATE_LAUNCH(c, k_rate_block, cnc, cm, grid, RT_WIDE, words * cap_full * 4, A, rl, cnt, cap_full, (u32 *)nullptr, dn,
                (u32 *)nullptr, (u32 *)nullptr, (u32 *)nullptr);
     };
-    block_tier(list2, nl, cap1);
+    block_tier(0, list2, nl, cap1);
     // tier: one block per node, up to 16384-slot table in dynamic smem
     nl = (u32)h[2];
-    block_tier(list3, nl, cap2);
+    block_tier(1, list3, nl, cap2);
     // tier: heavy nodes, tables in a global scratch slice per resident block
     nl = (u32)h[3];
     if (nl) {
@@ -874,11 +877,11 @@ void rating(Ctx &c, const DLevel &L, const u32 *wfx, u32 omega, u32 delta, u32 c
             else LAUNCH_AS(c, "k_rate_split_acc", k_rate_split_acc<false>, nl * splits, RT_BLOCK, 0, A, list4, nl, cap, splits, gtab);
             RATE_LAUNCH(c, k_rate_split_select, cnc, cm, nl, RT_BLOCK, 0, A, list4, nl, cap, gtab);
         } else if (by_node) {
-            direct_tier(list4, nl);
+            direct_tier(2, list4, nl);
         } else {
             u32 grid = nl < (u32)c.sms * 2 ? nl : (u32)c.sms * 2;
             u32 *gtab = c.arena.alloc<u32>((u64)grid * 3 * cap), *gused = c.arena.alloc<u32>((u64)grid * cap);
-            if (c.profiling("k_rate_block")) c.prof_bytes += 4 * tier_visits[2] + 8ull * cnc * nl;
+            add_bytes("k_rate_block", 2);
             RATE_LAUNCH(c, k_rate_block, cnc, cm, grid, RT_BLOCK, 0, A, list4, nl, cap, gtab, (const u32 *)nullptr, (u32 *)nullptr,
                    (u32 *)nullptr, gused);
         }

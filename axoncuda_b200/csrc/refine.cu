@@ -4837,7 +4837,7 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
         lp.huge_tot = fetch1(c, lp.huge_tab + lp.n_hhuge);
     }
     if (n) {
-        if (c.prof_on && c.prof_name.find("gain") != std::string::npos) {
+        if (c.prof_on && (c.prof_name.find("gain") != std::string::npos || c.prof_name.find("k_kway") == 0)) {
             unsigned long long *dg = c.arena.alloc<unsigned long long>(3);
             AXC_CUDA(cudaMemsetAsync(dg, 0, 24, c.stream));
             for (int t = 0; t < 3; ++t)
@@ -5291,6 +5291,13 @@ static void kway_gains_t(Ctx &c, const DLevel &L, const LevelPrep &lp, const Gai
     // planes: merging a warp's counters costs as much as a few dozen incidences the other way
     const bool planes = lp.uniform && kw.k > 8 && L.P / L.n >= 48;
     const auto grid = [&](u32 G) { return cdiv((u64)lp.ncount[0] * G, KW_THREADS); };
+    // kernel timer, per incidence: hyperedge id, a word of single pins, the present words, the weight
+    // where unequal
+    const auto add_bytes = [&](const char *kernel, int t) {
+        if (c.profiling(kernel))
+            c.prof_bytes += (8 + 4 * kw.mw + (lp.uniform ? 0 : 4)) * lp.tier_deg[t] + 16 * (u64)lp.ncount[t];
+    };
+    if (lp.ncount[0]) add_bytes(planes ? "k_kway_planes" : "k_kway_gain", 0);
     if (lp.ncount[0] && kw.k <= 4) {
         const u64 deg = L.P / L.n;
         if (deg < 8) LAUNCH_AS(c, "k_kway_gain", (k_kway_gain_few<4, T>), grid(4), KW_THREADS, 0, A, V);
@@ -5314,6 +5321,7 @@ static void kway_gains_t(Ctx &c, const DLevel &L, const LevelPrep &lp, const Gai
         V.list = lp.ntier[1];
         V.nl = lp.ncount[1];
         const bool wide = planes && lp.max_deg / (KW_THREADS / 32) + 1 < (1u << KP_PLANES_BLOCK);
+        add_bytes(wide ? "k_kway_planes_block" : "k_kway_gain_block", 1);
         kway_words(kw.mw, [&](auto mw) {
             if (wide)
                 LAUNCH_AS(c, "k_kway_planes_block", (k_kway_planes<decltype(mw)::value, true>), lp.ncount[1], KW_THREADS, 0, A,
@@ -5325,10 +5333,6 @@ static void kway_gains_t(Ctx &c, const DLevel &L, const LevelPrep &lp, const Gai
     }
 }
 static void kway_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainArgs &A, const KwayLevel &kw) {
-    // per incidence: hyperedge id, a word of single pins, the present words, the weight where unequal
-    for (int t = 0; t < 2; ++t)
-        if (c.profiling(t ? "k_kway_gain_block" : "k_kway_gain"))
-            c.prof_bytes += (8 + 4 * kw.mw + (lp.uniform ? 0 : 4)) * lp.tier_deg[t] + 16 * (u64)lp.ncount[t];
     if (lp.gain_bound < (1ull << 32)) kway_gains_t<u32>(c, L, lp, A, kw);
     else kway_gains_t<unsigned long long>(c, L, lp, A, kw);
 }

@@ -223,10 +223,13 @@ ROOFLINE_KERNELS = {"circuit-200k-k2": "k_kway_gain", "circuit-200k-k64": "k_kwa
 # algorithmic bytes per launch of the kernels the library's timer has a byte model for
 BYTE_MODELS = {
     "k_rate_block": "4 B per pin visit of the listed nodes (the pin id) + 8 B per candidate slot written",
+    "k_rate_direct": "as k_rate_block",
     "k_gain_warp": "8 B per incidence entry of the listed nodes + 16 B per listed node",
     "k_kway_gain": "per incidence of the listed nodes 8 B (hyperedge id, one word of single pins) + 4 B per word of "
                    "present partitions (one per 32) + 4 B (weight) where unequal; + 16 B per listed node",
     "k_kway_gain_block": "as k_kway_gain",
+    "k_kway_planes": "as k_kway_gain",
+    "k_kway_planes_block": "as k_kway_gain",
     "k_gain_mask_warp": "8 B per incidence entry of the listed nodes + 16 B per listed node",
     "k_gain_mask_block": "8 B per incidence entry of the listed nodes + 16 B per listed node",
     "k_census_direct_warp": "per hyperedge, counted by the kernel: 20 B (offsets, source count) + 8 B per pin (id, "

@@ -152,9 +152,9 @@ const char *axc_last_error(axc_ctx *ctx);   /* human-readable detail of the last
  * with host clocks, sources/main.cu:151-910) ------------------------------------------------------
  * While a kernel name is set, every launch of that kernel on the context stream is bracketed by a
  * pair of CUDA events, and launch sites with a byte model add the launch's algorithmic bytes:
- * k_rate_block and the gain kernels from host-side sizes; k_census_direct_warp and k_census_inc_warp
- * counted by the kernels themselves (they depend on each round's census). axc_profile_read
- * synchronizes the stream, returns the totals since the kernel was set and resets them.
+ * k_rate_block, k_rate_direct and the gain kernels from host-side sizes; k_census_direct_warp and
+ * k_census_inc_warp counted by the kernels themselves (they depend on each round's census).
+ * axc_profile_read synchronizes the stream, returns the totals since the kernel was set and resets them.
  * kernel = NULL switches the timer off. */
 typedef struct {
     uint32_t launches;  /* launches of the kernel seen */
