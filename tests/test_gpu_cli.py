@@ -2,7 +2,8 @@
 hgraph_gpu.exe: INCC with `-rfr 16 -cnc 4 -dtc -ipm -v 0` (hgraphs/run_snns.sh:20), k-way with
 `-rfr 16 -cnc 4 -dtc -v 0 -smh 0` (hgraphs/run_ispd.sh:20). Its result lines parse as the
 reference's (sources/main.cu:908-928), its -p file is accepted by the reference grader with the
-same lambda-1 as the library reports, and its -s file reads back as the quotient hypergraph."""
+same lambda-1 as the library reports (where the grader is not built, by the oracle's evaluation), and its
+-s file reads back as the quotient hypergraph."""
 import os
 import re
 import subprocess
@@ -56,8 +57,12 @@ def test_cli_result_lines_grader_and_quotient(tmp_path, i):
             lib_part, st = ctx.partition(g, params)
         np.testing.assert_array_equal(part, lib_part)
         assert abs(conn - st.connectivity) <= 1e-3 * max(1.0, st.connectivity)
-        gr = O.ref_grade(os.path.join(GOLDEN, name), str(pf), *grade_args)
-        assert gr["valid"] and abs(gr["Connectivity"] - st.connectivity) <= 1e-3 * max(1.0, st.connectivity)
+        if os.path.exists(O.ref_tool("hgrade.exe")):
+            gr = O.ref_grade(os.path.join(GOLDEN, name), str(pf), *grade_args)
+            assert gr["valid"] and abs(gr["Connectivity"] - st.connectivity) <= 1e-3 * max(1.0, st.connectivity)
+        else:  # the grader is compiled from the reference's sources; the oracle's evaluation is pinned to it
+            ev = oracle_evaluate(g, params, part)
+            assert ev["valid"] and ev["connectivity_fx"] == st.connectivity_fx
     # -s: the quotient hypergraph as written reads back equal to the library's construction
     q = ax.read(str(sf))
     qr = ax.quotient(g, part)
@@ -68,6 +73,13 @@ def test_cli_result_lines_grader_and_quotient(tmp_path, i):
     np.testing.assert_array_equal(q.pins, qr.pins)
     np.testing.assert_array_equal(q.nsrc, qr.nsrc)
     np.testing.assert_allclose(q.w, qr.w, rtol=1e-6)
+
+
+def oracle_evaluate(g, p, part):
+    off, pins, nsrc = O.dedupe(g.off, g.pins, g.nsrc)
+    kway = p.mode == ax.MODE_KWAY
+    return O.evaluate(g.n, off, pins, nsrc, g.w, part, ax.kway_omega(g.n, p.k, p.eps) if kway else p.omega,
+                      0x7FFFFFFF if kway else p.delta, p.k if kway else p.max_parts)
 
 
 def as_hmetis(q):
