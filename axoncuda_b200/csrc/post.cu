@@ -204,6 +204,7 @@ void evaluate(Ctx &c, const DLevel &L, const u32 *wfx, const u32 *part, u32 omeg
               axc_stats *st) {
     size_t mk = c.arena.mark();
     const u32 K = L.n ? reduce_max_u32(c, part, L.n) + 1 : 0;
+    if (L.n && !K) throw Error(AXC_EOVERFLOW, "a partition id of 2^32 - 1");
     Census cs = build_census(c, L, part, K);
     u64 *psize = c.arena.alloc<u64>(K ? K : 1), *pinb = c.arena.alloc<u64>(K ? K : 1);
     // validity counts nodes (not node weights), like sources/constr.cpp:95-115

@@ -189,7 +189,8 @@ int axc_partition_device(axc_ctx *ctx, const axc_hgraph *d_g, const axc_params *
 /* ---- validity and metrics on the device --------------------------------------------------------
  * Replaces Constraints::checkPartitionValidity (sources/constr.cpp:90-147) and the metrics of
  * includes/hgraph.hpp:214-280 as printed by sources/main.cu:917-928 and grading/grade.cpp:298-309.
- * `part` is host memory [g->n]. The hypergraph is used as given (no dedupe), like grade.cpp. */
+ * `part` is host memory [g->n]; an id of 2^32 - 1 gives AXC_EOVERFLOW. The hypergraph is used as given
+ * (no dedupe), like grade.cpp. */
 int axc_evaluate(axc_ctx *ctx, const axc_hgraph *g, const axc_params *p, const uint32_t *part,
                  axc_stats *stats);
 

@@ -11,7 +11,7 @@ from conftest import GOLDEN
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
-AXC_EINTERNAL = 10
+AXC_EINTERNAL, AXC_EOVERFLOW = 10, 11
 DEV_SPIN_LIMIT = 3
 
 
@@ -32,3 +32,20 @@ def test_bounded_wait_gives_up_and_the_context_recovers(ctx, spin_limit):
 
 def test_bounded_wait_rejects_a_zero_limit(ctx):
     assert ax.lib().axc_selftest_bounded_wait(ctx._h, 0) == 1  # AXC_EINVAL
+
+
+@pytest.mark.parametrize("hyperedges", [0, 1, 300])
+def test_evaluate_refuses_a_partition_id_without_a_count(ctx, hyperedges):
+    """Ids up to 2^32 - 2 have a partition count; 2^32 - 1 is refused on the host, before any kernel would
+    index by it."""
+    n = 400
+    g = ax.Hypergraph(n, np.arange(hyperedges + 1, dtype=np.uint64) * n, np.tile(np.arange(n, dtype=np.uint32), hyperedges),
+                      np.ones(hyperedges, np.uint32), np.ones(hyperedges, np.float32))
+    part = np.zeros(n, np.uint32)
+    part[7] = 0xFFFFFFFF
+    with pytest.raises(ax.AxcError) as err:
+        ctx.evaluate(g, ax.params_kway(2, 0.1), part)
+    assert err.value.code == AXC_EOVERFLOW
+    part[7] = 1
+    st = ctx.evaluate(g, ax.params_kway(2, 0.1), part)
+    assert st.num_parts == 2 and st.connectivity == hyperedges
