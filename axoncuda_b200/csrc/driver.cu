@@ -218,6 +218,21 @@ static u32 partition_core(Ctx &c, u32 n, u32 e, const u64 *d_off, const u32 *d_p
     return Kp;
 }
 
+// The staging of large uploads, made at the first; false where it cannot be had (the next call tries again).
+static bool stage_ready(Ctx &c) {
+    if (c.h_stage) return true;
+    for (cudaEvent_t &e : c.stage_free)
+        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            e = nullptr;
+            return false;
+        }
+    if (cudaHostAlloc((void **)&c.h_stage, 2 * STAGE_BYTES, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        c.h_stage = nullptr;
+    }
+    return c.h_stage != nullptr;
+}
 static void stage_destroy(Ctx &c) {
     if (c.h_stage) cudaFreeHost(c.h_stage);
     for (cudaEvent_t &e : c.stage_free) {
@@ -449,15 +464,7 @@ static void copy_in(Ctx &c, void *dst, const void *src, size_t bytes) {
     const bool pageable = bytes >= (2u << 20) &&
                           (cudaPointerGetAttributes(&at, src) != cudaSuccess || at.type == cudaMemoryTypeUnregistered);
     cudaGetLastError();  // an unknown pointer is pageable memory, not an error
-    if (pageable && !c.h_stage) {
-        if (cudaHostAlloc((void **)&c.h_stage, 2 * STAGE_BYTES, cudaHostAllocDefault) != cudaSuccess) {
-            cudaGetLastError();
-            c.h_stage = nullptr;
-        } else {
-            for (cudaEvent_t &e : c.stage_free) AXC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        }
-    }
-    if (!pageable || !c.h_stage) {
+    if (!pageable || !stage_ready(c)) {
         AXC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c.stream));
         return;
     }
