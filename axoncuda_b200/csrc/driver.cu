@@ -456,9 +456,9 @@ int axc_partition_device(axc_ctx *ctx, const axc_hgraph *d_g, const axc_params *
 }
 
 // Host memory to the device on the context's stream. The runtime stages pageable memory through one
-// thread (about 11 GB/s here); large arrays go through two pinned halves filled by a few threads
-// while the other half is on its way (1M-node netlist, 39 MB: 3.6 -> 1.5 ms). Pinned sources and
-// small arrays are copied directly, and any where no pinned memory is to be had.
+// thread (11 to 20 GB/s here); large arrays go through two pinned halves filled by a few threads
+// while the other half is on its way (1M-node netlist, 35 MB: 1.7 to 3.2 ms, by the box, and 1.2).
+// Pinned sources and small arrays are copied directly, and any where no pinned memory is to be had.
 static void copy_in(Ctx &c, void *dst, const void *src, size_t bytes) {
     cudaPointerAttributes at{};
     const bool pageable = bytes >= (2u << 20) &&

@@ -875,37 +875,6 @@ constexpr u32 GM_WARP_DEG = 4096;     // incidences one warp takes in the mask g
 // its lambda, against lambda hash updates in the general path. The node's saving from leaving
 // its own partition comes from the census pass (Census::save); candidates, connectivity and the
 // inbound count per candidate are the same quantities the general path accumulates.
-__global__ void k_census_masks(u32 e, const u64 *__restrict__ off, const u32 *__restrict__ lam,
-                               const u32 *__restrict__ cpart, const u32 *__restrict__ cdcnt, u32 MW,
-                               u32 *__restrict__ mask, u32 *__restrict__ dmask) {
-    const u32 h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (h >= e) return;
-    const u64 a = off[h];
-    const u32 lm = lam[h];
-    u32 mw[8], dw[8];
-#pragma unroll
-    for (u32 k = 0; k < 8; ++k) mw[k] = dw[k] = 0;
-    for (u32 j = lane; j < lm; j += 32) {
-        const u32 q = cpart[a + j], bit = 1u << (q & 31), wd = q >> 5;
-        const bool d = cdcnt[a + j] > 0;
-#pragma unroll
-        for (u32 k = 0; k < 8; ++k)
-            if (k == wd) {
-                mw[k] |= bit;
-                if (d) dw[k] |= bit;
-            }
-    }
-#pragma unroll
-    for (u32 k = 0; k < 8; ++k) {
-        if (k < MW) {
-            const u32 m = __reduce_or_sync(0xFFFFFFFFu, mw[k]), d = __reduce_or_sync(0xFFFFFFFFu, dw[k]);
-            if (lane == 0) {
-                mask[(u64)h * MW + k] = m;
-                dmask[(u64)h * MW + k] = d;
-            }
-        }
-    }
-}
 
 template <u32 MW>
 __device__ __forceinline__ void load_words(const u32 *p, u32 (&w)[MW]) {
@@ -2173,7 +2142,7 @@ struct CascadeArgs {
     unsigned long long *tdense;
     u32 dense_stride;
     u32 *status;
-    u32 K;  // partitions: with K <= CC_DIRECT_K the per-hyperedge tables are indexed by partition id
+    u32 K;  // partitions: with K <= CC_DIRECT_BLOCK_K the per-hyperedge tables are indexed by partition id
     // without a census (k-way levels of few partitions per copy): K partitions and ce hyperedges
     // of one copy; the tables hold copy-local partitions, counted from the pins (lam, cpart null)
     u32 ce;
@@ -2304,8 +2273,6 @@ __device__ __forceinline__ u32 cascade_cap32(u32 lm, u32 m) {
     return cap > (1ull << 31) ? (1u << 31) : (u32)cap;
 }
 
-// Hyperedges with at most CC_MOV movers, one warp each (hashed tables also need at most CC_TAB
-// slots); the others are appended to `big` for the block kernel.
 // The same sweep with a whole warp, 32 movers at a time (slots from cascade_slots required). The
 // counts a mover sees are the table's counts before its chunk plus what the chunk's earlier lanes
 // did to its two partitions: leaves of the same source (match_any), joins of the same target
@@ -5131,9 +5098,6 @@ static Census census_for_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, con
         cs.dmask = c.arena.alloc<u32>((u64)(L.e ? L.e : 1) * cs.mw);
     }
     run_census(c, L, lp, part, rp.K, cs);
-    if (direct && L.e && !lp.census_K)  // a hashed census: masks from its entries
-        LAUNCH(c, k_census_masks, cdiv((u64)L.e * 32, 256), 256, 0, L.e, L.off, cs.lam, cs.part, cs.dcnt, cs.mw,
-               cs.mask, cs.dmask);
     return cs;
 }
 
@@ -5591,7 +5555,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     }
     LAUNCH(c, k_gather_g2, cdiv(n, 256), 256, 0, mv, dM, n, g2, Gx);  // also zeroes Vs and Vi
     // size validity
-    if (!small) {
+    {
         size_t m1 = c.arena.mark();
         const u32 nemax = 2 * n;
         u32 *key = c.arena.alloc<u32>(nemax), *val = c.arena.alloc<u32>(nemax);
@@ -5607,7 +5571,7 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     }
     // inbound validity (INCC only): the transitions ordered by (partition, rank), the running
     // inbound-set size of each partition along them
-    if (track && !small) {
+    if (track) {
         size_t m1 = c.arena.mark();
         const u64 nt = tcap;
         const u32 rb = bits_for(n ? n - 1 : 0), pb = bits_for(rp.K ? rp.K - 1 : 0);

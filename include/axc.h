@@ -327,9 +327,9 @@ int axc_stage_refine(axc_ctx *ctx, const axc_hgraph *g, const uint32_t *part, ui
 
 /* ---- failure path of the bounded device waits (no reference counterpart: the reference's waits
  * are grid syncs and host synchronizations, which never time out) ------------------------------------
- * Runs one look-back wait of the single-pass scans (the only waits on other blocks' flags in this
- * library) against a tile flag that nothing publishes, polling it spin_limit times (the scans poll
- * 2^24 times). The wait gives up, the kernel sets the status word and returns, and the call reports
+ * Runs one look-back wait of the single-pass scans (the sorts' look-backs give up in the same way, and
+ * no other wait in this library polls another block's flag) against a tile flag that nothing
+ * publishes, polling it spin_limit times (scans and sorts poll 2^24 times). The wait gives up, the kernel sets the status word and returns, and the call reports
  * AXC_EINTERNAL with the status in axc_last_error; the context stays usable. Returns AXC_OK only
  * if the wait did not give up, which would be a defect. */
 int axc_selftest_bounded_wait(axc_ctx *ctx, uint32_t spin_limit);
