@@ -74,3 +74,49 @@ def test_multistart_without_moves(ctx):
     part, _ = ctx.partition(g, p)
     o, _, _, _ = O.partition(g.n, g.off, g.pins, g.nsrc, g.w, 1, k=4, eps=p.eps, cnc=4, rfr=4)
     np.testing.assert_array_equal(part, o)
+
+
+def dense_network(n, hubs):
+    """Equal weights and at least 48 incidences per node on average, where gains count in bit planes; `hubs`
+    nodes are in two hyperedges of three."""
+    g = ax.gen_snn(4, n // 4, 90, 0.3, 200, 0.7, n)
+    rng = np.random.default_rng(n)
+    nets = []
+    for a, b in zip(g.off[:-1], g.off[1:]):
+        p = g.pins[int(a):int(b)]
+        nets.append(np.concatenate([p, [v for v in range(hubs) if v not in p and rng.random() < 0.67]]).astype(np.uint32))
+    off = np.concatenate([[0], np.cumsum([len(p) for p in nets])]).astype(np.uint64)
+    off, pins, nsrc = O.dedupe(off, np.concatenate(nets), g.nsrc)
+    g = ax.Hypergraph(g.n, off, pins, nsrc, np.full(g.e, 1 / 3, np.float32))
+    assert g.P >= 48 * g.n
+    return g
+
+
+# one to eight words of partitions; a block per node (at most 1024 nodes), and a warp per node with the
+# hubs' more than 1024 incidences in blocks
+@pytest.mark.parametrize("n,hubs", [(800, 0), (3200, 3)])
+@pytest.mark.parametrize("K", [8, 9, 32, 33, 64, 65, 128, 129, 256])
+def test_kway_planes_match_oracle(ctx, n, hubs, K):
+    g = dense_network(n, hubs)
+    deg = np.bincount(g.pins, minlength=g.n)
+    assert (deg > 1024).sum() == hubs
+    check_refine(ctx, g, K, False, int(2.2 * n / K) + 3, NO_LIMIT, 3)
+
+
+@pytest.mark.parametrize("hub_degree", [131055, 131056, 131063, 131064])
+def test_kway_planes_at_their_capacity_match_oracle(ctx, hub_degree):
+    """A node of 2^17 incidences: the last whose eighth a block's counters hold, and the first that sums
+    by partition instead. All its neighbours are in one partition, where the counters reach their limit."""
+    n, K = 2000, 40
+    rng = np.random.default_rng(hub_degree)
+    pins = np.zeros((hub_degree, 2), np.uint32)
+    pins[:, 1] = 1 + rng.integers(0, n // 2, hub_degree)
+    g = ax.Hypergraph(n, np.arange(hub_degree + 1, dtype=np.uint64) * 2, pins.ravel(), np.ones(hub_degree, np.uint32),
+                      np.ones(hub_degree, np.float32))
+    part = np.where(np.arange(n) <= n // 2, 5, rng.integers(0, K, n)).astype(np.uint32)
+    part[0] = 7
+    ns = np.ones(n, np.uint32)
+    out, ran = ctx.stage_refine(g, part, K, ns, n, NO_LIMIT, False, 3, 3)
+    o = O.refine(g.n, g.off, g.pins, g.nsrc, O.wfx(g.w), ns, part, K, n, NO_LIMIT, False, 3, 3)
+    np.testing.assert_array_equal(out, o)
+    assert out[0] == 5
