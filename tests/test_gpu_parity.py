@@ -230,18 +230,15 @@ def test_cascade_middle_tier_matches_oracle(ctx):
     assert st.valid == 1 and st.num_parts > 256
 
 
-# Nodes whose gain-table bound passes 4096 slots (here about 2000 partitions of two neurons and
-# about 80 inbound hyperedges of about 80 pins) first try a shared-memory table and fall back to a
-# global one when they reach too many distinct partitions. With at most 4096 partitions the first
-# try always fits; AXC_GAIN_TRY_LIMIT=16 makes nearly every such node fall back.
-@pytest.mark.parametrize("try_limit", [None, "16"])
-def test_heavy_gain_tier_matches_oracle(ctx, monkeypatch, try_limit):
+# Nodes whose census entries pass 4096 (here about 2000 partitions of two neurons and about 80 inbound
+# hyperedges of about 80 pins) sum by partition index up to 4096 partitions: with equal weights in bit
+# planes, else in tables.
+@pytest.mark.parametrize("weighted", [False, True])
+def test_heavy_gain_tier_matches_oracle(ctx, weighted):
     g = ax.gen_snn(4, 1000, 80, 0.7, 300, 0.7, 31)
+    if weighted:
+        g.w = (np.random.default_rng(31).integers(1, 65, g.e) / 4.0).astype(np.float32)
     p = ax.params_incc(2, 4096, 1048576, cnc=4, rfr=4)
-    if try_limit is None:
-        monkeypatch.delenv("AXC_GAIN_TRY_LIMIT", raising=False)
-    else:
-        monkeypatch.setenv("AXC_GAIN_TRY_LIMIT", try_limit)
     part, st = ctx.partition(g, p)
     o_part, o_K, _, _ = oracle_partition(g, p)
     np.testing.assert_array_equal(part, o_part)
