@@ -734,10 +734,10 @@ __device__ __forceinline__ GainArgs gain_args_now(const GainArgs &A0) {
 // Per-level bounds of a node's gain work: the partitions adjacent to it in any round number at
 // most min(sum over incident hyperedges of min(|e|, K), K), which sizes its accumulator table; the
 // sum of incident weights bounds its gain. G lanes a node; the block takes those of more than
-// GB_HEAVY incidences a lane together.
+// GB_HEAVY incidences a lane (GB_HEAVY_WARP for a warp) together.
 // Measured: 1M nodes 169 us a level, 664 at the first (an atomic per node at one address), 45. A node of
 // 300,000 incidences among 120,000 of few: 10.3 ms with four lanes, 3.8 with a warp, 0.37 with the block.
-constexpr u32 GB_HEAVY = 64;
+constexpr u32 GB_HEAVY = 64, GB_HEAVY_WARP = 8192;
 template <u32 G>
 __global__ void __launch_bounds__(256) k_gain_bounds(u32 n, u32 K, const u64 *__restrict__ toff,
                                                      const u32 *__restrict__ touch, const u64 *__restrict__ off,
@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(256) k_gain_bounds(u32 n, u32 K, const u64 *__
     bool light = false;
     if (u < n) {
         const u64 t0 = toff[u], t1 = toff[u + 1];
-        light = t1 - t0 <= GB_HEAVY * G;
+        light = t1 - t0 <= (G == 32 ? GB_HEAVY_WARP : GB_HEAVY * G);
         if (light) add(t0 + own, t1, G);
         else if (own == 0) heavy[atomicAdd(&nheavy, 1u)] = u;
     }

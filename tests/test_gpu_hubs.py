@@ -7,7 +7,7 @@ import axoncuda_b200 as ax
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
-HUBS = [256, 257, 512, 513, 2048, 2049, 4096, 4097, 20000]
+HUBS = [256, 257, 512, 513, 2048, 2049, 4096, 4097, 8192, 8193, 20000]
 
 
 def hub_graph(n, mean, weighted):
