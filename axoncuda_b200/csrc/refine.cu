@@ -1244,12 +1244,15 @@ __device__ __forceinline__ void census_flat(const GainArgs &A, u32 u, u32 first,
 //  - k_gain_table: one shared add per census entry into K-entry tables. The connectivity is one
 //    u32 where no node's incident weights pass 2^32, else a low and a high word: 64-bit shared
 //    adds would be compare-and-swap loops. NT threads: 64 at moderate degrees, where more nodes in
-//    flight hide the loads' latency better than more threads per node.
+//    flight hide the loads' latency better than more threads per node, and no node of more than
+//    GT_SMALL_DEG incidences, whose walk by two warps would outlast the level's other nodes.
 //  - k_gain_planes: for equal weights and hyperedges of at least as many pins as mask words. A
 //    candidate's connectivity is then a count of incidences whose K-bit mask holds it. A lane owns
 //    one mask word and adds whole words into bit-plane counters (carry-save adders, eight
 //    incidences at a time): 32 partitions per instruction, whatever the number of entries.
-// Measured: 120k-node netlist 134 us hashed, 64 (64 threads) and 68 (256).
+// Measured: 120k-node netlist 134 us hashed, 64 (64 threads) and 68 (256); with a node of 300,000
+// incidences 20.8 ms (64) and 2.8 (256).
+constexpr u32 GT_SMALL_DEG = 4096;
 template <bool WIDE, u32 NT>
 __global__ void __launch_bounds__(NT) k_gain_table(GainArgs A0, const u32 *__restrict__ list, u32 nl) {
     const GainArgs A = gain_args_now(A0);
@@ -4980,7 +4983,7 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
             LAUNCH_AS(c, "k_gain_table", (k_gain_table<W, NT>), lp.ncount[1], NT, (size_t)A.K * (W ? 12 : 8), A,
                       lp.ntier[1], lp.ncount[1]);
         };
-        const bool wide = lp.gain_bound >= (1ull << 32), small = L.P / L.n <= 256;
+        const bool wide = lp.gain_bound >= (1ull << 32), small = L.P / L.n <= 256 && lp.max_deg <= GT_SMALL_DEG;
         const std::integral_constant<u32, 64> t64;
         const std::integral_constant<u32, GN_BLOCK> t256;
         if (wide && small) launch(std::true_type(), t64);
