@@ -5805,10 +5805,18 @@ static u32 refine_level_loop(Ctx &c, const DLevel &L, const LevelPrep &lp, const
     return done;
 }
 
-// Levels whose rounds run in one launch (k_small_rounds).
+// Blocks of k_small_rounds: a warp per two or so hyperedges and per node, at most one block per SM.
+static u32 small_rounds_grid(const Ctx &c, const DLevel &L) {
+    return std::max(1u, std::min<u32>((u32)c.sms, cdiv(std::max<u64>(L.e, L.n), 2 * (SR_THREADS / 32))));
+}
+
+// Levels whose rounds run in one launch (k_small_rounds). A node takes a warp there where the nodes are
+// many; a level with one of more than GM_WARP_DEG incidences then keeps the rounds' own launches, which
+// give such nodes a block (20,000 nodes, one of 300,000 incidences, 156 parts: 1500 ms in one launch, 360).
 static bool small_rounds_eligible(const Ctx &c, const DLevel &L, const LevelPrep &lp, const RefineParams &rp) {
     return rp.encourage && rp.copies == 1 && rp.K <= VS_MAX_K && L.n <= (u32)RSS_CAP && L.e && lp.max_len <= CM_LEN &&
-           c.coop_supported && !c.prof_on && round_loop_enabled();
+           (lp.max_deg <= GM_WARP_DEG || L.n <= small_rounds_grid(c, L) * (SR_THREADS / 32) / 2) && c.coop_supported &&
+           !c.prof_on && round_loop_enabled();
 }
 
 static u32 small_rounds(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *wfx, const RefineParams &rp, u32 *part) {
@@ -5850,8 +5858,7 @@ static u32 small_rounds(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 
     S.Vi = c.arena.alloc<unsigned long long>(n);
     S.R = rp.rounds; S.kb = bits_for(lp.gain_bound); S.gbound = lp.gain_bound;
     S.part = part; S.psize = psize; S.pinb = pinb; S.save = cs.save; S.rs = ctl; S.track = track ? 1 : 0;
-    // a warp per two or so hyperedges and per node, at most one block per SM
-    const u32 grid = std::max(1u, std::min<u32>((u32)c.sms, cdiv(std::max<u64>(L.e, n), 2 * (SR_THREADS / 32))));
+    const u32 grid = small_rounds_grid(c, L);
     S.V.per_warp = 32;
     while (S.V.per_warp > 2 && L.e / S.V.per_warp < grid * (SR_THREADS / 32)) S.V.per_warp >>= 1;
     const void *k = cs.mw == 1 ? (const void *)k_small_rounds<1> : cs.mw == 2 ? (const void *)k_small_rounds<2>
