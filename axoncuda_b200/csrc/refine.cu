@@ -4794,30 +4794,37 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
     u64 *dc = c.arena.alloc<u64>(16);
     AXC_CUDA(cudaMemsetAsync(dc, 0, 128, c.stream));
     lp.census_K = K <= CD_K || kway ? K : 0;
+    if (n) {
+        lp.work = c.arena.alloc<u64>(n);
+        for (u32 t = 0; t < (kway ? 2u : 3u); ++t) lp.ntier[t] = c.arena.alloc<u32>(n);
+    }
+    // what the counts may show to be needless comes last, and is given back then
+    const size_t before_wsum = c.arena.mark();
+    if (n && K > GS_K) lp.wsum = c.arena.alloc<u64>(n);
+    const size_t before_lists = c.arena.mark();
+    size_t before_long = before_lists;
     if (e) {
         // census: a warp, a block above CD_WARP_LEN pins (partition-indexed) or CS_WARP_CAP (hashed),
         // and hashed above CS_BLOCK_CAP a table in device memory
+        lp.hclass = c.arena.alloc<uint8_t>(e);
         lp.hblock = c.arena.alloc<u32>(e);
         if (!lp.census_K) lp.hhuge = c.arena.alloc<u32>(e);
+        before_long = c.arena.mark();
         lp.hlong = c.arena.alloc<u32>(e);
-        lp.hclass = c.arena.alloc<uint8_t>(e);
+        static_assert(CM_LEN <= CS_WARP_CAP && CM_LEN <= CD_WARP_LEN, "no long hyperedges: the other lists are empty too");
         LAUNCH(c, k_level_hedges, cdiv(e, 1024), 1024, 0, e, L.off, L.nsrc, wfx, lp.census_K ? (u64)CD_WARP_LEN : (u64)CS_WARP_CAP,
                lp.census_K ? ~0ull : (u64)CS_BLOCK_CAP, lp.hblock, lp.hhuge, lp.hlong, lp.hclass, dc);
     }
     if (n) {
-        u64 *work = c.arena.alloc<u64>(n);
-        lp.work = work;
-        if (K > GS_K) lp.wsum = c.arena.alloc<u64>(n);
         const auto bounds = [&](auto g) {  // lanes per node: as many as a mean node has incidences
             constexpr u32 G = decltype(g)::value;
             LAUNCH_AS(c, "k_gain_bounds", k_gain_bounds<G>, cdiv((u64)n * G, 256), 256, 0, n, K, L.toff, L.touch, L.off, wfx,
-                      work, lp.wsum, (unsigned long long *)(dc + 5));
+                      lp.work, lp.wsum, (unsigned long long *)(dc + 5));
         };
         if (L.P < 8ull * n) bounds(std::integral_constant<u32, 4>());
         else if (L.P < 32ull * n) bounds(std::integral_constant<u32, 8>());
         else bounds(std::integral_constant<u32, 32>());
-        for (u32 t = 0; t < (kway ? 2u : 3u); ++t) lp.ntier[t] = c.arena.alloc<u32>(n);
-        LAUNCH(c, k_tier_lists, cdiv(n, 1024), 1024, 0, n, K, work, L.toff, kway ? 1u : 0u, lp.ntier[0], lp.ntier[1],
+        LAUNCH(c, k_tier_lists, cdiv(n, 1024), 1024, 0, n, K, lp.work, L.toff, kway ? 1u : 0u, lp.ntier[0], lp.ntier[1],
                lp.ntier[2], dc + 2, (unsigned long long *)(dc + 6));
     }
     u64 h[16];
@@ -4832,6 +4839,15 @@ static LevelPrep prepare_level(Ctx &c, const DLevel &L, const u32 *wfx, u32 K, b
     lp.short_pins = h[13];
     lp.short_sq = h[14];
     lp.n_hlong = (u32)h[15];
+    if (lp.n_hlong) {
+        c.arena.release(before_long);
+        lp.hlong = c.arena.alloc<u32>(lp.n_hlong);  // same address, tighter size
+    } else {
+        lp.hclass = nullptr;
+        lp.hblock = lp.hhuge = lp.hlong = nullptr;
+        if (!lp.ncount[2]) lp.wsum = nullptr;
+        c.arena.release(lp.wsum ? before_lists : before_wsum);
+    }
     if (e && (u32)h[11] == ~(u32)h[12]) {
         lp.uniform = true;
         lp.weight = (u32)h[11];
@@ -4994,9 +5010,13 @@ static void run_gains(Ctx &c, const DLevel &L, const LevelPrep &lp, const GainAr
     if (A.K > GS_K && lp.ncount[1] + lp.ncount[2]) {  // the sampled rule (include/axc.h AXC_SPARSE_GAIN_*)
         size_t m = c.arena.mark();
         const u32 rows = lp.ncount[2];
-        CandAcc C{c.arena.alloc<u32>((u64)L.n * GS_C), c.arena.alloc<unsigned long long>((u64)L.n * GS_C),
-                  lp.uniform ? nullptr : c.arena.alloc<u32>((u64)L.n * GS_C), lp.wsum, lp.weight};
-        AXC_CUDA(cudaMemsetAsync(C.cand, 0xFF, (size_t)L.n * GS_C * 4, c.stream));  // NONE
+        CandAcc C{nullptr, nullptr, nullptr, lp.wsum, lp.weight};
+        if (rows) {  // tier 1 has no candidates: its nodes' samples are the whole nodes
+            C.cand = c.arena.alloc<u32>((u64)L.n * GS_C);
+            C.conn = c.arena.alloc<unsigned long long>((u64)L.n * GS_C);
+            if (!lp.uniform) C.dcon = c.arena.alloc<u32>((u64)L.n * GS_C);
+            AXC_CUDA(cudaMemsetAsync(C.cand, 0xFF, (size_t)L.n * GS_C * 4, c.stream));  // NONE
+        }
         u32 *room = c.arena.alloc<u32>(A.K);
         LAUNCH(c, k_part_room, cdiv(A.K, 256), 256, 0, A.K, A.omega, A.delta, A.psize, A.pinb, room);
         const auto sample = [&](auto uni, auto direct) {
@@ -5385,11 +5405,14 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
     const bool small = !slots && rp.K <= VS_MAX_K && n <= (u32)RSS_CAP && rp.copies == 1;
     CopyArgs ca{};
     // movers in id order, then ranked by (gain desc, id asc)
-    u32 *flag = c.arena.alloc<u32>(n), *mv = c.arena.alloc<u32>(n);
+    u32 *mv = c.arena.alloc<u32>(n);
     uint2 *state = (uint2 *)c.arena.alloc<u64>(n);
     unsigned long long *g2 = c.arena.alloc<unsigned long long>(n);  // cascaded gains, zeroed here
+    u32 *ck = rp.copies > 1 && !slots ? c.arena.alloc<u32>(n) : nullptr;  // copies: the copy of every rank, ascending
+    const size_t ranking = c.arena.mark();  // its scratch is given back once the movers are ranked
+    u32 *flag = slots ? nullptr : c.arena.alloc<u32>(n), *klo = slots ? nullptr : c.arena.alloc<u32>(n);
+    u32 *khi = flag;  // the flags are spent when the keys are made
     const u32 kb = bits_for(lp.gain_bound);
-    u32 *khi = flag, *klo = c.arena.alloc<u32>(n);  // the flags are spent when the keys are made
     const int packed = rp.K <= STATE_PACK_K ? 1 : 0;
     if (slots) {
         const u64 pbound = 2 * lp.gain_bound;
@@ -5435,13 +5458,12 @@ static u32 *round_body(Ctx &c, const DLevel &L, const LevelPrep &lp, const u32 *
             radix_sort_pairs_dn(c, khi, mv, dM, n, pb - 32);
         }
     }
-    u32 *ck = nullptr;  // copies: the copy of every rank, ascending
-    if (rp.copies > 1 && !slots) {
-        ck = c.arena.alloc<u32>(n);
+    if (ck) {
         LAUNCH(c, k_copy_keys, cdiv(n, 256), 256, 0, mv, dM, rp.copy_n, ck);
         radix_sort_pairs_dn(c, ck, mv, dM, n, bits_for(rp.copies - 1));
     }
     if (!slots && (!small || pairs || rp.copies > 1)) LAUNCH(c, k_set_rank, cdiv(n, 256), 256, 0, mv, dM, state, dSE);
+    if (!slots) c.arena.release(ranking);
     // cascade
 
     // inbound-set transitions (INCC): each destination pin of a mover gives at most two
