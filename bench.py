@@ -217,8 +217,9 @@ def barrier(world):
         dist.barrier()
 
 
-# the kernel with the largest share of device time (ncu launch lists in profiles/) per workload
-ROOFLINE_KERNELS = {"circuit-200k-k2": "k_kway_gain", "circuit-200k-k64": "k_kway_gain",
+# per workload the kernel with the largest share of device time (launch lists in profiles/) among those
+# with a byte model below
+ROOFLINE_KERNELS = {"circuit-200k-k2": "k_kway_gain", "circuit-200k-k64": "k_kway_planes",
                     "snn-8x512": "k_rate_block", "snn-1m-k128": "k_rate_block"}
 # algorithmic bytes per launch of the kernels the library's timer has a byte model for
 BYTE_MODELS = {
@@ -242,8 +243,8 @@ BYTE_MODELS = {
 }
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch from one ncu capture of the
 # kernel on the workload, recorded with its capture command in profiles/<kernel>-<workload>.md
-PROFILED_TRAFFIC = {("k_rate_block", "snn-8x512"): 616456, ("k_census_direct_warp", "circuit-200k-k2"): 67656819,
-                    ("k_census_inc_warp", "circuit-200k-k2"): 22632375, ("k_kway_gain", "circuit-200k-k2"): 17986452}
+PROFILED_TRAFFIC = {("k_rate_block", "snn-8x512"): 330701, ("k_kway_gain", "circuit-200k-k2"): 17986452,
+                    ("k_kway_planes", "circuit-200k-k64"): 45885978}
 STEP_MODEL = ("construction 8P+8(n+E); per rated level 4 B per rating pin visit + 4P_l + 16 n_l C (matching); "
               "per contraction 8P_l + 12P_(l+1); per refinement round 16P_l + 16n_l (moves not counted)")
 
