@@ -5834,7 +5834,7 @@ static u32 small_rounds_grid(const Ctx &c, const DLevel &L) {
 
 // Levels whose rounds run in one launch (k_small_rounds). A node takes a warp there where the nodes are
 // many; a level with one of more than GM_WARP_DEG incidences then keeps the rounds' own launches, which
-// give such nodes a block (20,000 nodes, one of 300,000 incidences, 156 parts: 1500 ms in one launch, 360).
+// give such nodes a block (20,000 nodes, one of 300,000 incidences, 156 parts: 1559 ms in one launch, 316).
 static bool small_rounds_eligible(const Ctx &c, const DLevel &L, const LevelPrep &lp, const RefineParams &rp) {
     return rp.encourage && rp.copies == 1 && rp.K <= VS_MAX_K && L.n <= (u32)RSS_CAP && L.e && lp.max_len <= CM_LEN &&
            (lp.max_deg <= GM_WARP_DEG || L.n <= small_rounds_grid(c, L) * (SR_THREADS / 32) / 2) && c.coop_supported &&
